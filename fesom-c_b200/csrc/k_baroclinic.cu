@@ -33,6 +33,7 @@ struct ColBlock {
 // hydrostatic sum per node in level order
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_pressure_col(Dev d) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const real gd0 = kG / d.density_0;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(1024) k_pressure_col(Dev d) {
 // the kernel is bounded to 64 registers (unbounded it takes 96, which a
 // block of more than 682 threads, i.e. L >= 43, could not launch with).
 __global__ void __launch_bounds__(1024) k_bpg_elem(Dev d) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L, NS = d.NS;
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(1024) k_bpg_elem(Dev d) {
 // vel_gradients (fv_gradients.F90:2-93), one thread per (element, level).
 // 64 registers: 32 resident warps per SM instead of 24 (11 % faster).
 __global__ void __maxnreg__(64) k_velgrad3d(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     GRID_LOOP(ii, total) {
         const int e = (int)(ii / d.L);
@@ -267,6 +270,7 @@ __device__ __forceinline__ void uvert_at(const Dev &d, int e, int k, const real4
 // by the edge's two elements in velrhs.  Thread per (edge, level), levels on
 // consecutive threads.
 __global__ void k_adv3_edge(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.Ed_in * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
@@ -311,6 +315,7 @@ __global__ void k_adv3_edge(Dev d) {
 // p1_elem gathers the mode-2 fluxes, times Je, into U_rhs_2D_3D.
 // ---------------------------------------------------------------------------
 __global__ void k_bih_edge(Dev d, const real *U, const real *V, int mode) {
+    pdl_enter();
     const long long total = (long long)d.Ed * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
@@ -365,6 +370,7 @@ __global__ void k_bih_edge(Dev d, const real *U, const real *V, int mode) {
 }
 
 __global__ void k_bih_uc(Dev d, int mode) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
@@ -384,6 +390,7 @@ __global__ void k_bih_uc(Dev d, int mode) {
 // (vel_gradients_puls)
 template <bool FREE_SLIP>
 __global__ void k_bih_grad(Dev d, const real *U, const real *V) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
@@ -435,6 +442,7 @@ __global__ void k_bih_grad(Dev d, const real *U, const real *V) {
 // (neighbour 4 only when it differs from neighbour 1), times K_bi.  velrhs
 // forms UV_rhs from the neighbours' U_c.
 __global__ void k_filt2x_uc(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     const int L = d.L;
     const real tau_inv = d.dt * d.tau_c / real(3600.0) / real(24.0);
@@ -477,6 +485,7 @@ __global__ void k_filt2x_uc(Dev d) {
 // spilled registers cost less than the lost warps (11 % faster than 3
 // blocks at 80 registers).
 __global__ void __launch_bounds__(256, 4) k_velrhs(Dev d, real ff) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     const int lane = threadIdx.x & 31;
     const long long nwarp = (long long)gridDim.x * (blockDim.x >> 5);
@@ -588,6 +597,7 @@ __global__ void __launch_bounds__(256, 4) k_velrhs(Dev d, real ff) {
 // ---------------------------------------------------------------------------
 template <int MAXL>
 __global__ void k_implvisc(Dev d) {
+    pdl_enter();
     GRID_LOOP(ii, d.E) {
         const int e = (int)ii;
         const int L = d.L, NS = d.NS;
@@ -715,6 +725,7 @@ __global__ void k_implvisc(Dev d) {
 
 // jacobian bookkeeping after the sub-cycle (fv_main.F90:2050): Jc_old <- Jc
 __global__ void k_jac_swap(Dev d) {
+    pdl_enter();
     GRID_LOOP(ii, d.N) {
         d.eta_jac_old[ii] = d.eta_jac[ii];
         d.eta_jac[ii] = d.eta_n[ii];
@@ -724,6 +735,7 @@ __global__ void k_jac_swap(Dev d) {
 // Je, Ze, ZBe of every (element, level) from eta_jac (jacobian,
 // fv_main.F90:1208-1267); at init, afterwards refreshed by update3d
 __global__ void k_je_elem(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     GRID_LOOP(ii, total) {
         const int e = (int)(ii / d.L);
@@ -744,6 +756,7 @@ __global__ void k_je_elem(Dev d) {
 constexpr int kU3Sc = 14;  // per element: U2p, V2p, uf, vf, w_cv(4), a(4), U_n_2D(2)
 // 48 registers: 4 resident column blocks per SM instead of 3 (15 % faster).
 __global__ void __maxnreg__(48) k_update3d(Dev d, real Mt_inv) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L;
@@ -822,6 +835,7 @@ __global__ void __maxnreg__(48) k_update3d(Dev d, real Mt_inv) {
 // transport divergence of (node, level) gathered over the node's edges in
 // edge order, then summed upward from the bottom per node.
 __global__ void k_wvel(Dev d) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L, NS = d.NS;
@@ -889,6 +903,7 @@ __host__ __device__ __forceinline__ int iv_odd(int x) { return x | 1; }
 
 template <int LC>
 __global__ void __launch_bounds__(kIvCols) k_implvisc_fic_tile(Dev d) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char iv_smem[];
     constexpr int L = LC, LP = LC | 1;
     const int NS = d.NS, KP = iv_odd(d.NS), E = d.E;
@@ -1033,63 +1048,63 @@ int config_columns(const Dev &d) {
     return e == cudaSuccess ? 0 : 1;
 }
 void launch_pressure_col(const Dev &d, cudaStream_t s) {
-    k_pressure_col<<<col_grid(d, d.N), col_b(d) * d.L, col_smem(d, 1, 0), s>>>(d);
+    launch_k(k_pressure_col, col_grid(d, d.N), col_b(d) * d.L, col_smem(d, 1, 0), s, d);
 }
 void launch_bpg_elem(const Dev &d, cudaStream_t s) {
-    k_bpg_elem<<<col_grid(d, d.E), col_b(d) * d.L, col_smem(d, 2, 0), s>>>(d);
+    launch_k(k_bpg_elem, col_grid(d, d.E), col_b(d) * d.L, col_smem(d, 2, 0), s, d);
 }
 void launch_velgrad3d(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_VELGRAD3D, 256);
-    k_velgrad3d<<<grid_for((long long)d.E * d.L, b), b, 0, s>>>(d);
+    launch_k(k_velgrad3d, grid_for((long long)d.E * d.L, b), b, 0, s, d);
 }
 void launch_adv3_edge(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ADV3, 256);
-    k_adv3_edge<<<grid_for((long long)d.Ed_in * d.L, b), b, 0, s>>>(d);
+    launch_k(k_adv3_edge, grid_for((long long)d.Ed_in * d.L, b), b, 0, s, d);
 }
 void launch_filt2x(const Dev &d, cudaStream_t s) {
-    k_filt2x_uc<<<grid_for((long long)d.E * d.L, 256), 256, 0, s>>>(d);
+    launch_k(k_filt2x_uc, grid_for((long long)d.E * d.L, 256), 256, 0, s, d);
 }
 void launch_bih(const Dev &d, cudaStream_t s) {
     const int ge = grid_for((long long)d.Ed * d.L, 256), gl = grid_for((long long)d.E * d.L, 256);
-    k_bih_edge<<<ge, 256, 0, s>>>(d, d.U_n, d.V_n, 0);
-    k_bih_uc<<<gl, 256, 0, s>>>(d, 0);
-    k_bih_grad<false><<<gl, 256, 0, s>>>(d, d.bihU, d.bihV);
-    k_bih_edge<<<ge, 256, 0, s>>>(d, d.bihU, d.bihV, 1);
+    launch_k(k_bih_edge, ge, 256, 0, s, d, d.U_n, d.V_n, 0);
+    launch_k(k_bih_uc, gl, 256, 0, s, d, 0);
+    launch_k(k_bih_grad<false>, gl, 256, 0, s, d, d.bihU, d.bihV);
+    launch_k(k_bih_edge, ge, 256, 0, s, d, d.bihU, d.bihV, 1);
 }
 void launch_bih_puls(const Dev &d, cudaStream_t s) {
     const int ge = grid_for((long long)d.Ed * d.L, 256), gl = grid_for((long long)d.E * d.L, 256);
-    k_bih_grad<true><<<gl, 256, 0, s>>>(d, d.U_puls, d.V_puls);
-    k_bih_edge<<<ge, 256, 0, s>>>(d, d.U_puls, d.V_puls, 0);
-    k_bih_uc<<<gl, 256, 0, s>>>(d, 1);
-    k_bih_grad<false><<<gl, 256, 0, s>>>(d, d.bihU, d.bihV);
-    k_bih_edge<<<ge, 256, 0, s>>>(d, d.bihU, d.bihV, 2);
+    launch_k(k_bih_grad<true>, gl, 256, 0, s, d, d.U_puls, d.V_puls);
+    launch_k(k_bih_edge, ge, 256, 0, s, d, d.U_puls, d.V_puls, 0);
+    launch_k(k_bih_uc, gl, 256, 0, s, d, 1);
+    launch_k(k_bih_grad<false>, gl, 256, 0, s, d, d.bihU, d.bihV);
+    launch_k(k_bih_edge, ge, 256, 0, s, d, d.bihU, d.bihV, 2);
 }
 void launch_velrhs(const Dev &d, real ff, cudaStream_t s) {
     const int b = tuned(d, TK_VELRHS, 256);
-    k_velrhs<<<grid_for((long long)d.E * d.L, b), b, 0, s>>>(d, ff);
+    launch_k(k_velrhs, grid_for((long long)d.E * d.L, b), b, 0, s, d, ff);
 }
 #define MAXL_DISPATCH(KERNEL, GRID, BLOCK, STREAM, ...)                                   \
     do {                                                                                   \
-        if (d.L <= 24) KERNEL<24><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__);                \
-        else if (d.L <= 48) KERNEL<48><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__);           \
-        else KERNEL<128><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__);                         \
+        if (d.L <= 24) launch_k(KERNEL<24>, GRID, BLOCK, 0, STREAM, __VA_ARGS__);                \
+        else if (d.L <= 48) launch_k(KERNEL<48>, GRID, BLOCK, 0, STREAM, __VA_ARGS__);           \
+        else launch_k(KERNEL<128>, GRID, BLOCK, 0, STREAM, __VA_ARGS__);                         \
     } while (0)
 void launch_implvisc(const Dev &d, cudaStream_t s) {
     if (implvisc_tiled(d)) {
         const long long tiles = ((long long)d.E + kIvCols - 1) / kIvCols;
         const int g = (int)(tiles < (1LL << 30) ? tiles : (1LL << 30));
-        if (d.L == 10) k_implvisc_fic_tile<10><<<g, kIvCols, implvisc_tile_smem(d), s>>>(d);
-        else k_implvisc_fic_tile<20><<<g, kIvCols, implvisc_tile_smem(d), s>>>(d);
+        if (d.L == 10) launch_k(k_implvisc_fic_tile<10>, g, kIvCols, implvisc_tile_smem(d), s, d);
+        else launch_k(k_implvisc_fic_tile<20>, g, kIvCols, implvisc_tile_smem(d), s, d);
         return;
     }
     MAXL_DISPATCH(k_implvisc, grid_for(d.E, 128), 128, s, d);
 }
-void launch_jac_swap(const Dev &d, cudaStream_t s) { k_jac_swap<<<grid_for(d.N, 256), 256, 0, s>>>(d); }
-void launch_je(const Dev &d, cudaStream_t s) { k_je_elem<<<grid_for((long long)d.E * d.L, 256), 256, 0, s>>>(d); }
+void launch_jac_swap(const Dev &d, cudaStream_t s) { launch_k(k_jac_swap, grid_for(d.N, 256), 256, 0, s, d); }
+void launch_je(const Dev &d, cudaStream_t s) { launch_k(k_je_elem, grid_for((long long)d.E * d.L, 256), 256, 0, s, d); }
 void launch_update3d(const Dev &d, real Mt_inv, cudaStream_t s) {
-    k_update3d<<<col_grid(d, d.E), col_b(d) * d.L, col_smem(d, 2, kU3Sc), s>>>(d, Mt_inv);
+    launch_k(k_update3d, col_grid(d, d.E), col_b(d) * d.L, col_smem(d, 2, kU3Sc), s, d, Mt_inv);
 }
-void launch_wvel(const Dev &d, cudaStream_t s) { k_wvel<<<col_grid(d, d.N), col_b(d) * d.L, col_smem(d, 1, 2), s>>>(d); }
+void launch_wvel(const Dev &d, cudaStream_t s) { launch_k(k_wvel, col_grid(d, d.N), col_b(d) * d.L, col_smem(d, 1, 2), s, d); }
 
 
 // Largest block (threads) each tunable kernel of this file can launch with

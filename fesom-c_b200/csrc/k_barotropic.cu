@@ -33,6 +33,7 @@ __device__ __forceinline__ real2 ab3v(real b, real2 x0, real2 x1, real2 x2) {
 // their AB3 again in this kernel).
 // ---------------------------------------------------------------------------
 __global__ void k_ab3_elem(Dev d) {
+    pdl_enter();
     GRID_LOOP(ii, d.E) {
         const int e = (int)ii;
         const real b = d.beta;
@@ -69,6 +70,7 @@ __device__ __forceinline__ real ssh_edge_flux(const Dev &d, int ed) {
 // the SSH edge flux of every edge, once, for both end nodes to gather (the
 // flux array stays in L2; a quarter faster than forming it per node)
 __global__ void k_ssh_edge(Dev d) {
+    pdl_enter();
     GRID_LOOP(ed, d.Ed) d.sshfl[ed] = ssh_edge_flux(d, (int)ed);
 }
 
@@ -83,6 +85,7 @@ __global__ void k_ssh_edge(Dev d) {
 // ---------------------------------------------------------------------------
 // 40 registers: 6 resident blocks per SM instead of 5 (3 % faster).
 __global__ void __maxnreg__(40) k_ssh_node(Dev d, int sub) {
+    pdl_enter();
     const double de = 0.614, ga = 0.088, ep = 0.013, fe = 1.0 - de - ga - ep;
     GRID_LOOP(ii, d.N) {
         const int n = (int)ii;
@@ -115,6 +118,7 @@ __global__ void __maxnreg__(40) k_ssh_node(Dev d, int sub) {
 // (fv_3D_vel.F90:257-307), one thread per (element, level).
 // ---------------------------------------------------------------------------
 __global__ void k_puls_elem(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     GRID_LOOP(ii, total) {
         const int e = (int)(ii / d.L);
@@ -133,6 +137,7 @@ __global__ void k_puls_elem(Dev d) {
 
 // compute_el2nodes_3D (fv_utilit.F90:644-700), one thread per (node, level)
 __global__ void k_el2nodes(Dev d, const real *Ue, const real *Ve, real *Un, real *Vn) {
+    pdl_enter();
     const long long total = (long long)d.N * d.L;
     GRID_LOOP(ii, total) {
         const int n = (int)(ii / d.L);
@@ -154,6 +159,7 @@ __global__ void k_el2nodes(Dev d, const real *Ue, const real *Ve, real *Un, real
 // uu*un, vv*un of every (internal edge, level), thread per (edge, level).
 // Stored in the adv3 buffer, which velrhs has finished with.
 __global__ void k_p1_edge(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.Ed_in * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
@@ -187,6 +193,7 @@ __global__ void k_p1_edge(Dev d) {
 // biharmonic terms level by level.
 constexpr int kP1Slots = 5;  // 4 internal-edge slots + the filter
 __global__ void k_p1_elem(Dev d) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const int L = d.L;
     const int B = (int)blockDim.x / L;
@@ -311,6 +318,7 @@ __device__ __forceinline__ void adv2d_edge(const Dev &d, int ed, real &uu, real 
 
 // momentum_adv_upwind_2D edge fluxes of the sub-step, once per internal edge
 __global__ void k_adv2d_edge(Dev d) {
+    pdl_enter();
     GRID_LOOP(ed, d.Ed_in) {
         real uu, vv;
         adv2d_edge(d, (int)ed, uu, vv);
@@ -325,6 +333,7 @@ __global__ void k_adv2d_edge(Dev d) {
 // fluxes; bih2d_grad: vel_gradients_2D(Ul) into vel_grad (adv2d_edge has
 // used the gradients of UAB by then).  u2d_elem gathers the second pass.
 __global__ void k_bih2d_edge(Dev d, const real2 *U) {
+    pdl_enter();
     GRID_LOOP(ii, d.Ed) {
         const int ed = (int)ii;
         const int2 et = d.edge_tri[ed];
@@ -368,6 +377,7 @@ __global__ void k_bih2d_edge(Dev d, const real2 *U) {
 }
 
 __global__ void k_bih2d_ul(Dev d) {
+    pdl_enter();
     GRID_LOOP(ii, d.E) {
         const int e = (int)ii;
         const int4 se = d.elem_sedges[e];
@@ -390,6 +400,7 @@ __global__ void k_bih2d_ul(Dev d) {
 // vel_gradients_2D (fv_gradients.F90:97-176, free slip) of U into vel_grad:
 // of UAB after ab3_elem in every sub-step, of Ul in biharmonic_2D
 __global__ void k_velgrad2d(Dev d, const real2 *U) {
+    pdl_enter();
     GRID_LOOP(ii, d.E) {
         const int e = (int)ii;
         const int4 en = d.elem_nodes[e];
@@ -431,6 +442,7 @@ __global__ void k_velgrad2d(Dev d, const real2 *U) {
 // u2d_elem forms UV2_rhs from the neighbours' U_c.  Runs before u2d_elem,
 // which rotates U_n_2D.
 __global__ void k_filt2x_2d(Dev d) {
+    pdl_enter();
     const real tau_inv = d.dt_2D * d.tau_c / real(3600.0) / real(24.0);
     GRID_LOOP(ii, d.E) {
         const int e = (int)ii;
@@ -457,6 +469,7 @@ __global__ void k_filt2x_2d(Dev d) {
 // ---------------------------------------------------------------------------
 // FP32: 8 resident blocks (at most 64 registers); FP64: 6.
 __global__ void __launch_bounds__(128, FESOMC_FP32 ? 8 : 6) k_u2d_elem(Dev d) {
+    pdl_enter();
     const real d0inv = real(1.0) / d.density_0;
     GRID_LOOP(ii, d.E) {
         const int e = (int)ii;
@@ -577,6 +590,7 @@ __global__ void __launch_bounds__(128, FESOMC_FP32 ? 8 : 6) k_u2d_elem(Dev d) {
 
 // eta time-level rotation (fv_main.F90:1547-1551)
 __global__ void k_rot_nodes(Dev d) {
+    pdl_enter();
     GRID_LOOP(ii, d.N) {
         const int n = (int)ii;
         const double e0 = d.eta_n[n], e1 = d.eta_n_1[n];
@@ -591,6 +605,7 @@ __global__ void k_rot_nodes(Dev d) {
 // sub-step (fv_average_dynamic.F90:262, 400-420; U_n is fixed during the
 // sub-cycle)
 __global__ void k_zero_filt(Dev d) {
+    pdl_enter();
     GRID_LOOP(ii, d.E) {
         d.U_filt_2D[ii] = real(0.0);
         d.V_filt_2D[ii] = real(0.0);
@@ -603,21 +618,21 @@ __global__ void k_zero_filt(Dev d) {
 // ---- launch wrappers --------------------------------------------------------
 void launch_ab3_elem(const Dev &d, cudaStream_t s) {
     const int b1 = tuned(d, TK_AB3, 256), b2 = tuned(d, TK_VELGRAD2D, 256);
-    k_ab3_elem<<<grid_for(d.E, b1), b1, 0, s>>>(d);
-    k_velgrad2d<<<grid_for(d.E, b2), b2, 0, s>>>(d, d.UAB);
+    launch_k(k_ab3_elem, grid_for(d.E, b1), b1, 0, s, d);
+    launch_k(k_velgrad2d, grid_for(d.E, b2), b2, 0, s, d, d.UAB);
 }
 void launch_ssh_node(const Dev &d, int sub, cudaStream_t s) {
     const int b1 = tuned(d, TK_SSHEDGE, 256), b2 = tuned(d, TK_SSHNODE, 256);
-    k_ssh_edge<<<grid_for(d.Ed, b1), b1, 0, s>>>(d);
-    k_ssh_node<<<grid_for(d.N, b2), b2, 0, s>>>(d, sub);
+    launch_k(k_ssh_edge, grid_for(d.Ed, b1), b1, 0, s, d);
+    launch_k(k_ssh_node, grid_for(d.N, b2), b2, 0, s, d, sub);
 }
 void launch_puls_elem(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_PULS, 256);
-    k_puls_elem<<<grid_for((long long)d.E * d.L, b), b, 0, s>>>(d);
+    launch_k(k_puls_elem, grid_for((long long)d.E * d.L, b), b, 0, s, d);
 }
 void launch_el2nodes(const Dev &d, const real *Ue, const real *Ve, real *Un, real *Vn, cudaStream_t s) {
     const int b = tuned(d, TK_EL2NODES, 256);
-    k_el2nodes<<<grid_for((long long)d.N * d.L, b), b, 0, s>>>(d, Ue, Ve, Un, Vn);
+    launch_k(k_el2nodes, grid_for((long long)d.N * d.L, b), b, 0, s, d, Ue, Ve, Un, Vn);
 }
 // B elements per block: B*L threads, at most 1024 and at most 32 elements;
 // per element its slot tile, 8 slot sums, 4 acc, dmean_n and 4 edge codes
@@ -632,35 +647,35 @@ int config_p1(const Dev &d) {
 }
 void launch_p1_edge(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_P1EDGE, 256);
-    k_p1_edge<<<grid_for((long long)d.Ed_in * d.L, b), b, 0, s>>>(d);
+    launch_k(k_p1_edge, grid_for((long long)d.Ed_in * d.L, b), b, 0, s, d);
 }
 void launch_p1_elem(const Dev &d, cudaStream_t s) {
     const int B = p1_elems(d);
     const long long blocks = ((long long)d.E + B - 1) / B;
-    k_p1_elem<<<(int)(blocks < 148LL * 16 ? blocks : 148LL * 16), B * d.L, p1_smem(d), s>>>(d);
+    launch_k(k_p1_elem, (int)(blocks < 148LL * 16 ? blocks : 148LL * 16), B * d.L, p1_smem(d), s, d);
 }
 void launch_adv2d_edge(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ADV2D, 256);
-    k_adv2d_edge<<<grid_for(d.Ed_in, b), b, 0, s>>>(d);
+    launch_k(k_adv2d_edge, grid_for(d.Ed_in, b), b, 0, s, d);
 }
-void launch_filt2x_2d(const Dev &d, cudaStream_t s) { k_filt2x_2d<<<grid_for(d.E, 256), 256, 0, s>>>(d); }
+void launch_filt2x_2d(const Dev &d, cudaStream_t s) { launch_k(k_filt2x_2d, grid_for(d.E, 256), 256, 0, s, d); }
 void launch_bih_2d(const Dev &d, cudaStream_t s) {
-    k_bih2d_edge<<<grid_for(d.Ed, 256), 256, 0, s>>>(d, d.UAB);
-    k_bih2d_ul<<<grid_for(d.E, 256), 256, 0, s>>>(d);
-    k_velgrad2d<<<grid_for(d.E, 256), 256, 0, s>>>(d, d.b2ul);
-    k_bih2d_edge<<<grid_for(d.Ed, 256), 256, 0, s>>>(d, d.b2ul);
+    launch_k(k_bih2d_edge, grid_for(d.Ed, 256), 256, 0, s, d, d.UAB);
+    launch_k(k_bih2d_ul, grid_for(d.E, 256), 256, 0, s, d);
+    launch_k(k_velgrad2d, grid_for(d.E, 256), 256, 0, s, d, d.b2ul);
+    launch_k(k_bih2d_edge, grid_for(d.Ed, 256), 256, 0, s, d, d.b2ul);
 }
 void launch_u2d_elem(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_U2D, 128);
-    k_u2d_elem<<<grid_for(d.E, b), b, 0, s>>>(d);
+    launch_k(k_u2d_elem, grid_for(d.E, b), b, 0, s, d);
 }
 void launch_rot_nodes(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ROT, 256);
-    k_rot_nodes<<<grid_for(d.N, b), b, 0, s>>>(d);
+    launch_k(k_rot_nodes, grid_for(d.N, b), b, 0, s, d);
 }
 void launch_zero_filt(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ZEROFILT, 256);
-    k_zero_filt<<<grid_for(d.E, b), b, 0, s>>>(d);
+    launch_k(k_zero_filt, grid_for(d.E, b), b, 0, s, d);
 }
 
 

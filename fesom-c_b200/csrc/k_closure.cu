@@ -64,6 +64,7 @@ __device__ __forceinline__ unsigned long long warp_append(bool take, unsigned lo
 // Inputs of every column, normalised into X; the envelope test; the list of
 // columns the plain closure takes (dry or outside the envelope); counters.
 __global__ void k_lc_features(Dev d, LcView c) {
+    pdl_enter();
     GRID_LOOP(ii, d.N) {
         const int node = (int)ii;
         float *x = c.X + (size_t)node * c.IN;
@@ -112,6 +113,7 @@ __device__ __forceinline__ void lc_state(const Dev &d, const LcView &c, int node
 
 // Network columns: bt, snu and Kv of the network's closure state.
 __global__ void k_lc_apply(Dev d, LcView c) {
+    pdl_enter();
     GRID_LOOP(ii, d.N) {
         const int node = (int)ii;
         if (!c.flag[node]) continue;
@@ -137,6 +139,7 @@ __global__ void k_lc_apply(Dev d, LcView c) {
 // one block turns the counts into first slots (an ordered scan from the
 // current count), and each block writes its columns at its slots.
 __global__ void k_lc_wetcount(Dev d, LcView c) {
+    pdl_enter();
     const int node = blockIdx.x * kLcHarvestBlock + threadIdx.x;
     const bool wet = node < d.N && d.mask_wd_node[node] != real(0.0);
     const int n = __syncthreads_count(wet);
@@ -146,6 +149,7 @@ __global__ void k_lc_wetcount(Dev d, LcView c) {
 // blk[b] <- the slot of block b's first wet column (capped at hcap);
 // hcount <- hcount + all wet columns.  One block of 1024 threads.
 __global__ void k_lc_slots(int nblk, LcView c) {
+    pdl_enter();
     __shared__ unsigned long long wsum[32];
     __shared__ unsigned long long base;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -180,6 +184,7 @@ __global__ void k_lc_slots(int nblk, LcView c) {
 }
 
 __global__ void k_lc_harvest(Dev d, LcView c) {
+    pdl_enter();
     __shared__ int wcount[kLcHarvestBlock / 32];
     const int node = blockIdx.x * kLcHarvestBlock + threadIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -200,6 +205,7 @@ __global__ void k_lc_harvest(Dev d, LcView c) {
 // judge: the plain closure ran on every column; compare the network's
 // viscosity on the columns it would have taken (log difference)
 __global__ void k_lc_judge(Dev d, LcView c) {
+    pdl_enter();
     double s2 = 0.0, n = 0.0, mx = 0.0;
     GRID_LOOP(ii, d.N) {
         const int node = (int)ii;
@@ -230,20 +236,20 @@ __global__ void k_lc_judge(Dev d, LcView c) {
 }
 
 void launch_lc_features(const Dev &d, const LcView &c, cudaStream_t s) {
-    k_lc_features<<<grid_for(d.N, 128), 128, 0, s>>>(d, c);
+    k_lc_features<<<grid_for(d.N, 128), 128, 0, s>>>(d, c);   // follows a memset
 }
 void launch_lc_apply(const Dev &d, const LcView &c, cudaStream_t s) {
-    k_lc_apply<<<grid_for(d.N, 128), 128, 0, s>>>(d, c);
+    launch_k(k_lc_apply, grid_for(d.N, 128), 128, 0, s, d, c);
 }
 int lc_harvest_blocks(int N) { return (N + kLcHarvestBlock - 1) / kLcHarvestBlock; }
 void launch_lc_harvest(const Dev &d, const LcView &c, cudaStream_t s) {
     const int nblk = lc_harvest_blocks(d.N);
-    k_lc_wetcount<<<nblk, kLcHarvestBlock, 0, s>>>(d, c);
-    k_lc_slots<<<1, 1024, 0, s>>>(nblk, c);
-    k_lc_harvest<<<nblk, kLcHarvestBlock, 0, s>>>(d, c);
+    launch_k(k_lc_wetcount, nblk, kLcHarvestBlock, 0, s, d, c);
+    launch_k(k_lc_slots, 1, 1024, 0, s, nblk, c);
+    launch_k(k_lc_harvest, nblk, kLcHarvestBlock, 0, s, d, c);
 }
 void launch_lc_judge(const Dev &d, const LcView &c, cudaStream_t s) {
-    k_lc_judge<<<grid_for(d.N, 128), 128, 0, s>>>(d, c);
+    launch_k(k_lc_judge, grid_for(d.N, 128), 128, 0, s, d, c);
 }
 
 FESOMC_PREC_END

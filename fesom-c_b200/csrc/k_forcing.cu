@@ -15,12 +15,14 @@ namespace fesomc {
 
 // time_jd = time_jd + dt/86400 (one thread)
 __global__ void k_forcing_clock(ForcingDev f) {
+    pdl_enter();
     if (blockIdx.x == 0 && threadIdx.x == 0) f.clock[0] = f.clock[0] + f.dt / 86400.0;
 }
 
 // open-boundary elevation of the Mt sub-steps (slot sub*nobn + q) and the
 // river runoff of the step
 __global__ void k_forcing_values(ForcingDev f) {
+    pdl_enter();
     const double time_jd = f.clock[0];
     const double time = time_jd * 86400.0;
     const long long n_ob = f.tides_on ? (long long)f.Mt * f.nobn : 0;
@@ -58,6 +60,7 @@ __device__ __forceinline__ double control_360(double fr) {
 // the phases sxi depend on the step only; every thread forms them itself
 // (a few dozen operations against the 11 cosines of a node).
 __global__ void k_potential(PotentialDev p) {
+    pdl_enter();
     const double Apt[11] = {0.242334, 0.112841, 0.046398, 0.030704, 0.141565, 0.100514,
                             0.046843, 0.019256, 0.041742, 0.022026, 0.019446};
     const double Fpt[11] = {1.40519e-4, 1.45444e-4, 1.37880e-4, 1.45842e-4, 0.72921e-4, 0.67598e-4,
@@ -108,17 +111,17 @@ void launch_potential(const PotentialDev &p, cudaStream_t s) {
     long long g = ((long long)p.N + block - 1) / block;
     if (g < 1) g = 1;
     if (g > 148 * 8) g = 148 * 8;
-    k_potential<<<(int)g, block, 0, s>>>(p);
+    launch_k(k_potential, (int)g, block, 0, s, p);
 }
 
 void launch_forcing(const ForcingDev &f, cudaStream_t s) {
-    k_forcing_clock<<<1, 32, 0, s>>>(f);
+    launch_k(k_forcing_clock, 1, 32, 0, s, f);
     const long long n = (f.tides_on ? (long long)f.Mt * f.nobn : 0) + (f.rivers_on ? f.n_rivers : 0);
     const int block = 128;
     long long g = (n + block - 1) / block;
     if (g < 1) g = 1;
     if (g > 148) g = 148;
-    k_forcing_values<<<(int)g, block, 0, s>>>(f);
+    launch_k(k_forcing_values, (int)g, block, 0, s, f);
 }
 
 }  // namespace fesomc

@@ -50,6 +50,7 @@ __device__ __forceinline__ bool d3_above_tol(real a, real b) {
 // columns the learned closure hands back to the plain one).
 template <int ARR, bool kList>
 __global__ void k_d3end(Dev d, const int *list, const unsigned long long *count) {
+    pdl_enter();
     const real t_inv = real(1.0) / d.dt;
     const real cka = d.cka;
     const real B1cka2 = real(16.6) * (cka * cka);
@@ -210,6 +211,7 @@ __host__ __device__ inline int d3end_values(int NS) { return 7 * NS - 8; }
 
 template <bool kList>
 __global__ void __launch_bounds__(kD3Block, 6) k_d3end_sm(Dev d, const int *list, const unsigned long long *count) {
+    pdl_enter();
     extern __shared__ unsigned char d3_smem[];
     constexpr int B = kD3Block;
     const int NS = d.NS, L = d.L;
@@ -386,6 +388,7 @@ constexpr int kD3Tile = 32;
 constexpr int kD3SetupThreads = 256;
 
 __global__ void __launch_bounds__(kD3SetupThreads) k_d3end_setup(Dev d) {
+    pdl_enter();
     extern __shared__ unsigned char d3s_smem[];
     const int NS = d.NS, L = d.L, N = d.N;
     real *sm = reinterpret_cast<real *>(d3s_smem);
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(kD3SetupThreads) k_d3end_setup(Dev d) {
 // constants; the same arithmetic as k_d3end, in the same order.
 template <int ARR, bool kList>
 __global__ void k_d3end_sweep(Dev d, const int *list, const unsigned long long *count) {
+    pdl_enter();
     const real t_inv = real(1.0) / d.dt;
     const real cka = d.cka;
     const real B1cka2 = real(16.6) * (cka * cka);
@@ -584,6 +588,7 @@ __global__ void k_d3end_sweep(Dev d, const int *list, const unsigned long long *
 // [thread] (launch-shape knob "d3end_arrays" = 4): no local memory at all,
 // 4*NS - 2 values per column, blocks of kD3Block columns.
 __global__ void __launch_bounds__(kD3Block) k_d3end_sweep_sm(Dev d) {
+    pdl_enter();
     extern __shared__ unsigned char d3w_smem[];
     constexpr int B = kD3Block;
     const real t_inv = real(1.0) / d.dt;
@@ -775,6 +780,7 @@ __device__ __forceinline__ bool d3_sweep_reg(const Dev &d, size_t N, int node, c
 // 8 (128 registers, a few spilled)
 template <int NSC, int MINB>
 __global__ void __launch_bounds__(64, MINB) k_d3end_sweep_reg(Dev d) {
+    pdl_enter();
     const real t_inv = real(1.0) / d.dt;
     const real cka = d.cka;
     const real B1cka2 = real(16.6) * (cka * cka);
@@ -849,6 +855,7 @@ __global__ void __launch_bounds__(64, MINB) k_d3end_sweep_reg(Dev d) {
 
 // Av(nz,elem) = sum(w_cv*snu(nz,nodes)) (fv_mixing.F90:308-313)
 __global__ void k_av(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.E * d.NS;
     GRID_LOOP(ii, total) {
         const int e = (int)(ii / d.NS);
@@ -880,41 +887,41 @@ int config_d3end(const Dev &d) {
 }
 static void launch_d3end_split(const Dev &d, cudaStream_t s) {
     const int tiles = (d.N + kD3Tile - 1) / kD3Tile;
-    k_d3end_setup<<<tiles < 148 * 16 ? tiles : 148 * 16, kD3SetupThreads, d3end_setup_smem(d), s>>>(d);
+    launch_k(k_d3end_setup, tiles < 148 * 16 ? tiles : 148 * 16, kD3SetupThreads, d3end_setup_smem(d), s, d);
     if (d3end_reg(d)) {
         const bool b8 = d.tune[TK_D3END] == 6;
-        if (d.NS == 11 && b8) k_d3end_sweep_reg<11, 8><<<grid_for(d.N, 64), 64, 0, s>>>(d);
-        else if (d.NS == 11) k_d3end_sweep_reg<11, 6><<<grid_for(d.N, 64), 64, 0, s>>>(d);
-        else if (b8) k_d3end_sweep_reg<21, 8><<<grid_for(d.N, 64), 64, 0, s>>>(d);
-        else k_d3end_sweep_reg<21, 6><<<grid_for(d.N, 64), 64, 0, s>>>(d);
+        if (d.NS == 11 && b8) launch_k(k_d3end_sweep_reg<11, 8>, grid_for(d.N, 64), 64, 0, s, d);
+        else if (d.NS == 11) launch_k(k_d3end_sweep_reg<11, 6>, grid_for(d.N, 64), 64, 0, s, d);
+        else if (b8) launch_k(k_d3end_sweep_reg<21, 8>, grid_for(d.N, 64), 64, 0, s, d);
+        else launch_k(k_d3end_sweep_reg<21, 6>, grid_for(d.N, 64), 64, 0, s, d);
     }
-    else if (d.tune[TK_D3END] == 4) k_d3end_sweep_sm<<<grid_for(d.N, kD3Block), kD3Block, d3end_sweep_smem(d), s>>>(d);
-    else if (d.NS <= 11) k_d3end_sweep<12, false><<<grid_for(d.N, 64), 64, 0, s>>>(d, nullptr, nullptr);
-    else if (d.NS <= 21) k_d3end_sweep<22, false><<<grid_for(d.N, 64), 64, 0, s>>>(d, nullptr, nullptr);
-    else k_d3end_sweep<41, false><<<grid_for(d.N, 64), 64, 0, s>>>(d, nullptr, nullptr);
+    else if (d.tune[TK_D3END] == 4) launch_k(k_d3end_sweep_sm, grid_for(d.N, kD3Block), kD3Block, d3end_sweep_smem(d), s, d);
+    else if (d.NS <= 11) launch_k(k_d3end_sweep<12, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
+    else if (d.NS <= 21) launch_k(k_d3end_sweep<22, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
+    else launch_k(k_d3end_sweep<41, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
 }
 void launch_d3end(const Dev &d, cudaStream_t s) {
     if (d3end_split(d)) launch_d3end_split(d, s);
-    else if (d.tune[TK_D3END] == 2) k_d3end_sm<false><<<grid_for(d.N, kD3Block), kD3Block, d3end_smem(d), s>>>(d, nullptr, nullptr);
-    else if (d.NS <= 11) k_d3end<12, false><<<grid_for(d.N, 64), 64, 0, s>>>(d, nullptr, nullptr);
-    else if (d.NS <= 21) k_d3end<22, false><<<grid_for(d.N, 64), 64, 0, s>>>(d, nullptr, nullptr);
-    else if (d.NS <= 40) k_d3end<41, false><<<grid_for(d.N, 64), 64, 0, s>>>(d, nullptr, nullptr);
-    else k_d3end<128, false><<<grid_for(d.N, 64), 64, 0, s>>>(d, nullptr, nullptr);
+    else if (d.tune[TK_D3END] == 2) launch_k(k_d3end_sm<false>, grid_for(d.N, kD3Block), kD3Block, d3end_smem(d), s, d, nullptr, nullptr);
+    else if (d.NS <= 11) launch_k(k_d3end<12, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
+    else if (d.NS <= 21) launch_k(k_d3end<22, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
+    else if (d.NS <= 40) launch_k(k_d3end<41, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
+    else launch_k(k_d3end<128, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
 }
 // the plain closure on the listed columns (count read on the device, so the
 // launch covers every node and the grid-stride loop stops at the count)
 // (the two-kernel form sets up every column, so the listed columns take the
 // one-kernel forms, which leave the others' Ri alone)
 void launch_d3end_list(const Dev &d, const int *list, const unsigned long long *count, cudaStream_t s) {
-    if (d.tune[TK_D3END] == 2) k_d3end_sm<true><<<grid_for(d.N, kD3Block), kD3Block, d3end_smem(d), s>>>(d, list, count);
-    else if (d.NS <= 11) k_d3end<12, true><<<grid_for(d.N, 64), 64, 0, s>>>(d, list, count);
-    else if (d.NS <= 21) k_d3end<22, true><<<grid_for(d.N, 64), 64, 0, s>>>(d, list, count);
-    else if (d.NS <= 40) k_d3end<41, true><<<grid_for(d.N, 64), 64, 0, s>>>(d, list, count);
-    else k_d3end<128, true><<<grid_for(d.N, 64), 64, 0, s>>>(d, list, count);
+    if (d.tune[TK_D3END] == 2) launch_k(k_d3end_sm<true>, grid_for(d.N, kD3Block), kD3Block, d3end_smem(d), s, d, list, count);
+    else if (d.NS <= 11) launch_k(k_d3end<12, true>, grid_for(d.N, 64), 64, 0, s, d, list, count);
+    else if (d.NS <= 21) launch_k(k_d3end<22, true>, grid_for(d.N, 64), 64, 0, s, d, list, count);
+    else if (d.NS <= 40) launch_k(k_d3end<41, true>, grid_for(d.N, 64), 64, 0, s, d, list, count);
+    else launch_k(k_d3end<128, true>, grid_for(d.N, 64), 64, 0, s, d, list, count);
 }
 void launch_av(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_AV, 256);
-    k_av<<<grid_for((long long)d.E * d.NS, b), b, 0, s>>>(d);
+    launch_k(k_av, grid_for((long long)d.E * d.NS, b), b, 0, s, d);
 }
 
 

@@ -28,6 +28,7 @@ constexpr int kRedGrid = 592;  // 4 x 148 SMs
 // One partial per (block, member): blockIdx.y is the member, whose nodes
 // are member_node_off[m] .. member_node_off[m+1] (all nodes for one member).
 __global__ void k_minmax_part(Dev d) {
+    pdl_enter();
     __shared__ real s[4][kRedBlock];
     const int mb = blockIdx.y;
     const long long n0 = d.member_node_off ? d.member_node_off[mb] : 0;
@@ -58,6 +59,7 @@ __global__ void k_minmax_part(Dev d) {
 // one warp per member; min / max are exact, so the order in which the
 // partials are combined does not change the result
 __global__ void k_minmax_final(Dev d, int nparts) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const real *part = d.mm_part + (size_t)blockIdx.x * nparts * 4;
     real tmin = part[0], tmax = part[1], smin = part[2], smax = part[3];
@@ -187,6 +189,7 @@ __device__ __forceinline__ void tvert_upwind2(const Dev &d, int k, real a, const
 // AB2 tracers of this step minus their means, stored once per (node, level)
 // for the gathers below (fv_tracer.F90:433,435 and :39-47)
 __global__ void k_ab2_node(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.N * d.L;
     GRID_LOOP(i, total) {
         const int n = (int)(i / d.L);
@@ -200,6 +203,7 @@ __global__ void k_ab2_node(Dev d) {
 // lanes of a flat index (no lane idles when L < 32); level data coalesced.
 // ---------------------------------------------------------------------------
 __global__ void k_upwind_h(Dev d) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int L = d.L, NS = d.NS;
     const long long total = (long long)d.N * L;
@@ -297,6 +301,7 @@ __global__ void k_upwind_h(Dev d) {
 // ---------------------------------------------------------------------------
 // tracer_gradient_elements of the AB2 tracer, thread per (element, level)
 __global__ void k_muscl_egrad(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     GRID_LOOP(ii, total) {
         const int e = (int)(ii / d.L);
@@ -318,6 +323,7 @@ __global__ void k_muscl_egrad(Dev d) {
 // area-weighted node mean of the element gradients (fill_up_dn_grad fallback,
 // fv_gradients.F90:292-318: tx/tvol with running sums)
 __global__ void k_muscl_ngrad(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.N * d.L;
     GRID_LOOP(ii, total) {
         const int n = (int)(ii / d.L);
@@ -439,6 +445,7 @@ __device__ __forceinline__ real muscl_mean(bool upw2, real Tm1, real Tm2) {
 // end nodes below.  64 registers: 32 resident warps per SM instead of 24
 // (17 % faster).
 __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.Ed * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
@@ -511,6 +518,7 @@ __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
 // together; the sums stay in edge order.  The vertical flux at interface
 // z+1 comes from the next lane when that lane holds the same node.
 __global__ void __launch_bounds__(128, 8) k_muscl_h(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.N * d.L;
     const int lane = threadIdx.x & 31;
     const int L = d.L, NS = d.NS;
@@ -585,6 +593,7 @@ __global__ void __launch_bounds__(128, 8) k_muscl_h(Dev d) {
 // advection-order mask of adv_tracer_mask (fv_main.F90:1309-1335,
 // H_advtr_crit = 0.1, H_advtr_min = 0)
 __global__ void k_miura_prep(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.N * d.L;
     GRID_LOOP(i, total) {
         const real T_aver = t_aver_of(d, (int)(i / d.L));
@@ -605,6 +614,7 @@ __global__ void k_miura_prep(Dev d) {
 
 // tracer_gradient_elements of T - T_aver (fv_gradients.F90:180-214)
 __global__ void k_miura_egrad(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.E * d.L;
     GRID_LOOP(ii, total) {
         const int e = (int)(ii / d.L);
@@ -621,6 +631,7 @@ __global__ void k_miura_egrad(Dev d) {
 // tracer_gradient_nodes (fv_gradients.F90:217-260): area-weighted sums
 // times the reciprocal of the summed area
 __global__ void k_miura_ngrad(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.N * d.L;
     GRID_LOOP(ii, total) {
         const int n = (int)(ii / d.L);
@@ -644,6 +655,7 @@ __global__ void k_miura_ngrad(Dev d) {
 // Miura segment fluxes of one (edge, level) (fv_tracer.F90:1010-1140) and the
 // continuity terms (:1141-1168); thread per (edge, level)
 __global__ void k_miura_edge(Dev d) {
+    pdl_enter();
     const long long total = (long long)d.Ed * d.L;
     const int L = d.L;
     const real dt = d.dt;
@@ -710,6 +722,7 @@ __global__ void k_miura_edge(Dev d) {
 // salinity passed through; one thread per (node, level), levels on
 // consecutive lanes of a flat index
 __global__ void __launch_bounds__(128, 8) k_miura_h(Dev d) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int L = d.L, NS = d.NS;
     const long long total = (long long)d.N * L;
@@ -914,6 +927,7 @@ __device__ real evap_precip(const Dev &d, int n, real aj, real T0, real S0, real
 // its register count without them
 template <bool kAtm>
 __global__ void __launch_bounds__(kVdBlock) k_vdiff_col(Dev d) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L, NS = d.NS;
@@ -1010,6 +1024,7 @@ struct KSum {
 };
 
 __global__ void k_energy_part(Dev d, double *part) {
+    pdl_enter();
     __shared__ double sh[3][kRedBlock];
     KSum pe{0.0, 0.0}, ke{0.0, 0.0}, ar{0.0, 0.0};
     GRID_LOOP(i, d.N) {
@@ -1041,6 +1056,7 @@ __global__ void k_energy_part(Dev d, double *part) {
 }
 
 __global__ void k_energy_final(const double *part, int nparts, double *out) {
+    pdl_enter();
     if (threadIdx.x < 3 && blockIdx.x == 0) {
         KSum t{0.0, 0.0};
         for (int b = 0; b < nparts; ++b) t.add(part[(size_t)b * 3 + threadIdx.x]);
@@ -1054,8 +1070,8 @@ __global__ void k_energy_final(const double *part, int nparts, double *out) {
 int minmax_parts(int n_members) { return n_members <= 1 ? kRedGrid : (kRedGrid / n_members > 8 ? kRedGrid / n_members : 8); }
 void launch_minmax(const Dev &d, cudaStream_t s) {
     const int parts = minmax_parts(d.n_members);
-    k_minmax_part<<<dim3(parts, d.n_members), kRedBlock, 0, s>>>(d);
-    k_minmax_final<<<d.n_members, 32, 0, s>>>(d, parts);
+    launch_k(k_minmax_part, dim3(parts, d.n_members), kRedBlock, 0, s, d);
+    launch_k(k_minmax_final, d.n_members, 32, 0, s, d, parts);
 }
 // ---- sbc_do on the device: bulk surface fluxes ------------------------------
 // psi_h / psi_m of Large & Yeager (2004), eq. 8c-8e (fv_sbc.F90:620-662);
@@ -1139,6 +1155,7 @@ __device__ void sbc_core_coeff_2z(double zt, double zu, double sst, double T_zt,
 // subtracts the surface Unode / Vnode of the previous step, the surface
 // temperature is TF's top layer.  rhoa, albo, emiss_wat are REAL(4).
 __global__ void k_atm_nodes(Dev d, AtmDev a) {
+    pdl_enter();
     const double now_date = a.clock[0];
     const double rhoa = (double)1.3f, cpa = 1005.0, Lv = 2.5e6, Stef = 5.67e-8, albo = (double)0.1f,
                  emiss_wat = (double)0.97f;
@@ -1176,6 +1193,7 @@ __global__ void k_atm_nodes(Dev d, AtmDev a) {
 }
 // the stress per element: sum(w_cv * taux_node(elem2D_nodes)) in node order
 __global__ void k_atm_stress(Dev d, AtmDev a) {
+    pdl_enter();
     GRID_LOOP(ee, d.E) {
         const int e = (int)ee;
         const int4 en = d.elem_nodes[e];
@@ -1193,52 +1211,53 @@ __global__ void k_atm_stress(Dev d, AtmDev a) {
     }
 }
 void launch_atm(const Dev &d, const AtmDev &a, cudaStream_t s) {
-    k_atm_nodes<<<grid_for(d.N, 128), 128, 0, s>>>(d, a);
-    k_atm_stress<<<grid_for(d.E, 256), 256, 0, s>>>(d, a);
+    launch_k(k_atm_nodes, grid_for(d.N, 128), 128, 0, s, d, a);
+    launch_k(k_atm_stress, grid_for(d.E, 256), 256, 0, s, d, a);
 }
 
 // T_aver / S_aver from a range the host gives (fesomc_gpu_set_tracer_range:
 // the min / max over the whole domain of a decomposed mesh), with
 // k_minmax_final's expression
 __global__ void k_aver_from_range(Dev d, const double *r) {
+    pdl_enter();
     if (threadIdx.x == 0) {
         d.aver[0] = real(0.5) * ((real)r[0] + (real)r[1]);
         d.aver[1] = real(0.5) * ((real)r[2] + (real)r[3]);
     }
 }
 void launch_aver_from_range(const Dev &d, const double *range, cudaStream_t s) {
-    k_aver_from_range<<<1, 32, 0, s>>>(d, range);
+    launch_k(k_aver_from_range, 1, 32, 0, s, d, range);
 }
 void launch_ab2(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_AB2, 256);
-    k_ab2_node<<<grid_for((long long)d.N * d.L, b), b, 0, s>>>(d);
+    launch_k(k_ab2_node, grid_for((long long)d.N * d.L, b), b, 0, s, d);
 }
 void launch_upwind(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_UPWIND, 128);
-    k_upwind_h<<<grid_for((long long)d.N * d.L, b), b, 0, s>>>(d);
+    launch_k(k_upwind_h, grid_for((long long)d.N * d.L, b), b, 0, s, d);
 }
 void launch_muscl_egrad(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_MEGRAD, 256);
-    k_muscl_egrad<<<grid_for((long long)d.E * d.L, b), b, 0, s>>>(d);
+    launch_k(k_muscl_egrad, grid_for((long long)d.E * d.L, b), b, 0, s, d);
 }
 void launch_muscl_ngrad(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_MNGRAD, 256);
-    k_muscl_ngrad<<<grid_for((long long)d.N * d.L, b), b, 0, s>>>(d);
+    launch_k(k_muscl_ngrad, grid_for((long long)d.N * d.L, b), b, 0, s, d);
 }
 void launch_miura(const Dev &d, cudaStream_t s) {
-    k_miura_prep<<<grid_for((long long)d.N * d.L, 256), 256, 0, s>>>(d);
-    k_miura_egrad<<<grid_for((long long)d.E * d.L, 256), 256, 0, s>>>(d);
-    k_miura_ngrad<<<grid_for((long long)d.N * d.L, 256), 256, 0, s>>>(d);
-    k_miura_edge<<<grid_for((long long)d.Ed * d.L, 256), 256, 0, s>>>(d);
-    k_miura_h<<<grid_for((long long)d.N * d.L, 128), 128, 0, s>>>(d);
+    launch_k(k_miura_prep, grid_for((long long)d.N * d.L, 256), 256, 0, s, d);
+    launch_k(k_miura_egrad, grid_for((long long)d.E * d.L, 256), 256, 0, s, d);
+    launch_k(k_miura_ngrad, grid_for((long long)d.N * d.L, 256), 256, 0, s, d);
+    launch_k(k_miura_edge, grid_for((long long)d.Ed * d.L, 256), 256, 0, s, d);
+    launch_k(k_miura_h, grid_for((long long)d.N * d.L, 128), 128, 0, s, d);
 }
 void launch_muscl_edge(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_MEDGE, 256);
-    k_muscl_edge<<<grid_for((long long)d.Ed * d.L, b), b, 0, s>>>(d);
+    launch_k(k_muscl_edge, grid_for((long long)d.Ed * d.L, b), b, 0, s, d);
 }
 void launch_muscl_h(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_MH, 128);
-    k_muscl_h<<<grid_for((long long)d.N * d.L, b), b, 0, s>>>(d);
+    launch_k(k_muscl_h, grid_for((long long)d.N * d.L, b), b, 0, s, d);
 }
 // ---- tracer_impl_vert_diff on tiles of columns (knob vdiff_form = 2) -------
 // k_vdiff_col reads each column with one thread, so a warp's loads of one
@@ -1258,6 +1277,7 @@ __host__ __device__ __forceinline__ int vd_odd(int x) { return x | 1; }
 
 template <bool kAtm, int LC, int kVtCols>
 __global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char vt_smem[];
     constexpr int L = LC, LP = LC | 1;
     const int NS = d.NS, KP = vd_odd(d.NS), N = d.N;
@@ -1415,8 +1435,8 @@ template <int LC, int C>
 static void launch_vdiff_tile(const Dev &d, cudaStream_t s) {
     const long long tiles = ((long long)d.N + C - 1) / C;
     const int g = (int)(tiles < (1LL << 30) ? tiles : (1LL << 30));
-    if (d.key_atm) k_vdiff_tile<true, LC, C><<<g, C, vdiff_tile_smem(d, C, true), s>>>(d);
-    else k_vdiff_tile<false, LC, C><<<g, C, vdiff_tile_smem(d, C, false), s>>>(d);
+    if (d.key_atm) launch_k(k_vdiff_tile<true, LC, C>, g, C, vdiff_tile_smem(d, C, true), s, d);
+    else launch_k(k_vdiff_tile<false, LC, C>, g, C, vdiff_tile_smem(d, C, false), s, d);
 }
 void launch_vdiff(const Dev &d, cudaStream_t s) {
     if (vdiff_tiled(d)) {
@@ -1427,13 +1447,13 @@ void launch_vdiff(const Dev &d, cudaStream_t s) {
         else launch_vdiff_tile<20, 128>(d, s);
         return;
     }
-    if (d.key_atm) k_vdiff_col<true><<<grid_for(d.N, vdiff_block(d)), vdiff_block(d), vdiff_smem(d), s>>>(d);
-    else k_vdiff_col<false><<<grid_for(d.N, vdiff_block(d)), vdiff_block(d), vdiff_smem(d), s>>>(d);
+    if (d.key_atm) launch_k(k_vdiff_col<true>, grid_for(d.N, vdiff_block(d)), vdiff_block(d), vdiff_smem(d), s, d);
+    else launch_k(k_vdiff_col<false>, grid_for(d.N, vdiff_block(d)), vdiff_block(d), vdiff_smem(d), s, d);
 }
 int energy_parts() { return kRedGrid; }
 void launch_energy(const Dev &d, double *part, double *out, cudaStream_t s) {
-    k_energy_part<<<kRedGrid, kRedBlock, 0, s>>>(d, part);
-    k_energy_final<<<1, 32, 0, s>>>(part, kRedGrid, out);
+    launch_k(k_energy_part, kRedGrid, kRedBlock, 0, s, d, part);
+    launch_k(k_energy_final, 1, 32, 0, s, part, kRedGrid, out);
 }
 
 

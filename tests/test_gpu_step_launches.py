@@ -1,0 +1,33 @@
+"""The step's launch rules against the oracle, bit for bit: meshes whose
+grids lie on both sides of the size up to which kernels are started early
+(programmatic dependent launch), in eager and captured steps."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _compare(case_of, steps):
+    import pyoracle
+    from fesomc import abi, cases, model
+    g = model.GpuModel(case_of(None))
+    o = pyoracle.Oracle(case_of(pyoracle.MeshLib(abi)), abi, cases)
+    try:
+        g.step(steps)
+        o.step(steps)
+        sg, so = g.state(), o.state()
+        for f in ("eta_n", "eta_n_1", "eta_n_2", "U_n_2D", "U_n_1", "U_n_2", "U_filt_2D", "U_n", "V_n", "TF", "SF",
+                  "bt", "snu", "Kv", "Av", "Wvel", "mask_wd", "mask_wd_node"):
+            assert np.array_equal(sg[f], so[f]), f
+    finally:
+        g.close()
+        o.close()
+
+
+# elements per 256-thread block of the 2D kernels, times 2 blocks per SM on
+# 148 SMs: 75,776 threads; the level kernels cross it at a few thousand
+# elements
+@pytest.mark.parametrize("nx,ny", [(9, 9), (100, 57), (310, 180)])
+def test_early_launch_sizes(built, nx, ny):
+    from fesomc import cases
+    _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, 11, 2.0, 25.0, stress=(0.0, 0.05), lib=lib), 3)
