@@ -12,7 +12,7 @@
 //                  (momentum_vert_impl_visc_tmp / momentum_vert_impl_visc)
 //   update3d     : update_3D_vel per element column; stores the new Je, Ze, ZBe
 //   wvel         : vert_vel_sigma per node column (edge gather + reverse scan)
-//   jac_swap     : jacobian bookkeeping (eta at the previous / last call)
+//   jac_swap     : last elevation rotation of the sub-cycle, jacobian elevation
 //   je_elem      : Je, Ze, ZBe at init
 #include "device_common.cuh"
 
@@ -723,12 +723,18 @@ __global__ void k_implvisc(Dev d) {
     }
 }
 
-// jacobian bookkeeping after the sub-cycle (fv_main.F90:2050): Jc_old <- Jc
+// after the sub-cycle: the last sub-step's rotation of the elevation's time
+// levels (fv_main.F90:1547-1551; those before it are made by the next
+// sub-step's ssh_node), and the elevation of the jacobian call
+// (fv_main.F90:2050)
 __global__ void k_jac_swap(Dev d) {
     pdl_enter();
     GRID_LOOP(ii, d.N) {
-        d.eta_jac_old[ii] = d.eta_jac[ii];
-        d.eta_jac[ii] = d.eta_n[ii];
+        const double e0 = d.eta_n[ii], e1 = d.eta_n_1[ii], en = d.eta_new[ii];
+        d.eta_n_2[ii] = e1;
+        d.eta_n_1[ii] = e0;
+        d.eta_n[ii] = en;
+        d.eta_jac[ii] = en;
     }
 }
 
@@ -1099,7 +1105,10 @@ void launch_implvisc(const Dev &d, cudaStream_t s) {
     }
     MAXL_DISPATCH(k_implvisc, grid_for(d.E, 128), 128, s, d);
 }
-void launch_jac_swap(const Dev &d, cudaStream_t s) { launch_k(k_jac_swap, grid_for(d.N, 256), 256, 0, s, d); }
+void launch_jac_swap(const Dev &d, cudaStream_t s) {
+    const int b = tuned(d, TK_ROT, 256);
+    launch_k(k_jac_swap, grid_for(d.N, b), b, 0, s, d);
+}
 void launch_je(const Dev &d, cudaStream_t s) { launch_k(k_je_elem, grid_for((long long)d.E * d.L, 256), 256, 0, s, d); }
 void launch_update3d(const Dev &d, real Mt_inv, cudaStream_t s) {
     launch_k(k_update3d, col_grid(d, d.E), col_b(d) * d.L, col_smem(d, 2, kU3Sc), s, d, Mt_inv);

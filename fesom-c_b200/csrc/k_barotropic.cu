@@ -1,15 +1,22 @@
 // External-mode (barotropic) sub-cycle kernels: one sub-step of
 // timestep_AB_2D (src/fv_main.F90:1372-1634) is
-//   ab3_elem  : AB3 extrapolation of U, element mean total depth (aux_elem)
-//               and the least-squares velocity gradients of UAB
+//   sub_edge  : SSH flux per edge and the least-squares velocity gradients
+//               of UAB per element, both from UAB and aux_elem, in one launch
 //   ssh_node  : edge-flux divergence gathered per node in edge order
-//               (compute_ssh_rhs_elem), rivers, OB tide, eta update, AM4
+//               (compute_ssh_rhs_elem), rivers, OB tide, eta update, AM4;
+//               first the previous sub-step's rotation of the time levels
 //   [sub-step 1 only: puls_elem, el2nodes, p1_elem]
 //   u2d_elem  : update_2D_vel (pressure gradient, Coriolis, wind, upwind
 //               momentum advection gathered per element, filter viscosity,
 //               3D->2D forcing, implicit friction, wet/dry mask) fused with
-//               the time-level rotation of U and the U_filt accumulation
-//   rot_nodes : eta time-level rotation
+//               the time-level rotation of U, the U_filt accumulation and
+//               the next sub-step's AB3 velocity and mean total depth
+//   Before the first sub-step ab3_elem forms those two from the state; after
+//   the last one jac_swap rotates the elevation.
+// Per sub-step 4 launches.  With AB3, gradients and rotation in kernels of
+// their own (7 launches) a step took 0.328 instead of 0.292 ms on 697 nodes,
+// 0.440 / 0.398 ms on 16 k, 1.634 / 1.552 ms on 42 k (biharmonic viscosity)
+// and 18.15 / 18.01 ms on 1.05 M nodes.
 // All kernels are HBM-bandwidth bound.  Both precision forms compile them:
 // the elevation, total depths and the wet/dry tests are FP64 in both (the
 // *_d scalars, wsum_d / wexp_d), the 2D momentum follows 'real'.
@@ -27,30 +34,45 @@ __device__ __forceinline__ real2 ab3v(real b, real2 x0, real2 x1, real2 x2) {
 }
 
 // ---------------------------------------------------------------------------
-// ab3_elem: UAB (fv_main.F90:1407-1410) and aux_elem
-// (fv_average_dynamic.F90:66-86); vel_gradients_2D(UAB) follows in
-// k_velgrad2d, which reads the neighbours' UAB (a third faster than forming
-// their AB3 again in this kernel).
+// UAB (fv_main.F90:1407-1410) and aux_elem (fv_average_dynamic.F90:66-86) of
+// element e from the three time levels of its velocity and of its nodes'
+// elevation
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ real aux_of(const Dev &d, const real4 &w, const double (&e0)[4], const double (&e1)[4],
+                                       const double (&e2)[4], const double (&dep)[4]) {
+    double ad[4];
+    for (int i = 0; i < 4; ++i) {
+        const double etaab = ab3<double>(d.beta_d, e0[i], e1[i], e2[i]);
+        ad[i] = d.Dmin_d;
+        const double ttl = etaab + dep[i];
+        if (ttl > d.Dmin_d) ad[i] = ttl;
+    }
+    return (real)wexp_d(w, ad[0], ad[1], ad[2], ad[3]);
+}
+
+// ab3_elem, before the first sub-step: UAB and aux_elem; U_filt_2D =
+// V_filt_2D = 0; the bottom velocity and quadratic drag a_Cd*|U_b| that
+// update_2D_vel uses in every sub-step (fv_average_dynamic.F90:262, 400-420;
+// U_n is fixed during the sub-cycle)
 __global__ void k_ab3_elem(Dev d) {
     pdl_enter();
     GRID_LOOP(ii, d.E) {
         const int e = (int)ii;
-        const real b = d.beta;
-        const real2 uab = ab3v(b, d.U_n_2D[e], d.U_n_1[e], d.U_n_2[e]);
-        d.UAB[e] = uab;
+        d.UAB[e] = ab3v(d.beta, d.U_n_2D[e], d.U_n_1[e], d.U_n_2[e]);
         const int4 en = d.elem_nodes[e];
         const int nd[4] = {en.x, en.y, en.z, en.w};
-        double ad[4];
+        double e0[4], e1[4], e2[4], dep[4];
         for (int i = 0; i < 4; ++i) {
             const int n = nd[i];
-            const double etaab = ab3<double>(d.beta_d, d.eta_n[n], d.eta_n_1[n], d.eta_n_2[n]);
-            ad[i] = d.Dmin_d;
-            const double ttl = etaab + (double)d.depth[n];
-            if (ttl > d.Dmin_d) ad[i] = ttl;
+            e0[i] = d.eta_n[n]; e1[i] = d.eta_n_1[n]; e2[i] = d.eta_n_2[n];
+            dep[i] = (double)d.depth[n];
         }
-        const real4 w = d.w_cv[e];
-        d.aux_elem[e] = (real)wexp_d(w, ad[0], ad[1], ad[2], ad[3]);
+        d.aux_elem[e] = aux_of(d, d.w_cv[e], e0, e1, e2, dep);
+        d.U_filt_2D[e] = real(0.0);
+        d.V_filt_2D[e] = real(0.0);
+        const real a_Cd = d.C_d * ((real(1.0) - d.elem_acc[e]) * d.Cd_bz + real(1.0));
+        const real ub = d.U_n[(size_t)e * d.L + d.L - 1], vb = d.V_n[(size_t)e * d.L + d.L - 1];
+        d.bfric[e] = make_real4(ub, vb, a_Cd * sqrt(ub * ub + vb * vb), real(0.0));
     }
 }
 
@@ -65,13 +87,6 @@ __device__ __forceinline__ real ssh_edge_flux(const Dev &d, int ed) {
         c1 = c1 + (-u2.y * X.z + u2.x * X.w) * d.aux_elem[et.y];
     }
     return c1;
-}
-
-// the SSH edge flux of every edge, once, for both end nodes to gather (the
-// flux array stays in L2; a quarter faster than forming it per node)
-__global__ void k_ssh_edge(Dev d) {
-    pdl_enter();
-    GRID_LOOP(ed, d.Ed) d.sshfl[ed] = ssh_edge_flux(d, (int)ed);
 }
 
 // ---------------------------------------------------------------------------
@@ -103,11 +118,20 @@ __global__ void __maxnreg__(40) k_ssh_node(Dev d, int sub) {
         }
         const int q = d.obn_of_node[n];
         if (d.TF_presence && q >= 0) acc = d.ob_val[(size_t)sub * d.nobn + q];
-        const double en = d.eta_n[n];
+        // the previous sub-step's rotation of the time levels
+        // (fv_main.F90:1547-1551)
+        const double en = sub > 0 ? d.eta_new[n] : d.eta_n[n];
+        const double em1 = sub > 0 ? d.eta_n[n] : d.eta_n_1[n];
+        const double em2 = sub > 0 ? d.eta_n_1[n] : d.eta_n_2[n];
+        if (sub > 0) {
+            d.eta_n[n] = en;
+            d.eta_n_1[n] = em1;
+            d.eta_n_2[n] = em2;
+        }
         double enew = acc;
         if (d.index_nod2D[n] < 2) enew = en + d.dt_2D_d * acc / (double)d.area[n];
         d.eta_new[n] = enew;
-        const double eab = de * enew + fe * en + ga * d.eta_n_1[n] + ep * d.eta_n_2[n];
+        const double eab = de * enew + fe * en + ga * em1 + ep * em2;
         d.etaAB[n] = eab;
         if (d.wet_dry_on) d.mask_wd_node[n] = ((double)d.depth[n] + eab > d.Dmin_d) ? real(1.0) : real(0.0);
     }
@@ -398,11 +422,9 @@ __global__ void k_bih2d_ul(Dev d) {
 }
 
 // vel_gradients_2D (fv_gradients.F90:97-176, free slip) of U into vel_grad:
-// of UAB after ab3_elem in every sub-step, of Ul in biharmonic_2D
-__global__ void k_velgrad2d(Dev d, const real2 *U) {
-    pdl_enter();
-    GRID_LOOP(ii, d.E) {
-        const int e = (int)ii;
+// of UAB in every sub-step (sub_edge), of Ul in biharmonic_2D
+__device__ __forceinline__ void velgrad2d_elem(const Dev &d, const real2 *U, int e) {
+    {
         const int4 en = d.elem_nodes[e];
         const int4 nb = d.elem_nb[e];
         const int4 ee = d.elem_edges[e];
@@ -434,6 +456,24 @@ __global__ void k_velgrad2d(Dev d, const real2 *U) {
             }
         }
         d.vel_grad[e] = make_real4(g1, g2, g3, g4);
+    }
+}
+__global__ void k_velgrad2d(Dev d, const real2 *U) {
+    pdl_enter();
+    GRID_LOOP(ii, d.E) velgrad2d_elem(d, U, (int)ii);
+}
+
+// sub_edge: the SSH flux of every edge, once, for both end nodes to gather
+// (the flux array stays in L2; a quarter faster than forming it per node),
+// and the gradients of UAB of every element.  Both need only UAB and
+// aux_elem, so they share a launch: threads [0, Ed) take an edge, the rest
+// an element.
+__global__ void k_sub_edge(Dev d) {
+    pdl_enter();
+    const long long Ed = d.Ed;
+    GRID_LOOP(i, Ed + d.E) {
+        if (i < Ed) d.sshfl[i] = ssh_edge_flux(d, (int)i);
+        else velgrad2d_elem(d, d.UAB, (int)(i - Ed));
     }
 }
 
@@ -468,7 +508,7 @@ __global__ void k_filt2x_2d(Dev d) {
 // (fv_main.F90:1568-1606).
 // ---------------------------------------------------------------------------
 // FP32: 8 resident blocks (at most 64 registers); FP64: 6.
-__global__ void __launch_bounds__(128, FESOMC_FP32 ? 8 : 6) k_u2d_elem(Dev d) {
+__global__ void __launch_bounds__(128, FESOMC_FP32 ? 8 : 6) k_u2d_elem(Dev d, int next) {
     pdl_enter();
     const real d0inv = real(1.0) / d.density_0;
     GRID_LOOP(ii, d.E) {
@@ -578,53 +618,36 @@ __global__ void __launch_bounds__(128, FESOMC_FP32 ? 8 : 6) k_u2d_elem(Dev d) {
         const real nx = mwd * ((dmo * u0.x - dt2 * friction * (ub - u0.x) + dt2 * bp.x + dt2 * rx / ar) * ff + uvx);
         const real ny = mwd * ((dmo * u0.y - dt2 * friction * (vb - u0.y) + dt2 * bp.y + dt2 * ry / ar) * ff + uvy);
         // rotate U_n_2 <- U_n_1 <- U_n_2D <- new (fv_main.F90:1569-1578)
-        d.U_n_2[e] = d.U_n_1[e];
+        const real2 u1 = d.U_n_1[e];
+        d.U_n_2[e] = u1;
         d.U_n_1[e] = u0;
         d.U_n_2D[e] = make_real2(nx, ny);
         // U_filt accumulation with the new elevation (fv_main.F90:1596-1605)
         const real dmn = (real)dmax(d.Dmin_d, wexp_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]));
         d.U_filt_2D[e] = d.U_filt_2D[e] + nx * dmn;
         d.V_filt_2D[e] = d.V_filt_2D[e] + ny * dmn;
-    }
-}
-
-// eta time-level rotation (fv_main.F90:1547-1551)
-__global__ void k_rot_nodes(Dev d) {
-    pdl_enter();
-    GRID_LOOP(ii, d.N) {
-        const int n = (int)ii;
-        const double e0 = d.eta_n[n], e1 = d.eta_n_1[n];
-        d.eta_n_2[n] = e1;
-        d.eta_n_1[n] = e0;
-        d.eta_n[n] = d.eta_new[n];
-    }
-}
-
-// U_filt_2D = V_filt_2D = 0 at the start of the sub-cycle, and the bottom
-// velocity and quadratic drag a_Cd*|U_b| that update_2D_vel uses in every
-// sub-step (fv_average_dynamic.F90:262, 400-420; U_n is fixed during the
-// sub-cycle)
-__global__ void k_zero_filt(Dev d) {
-    pdl_enter();
-    GRID_LOOP(ii, d.E) {
-        d.U_filt_2D[ii] = real(0.0);
-        d.V_filt_2D[ii] = real(0.0);
-        const real a_Cd = d.C_d * ((real(1.0) - d.elem_acc[ii]) * d.Cd_bz + real(1.0));
-        const real ub = d.U_n[(size_t)ii * d.L + d.L - 1], vb = d.V_n[(size_t)ii * d.L + d.L - 1];
-        d.bfric[ii] = make_real4(ub, vb, a_Cd * sqrt(ub * ub + vb * vb), real(0.0));
+        // the next sub-step's AB3 velocity and mean total depth
+        if (next) {
+            d.UAB_next[e] = ab3v(d.beta, make_real2(nx, ny), u0, u1);
+            double em[4];
+            for (int k = 0; k < 4; ++k) em[k] = d.eta_n_1[nd[k]];
+            d.aux_elem[e] = aux_of(d, w, enw, eo, em, dep);
+        }
     }
 }
 
 // ---- launch wrappers --------------------------------------------------------
 void launch_ab3_elem(const Dev &d, cudaStream_t s) {
-    const int b1 = tuned(d, TK_AB3, 256), b2 = tuned(d, TK_VELGRAD2D, 256);
-    launch_k(k_ab3_elem, grid_for(d.E, b1), b1, 0, s, d);
-    launch_k(k_velgrad2d, grid_for(d.E, b2), b2, 0, s, d, d.UAB);
+    const int b = tuned(d, TK_AB3, 256);
+    launch_k(k_ab3_elem, grid_for(d.E, b), b, 0, s, d);
+}
+void launch_sub_edge(const Dev &d, cudaStream_t s) {
+    const int b = tuned(d, TK_SSHEDGE, 256);
+    launch_k(k_sub_edge, grid_for((long long)d.Ed + d.E, b), b, 0, s, d);
 }
 void launch_ssh_node(const Dev &d, int sub, cudaStream_t s) {
-    const int b1 = tuned(d, TK_SSHEDGE, 256), b2 = tuned(d, TK_SSHNODE, 256);
-    launch_k(k_ssh_edge, grid_for(d.Ed, b1), b1, 0, s, d);
-    launch_k(k_ssh_node, grid_for(d.N, b2), b2, 0, s, d, sub);
+    const int b = tuned(d, TK_SSHNODE, 256);
+    launch_k(k_ssh_node, grid_for(d.N, b), b, 0, s, d, sub);
 }
 void launch_puls_elem(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_PULS, 256);
@@ -660,22 +683,15 @@ void launch_adv2d_edge(const Dev &d, cudaStream_t s) {
 }
 void launch_filt2x_2d(const Dev &d, cudaStream_t s) { launch_k(k_filt2x_2d, grid_for(d.E, 256), 256, 0, s, d); }
 void launch_bih_2d(const Dev &d, cudaStream_t s) {
+    const int bg = tuned(d, TK_VELGRAD2D, 256);
     launch_k(k_bih2d_edge, grid_for(d.Ed, 256), 256, 0, s, d, d.UAB);
     launch_k(k_bih2d_ul, grid_for(d.E, 256), 256, 0, s, d);
-    launch_k(k_velgrad2d, grid_for(d.E, 256), 256, 0, s, d, d.b2ul);
+    launch_k(k_velgrad2d, grid_for(d.E, bg), bg, 0, s, d, d.b2ul);
     launch_k(k_bih2d_edge, grid_for(d.Ed, 256), 256, 0, s, d, d.b2ul);
 }
-void launch_u2d_elem(const Dev &d, cudaStream_t s) {
+void launch_u2d_elem(const Dev &d, int next, cudaStream_t s) {
     const int b = tuned(d, TK_U2D, 128);
-    launch_k(k_u2d_elem, grid_for(d.E, b), b, 0, s, d);
-}
-void launch_rot_nodes(const Dev &d, cudaStream_t s) {
-    const int b = tuned(d, TK_ROT, 256);
-    launch_k(k_rot_nodes, grid_for(d.N, b), b, 0, s, d);
-}
-void launch_zero_filt(const Dev &d, cudaStream_t s) {
-    const int b = tuned(d, TK_ZEROFILT, 256);
-    launch_k(k_zero_filt, grid_for(d.E, b), b, 0, s, d);
+    launch_k(k_u2d_elem, grid_for(d.E, b), b, 0, s, d, next);
 }
 
 
@@ -688,15 +704,13 @@ static void tune_lower(int *lim, int knob, const void *k) {
 void tune_limits_barotropic(int *lim) {
     tune_lower(lim, TK_AB3, (const void *)k_ab3_elem);
     tune_lower(lim, TK_VELGRAD2D, (const void *)k_velgrad2d);
-    tune_lower(lim, TK_SSHEDGE, (const void *)k_ssh_edge);
+    tune_lower(lim, TK_SSHEDGE, (const void *)k_sub_edge);
     tune_lower(lim, TK_SSHNODE, (const void *)k_ssh_node);
     tune_lower(lim, TK_PULS, (const void *)k_puls_elem);
     tune_lower(lim, TK_EL2NODES, (const void *)k_el2nodes);
     tune_lower(lim, TK_P1EDGE, (const void *)k_p1_edge);
     tune_lower(lim, TK_ADV2D, (const void *)k_adv2d_edge);
     tune_lower(lim, TK_U2D, (const void *)k_u2d_elem);
-    tune_lower(lim, TK_ROT, (const void *)k_rot_nodes);
-    tune_lower(lim, TK_ZEROFILT, (const void *)k_zero_filt);
 }
 
 FESOMC_PREC_END

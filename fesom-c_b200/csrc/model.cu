@@ -26,9 +26,8 @@ namespace fesomc {
     void launch_p1_edge(const Dev &, cudaStream_t); \
     void launch_p1_elem(const Dev &, cudaStream_t); \
     void launch_adv2d_edge(const Dev &, cudaStream_t); \
-    void launch_u2d_elem(const Dev &, cudaStream_t); \
-    void launch_rot_nodes(const Dev &, cudaStream_t); \
-    void launch_zero_filt(const Dev &, cudaStream_t); \
+    void launch_sub_edge(const Dev &, cudaStream_t); \
+    void launch_u2d_elem(const Dev &, int, cudaStream_t); \
     void launch_pressure_col(const Dev &, cudaStream_t); \
     void launch_bpg_elem(const Dev &, cudaStream_t); \
     void launch_velgrad3d(const Dev &, cudaStream_t); \
@@ -729,8 +728,7 @@ int alloc_2d(fesomc_model *m) {
     Dev &d = m->d;
     const size_t N = d.N;
     int rc = 0;
-    double **nodes[] = {&d.eta_n, &d.eta_n_1, &d.eta_n_2, &d.eta_new, &d.etaAB, &d.ssh_gp, &d.eta_jac,
-                        &d.eta_jac_old};
+    double **nodes[] = {&d.eta_n, &d.eta_n_1, &d.eta_n_2, &d.eta_new, &d.etaAB, &d.ssh_gp, &d.eta_jac};
     for (auto p : nodes) if ((rc = dalloc(m, p, N))) return rc;
     if ((rc = dalloc(m, &d.runoff, (size_t)(d.n_rivers > 0 ? d.n_rivers : 1)))) return rc;
     if ((rc = dalloc(m, &d.ob_val, (size_t)(d.nobn > 0 ? d.nobn : 1) * (m->p.Mt > 0 ? m->p.Mt : 1)))) return rc;
@@ -762,7 +760,7 @@ int alloc_mom2d(fesomc_model *m, D &d) {
     for (auto p : nodes) if ((rc = dalloc(m, p, N))) return rc;
     decltype(&d.mask_wd) elems[] = {&d.aux_elem, &d.dmean_n, &d.U_filt_2D, &d.V_filt_2D, &d.mask_wd, &d.taux, &d.tauy};
     for (auto p : elems) if ((rc = dalloc(m, p, E))) return rc;
-    decltype(&d.UAB) e2[] = {&d.U_n_2D, &d.U_n_1, &d.U_n_2, &d.UAB, &d.U_rhs_2D_3D, &d.Bar_pr_2D};
+    decltype(&d.UAB) e2[] = {&d.U_n_2D, &d.U_n_1, &d.U_n_2, &d.UAB, &d.UAB_next, &d.U_rhs_2D_3D, &d.Bar_pr_2D};
     for (auto p : e2) if ((rc = dalloc(m, p, E))) return rc;
     if ((rc = dalloc(m, &d.vel_grad, E))) return rc;
     if ((rc = dalloc(m, &d.bfric, E))) return rc;
@@ -876,7 +874,7 @@ void share_2d(fesomc_model *m) {
     const Dev &a = m->d;
     fesomc::f32::Dev &b = m->d32;
     b.eta_n = a.eta_n; b.eta_n_1 = a.eta_n_1; b.eta_n_2 = a.eta_n_2; b.eta_new = a.eta_new; b.etaAB = a.etaAB;
-    b.ssh_gp = a.ssh_gp; b.eta_jac = a.eta_jac; b.eta_jac_old = a.eta_jac_old;
+    b.ssh_gp = a.ssh_gp; b.eta_jac = a.eta_jac;
     b.runoff = a.runoff; b.ob_val = a.ob_val; b.status = a.status; b.notconv = a.notconv;
     b.mslp = a.mslp; b.emp = a.emp; b.qsr = a.qsr; b.qns = a.qns; b.Rj = a.Rj; b.aj = a.aj; b.bj = a.bj;
 }
@@ -919,21 +917,22 @@ double kernel_bytes_fp64(const fesomc_model *m, const std::string &k) {
     if (k == "bih_2d") return 2 * (Ed * (16 + 8 + 32 + 8 + 16) + E * 32 + Ed * 16) + E * (16 + 16 + 8 + 8 + 16) +
                               E * (16 + 16 + 64 + 16 + 32);
     if (k == "forcing") return (double)d.nobn * (m->p.Mt * 8 + 12 * 16) + 36 * 8 + d.n_rivers * 16.0 + 16;
-    // ab3_elem (AB3 levels, w_cv, nodes; eta levels and depth; UAB, aux out)
-    // and velgrad2d (UAB, neighbours, edges, gradients, cos; vel_grad out)
-    if (k == "ab3_elem") return E * (48 + 32 + 16) + N * 32 + E * (16 + 8) + E * (16 + 16 + 16 + 64 + 8) + E * 32;
-    // ssh_edge (edge geometry, UAB, aux; the flux out) and ssh_node (CSR,
-    // the fluxes, node fields)
-    if (k == "ssh_node") return N * (4 + 4 + 4 + 24 + 8 + 8 + 16) + 4 * nnz_ne + Ed * (8 + 32) + E * 24 + Ed * 16;
+    // AB3 levels, w_cv, nodes; eta levels and depth; UAB, aux out; bottom
+    // velocity and drag, U_filt reset
+    if (k == "ab3_elem") return E * (48 + 32 + 16) + N * 32 + E * (16 + 8) + E * (16 + 8 + 16 + 32);
+    // SSH edge flux (edge geometry, UAB, aux; the flux out) and the gradients
+    // of UAB (neighbours, nodes, edges, gradients, cos; vel_grad out)
+    if (k == "sub_edge") return Ed * (8 + 32 + 8) + E * 24 + E * (16 + 16 + 16 + 64 + 8 + 32);
+    // CSR, the fluxes, node fields (three time levels moved on)
+    if (k == "ssh_node") return N * (4 + 4 + 4 + 24 + 8 + 8 + 16 + 24) + 4 * nnz_ne + Ed * 8;
     // per internal edge: nodes (etaAB, depth, ac), elements (UAB, vel_grad,
     // cos), geometry; one flux pair written
     if (k == "adv2d_edge") return N * 24 + E * (16 + 32 + 8) + Ei * (8 + 8 + 32 + 16 + 16);
     // per element: 4 nodes' etaAB, depth, atp1/2, ssh_gp, eta_n, eta_new;
     // element fields read / written once; edge fluxes of its internal edges
     if (k == "u2d_elem")
-        return N * 56 + E * (16 + 8 + 32 + 8 + 64 + 16 + 8 + 16 + 16 + 16 + 16 + 32 + 16 + 16 + 16 + 16) +
-               Ei * 16 + E * (8 + 16 + 16 + 16 + 16);
-    if (k == "rot_nodes") return N * 48;
+        return N * 64 + E * (16 + 8 + 32 + 8 + 64 + 16 + 8 + 16 + 16 + 16 + 16 + 32 + 16 + 16 + 16 + 16) +
+               Ei * 16 + E * (8 + 16 + 16 + 16 + 16 + 24);
     if (k == "pressure_col") return L * N * 16 + N * 16 + L * N * 8 + NS * N * 8;
     if (k == "bpg_elem") return NS * N * 8 + N * 48 + E * (96 + 16 + 8 + 8) + L * E * 8 + L * E * 16 + E * 32;
     if (k == "el2nodes" || k == "el2nodes_p") return L * E * 16 + N * 12 + 4 * (4.0 * E) + E * 8 + L * N * 16;
@@ -944,13 +943,12 @@ double kernel_bytes_fp64(const fesomc_model *m, const std::string &k) {
     if (k == "velrhs")
         return L * E * (48 + 24) + L * Ei * 16 + NS * N * 8 + N * 16 + E * 168 + L * E * 32;
     if (k == "implvisc") return L * E * 16 + NS * E * 8 + E * (16 + 16 + 16) + L * E * 16 + L * E * 16;
-    if (k == "zero_filt") return E * 16 + E * 8 + E * 16 + E * 32;
     if (k == "puls_elem") return L * E * 16 + E * 16 + N * 24 + E * 48 + L * E * 16 + E * 8;
     if (k == "p1_edge") return L * N * 16 + N * 16 + Ei * 32 + E * 8 + L * Ei * 16;
     if (k == "p1_elem")
         return L * Ei * 16 + E * (16 + 16 + 16) + Ei * 8 + N * 8 + L * E * 8 +
                (d.filt_3D ? L * E * 16 + E * 24 : 0.0);
-    if (k == "jac_swap") return N * 32;
+    if (k == "jac_swap") return N * 56;
     if (k == "update3d") return L * E * (16 + 8 + 32 + 24) + N * 24 + E * 48 + E * 32 + E * 16;
     if (k == "wvel") return N * 4 + 4 * nnz_ne + Ed * 40 + E * 16 + L * E * 24 + N * 8 + NS * N * 8;
     if (k == "minmax") return L * N * 16;
@@ -982,11 +980,11 @@ double kernel_bytes_fp64(const fesomc_model *m, const std::string &k) {
 
 // In the FP32 form the 3D kernels and the 2D momentum kernels move their
 // fields (almost all of their bytes) at half the size; the elevation
-// kernels (ssh_node, rot_nodes, jac_swap) keep FP64 and are counted as such.
+// kernels (ssh_node, jac_swap) keep FP64 and are counted as such.
 double kernel_bytes(const fesomc_model *m, const std::string &k) {
     const double b = kernel_bytes_fp64(m, k);
     if (!m->fp32) return b;
-    if (k == "ssh_node" || k == "rot_nodes" || k == "jac_swap" || k == "forcing" || k == "potential") return b;
+    if (k == "ssh_node" || k == "jac_swap" || k == "forcing" || k == "potential") return b;
     return 0.5 * b;
 }
 
@@ -1047,8 +1045,9 @@ ForcingDev forcing_view(const fesomc_model *m) {
 }
 
 int enqueue_step(fesomc_model *m, double ff) {
-    const Dev &d = m->d;
-    const fesomc::f32::Dev &q = m->d32;
+    const Dev &d0 = m->d;
+    Dev d = d0;                       // the sub-cycle swaps its buffers here
+    fesomc::f32::Dev q = m->d32;
     const bool f = m->fp32;
     cudaStream_t s = m->stream;
     int n = 0;
@@ -1118,12 +1117,18 @@ int enqueue_step(fesomc_model *m, double ff) {
     rec(m, "velrhs", [&] { K3(launch_velrhs, ff, s); });
     n += 1;
     if (d.im_vert_visc || d.im_vert_visc_fic) { rec(m, "implvisc", [&] { K3(launch_implvisc, s); }); n += 1; }
-    rec(m, "zero_filt", [&] { K3(launch_zero_filt, s); });
+    // the AB3 velocity of a sub-step is formed by the u2d_elem of the one
+    // before (its neighbours still read this sub-step's: two buffers in turn)
+    rec(m, "ab3_elem", [&] { K3(launch_ab3_elem, s); });
     n += 1;
-    for (int sub = 0; sub < d.Mt; ++sub) {
-        rec(m, "ab3_elem", [&] { K3(launch_ab3_elem, s); });
+    for (int sub = 0; sub < d0.Mt; ++sub) {
+        if (sub > 0) {
+            std::swap(d.UAB, d.UAB_next);
+            std::swap(q.UAB, q.UAB_next);
+        }
+        rec(m, "sub_edge", [&] { K3(launch_sub_edge, s); });
         rec(m, "ssh_node", [&] { K3(launch_ssh_node, sub, s); });
-        n += 4;
+        n += 2;
         if (sub == 0) {
             rec(m, "puls_elem", [&] { K3(launch_puls_elem, s); });
             rec(m, "el2nodes_p", [&] { K3E2N(U_puls, V_puls, Unode_p, Vnode_p); });
@@ -1135,9 +1140,8 @@ int enqueue_step(fesomc_model *m, double ff) {
         if (d.mom_adv_2D == 2) { rec(m, "adv2d_edge", [&] { K3(launch_adv2d_edge, s); }); n += 1; }
         if (d.filt_bi_2D) { rec(m, "filt2x_2d", [&] { K3(launch_filt2x_2d, s); }); n += 1; }
         if (d.bih_2D) { rec(m, "bih_2d", [&] { K3(launch_bih_2d, s); }); n += 4; }
-        rec(m, "u2d_elem", [&] { K3(launch_u2d_elem, s); });
-        rec(m, "rot_nodes", [&] { K3(launch_rot_nodes, s); });
-        n += 2;
+        rec(m, "u2d_elem", [&] { K3(launch_u2d_elem, sub + 1 < d0.Mt, s); });
+        n += 1;
     }
     rec(m, "jac_swap", [&] { launch_jac_swap(d, s); });
     rec(m, "update3d", [&] { K3(launch_update3d, 1.0 / (double)d.Mt, s); });
@@ -1467,8 +1471,7 @@ int fesomc_gpu_init_packed(const fesomc_mesh *mesh, const fesomc_params *par, co
         if ((rc = field_from_host(m, dev, m->fp32, ones.size(), ones.data(), ENT_NODE))) return fail(rc);
     }
     // jacobian state before the main loop: both calls see the initial eta
-    if (cudaMemcpy(m->d.eta_jac, m->d.eta_n, sizeof(double) * mesh->nod2D, cudaMemcpyDeviceToDevice) ||
-        cudaMemcpy(m->d.eta_jac_old, m->d.eta_n, sizeof(double) * mesh->nod2D, cudaMemcpyDeviceToDevice))
+    if (cudaMemcpy(m->d.eta_jac, m->d.eta_n, sizeof(double) * mesh->nod2D, cudaMemcpyDeviceToDevice))
         return fail(FESOMC_ECUDA);
     if (m->fp32) fesomc::f32::launch_je(m->d32, m->stream);
     else launch_je(m->d, m->stream);
@@ -1623,7 +1626,6 @@ int fesomc_gpu_sync_from_host(fesomc_model *m, uint32_t mask, const fesomc_state
         // a running model holds the same at every step boundary
         const size_t N = (size_t)m->d.N;
         CK(cudaMemcpy(m->d.eta_jac, m->d.eta_n, sizeof(double) * N, cudaMemcpyDeviceToDevice));
-        CK(cudaMemcpy(m->d.eta_jac_old, m->d.eta_n, sizeof(double) * N, cudaMemcpyDeviceToDevice));
         if (m->fp32) fesomc::f32::launch_je(m->d32, m->stream);
         else launch_je(m->d, m->stream);
         CK(cudaGetLastError());
@@ -1724,7 +1726,6 @@ int fesomc_gpu_halo_unpack(fesomc_model *m, const fesomc_halo *h, const double *
     // running model holds eta_jac = eta_n at every step boundary
     const size_t N = (size_t)m->d.N;
     CK(cudaMemcpyAsync(m->d.eta_jac, m->d.eta_n, sizeof(double) * N, cudaMemcpyDeviceToDevice, m->stream));
-    CK(cudaMemcpyAsync(m->d.eta_jac_old, m->d.eta_n, sizeof(double) * N, cudaMemcpyDeviceToDevice, m->stream));
     if (m->fp32) fesomc::f32::launch_je(m->d32, m->stream);
     else launch_je(m->d, m->stream);
     CK(cudaGetLastError());
@@ -2033,9 +2034,9 @@ struct KnobInfo {
 const KnobInfo kKnobs[fesomc::kTuneKnobs] = {
     {"velrhs", "velrhs", 256}, {"velgrad3d", "velgrad3d", 256}, {"adv3_edge", "adv3_edge", 256},
     {"puls_elem", "puls_elem", 256}, {"el2nodes", "el2nodes,el2nodes_p", 256}, {"p1_edge", "p1_edge", 256},
-    {"ab3_elem", "ab3_elem", 256}, {"velgrad2d", "ab3_elem", 256}, {"ssh_edge", "ssh_node", 256},
+    {"ab3_elem", "ab3_elem", 256}, {"velgrad2d", "bih_2d", 256}, {"ssh_edge", "sub_edge", 256},
     {"ssh_node", "ssh_node", 256}, {"adv2d_edge", "adv2d_edge", 256}, {"u2d_elem", "u2d_elem", 128},
-    {"rot_nodes", "rot_nodes", 256}, {"zero_filt", "zero_filt", 256}, {"ab2_node", "ab2_node", 256},
+    {"rot_nodes", "jac_swap", 256}, {"zero_filt", "ab3_elem", 256}, {"ab2_node", "ab2_node", 256},
     {"muscl_egrad", "muscl_egrad", 256}, {"muscl_ngrad", "muscl_ngrad", 256}, {"muscl_edge", "muscl_edge", 256},
     {"muscl_h", "muscl_h", 128}, {"upwind_h", "upwind_h", 128}, {"av", "av", 256},
     {"columns", "pressure_col,bpg_elem,update3d,wvel", 0},

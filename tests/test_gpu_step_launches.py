@@ -1,6 +1,9 @@
 """The step's launch rules against the oracle, bit for bit: meshes whose
 grids lie on both sides of the size up to which kernels are started early
-(programmatic dependent launch), in eager and captured steps."""
+(programmatic dependent launch), in eager and captured steps; and sub-cycles
+of one, two, three and ten external steps, whose AB3 velocities alternate
+between two buffers and whose elevation is rotated by the next sub-step or,
+after the last, by the jacobian kernel."""
 import numpy as np
 import pytest
 
@@ -31,3 +34,14 @@ def _compare(case_of, steps):
 def test_early_launch_sizes(built, nx, ny):
     from fesomc import cases
     _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, 11, 2.0, 25.0, stress=(0.0, 0.05), lib=lib), 3)
+
+
+@pytest.mark.parametrize("sub", [1, 2, 3])
+def test_sub_cycle_lengths(built, sub):
+    from fesomc import cases
+
+    def case_of(lib):
+        return cases.estuary_case("e", 23, 14, 300.0, 11, 2.0, 25.0, stress=(0.0, 0.05), lib=lib, dt=2.0 * sub)
+
+    assert case_of(None).params.Mt == sub
+    _compare(case_of, 4)
