@@ -25,7 +25,8 @@ FESOMC_PREC_BEGIN
 // entity, in level order.
 struct ColBlock {
     int L, B, jl, z;
-    __device__ ColBlock(int L_) : L(L_), B((int)blockDim.x / L_), jl((int)threadIdx.x / L_), z((int)threadIdx.x % L_) {}
+    __device__ ColBlock(const Dev &d)
+        : L(d.L), B(d.by_L.div(blockDim.x)), jl(d.by_L.div(threadIdx.x)), z((int)threadIdx.x - jl * d.L) {}
 };
 
 // ---------------------------------------------------------------------------
@@ -38,7 +39,7 @@ __global__ void __launch_bounds__(1024) k_pressure_col(Dev d) {
     real *sm = reinterpret_cast<real *>(sm_raw);
     const real gd0 = kG / d.density_0;
     const int L = d.L, NS = d.NS;
-    const ColBlock cb(L);
+    const ColBlock cb(d);
     const int S = L | 1;
     for (long long nb = (long long)blockIdx.x * cb.B; nb < d.N; nb += (long long)gridDim.x * cb.B) {
         const long long n_ = nb + cb.jl;
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(1024) k_bpg_elem(Dev d) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L, NS = d.NS;
-    const ColBlock cb(L);
+    const ColBlock cb(d);
     const int S = 2 * L + 1;
     for (long long eb = (long long)blockIdx.x * cb.B; eb < d.E; eb += (long long)gridDim.x * cb.B) {
         const long long e_ = eb + cb.jl;
@@ -158,10 +159,10 @@ __global__ void __launch_bounds__(1024) k_bpg_elem(Dev d) {
 // 64 registers: 32 resident warps per SM instead of 24 (11 % faster).
 __global__ void __maxnreg__(64) k_velgrad3d(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / d.L);
-        const int z = (int)(ii % d.L);
+        const int e = d.by_L.div(ii);
+        const int z = (int)ii - e * d.L;
         const int L = d.L;
         const int4 en = d.elem_nodes[e];
         const int4 nb = d.elem_nb[e];
@@ -271,11 +272,11 @@ __device__ __forceinline__ void uvert_at(const Dev &d, int e, int k, const real4
 // consecutive threads.
 __global__ void k_adv3_edge(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.Ed_in * d.L;
+    const unsigned total = (unsigned)d.Ed_in * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
-        const int ed = (int)(ii / L);
-        const int z = (int)(ii % L);
+        const int ed = d.by_L.div(ii);
+        const int z = (int)ii - ed * L;
         const int2 nn = d.edge_nodes[ed];
         const int2 et = d.edge_tri[ed];
         const real acc = real(0.5) * (d.ac[nn.x] + d.ac[nn.y]);
@@ -316,11 +317,11 @@ __global__ void k_adv3_edge(Dev d) {
 // ---------------------------------------------------------------------------
 __global__ void k_bih_edge(Dev d, const real *U, const real *V, int mode) {
     pdl_enter();
-    const long long total = (long long)d.Ed * d.L;
+    const unsigned total = (unsigned)d.Ed * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
-        const int ed = (int)(ii / L);
-        const int z = (int)(ii % L);
+        const int ed = d.by_L.div(ii);
+        const int z = (int)ii - ed * L;
         const int2 nn = d.edge_nodes[ed];
         const int2 et = d.edge_tri[ed];
         const real2 dxy = d.edge_dxdy[ed];
@@ -371,11 +372,11 @@ __global__ void k_bih_edge(Dev d, const real *U, const real *V, int mode) {
 
 __global__ void k_bih_uc(Dev d, int mode) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / L);
-        const int z = (int)(ii % L);
+        const int e = d.by_L.div(ii);
+        const int z = (int)ii - e * L;
         const real2 c = bih_gather(d, e, z);
         const real sa = scale_area_of(d, e);
         const real Ah = (mode == 0) ? -d.Abh0 * sqrt(d.elem_area[e] / sa) / sa
@@ -391,11 +392,11 @@ __global__ void k_bih_uc(Dev d, int mode) {
 template <bool FREE_SLIP>
 __global__ void k_bih_grad(Dev d, const real *U, const real *V) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / L);
-        const int z = (int)(ii % L);
+        const int e = d.by_L.div(ii);
+        const int z = (int)ii - e * L;
         const int4 en = d.elem_nodes[e];
         const int4 nb = d.elem_nb[e];
         const int4 ee = d.elem_edges[e];
@@ -443,12 +444,12 @@ __global__ void k_bih_grad(Dev d, const real *U, const real *V) {
 // forms UV_rhs from the neighbours' U_c.
 __global__ void k_filt2x_uc(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     const int L = d.L;
     const real tau_inv = d.dt * d.tau_c / real(3600.0) / real(24.0);
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / L);
-        const int z = (int)(ii % L);
+        const int e = d.by_L.div(ii);
+        const int z = (int)ii - e * L;
         const int4 nb = d.elem_nb[e];
         const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
         const real K_bi = tau_inv * sqrt(scale_area_of(d, e) / d.elem_area[e]);
@@ -486,15 +487,15 @@ __global__ void k_filt2x_uc(Dev d) {
 // blocks at 80 registers).
 __global__ void __launch_bounds__(256, 4) k_velrhs(Dev d, real ff) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     const int lane = threadIdx.x & 31;
-    const long long nwarp = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 31 < total; c += nwarp) {
-        const long long iw = c * 31 + lane;
+    const unsigned nwarp = gridDim.x * (blockDim.x >> 5);
+    for (unsigned c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 31 < total; c += nwarp) {
+        const unsigned iw = c * 31 + lane;
         const bool valid = lane < 31 && iw < total;
-        const long long ii = iw < total ? iw : total - 1;
-        const int e = (int)(ii / d.L);
-        const int z = (int)(ii % d.L);
+        const unsigned ii = iw < total ? iw : total - 1;
+        const int e = d.by_L.div(ii);
+        const int z = (int)ii - e * d.L;
         const int L = d.L;
         const int4 en = d.elem_nodes[e];
         const real4 w = d.w_cv[e];
@@ -742,10 +743,10 @@ __global__ void k_jac_swap(Dev d) {
 // fv_main.F90:1208-1267); at init, afterwards refreshed by update3d
 __global__ void k_je_elem(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / d.L);
-        const int z = (int)(ii % d.L);
+        const int e = d.by_L.div(ii);
+        const int z = (int)ii - e * d.L;
         const real4 w = d.w_cv[e];
         const real4 a = elem_jac_a(d, d.eta_jac, d.elem_nodes[e]);
         d.Je[ii] = je_of(d, w, a, z);
@@ -766,7 +767,7 @@ __global__ void __maxnreg__(48) k_update3d(Dev d, real Mt_inv) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L;
-    const ColBlock cb(L);
+    const ColBlock cb(d);
     const int S = 2 * L + 1;
     real *sc = sm + (size_t)cb.B * S;  // kU3Sc scalars per element
     for (long long eb = (long long)blockIdx.x * cb.B; eb < d.E; eb += (long long)gridDim.x * cb.B) {
@@ -845,7 +846,7 @@ __global__ void k_wvel(Dev d) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L, NS = d.NS;
-    const ColBlock cb(L);
+    const ColBlock cb(d);
     const int S = L | 1;
     real *sc = sm + (size_t)cb.B * S;  // per node: bottom Wvel, 1/area
     for (long long nb = (long long)blockIdx.x * cb.B; nb < d.N; nb += (long long)gridDim.x * cb.B) {
@@ -929,7 +930,7 @@ __global__ void __launch_bounds__(kIvCols) k_implvisc_fic_tile(Dev d) {
             }
 #pragma unroll
             for (int u = 0; u < kIvBatch; ++u) {
-                const int i = i0 + u * kIvCols, j = i / NS;
+                const int i = i0 + u * kIvCols, j = d.by_NS.div(i);
                 if (i < nt * NS) sA[j * KP + (i - j * NS)] = av[u];
             }
         }

@@ -143,9 +143,9 @@ __global__ void __maxnreg__(40) k_ssh_node(Dev d, int sub) {
 // ---------------------------------------------------------------------------
 __global__ void k_puls_elem(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / d.L);
+        const int e = d.by_L.div(ii);
         const int4 en = d.elem_nodes[e];
         const real4 w = d.w_cv[e];
         const real dmn = dmax(d.Dmin, wexp(w, d.eta_n[en.x] + d.depth[en.x], d.eta_n[en.y] + d.depth[en.y],
@@ -155,17 +155,17 @@ __global__ void k_puls_elem(Dev d) {
         const real2 u2 = d.U_n_2D[e];
         d.U_puls[ii] = d.U_n[ii] - a * u2.x;
         d.V_puls[ii] = d.V_n[ii] - a * u2.y;
-        if (ii % d.L == 0) d.dmean_n[e] = dmn;
+        if ((int)ii == e * d.L) d.dmean_n[e] = dmn;
     }
 }
 
 // compute_el2nodes_3D (fv_utilit.F90:644-700), one thread per (node, level)
 __global__ void k_el2nodes(Dev d, const real *Ue, const real *Ve, real *Un, real *Vn) {
     pdl_enter();
-    const long long total = (long long)d.N * d.L;
+    const unsigned total = (unsigned)d.N * d.L;
     GRID_LOOP(ii, total) {
-        const int n = (int)(ii / d.L);
-        const int z = (int)(ii % d.L);
+        const int n = d.by_L.div(ii);
+        const int z = (int)ii - n * d.L;
         const real tvol_inv = real(1.0) / d.node_tvol[n];
         real su = real(0.0), sv = real(0.0);
         for (int p = d.node_nptr[n]; p < d.node_nptr[n + 1]; ++p) {
@@ -184,11 +184,11 @@ __global__ void k_el2nodes(Dev d, const real *Ue, const real *Ve, real *Un, real
 // Stored in the adv3 buffer, which velrhs has finished with.
 __global__ void k_p1_edge(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.Ed_in * d.L;
+    const unsigned total = (unsigned)d.Ed_in * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
-        const int ed = (int)(ii / L);
-        const int z = (int)(ii % L);
+        const int ed = d.by_L.div(ii);
+        const int z = (int)ii - ed * L;
         const int2 nn = d.edge_nodes[ed];
         const int2 et = d.edge_tri[ed];
         const real2 dxy = d.edge_dxdy[ed];
@@ -220,7 +220,7 @@ __global__ void k_p1_elem(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const int L = d.L;
-    const int B = (int)blockDim.x / L;
+    const int B = d.by_L.div(blockDim.x);
     const int nsl = kP1Slots + (d.bih_3D ? 1 : 0);  // + biharmonic_viscosity_3D_to_2D
     const int S = 2 * nsl * L + 1;  // per-element stride, odd: conflict-free
     real *sm = reinterpret_cast<real *>(sm_raw);
@@ -228,7 +228,7 @@ __global__ void k_p1_elem(Dev d) {
     real *accs = sums + (size_t)B * 8;   // [B][4]: acc of the edge slots
     real *dms = accs + (size_t)B * 4;    // [B]: dmean_n
     int *cds = reinterpret_cast<int *>(dms + B);  // [B][4]: edge codes
-    const int jl = (int)threadIdx.x / L, z = (int)threadIdx.x % L;
+    const int jl = d.by_L.div(threadIdx.x), z = (int)threadIdx.x - jl * L;
     const int nt = (int)blockDim.x;
     for (long long eb = (long long)blockIdx.x * B; eb < d.E; eb += (long long)gridDim.x * B) {
         const long long e_ = eb + jl;

@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kD3SetupThreads) k_d3end_setup(Dev d) {
     for (long long n0 = (long long)blockIdx.x * kD3Tile; n0 < N; n0 += (long long)gridDim.x * kD3Tile) {
         const int nt = (int)(N - n0 < kD3Tile ? N - n0 : kD3Tile);
         for (int i = threadIdx.x; i < nt * L; i += blockDim.x) {
-            const int j = i / L, k = i - j * L;
+            const int j = d.by_L.div(i), k = i - j * L;
             const size_t g = (size_t)n0 * L + i;
             sU[j * NS + k] = d.Unode[g];
             sV[j * NS + k] = d.Vnode[g];
@@ -856,10 +856,10 @@ __global__ void __launch_bounds__(64, MINB) k_d3end_sweep_reg(Dev d) {
 // Av(nz,elem) = sum(w_cv*snu(nz,nodes)) (fv_mixing.F90:308-313)
 __global__ void k_av(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.E * d.NS;
+    const unsigned total = (unsigned)d.E * d.NS;
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / d.NS);
-        const int z = (int)(ii % d.NS);
+        const int e = d.by_NS.div(ii);
+        const int z = (int)ii - e * d.NS;
         const int4 en = d.elem_nodes[e];
         const real4 w = d.w_cv[e];
         const int NS = d.NS;

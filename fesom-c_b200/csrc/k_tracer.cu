@@ -190,9 +190,9 @@ __device__ __forceinline__ void tvert_upwind2(const Dev &d, int k, real a, const
 // for the gathers below (fv_tracer.F90:433,435 and :39-47)
 __global__ void k_ab2_node(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.N * d.L;
+    const unsigned total = (unsigned)d.N * d.L;
     GRID_LOOP(i, total) {
-        const int n = (int)(i / d.L);
+        const int n = d.by_L.div(i);
         d.ttfold[i] = ab2(d, d.TF, d.T_old, i, t_aver_of(d, n));
         d.stfold[i] = ab2(d, d.SF, d.S_old, i, s_aver_of(d, n));
     }
@@ -206,17 +206,17 @@ __global__ void k_upwind_h(Dev d) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int L = d.L, NS = d.NS;
-    const long long total = (long long)d.N * L;
+    const unsigned total = (unsigned)d.N * d.L;
     // each warp takes 31 (node, level) outputs; lane 31 forms the flux at its
     // own index, the interface below lane 30's layer, for the shuffle, so no
     // lane forms a second flux
-    const long long nwarp = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 31 < total; c += nwarp) {
-        const long long iw = c * 31 + lane;
+    const unsigned nwarp = gridDim.x * (blockDim.x >> 5);
+    for (unsigned c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 31 < total; c += nwarp) {
+        const unsigned iw = c * 31 + lane;
         const bool valid = lane < 31 && iw < total;
-        const long long i_ = iw < total ? iw : total - 1;
-        const int n = (int)(i_ / L);
-        const int z = (int)(i_ % L), zc = z;
+        const unsigned i_ = iw < total ? iw : total - 1;
+        const int n = d.by_L.div(i_);
+        const int z = (int)i_ - n * L, zc = z;
         const real T_aver = t_aver_of(d, n), S_aver = s_aver_of(d, n);
         const real a = jac_a(d, d.eta_jac, n);
         const real *W = d.Wvel + (size_t)n * NS;
@@ -302,10 +302,10 @@ __global__ void k_upwind_h(Dev d) {
 // tracer_gradient_elements of the AB2 tracer, thread per (element, level)
 __global__ void k_muscl_egrad(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / d.L);
-        const int z = (int)(ii % d.L);
+        const int e = d.by_L.div(ii);
+        const int z = (int)ii - e * d.L;
         const int L = d.L;
         const int4 en = d.elem_nodes[e];
         const size_t i1 = (size_t)en.x * L + z, i2 = (size_t)en.y * L + z, i3 = (size_t)en.z * L + z,
@@ -324,10 +324,10 @@ __global__ void k_muscl_egrad(Dev d) {
 // fv_gradients.F90:292-318: tx/tvol with running sums)
 __global__ void k_muscl_ngrad(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.N * d.L;
+    const unsigned total = (unsigned)d.N * d.L;
     GRID_LOOP(ii, total) {
-        const int n = (int)(ii / d.L);
-        const int z = (int)(ii % d.L);
+        const int n = d.by_L.div(ii);
+        const int z = (int)ii - n * d.L;
         const int L = d.L;
         real tvol = real(0.0), a = real(0.0), b = real(0.0), c = real(0.0), e4 = real(0.0);
         for (int p = d.node_nptr[n]; p < d.node_nptr[n + 1]; ++p) {
@@ -446,11 +446,11 @@ __device__ __forceinline__ real muscl_mean(bool upw2, real Tm1, real Tm2) {
 // (17 % faster).
 __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.Ed * d.L;
+    const unsigned total = (unsigned)d.Ed * d.L;
     const int L = d.L;
     GRID_LOOP(ii, total) {
-        const int ed = (int)(ii / L);
-        const int z = (int)(ii % L);
+        const int ed = d.by_L.div(ii);
+        const int z = (int)ii - ed * L;
         const int2 nn = d.edge_nodes[ed];
         const int2 et = d.edge_tri[ed];
         const int2 ud = d.edge_updn[ed];
@@ -519,19 +519,19 @@ __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
 // z+1 comes from the next lane when that lane holds the same node.
 __global__ void __launch_bounds__(128, 8) k_muscl_h(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.N * d.L;
+    const unsigned total = (unsigned)d.N * d.L;
     const int lane = threadIdx.x & 31;
     const int L = d.L, NS = d.NS;
     // each warp takes 31 (node, level) outputs; lane 31 forms the flux at its
     // own index, the interface below lane 30's layer, for the shuffle, so no
     // lane forms a second flux
-    const long long nwarp = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 31 < total; c += nwarp) {
-        const long long iw = c * 31 + lane;
+    const unsigned nwarp = gridDim.x * (blockDim.x >> 5);
+    for (unsigned c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 31 < total; c += nwarp) {
+        const unsigned iw = c * 31 + lane;
         const bool valid = lane < 31 && iw < total;
-        const long long i_ = iw < total ? iw : total - 1;
-        const int n = (int)(i_ / L);
-        const int z = (int)(i_ % L);
+        const unsigned i_ = iw < total ? iw : total - 1;
+        const int n = d.by_L.div(i_);
+        const int z = (int)i_ - n * L;
         const real T_aver = t_aver_of(d, n), S_aver = s_aver_of(d, n);
         const real an = jac_a(d, d.eta_jac, n);
         const real *W = d.Wvel + (size_t)n * NS;
@@ -594,13 +594,13 @@ __global__ void __launch_bounds__(128, 8) k_muscl_h(Dev d) {
 // H_advtr_crit = 0.1, H_advtr_min = 0)
 __global__ void k_miura_prep(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.N * d.L;
+    const unsigned total = (unsigned)d.N * d.L;
     GRID_LOOP(i, total) {
-        const real T_aver = t_aver_of(d, (int)(i / d.L));
+        const int n = d.by_L.div(i);
+        const real T_aver = t_aver_of(d, n);
         d.ttfold[i] = ab2(d, d.TF, d.T_old, i, T_aver);
         d.tnow[i] = d.TF[i] - T_aver;
-        if (i % d.L == 0) {
-            const int n = (int)(i / d.L);
+        if ((int)i == n * d.L) {
             const real crit = real(0.1), hmin = real(0.0);
             const real dmean = dmax<real>(d.Dmin, d.depth[n] + d.eta_n[n]);
             real m;
@@ -615,10 +615,10 @@ __global__ void k_miura_prep(Dev d) {
 // tracer_gradient_elements of T - T_aver (fv_gradients.F90:180-214)
 __global__ void k_miura_egrad(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.E * d.L;
+    const unsigned total = (unsigned)d.E * d.L;
     GRID_LOOP(ii, total) {
-        const int e = (int)(ii / d.L);
-        const int z = (int)(ii % d.L);
+        const int e = d.by_L.div(ii);
+        const int z = (int)ii - e * d.L;
         const int L = d.L;
         const int4 en = d.elem_nodes[e];
         const real t1 = d.tnow[(size_t)en.x * L + z], t2 = d.tnow[(size_t)en.y * L + z];
@@ -632,10 +632,10 @@ __global__ void k_miura_egrad(Dev d) {
 // times the reciprocal of the summed area
 __global__ void k_miura_ngrad(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.N * d.L;
+    const unsigned total = (unsigned)d.N * d.L;
     GRID_LOOP(ii, total) {
-        const int n = (int)(ii / d.L);
-        const int z = (int)(ii % d.L);
+        const int n = d.by_L.div(ii);
+        const int z = (int)ii - n * d.L;
         const int L = d.L;
         real s = real(0.0);
         for (int p = d.node_nptr[n]; p < d.node_nptr[n + 1]; ++p) s = s + d.elem_area[d.node_nidx[p]];
@@ -656,12 +656,12 @@ __global__ void k_miura_ngrad(Dev d) {
 // continuity terms (:1141-1168); thread per (edge, level)
 __global__ void k_miura_edge(Dev d) {
     pdl_enter();
-    const long long total = (long long)d.Ed * d.L;
+    const unsigned total = (unsigned)d.Ed * d.L;
     const int L = d.L;
     const real dt = d.dt;
     GRID_LOOP(ii, total) {
-        const int ed = (int)(ii / L);
-        const int z = (int)(ii % L);
+        const int ed = d.by_L.div(ii);
+        const int z = (int)ii - ed * L;
         const int2 nn = d.edge_nodes[ed];
         const int2 et = d.edge_tri[ed];
         const real4 X = d.edge_cross[ed];
@@ -725,17 +725,17 @@ __global__ void __launch_bounds__(128, 8) k_miura_h(Dev d) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int L = d.L, NS = d.NS;
-    const long long total = (long long)d.N * L;
+    const unsigned total = (unsigned)d.N * d.L;
     // each warp takes 31 (node, level) outputs; lane 31 forms the flux at its
     // own index, the interface below lane 30's layer, for the shuffle, so no
     // lane forms a second flux
-    const long long nwarp = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 31 < total; c += nwarp) {
-        const long long iw = c * 31 + lane;
+    const unsigned nwarp = gridDim.x * (blockDim.x >> 5);
+    for (unsigned c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 31 < total; c += nwarp) {
+        const unsigned iw = c * 31 + lane;
         const bool valid = lane < 31 && iw < total;
-        const long long i_ = iw < total ? iw : total - 1;
-        const int n = (int)(i_ / L);
-        const int z = (int)(i_ % L), zc = z;
+        const unsigned i_ = iw < total ? iw : total - 1;
+        const int n = d.by_L.div(i_);
+        const int z = (int)i_ - n * L, zc = z;
         const real T_aver = t_aver_of(d, n);
         const real an = jac_a(d, d.eta_jac, n);
         const real *W = d.Wvel + (size_t)n * NS;
@@ -1301,7 +1301,7 @@ __global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
             }
 #pragma unroll
             for (int u = 0; u < kVtBatch; ++u) {
-                const int i = i0 + u * kVtCols, j = i / NS;
+                const int i = i0 + u * kVtCols, j = d.by_NS.div(i);
                 if (i < nt * NS) sK[j * KP + (i - j * NS)] = kv[u];
             }
         }

@@ -528,6 +528,10 @@ int build_mesh(fesomc_model *m, const fesomc_mesh *msh) {
     const int L = NS - 1;
     d.N = N; d.E = E; d.Ed = Ed; d.Ed_in = Ed_in; d.L = L; d.NS = NS;
     d.nobn = msh->nobn; d.n_rivers = msh->n_rivers;
+    d.by_L.set(L); d.by_NS.set(NS);
+    // the kernels' flat indices are 31 bits; a mesh beyond that needs several
+    // times the device's memory
+    if ((long long)std::max(std::max(N, E), Ed) * NS >= (1LL << 31)) return FESOMC_ENOMEM;
     std::vector<double> sig(msh->sigma, msh->sigma + NS), dsig(L);
     for (int k = 0; k < L; ++k) dsig[k] = sig[k] - sig[k + 1];
     int rc;
@@ -843,6 +847,7 @@ int setup_f32_view(fesomc_model *m) {
     fesomc::f32::Dev &b = m->d32;
     b.N = a.N; b.E = a.E; b.Ed = a.Ed; b.Ed_in = a.Ed_in; b.L = a.L; b.NS = a.NS;
     b.nobn = a.nobn; b.n_rivers = a.n_rivers;
+    b.by_L = a.by_L; b.by_NS = a.by_NS;
     b.elem_nodes = a.elem_nodes; b.elem_nb = a.elem_nb; b.elem_edges = a.elem_edges; b.elem_iedges = a.elem_iedges;
     b.elem_sedges = a.elem_sedges;
     b.edge_nodes = a.edge_nodes; b.edge_tri = a.edge_tri; b.edge_updn = a.edge_updn;
