@@ -76,10 +76,8 @@ __host__ __device__ __forceinline__ float4 make_real4(float x, float y, float z,
 // whose results do not depend on the block shape (one thread per entity or
 // per (entity, level), grid-stride, no block-level reduction), and entities
 // per block of the column kernels (pressure_col, bpg_elem, update3d, wvel),
-// and the form of d3_end (1 column arrays in local memory, 2 in shared
-// memory, 3 a level-parallel set-up kernel and a sweep kernel, 4 the same
-// with the sweep's arrays in shared memory, 5 and 6 in registers for 11 or
-// 21 levels), and the form of the tracers'
+// and the form of d3_end (1 one thread per column, 2 to 6 tiles of columns
+// in shared memory), and the form of the tracers'
 // implicit vertical diffusion (1 one thread per column reading the fields
 // directly, 2 and 3 tiles of 128 or 64 columns staged in shared memory, for
 // 10 or 20 layers; other layer counts take form 1), and the form of the

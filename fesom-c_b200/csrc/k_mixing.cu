@@ -1,5 +1,5 @@
-// Vertical turbulence closure d3_end (src/fv_mixing.F90:73-347): one thread
-// per node column.  Each column iterates its implicit turbulence-energy
+// Vertical turbulence closure d3_end (src/fv_mixing.F90:73-347) on tiles of
+// node columns, or with one thread per node column.  Each column iterates its implicit turbulence-energy
 // sweep up to 200 times (relative tolerance 1e-6); columns that reach the cap
 // are counted in the device status (the reference silently continues).
 // Compute / latency bound (FP64 divisions, log, sqrt).
@@ -24,6 +24,15 @@ __device__ __forceinline__ bool d3_above_tol(real a, real b) {
     return fabs(a / b) >= real(1.0e-6);
 }
 
+// x / d for d > 0: a zero x gives itself (the quotient's sign is x's).  The
+// division routine leaves its short path for a zero numerator; x is
+// replaced by 1 before the division instead.
+__device__ __forceinline__ real div_pos(real x, real d) {
+    const real q = (x == real(0.0) ? real(1.0) : x) / d;
+    return x == real(0.0) ? x : q;
+}
+
+#if !FESOMC_FP32
 // d3_end per node column (local-memory arrays indexed 1..NS like the Fortran
 // ones, ARR >= NS + 1 entries each).  The kernel is bound by the traffic of
 // those arrays: the working set of the resident columns does not fit in L2,
@@ -41,10 +50,7 @@ __device__ __forceinline__ bool d3_above_tol(real a, real b) {
 //   * both sweeps load the next level's array values one level ahead, so
 //     that their latency overlaps the current level's division chain (3 %
 //     faster; unrolling by 4 instead was 9 % slower).
-// (The same arrays in shared memory, [array][level][thread], take the DRAM
-// traffic down to the algorithmic bytes but leave room for 6 warps per SM
-// only, and the kernel then waits on its FP64 chains: 3.85 against 2.54 ms
-// on cfg1.)
+// The form for level counts whose tiles (below) do not fit well.
 //
 // kList: the columns are list[0 .. *count) instead of every node (the
 // columns the learned closure hands back to the plain one).
@@ -191,665 +197,218 @@ __global__ void k_d3end(Dev d, const int *list, const unsigned long long *count)
         }
     }
 }
+#endif
 
-// The same closure with the column arrays in shared memory, laid out
-// [array][level][thread] so that a warp's access to one level is 32
-// consecutive words (launch-shape knob "d3end_arrays" = 2):
-//   sn        snu(nz), nz = 1..NS                 (constant over the iteration)
-//   bA, bB    btr / btr1 / xx1, nz = 1..NS        (alternating; the back
-//             substitution writes btr1(k) into the xx1(k) slot it has just
-//             read, xx1(2) = 1 and yy1(2) = y2 being constants)
-//   yy1       yy1(nz), nz = 3..NS
-//   pb, qb, c2  -b1-b2, t_inv*bt and c2, nz = 2..NS-1 (constant)
-// i.e. 7*NS - 8 values per column: its DRAM traffic is the algorithmic
-// bytes, but only 6 warps of 32 columns fit an SM, so the set-up and final
-// level loops are unrolled for independent work per thread.  The same
-// arithmetic as k_d3end, in the same order.
-constexpr int kD3Block = 32;
+// ---- d3_end on tiles of columns in shared memory ----------------------------
+// A block takes kT3Cols consecutive (or listed) node columns and keeps all
+// of a column's arrays in shared memory for the whole closure.  What is
+// independent across interfaces is done by all threads, one (column,
+// interface) each: the set-up (the two densityJM and the divisions of b1,
+// b2, c2, Ri: most of the FP64 work), the sweep-invariant am and cm, in
+// every sweep the divisions of c1 and bm, and the final bt, snu, Kv and
+// tke_dissip.  Only the recurrences of the sweep (two divisions per level,
+// in parallel) and the back substitution are left to one thread per column,
+// all of one warp; which warp alternates between the blocks of an SM, so
+// that their chains run on different schedulers.  The arithmetic and its
+// order are k_d3end's.
+//
+// Shared memory, [array][interface][column] with an odd column stride, so
+// that both a warp over the columns of one interface and a warp over the
+// interfaces of one column (the coalesced global accesses) are free of bank
+// conflicts: snu, btr and its successor (alternating), -b1-b2, t_inv*bt, c2,
+// am, cm, and one array for fr, then yy1.  The successor's slot of interface
+// m holds bm(m), then xx1(m+1), then btr1(m), each written when the one
+// before has been read.
+//
+// Bound by latency: the FP64 chains of the recurrences and of the set-up
+// (FP64 pipe 29 %, barrier and dependency waits) at the 4 blocks of 32
+// columns (21 interfaces, FP64) that shared memory holds per SM; 256 threads
+// and 64 registers for the most warps on the set-up.  FP32 tiles are half
+// the size: 128 threads, more blocks.  Against one thread per column with its arrays in
+// local memory (whose traffic streamed through DRAM): 1.05 M nodes FP64 2.71
+// -> 2.30 ms, 232 k FP32 0.31 -> 0.18, 40 k with 31 interfaces 0.23 -> 0.18,
+// 16 k with 11 0.046 -> 0.031, 4.5 k with 40 0.196 -> 0.050 ms.  A set-up
+// kernel and a sweep kernel with the sweep's arrays in local memory, shared
+// memory or registers took 2.32-2.54 ms, 0.25-0.30, 0.19, 0.046-0.055 and
+// 0.11 ms.  128 threads or tiles of 16 at 1.05 M nodes: 2.54 and 2.65 ms.
+constexpr int kT3Arrays = 9;
+constexpr int kT3Threads = FESOMC_FP32 ? 128 : 256;
+#if FESOMC_FP32
+#define D3_TILE_BOUNDS __launch_bounds__(kT3Threads)
+#else
+#define D3_TILE_BOUNDS __launch_bounds__(kT3Threads, 4)
+#endif
+static size_t d3end_tile_smem(const Dev &d, int cols) {
+    return ((size_t)kT3Arrays * d.NS * (cols + 1) + 2 * cols) * sizeof(real) + 3 * cols * sizeof(int);
+}
 
-__host__ __device__ inline int d3end_values(int NS) { return 7 * NS - 8; }
-
-template <bool kList>
-__global__ void __launch_bounds__(kD3Block, 6) k_d3end_sm(Dev d, const int *list, const unsigned long long *count) {
+template <int C, bool kList>
+__global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsigned long long *count) {
     pdl_enter();
-    extern __shared__ unsigned char d3_smem[];
-    constexpr int B = kD3Block;
+    extern __shared__ __align__(16) unsigned char d3t_smem[];
+    constexpr int CP = C + 1;
     const int NS = d.NS, L = d.L;
-    real *const base = reinterpret_cast<real *>(d3_smem) + threadIdx.x;
-    // per-array views: element nz of an array at [(nz - first) * B]
-    real *const s_sn = base - 1 * B;                     // nz = 1..NS
-    real *const s_bA = base + (NS - 1) * B;              // nz = 1..NS
-    real *const s_bB = base + (2 * NS - 1) * B;          // nz = 1..NS
-    real *const s_yy = base + (3 * NS - 3) * B;          // nz = 3..NS
-    real *const s_pb = base + (4 * NS - 4) * B;          // nz = 2..NS-1
-    real *const s_qb = base + (5 * NS - 6) * B;          // nz = 2..NS-1
-    real *const s_c2 = base + (6 * NS - 8) * B;          // nz = 2..NS-1
-#define D3(a, nz) a[(size_t)(nz) * B]
+    real *const s_sn = reinterpret_cast<real *>(d3t_smem);   // interface k (0-based) at [k * CP + column]
+    const int A = NS * CP;
+    real *const s_b[2] = {s_sn + A, s_sn + 2 * A};
+    real *const s_pb = s_sn + 3 * A, *const s_qb = s_sn + 4 * A, *const s_c2 = s_sn + 5 * A;
+    real *const s_am = s_sn + 6 * A, *const s_cm = s_sn + 7 * A, *const s_fy = s_sn + 8 * A;
+    real *const s_dm = s_sn + 9 * A, *const s_aj = s_dm + C;
+    int *const s_node = reinterpret_cast<int *>(s_aj + C), *const s_done = s_node + C, *const s_par = s_done + C;
     const real t_inv = real(1.0) / d.dt;
     const real cka = d.cka;
     const real B1cka2 = real(16.6) * (cka * cka);
-    const long long ncol = kList ? (long long)*count : (long long)d.N;
-    GRID_LOOP(ii, ncol) {
-        const int node = kList ? list[ii] : (int)ii;
-        const real *bt = d.bt + (size_t)node * NS;
-        const real *snu = d.snu + (size_t)node * NS;
-        const real *Kv = d.Kv + (size_t)node * NS;
-        const real *Un = d.Unode + (size_t)node * L;
-        const real *Vn = d.Vnode + (size_t)node * L;
-        const real *T = d.TF + (size_t)node * L;
-        const real *S = d.SF + (size_t)node * L;
-        real *Ri = d.Ri + (size_t)node * NS;
-        real *tke = d.tke_dissip + (size_t)node * NS;
-        const real dmean = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
-        const real dmean2 = dmean * dmean;
-        const real ajac = jac_a(d, d.eta_jac, node);
-        for (int nz = 1; nz <= NS; ++nz) {
-            D3(s_bA, nz) = bt[nz - 1];
-            D3(s_sn, nz) = snu[nz - 1];
-        }
-        Ri[0] = real(0.0);
-        Ri[NS - 1] = real(0.0);
-#pragma unroll 4
-        for (int nz = 2; nz <= NS - 1; ++nz) {
-            const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
-            const real d1 = s_m - s_0;
-            const real d2 = s_0 - s_p;
-            const real dd = real(0.5) * (d1 + d2);
-            real ap1 = Un[nz - 2] - Un[nz - 1];
-            const real ap2 = Vn[nz - 2] - Vn[nz - 1];
-            const real sn_m = snu[nz - 2], sn_0 = snu[nz - 1], sn_p = snu[nz];
-            real b1 = sn_0 * (ap1 * ap1 + ap2 * ap2) / (dd * dd);
-            b1 = b1 / dmean2;
-            const real zb = zbar_of(d, ajac, nz - 1);
-            const real rho_up = density_jm(T[nz - 2], S[nz - 2], -zb, d.density_0);
-            const real rho_dn = density_jm(T[nz - 1], S[nz - 1], -zb, d.density_0);
-            ap1 = (rho_up - rho_dn) / dd;
-            const real b2 = -real(0.5) * kG * Kv[nz - 1] * ap1 / (d.density_0 * dmean);
-            const real snu_p = real(0.5) * (sn_m + sn_0);
-            const real snu_m = real(0.5) * (sn_0 + sn_p);
-            const real cc = real(0.5) * real(0.73) * (snu_p * (bt[nz - 2] - bt[nz - 1]) / d1 - snu_m * (bt[nz - 1] - bt[nz]) / d2) / dd;
-            D3(s_c2, nz) = cc / dmean2;
-            if (b1 > real(0.0)) Ri[nz - 1] = -kG * ap1 / (d.density_0 * dmean) / b1 * sn_0;
-            else Ri[nz - 1] = real(10000.0);
-            D3(s_pb, nz) = -b1 - b2;
-            D3(s_qb, nz) = t_inv * bt[nz - 1];
-        }
-        real y2;
-        {
-            const real d1 = real(0.5) * (__ldg(d.sig + NS - 2) - __ldg(d.sig + NS - 1));
-            const real wx = d.windx[node], wy = d.windy[node];
-            const real u_din_sur = real(0.05) * (wx * wx + wy * wy);
-            const real snu_m = real(0.5) * (snu[NS - 1] + snu[NS - 2]);
-            y2 = (real(0.4e-3) * (u_din_sur * u_din_sur * u_din_sur) * dmean * d1) / (snu_m * real(0.76));
-        }
-        // bottom boundary value (independent of the iteration)
-        const real delta_b = jc_of(d, ajac, NS - 2) + d.z0b_min;
-        const real lg = fesomc_log(delta_b / d.z0b_min);
-        const real bott_R = B1cka2 / (lg * lg);
-        const real ubt = Un[L - 1], vbt = Vn[L - 1];
-        const real bot = bott_R * (ubt * ubt + vbt * vbt);
-        real *btr = s_bA, *xq = s_bB;   // xq: this iteration's xx1, then its btr1
-        bool converged = false;
-        int iters = 200;
-        for (int it = 1; it <= 200; ++it) {
-            real x = real(1.0), y = y2;
-            real s_lo = D3(s_sn, 1), s_mid = D3(s_sn, 2);
-            real b_n = D3(btr, 2), pb_n = D3(s_pb, 2), qb_n = D3(s_qb, 2), c2_n = D3(s_c2, 2), sh_n = D3(s_sn, 3);
-            for (int nz = 2; nz <= NS - 1; ++nz) {
-                const real s_hi = sh_n;
-                const real b = b_n, pbv = pb_n, qbv = qb_n, c2v = c2_n;
-                if (nz + 1 <= NS - 1) {
-                    b_n = D3(btr, nz + 1); pb_n = D3(s_pb, nz + 1); qb_n = D3(s_qb, nz + 1);
-                    c2_n = D3(s_c2, nz + 1); sh_n = D3(s_sn, nz + 2);
-                }
-                const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
-                const real dd1 = s_m - s_0;
-                const real dd2 = s_0 - s_p;
-                const real dd = real(0.5) * (dd1 + dd2);
-                const real c1 = real(0.046) * (b * b) / s_mid;
-                if (it == 200) tke[nz - 1] = c1;
-                const real fr = pbv - c1 - qbv - c2v;
-                const real snu_p = real(0.5) * (s_lo + s_mid);
-                const real snu_mm = real(0.5) * (s_mid + s_hi);
-                const real am = real(0.5) * (snu_p * real(0.73)) / (dmean2 * dd1 * dd);
-                const real cm = real(0.5) * (snu_mm * real(0.73)) / (dmean2 * dd2 * dd);
-                const real bm = am + cm + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
-                const real a = bm - am * x;
-                const real xn = cm / a;
-                const real yn = (am * y - fr) / a;
-                D3(xq, nz + 1) = xn;
-                D3(s_yy, nz + 1) = yn;
-                x = xn;
-                y = yn;
-                s_lo = s_mid;
-                s_mid = s_hi;
-            }
-            real b1v = bot;  // btr1(NS)
-            real x_n = D3(xq, NS), y_n = D3(s_yy, NS), o_n = D3(btr, NS - 1);
-            const real top = D3(btr, NS);
-            D3(xq, NS) = b1v;
-            bool above = d3_above_tol(top - b1v, dmax(b1v, top) + real(1.0e-8));
-            for (int nz = NS; nz >= 2; --nz) {
-                const real xv = x_n, yv = y_n, ov = o_n;
-                if (nz - 1 >= 3) { x_n = D3(xq, nz - 1); y_n = D3(s_yy, nz - 1); o_n = D3(btr, nz - 2); }
-                else if (nz - 1 == 2) { x_n = real(1.0); y_n = y2; o_n = D3(btr, nz - 2); }
-                b1v = b1v * xv + yv;  // btr1(nz-1), into the xx1(nz-1) slot already read
-                D3(xq, nz - 1) = b1v;
-                above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
-            }
-            if (!above) { converged = true; iters = it; break; }
-            real *t = btr;
-            btr = xq;
-            xq = t;
-        }
-        if (d.d3_iters) d.d3_iters[node] = iters;   // measurement only (fesomc_gpu_d3end_iterations)
-        if (converged) {
-            for (int nz = 2; nz <= NS - 1; ++nz) {
-                const real b = D3(btr, nz);
-                tke[nz - 1] = real(0.046) * (b * b) / D3(s_sn, nz);
-            }
-        } else {
-            atomicAdd(d.notconv, 1);
-        }
-        real *btw = d.bt + (size_t)node * NS;
-        real *snw = d.snu + (size_t)node * NS;
-        real *Kvw = d.Kv + (size_t)node * NS;
-#pragma unroll 4
-        for (int nz = 1; nz <= NS; ++nz) {
-            const real btn = dmax(D3(btr, nz), real(1.0e-8));
-            btw[nz - 1] = btn;
-            const real zt = __ldg(d.sig + nz - 1) * dmean;
-            const real Zh = zt + d.z0b_min;
-            const real Zd = fabs(dmean - zt) + d.z0s_min;
-            const real Z0 = real(1.0) - d.beta_scale * Zh * Zd / (dmean * dmean);
-            const real scale_t = cka * Zh * Zd * Z0 / dmean;
-            real s = scale_t * sqrt(btn) + d.snul;
-            if (s >= real(0.2)) s = real(0.2);
-            snw[nz - 1] = s;
-            Kvw[nz - 1] = d.Pr_num * s;
-        }
-    }
-#undef D3
-}
-
-// ---- d3_end in two kernels (launch-shape knob "d3end_arrays" = 3) ----------
-// The set-up of a column (its per-interface constants, which take most of the
-// FP64 work: two densityJM per interface and the divisions of b1, b2, c2,
-// Ri) does not depend on the sweep, and its interfaces are independent.  The
-// set-up kernel takes blocks of kD3Tile consecutive nodes, stages their
-// columns in shared memory with coalesced loads, forms the constants with
-// one thread per (node, interface) exactly as k_d3end's first loop does, and
-// writes -b1-b2, t_inv*bt, c2 and snu level-major ([interface][node]: a warp
-// of 32 consecutive nodes reads 256 contiguous bytes of one interface) and
-// Ri in the column layout.  The sweep kernel then keeps only xx1, yy1 and
-// the btr pair in local memory (4 arrays instead of 8: the working set of
-// the resident columns fits in L2) and reads the constants level-major.
-constexpr int kD3Tile = 32;
-constexpr int kD3SetupThreads = 256;
-
-__global__ void __launch_bounds__(kD3SetupThreads) k_d3end_setup(Dev d) {
-    pdl_enter();
-    extern __shared__ unsigned char d3s_smem[];
-    const int NS = d.NS, L = d.L, N = d.N;
-    real *sm = reinterpret_cast<real *>(d3s_smem);
-    // per node j of the tile, stride NS: U, V, T, S (L levels), bt, snu, Kv, Ri (NS)
-    real *sU = sm, *sV = sm + 1 * kD3Tile * NS, *sT = sm + 2 * kD3Tile * NS, *sS = sm + 3 * kD3Tile * NS;
-    real *sB = sm + 4 * kD3Tile * NS, *sN = sm + 5 * kD3Tile * NS, *sK = sm + 6 * kD3Tile * NS;
-    real *sR = sm + 7 * kD3Tile * NS;
-    real *sDm = sm + 8 * kD3Tile * NS, *sAj = sDm + kD3Tile;
-    const real t_inv = real(1.0) / d.dt;
-    for (long long n0 = (long long)blockIdx.x * kD3Tile; n0 < N; n0 += (long long)gridDim.x * kD3Tile) {
-        const int nt = (int)(N - n0 < kD3Tile ? N - n0 : kD3Tile);
-        for (int i = threadIdx.x; i < nt * L; i += blockDim.x) {
-            const int j = d.by_L.div(i), k = i - j * L;
-            const size_t g = (size_t)n0 * L + i;
-            sU[j * NS + k] = d.Unode[g];
-            sV[j * NS + k] = d.Vnode[g];
-            sT[j * NS + k] = d.TF[g];
-            sS[j * NS + k] = d.SF[g];
-        }
-        for (int i = threadIdx.x; i < nt * NS; i += blockDim.x) {
-            const size_t g = (size_t)n0 * NS + i;
-            sB[i] = d.bt[g];
-            sN[i] = d.snu[g];
-            sK[i] = d.Kv[g];
-        }
+    const int ncol = kList ? (int)*count : d.N;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool mine = warp == (int)((blockIdx.x / 148) % (kT3Threads / 32));   // the warp of the recurrences
+    for (int n0 = blockIdx.x * C; n0 < ncol; n0 += gridDim.x * C) {
+        const int nt = ncol - n0 < C ? ncol - n0 : C;
         if ((int)threadIdx.x < nt) {
-            const int node = (int)n0 + threadIdx.x;
-            sDm[threadIdx.x] = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
-            sAj[threadIdx.x] = jac_a(d, d.eta_jac, node);
+            const int node = kList ? list[n0 + threadIdx.x] : n0 + (int)threadIdx.x;
+            s_node[threadIdx.x] = node;
+            s_dm[threadIdx.x] = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
+            s_aj[threadIdx.x] = jac_a(d, d.eta_jac, node);
+            s_done[threadIdx.x] = 0;
         }
         __syncthreads();
-        // snu level-major, and Ri(1) = Ri(NS) = 0
-        for (int i = threadIdx.x; i < kD3Tile * NS; i += blockDim.x) {
-            const int j = i % kD3Tile, k = i / kD3Tile;   // node fastest
-            if (j < nt) d.d3_sn[(size_t)k * N + n0 + j] = sN[j * NS + k];
-        }
-        for (int j = threadIdx.x; j < nt; j += blockDim.x) {
-            sR[j * NS] = real(0.0);
-            sR[j * NS + NS - 1] = real(0.0);
-        }
-        // the interfaces nz = 2..NS-1, node fastest (k_d3end's first loop)
-        for (int i = threadIdx.x; i < kD3Tile * (NS - 2); i += blockDim.x) {
-            const int j = i % kD3Tile, nz = 2 + i / kD3Tile;
-            if (j >= nt) continue;
-            const real *Un = sU + j * NS, *Vn = sV + j * NS, *T = sT + j * NS, *S = sS + j * NS;
-            const real *bt = sB + j * NS, *Kv = sK + j * NS, *snc = sN + j * NS;
-            const real dmean = sDm[j], dmean2 = dmean * dmean, ajac = sAj[j];
-            const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
+        // set-up, one (column, interface) per thread; k = nz - 1
+        for (int i = threadIdx.x; i < nt * NS; i += kT3Threads) {
+            const int j = d.by_NS.div(i), k = i - j * NS;
+            const int node = s_node[j];
+            const size_t g = (size_t)node * NS + k;
+            const real b_0 = d.bt[g], sn_0 = d.snu[g];
+            const int o = k * CP + j;
+            s_sn[o] = sn_0;
+            s_b[0][o] = b_0;
+            if (k == 0 || k == NS - 1) {
+                d.Ri[g] = real(0.0);
+                continue;
+            }
+            const size_t gl = (size_t)node * L + k;
+            const real b_m = d.bt[g - 1], b_p = d.bt[g + 1], sn_m = d.snu[g - 1], sn_p = d.snu[g + 1];
+            const real dmean = s_dm[j], dmean2 = dmean * dmean;
+            const real s_m = __ldg(d.sig + k - 1), s_0 = __ldg(d.sig + k), s_p = __ldg(d.sig + k + 1);
             const real d1 = s_m - s_0;
             const real d2 = s_0 - s_p;
             const real dd = real(0.5) * (d1 + d2);
-            real ap1 = Un[nz - 2] - Un[nz - 1];
-            const real ap2 = Vn[nz - 2] - Vn[nz - 1];
-            const real sn_m = snc[nz - 2], sn_0 = snc[nz - 1], sn_p = snc[nz];
-            real b1 = sn_0 * (ap1 * ap1 + ap2 * ap2) / (dd * dd);
-            b1 = b1 / dmean2;
-            const real zb = zbar_of(d, ajac, nz - 1);
-            const real rho_up = density_jm(T[nz - 2], S[nz - 2], -zb, d.density_0);
-            const real rho_dn = density_jm(T[nz - 1], S[nz - 1], -zb, d.density_0);
-            ap1 = (rho_up - rho_dn) / dd;
-            const real b2 = -real(0.5) * kG * Kv[nz - 1] * ap1 / (d.density_0 * dmean);
+            real ap1 = d.Unode[gl - 1] - d.Unode[gl];
+            const real ap2 = d.Vnode[gl - 1] - d.Vnode[gl];
+            real b1 = div_pos(sn_0 * (ap1 * ap1 + ap2 * ap2), dd * dd);
+            b1 = div_pos(b1, dmean2);
+            const real zb = zbar_of(d, s_aj[j], k);
+            const real rho_up = density_jm(d.TF[gl - 1], d.SF[gl - 1], -zb, d.density_0);
+            const real rho_dn = density_jm(d.TF[gl], d.SF[gl], -zb, d.density_0);
+            ap1 = div_pos(rho_up - rho_dn, dd);
+            const real b2 = div_pos(-real(0.5) * kG * d.Kv[g] * ap1, d.density_0 * dmean);
             const real snu_p = real(0.5) * (sn_m + sn_0);
             const real snu_m = real(0.5) * (sn_0 + sn_p);
-            const real cc = real(0.5) * real(0.73) * (snu_p * (bt[nz - 2] - bt[nz - 1]) / d1 - snu_m * (bt[nz - 1] - bt[nz]) / d2) / dd;
-            const size_t o = (size_t)(nz - 2) * N + n0 + j;
-            d.d3_c2[o] = cc / dmean2;
-            if (b1 > real(0.0)) sR[j * NS + nz - 1] = -kG * ap1 / (d.density_0 * dmean) / b1 * sn_0;
-            else sR[j * NS + nz - 1] = real(10000.0);
-            d.d3_pb[o] = -b1 - b2;
-            d.d3_qb[o] = t_inv * bt[nz - 1];
+            const real cn = real(0.5) * real(0.73) * (div_pos(snu_p * (b_m - b_0), d1) - div_pos(snu_m * (b_0 - b_p), d2));
+            s_c2[o] = div_pos(div_pos(cn, dd), dmean2);
+            if (b1 > real(0.0)) d.Ri[g] = div_pos(div_pos(-kG * ap1, d.density_0 * dmean), b1) * sn_0;
+            else d.Ri[g] = real(10000.0);
+            s_pb[o] = -b1 - b2;
+            s_qb[o] = t_inv * b_0;
+            s_am[o] = real(0.5) * (snu_p * real(0.73)) / (dmean2 * d1 * dd);
+            s_cm[o] = real(0.5) * (snu_m * real(0.73)) / (dmean2 * d2 * dd);
+        }
+        // the boundary values of a column, kept by the thread of its recurrences
+        real y2 = real(0.0), bot = real(0.0);
+        __syncthreads();
+        const bool col = mine && lane < nt;
+        if (col) {
+            const int node = s_node[lane];
+            const real dmean = s_dm[lane];
+            const real d1 = real(0.5) * (__ldg(d.sig + NS - 2) - __ldg(d.sig + NS - 1));
+            const real wx = d.windx[node], wy = d.windy[node];
+            const real u_din_sur = real(0.05) * (wx * wx + wy * wy);
+            const real snu_m = real(0.5) * (s_sn[(NS - 1) * CP + lane] + s_sn[(NS - 2) * CP + lane]);
+            y2 = (real(0.4e-3) * (u_din_sur * u_din_sur * u_din_sur) * dmean * d1) / (snu_m * real(0.76));
+            const real delta_b = jc_of(d, s_aj[lane], NS - 2) + d.z0b_min;
+            const real lg = fesomc_log(delta_b / d.z0b_min);
+            const real bott_R = B1cka2 / (lg * lg);
+            const real ubt = d.Unode[(size_t)node * L + L - 1], vbt = d.Vnode[(size_t)node * L + L - 1];
+            bot = bott_R * (ubt * ubt + vbt * vbt);
+        }
+        bool open = col;   // this thread's column has not converged
+        int par = 0;
+        for (int it = 1; it <= 200; ++it) {
+            const real *const bt = s_b[par];
+            real *const bx = s_b[par ^ 1];
+            for (int i = threadIdx.x; i < C * (NS - 2); i += kT3Threads) {
+                const int j = i % C, k = 1 + i / C;
+                if (j >= nt || s_done[j]) continue;
+                const int o = k * CP + j;
+                const real b = bt[o], s_mid = s_sn[o];
+                const real c1 = real(0.046) * (b * b) / s_mid;
+                if (it == 200) d.tke_dissip[(size_t)s_node[j] * NS + k] = c1;
+                s_fy[o] = s_pb[o] - c1 - s_qb[o] - s_c2[o];
+                bx[o] = s_am[o] + s_cm[o] + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
+            }
+            __syncthreads();
+            if (open) {
+                const real *am_ = s_am + lane, *cm_ = s_cm + lane, *bo = bt + lane;
+                real *X = bx + lane, *Y = s_fy + lane;
+                real x = real(1.0), y = y2;
+                real am_n = am_[CP], cm_n = cm_[CP], bm_n = X[CP], fr_n = Y[CP];
+                for (int k = 1; k <= NS - 2; ++k) {
+                    const real am = am_n, cm = cm_n, bm = bm_n, fr = fr_n;
+                    const int kn = (k < NS - 2 ? k + 1 : k) * CP;
+                    am_n = am_[kn]; cm_n = cm_[kn]; bm_n = X[kn]; fr_n = Y[kn];
+                    const real a = bm - am * x;
+                    const real xn = cm / a;
+                    const real yn = (am * y - fr) / a;
+                    X[k * CP] = xn;   // xx1(nz+1), nz = k + 1
+                    Y[k * CP] = yn;
+                    x = xn;
+                    y = yn;
+                }
+                real b1v = bot;  // btr1(NS)
+                const real top = bo[(NS - 1) * CP];
+                bool above = d3_above_tol(top - b1v, dmax(b1v, top) + real(1.0e-8));
+                X[(NS - 1) * CP] = b1v;
+                for (int k = NS - 2; k >= 1; --k) {
+                    const real xv = X[k * CP], yv = Y[k * CP], ov = bo[k * CP];
+                    b1v = b1v * xv + yv;  // btr1(k+1), into the slot of xx1(k+2)
+                    X[k * CP] = b1v;
+                    above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
+                }
+                b1v = b1v * real(1.0) + y2;
+                X[0] = b1v;
+                above |= d3_above_tol(bo[0] - b1v, dmax(b1v, bo[0]) + real(1.0e-8));
+                if (!above || it == 200) {
+                    // the final btr: the previous iterate when the sweep
+                    // converges, else the last sweep's
+                    s_par[lane] = above ? par ^ 1 : par;
+                    s_done[lane] = above ? 2 : 1;
+                    if (above) atomicAdd(d.notconv, 1);
+                    if (d.d3_iters) d.d3_iters[s_node[lane]] = it;   // measurement only (fesomc_gpu_d3end_iterations)
+                    open = false;
+                }
+            }
+            par ^= 1;
+            if (!__syncthreads_or(open)) break;
+        }
+        // bt, snu, Kv and tke_dissip of every interface
+        for (int i = threadIdx.x; i < nt * NS; i += kT3Threads) {
+            const int j = d.by_NS.div(i), k = i - j * NS;
+            const int o = k * CP + j;
+            const size_t g = (size_t)s_node[j] * NS + k;
+            const real b = s_b[s_par[j]][o];
+            if (s_done[j] == 1 && k > 0 && k < NS - 1) d.tke_dissip[g] = real(0.046) * (b * b) / s_sn[o];
+            const real dmean = s_dm[j];
+            const real btn = dmax(b, real(1.0e-8));
+            d.bt[g] = btn;
+            const real zt = __ldg(d.sig + k) * dmean;
+            const real Zh = zt + d.z0b_min;
+            const real Zd = fabs(dmean - zt) + d.z0s_min;
+            const real Z0 = real(1.0) - d.beta_scale * Zh * Zd / (dmean * dmean);
+            const real scale_t = cka * Zh * Zd * Z0 / dmean;
+            real s = scale_t * sqrt(btn) + d.snul;
+            if (s >= real(0.2)) s = real(0.2);
+            d.snu[g] = s;
+            d.Kv[g] = d.Pr_num * s;
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < nt * NS; i += blockDim.x) d.Ri[(size_t)n0 * NS + i] = sR[i];
-        __syncthreads();
-    }
-}
-
-// The sweeps of d3_end per node column, from the set-up's level-major
-// constants; the same arithmetic as k_d3end, in the same order.
-template <int ARR, bool kList>
-__global__ void k_d3end_sweep(Dev d, const int *list, const unsigned long long *count) {
-    pdl_enter();
-    const real t_inv = real(1.0) / d.dt;
-    const real cka = d.cka;
-    const real B1cka2 = real(16.6) * (cka * cka);
-    const long long ncol = kList ? (long long)*count : (long long)d.N;
-    const size_t N = d.N;
-    GRID_LOOP(ii, ncol) {
-        const int node = kList ? list[ii] : (int)ii;
-        const int NS = d.NS, L = d.L;
-        const real *bt = d.bt + (size_t)node * NS;
-        const real *Un = d.Unode + (size_t)node * L;
-        const real *Vn = d.Vnode + (size_t)node * L;
-        real *tke = d.tke_dissip + (size_t)node * NS;
-        // constants of interface nz (2..NS-1) and snu(nz) (1..NS), level-major
-        auto PB = [&](int nz) { return d.d3_pb[(size_t)(nz - 2) * N + node]; };
-        auto QB = [&](int nz) { return d.d3_qb[(size_t)(nz - 2) * N + node]; };
-        auto C2 = [&](int nz) { return d.d3_c2[(size_t)(nz - 2) * N + node]; };
-        auto SN = [&](int nz) { return d.d3_sn[(size_t)(nz - 1) * N + node]; };
-        real xx1[ARR], yy1[ARR], bA[ARR], bB[ARR];
-        const real dmean = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
-        const real dmean2 = dmean * dmean;
-        const real ajac = jac_a(d, d.eta_jac, node);
-        for (int nz = 1; nz <= NS; ++nz) bA[nz] = bt[nz - 1];
-        real y2;
-        {
-            const real d1 = real(0.5) * (__ldg(d.sig + NS - 2) - __ldg(d.sig + NS - 1));
-            const real wx = d.windx[node], wy = d.windy[node];
-            const real u_din_sur = real(0.05) * (wx * wx + wy * wy);
-            const real snu_m = real(0.5) * (SN(NS) + SN(NS - 1));
-            y2 = (real(0.4e-3) * (u_din_sur * u_din_sur * u_din_sur) * dmean * d1) / (snu_m * real(0.76));
-        }
-        xx1[2] = real(1.0);
-        yy1[2] = y2;
-        const real delta_b = jc_of(d, ajac, NS - 2) + d.z0b_min;
-        const real lg = fesomc_log(delta_b / d.z0b_min);
-        const real bott_R = B1cka2 / (lg * lg);
-        const real ubt = Un[L - 1], vbt = Vn[L - 1];
-        const real bot = bott_R * (ubt * ubt + vbt * vbt);
-        real *btr = bA, *btr1 = bB;
-        bool converged = false;
-        int iters = 200;
-        for (int it = 1; it <= 200; ++it) {
-            real x = real(1.0), y = y2;
-            real s_lo = SN(1), s_mid = SN(2);
-            real b_n = btr[2], pb_n = PB(2), qb_n = QB(2), c2_n = C2(2), sh_n = SN(3);
-            for (int nz = 2; nz <= NS - 1; ++nz) {
-                const real s_hi = sh_n;
-                const real b = b_n, pbv = pb_n, qbv = qb_n, c2v = c2_n;
-                if (nz + 1 <= NS - 1) {
-                    b_n = btr[nz + 1]; pb_n = PB(nz + 1); qb_n = QB(nz + 1); c2_n = C2(nz + 1); sh_n = SN(nz + 2);
-                }
-                const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
-                const real dd1 = s_m - s_0;
-                const real dd2 = s_0 - s_p;
-                const real dd = real(0.5) * (dd1 + dd2);
-                const real c1 = real(0.046) * (b * b) / s_mid;
-                if (it == 200) tke[nz - 1] = c1;
-                const real fr = pbv - c1 - qbv - c2v;
-                const real snu_p = real(0.5) * (s_lo + s_mid);
-                const real snu_mm = real(0.5) * (s_mid + s_hi);
-                const real am = real(0.5) * (snu_p * real(0.73)) / (dmean2 * dd1 * dd);
-                const real cm = real(0.5) * (snu_mm * real(0.73)) / (dmean2 * dd2 * dd);
-                const real bm = am + cm + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
-                const real a = bm - am * x;
-                const real xn = cm / a;
-                const real yn = (am * y - fr) / a;
-                xx1[nz + 1] = xn;
-                yy1[nz + 1] = yn;
-                x = xn;
-                y = yn;
-                s_lo = s_mid;
-                s_mid = s_hi;
-            }
-            real b1v = bot;  // btr1(NS)
-            btr1[NS] = b1v;
-            bool above = d3_above_tol(btr[NS] - b1v, dmax(b1v, btr[NS]) + real(1.0e-8));
-            real x_n = xx1[NS], y_n = yy1[NS], o_n = btr[NS - 1];
-            for (int nz = NS; nz >= 2; --nz) {
-                const real xv = x_n, yv = y_n, ov = o_n;
-                if (nz - 1 >= 2) { x_n = xx1[nz - 1]; y_n = yy1[nz - 1]; o_n = btr[nz - 2]; }
-                b1v = b1v * xv + yv;  // btr1(nz-1)
-                btr1[nz - 1] = b1v;
-                above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
-            }
-            if (!above) { converged = true; iters = it; break; }
-            real *t = btr;
-            btr = btr1;
-            btr1 = t;
-        }
-        if (d.d3_iters) d.d3_iters[node] = iters;   // measurement only (fesomc_gpu_d3end_iterations)
-        if (converged) {
-            for (int nz = 2; nz <= NS - 1; ++nz) tke[nz - 1] = real(0.046) * (btr[nz] * btr[nz]) / SN(nz);
-        } else {
-            atomicAdd(d.notconv, 1);
-        }
-        real *btw = d.bt + (size_t)node * NS;
-        real *snw = d.snu + (size_t)node * NS;
-        real *Kvw = d.Kv + (size_t)node * NS;
-        for (int nz = 1; nz <= NS; ++nz) {
-            const real btn = dmax(btr[nz], real(1.0e-8));
-            btw[nz - 1] = btn;
-            const real zt = __ldg(d.sig + nz - 1) * dmean;
-            const real Zh = zt + d.z0b_min;
-            const real Zd = fabs(dmean - zt) + d.z0s_min;
-            const real Z0 = real(1.0) - d.beta_scale * Zh * Zd / (dmean * dmean);
-            const real scale_t = cka * Zh * Zd * Z0 / dmean;
-            real s = scale_t * sqrt(btn) + d.snul;
-            if (s >= real(0.2)) s = real(0.2);
-            snw[nz - 1] = s;
-            Kvw[nz - 1] = d.Pr_num * s;
-        }
-    }
-}
-
-// The sweeps with xx1, yy1 and the btr pair in shared memory, [array][level]
-// [thread] (launch-shape knob "d3end_arrays" = 4): no local memory at all,
-// 4*NS - 2 values per column, blocks of kD3Block columns.
-__global__ void __launch_bounds__(kD3Block) k_d3end_sweep_sm(Dev d) {
-    pdl_enter();
-    extern __shared__ unsigned char d3w_smem[];
-    constexpr int B = kD3Block;
-    const real t_inv = real(1.0) / d.dt;
-    const real cka = d.cka;
-    const real B1cka2 = real(16.6) * (cka * cka);
-    const size_t N = d.N;
-    const int NS = d.NS, L = d.L;
-    real *const base = reinterpret_cast<real *>(d3w_smem) + threadIdx.x;
-    // element nz of an array at [(nz - first) * B]
-    real *const s_x = base - 2 * B;                      // xx1, nz = 2..NS
-    real *const s_y = base + (NS - 1 - 2) * B;           // yy1, nz = 2..NS
-    real *const s_bA = base + (2 * NS - 2 - 1) * B;      // nz = 1..NS
-    real *const s_bB = base + (3 * NS - 2 - 1) * B;      // nz = 1..NS
-#define W3(a, nz) a[(size_t)(nz) * B]
-    GRID_LOOP(ii, (long long)d.N) {
-        const int node = (int)ii;
-        const real *bt = d.bt + (size_t)node * NS;
-        const real *Un = d.Unode + (size_t)node * L;
-        const real *Vn = d.Vnode + (size_t)node * L;
-        real *tke = d.tke_dissip + (size_t)node * NS;
-        // constants of interface nz (2..NS-1) and snu(nz) (1..NS), level-major
-        auto PB = [&](int nz) { return d.d3_pb[(size_t)(nz - 2) * N + node]; };
-        auto QB = [&](int nz) { return d.d3_qb[(size_t)(nz - 2) * N + node]; };
-        auto C2 = [&](int nz) { return d.d3_c2[(size_t)(nz - 2) * N + node]; };
-        auto SN = [&](int nz) { return d.d3_sn[(size_t)(nz - 1) * N + node]; };
-        const real dmean = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
-        const real dmean2 = dmean * dmean;
-        const real ajac = jac_a(d, d.eta_jac, node);
-        for (int nz = 1; nz <= NS; ++nz) W3(s_bA, nz) = bt[nz - 1];
-        real y2;
-        {
-            const real d1 = real(0.5) * (__ldg(d.sig + NS - 2) - __ldg(d.sig + NS - 1));
-            const real wx = d.windx[node], wy = d.windy[node];
-            const real u_din_sur = real(0.05) * (wx * wx + wy * wy);
-            const real snu_m = real(0.5) * (SN(NS) + SN(NS - 1));
-            y2 = (real(0.4e-3) * (u_din_sur * u_din_sur * u_din_sur) * dmean * d1) / (snu_m * real(0.76));
-        }
-        W3(s_x, 2) = real(1.0);
-        W3(s_y, 2) = y2;
-        const real delta_b = jc_of(d, ajac, NS - 2) + d.z0b_min;
-        const real lg = fesomc_log(delta_b / d.z0b_min);
-        const real bott_R = B1cka2 / (lg * lg);
-        const real ubt = Un[L - 1], vbt = Vn[L - 1];
-        const real bot = bott_R * (ubt * ubt + vbt * vbt);
-        real *btr = s_bA, *btr1 = s_bB;
-        bool converged = false;
-        int iters = 200;
-        for (int it = 1; it <= 200; ++it) {
-            real x = real(1.0), y = y2;
-            real s_lo = SN(1), s_mid = SN(2);
-            real b_n = W3(btr, 2), pb_n = PB(2), qb_n = QB(2), c2_n = C2(2), sh_n = SN(3);
-            for (int nz = 2; nz <= NS - 1; ++nz) {
-                const real s_hi = sh_n;
-                const real b = b_n, pbv = pb_n, qbv = qb_n, c2v = c2_n;
-                if (nz + 1 <= NS - 1) {
-                    b_n = W3(btr, nz + 1); pb_n = PB(nz + 1); qb_n = QB(nz + 1); c2_n = C2(nz + 1); sh_n = SN(nz + 2);
-                }
-                const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
-                const real dd1 = s_m - s_0;
-                const real dd2 = s_0 - s_p;
-                const real dd = real(0.5) * (dd1 + dd2);
-                const real c1 = real(0.046) * (b * b) / s_mid;
-                if (it == 200) tke[nz - 1] = c1;
-                const real fr = pbv - c1 - qbv - c2v;
-                const real snu_p = real(0.5) * (s_lo + s_mid);
-                const real snu_mm = real(0.5) * (s_mid + s_hi);
-                const real am = real(0.5) * (snu_p * real(0.73)) / (dmean2 * dd1 * dd);
-                const real cm = real(0.5) * (snu_mm * real(0.73)) / (dmean2 * dd2 * dd);
-                const real bm = am + cm + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
-                const real a = bm - am * x;
-                const real xn = cm / a;
-                const real yn = (am * y - fr) / a;
-                W3(s_x, nz + 1) = xn;
-                W3(s_y, nz + 1) = yn;
-                x = xn;
-                y = yn;
-                s_lo = s_mid;
-                s_mid = s_hi;
-            }
-            real b1v = bot;  // btr1(NS)
-            const real top = W3(btr, NS);
-            W3(btr1, NS) = b1v;
-            bool above = d3_above_tol(top - b1v, dmax(b1v, top) + real(1.0e-8));
-            real x_n = W3(s_x, NS), y_n = W3(s_y, NS), o_n = W3(btr, NS - 1);
-            for (int nz = NS; nz >= 2; --nz) {
-                const real xv = x_n, yv = y_n, ov = o_n;
-                if (nz - 1 >= 2) { x_n = W3(s_x, nz - 1); y_n = W3(s_y, nz - 1); o_n = W3(btr, nz - 2); }
-                b1v = b1v * xv + yv;  // btr1(nz-1)
-                W3(btr1, nz - 1) = b1v;
-                above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
-            }
-            if (!above) { converged = true; iters = it; break; }
-            real *t = btr;
-            btr = btr1;
-            btr1 = t;
-        }
-        if (d.d3_iters) d.d3_iters[node] = iters;   // measurement only (fesomc_gpu_d3end_iterations)
-        if (converged) {
-            for (int nz = 2; nz <= NS - 1; ++nz) {
-                const real b = W3(btr, nz);
-                tke[nz - 1] = real(0.046) * (b * b) / SN(nz);
-            }
-        } else {
-            atomicAdd(d.notconv, 1);
-        }
-        real *btw = d.bt + (size_t)node * NS;
-        real *snw = d.snu + (size_t)node * NS;
-        real *Kvw = d.Kv + (size_t)node * NS;
-        for (int nz = 1; nz <= NS; ++nz) {
-            const real btn = dmax(W3(btr, nz), real(1.0e-8));
-            btw[nz - 1] = btn;
-            const real zt = __ldg(d.sig + nz - 1) * dmean;
-            const real Zh = zt + d.z0b_min;
-            const real Zd = fabs(dmean - zt) + d.z0s_min;
-            const real Z0 = real(1.0) - d.beta_scale * Zh * Zd / (dmean * dmean);
-            const real scale_t = cka * Zh * Zd * Z0 / dmean;
-            real s = scale_t * sqrt(btn) + d.snul;
-            if (s >= real(0.2)) s = real(0.2);
-            snw[nz - 1] = s;
-            Kvw[nz - 1] = d.Pr_num * s;
-        }
-    }
-#undef W3
-}
-
-
-// ---- the sweeps in registers (launch-shape knob "d3end_arrays" = 5, 6) -----
-// For a level count fixed at compile time (NSC) every loop over the levels
-// unrolls, so the column arrays live in registers and the sweep touches no
-// local memory.  Three arrays instead of four: the back substitution writes
-// btr1(m) into the slot of xx1(m + 1) it has just read (xx1(2) = 1 is a
-// constant), so with btr(m) = P[m] the sweep leaves btr1(m) in Q[m + 1],
-// copied back into P when the column has not converged.  yy1 keeps its own
-// array (yy1(2) = y2 a constant).  The arithmetic is k_d3end_sweep's, in
-// the same order; the constants are read level-major through the
-// read-only path.
-template <int NSC>
-__device__ __forceinline__ bool d3_sweep_reg(const Dev &d, size_t N, int node, const real (&P)[NSC + 2],
-                                             real (&Q)[NSC + 2], real (&Y)[NSC + 2], real y2, real bot, real dmean2,
-                                             real t_inv, bool last, real *tke) {
-    constexpr int PO = 0, QO = 0;
-    const real *pb = d.d3_pb + node, *qb = d.d3_qb + node, *c2 = d.d3_c2 + node, *sn = d.d3_sn + node;
-    real x = real(1.0), y = y2;
-    real s_lo = __ldg(sn), s_mid = __ldg(sn + N);
-#pragma unroll
-    for (int nz = 2; nz <= NSC - 1; ++nz) {
-        const real s_hi = __ldg(sn + (size_t)nz * N);
-        const real b = P[nz + PO];
-        const real pbv = __ldg(pb + (size_t)(nz - 2) * N), qbv = __ldg(qb + (size_t)(nz - 2) * N);
-        const real c2v = __ldg(c2 + (size_t)(nz - 2) * N);
-        const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
-        const real dd1 = s_m - s_0;
-        const real dd2 = s_0 - s_p;
-        const real dd = real(0.5) * (dd1 + dd2);
-        const real c1 = real(0.046) * (b * b) / s_mid;
-        if (last) tke[nz - 1] = c1;
-        const real fr = pbv - c1 - qbv - c2v;
-        const real snu_p = real(0.5) * (s_lo + s_mid);
-        const real snu_mm = real(0.5) * (s_mid + s_hi);
-        const real am = real(0.5) * (snu_p * real(0.73)) / (dmean2 * dd1 * dd);
-        const real cm = real(0.5) * (snu_mm * real(0.73)) / (dmean2 * dd2 * dd);
-        const real bm = am + cm + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
-        const real a = bm - am * x;
-        const real xn = cm / a;
-        const real yn = (am * y - fr) / a;
-        Q[nz + 1 + QO] = xn;
-        Y[nz + 1] = yn;
-        x = xn;
-        y = yn;
-        s_lo = s_mid;
-        s_mid = s_hi;
-    }
-    real b1v = bot;  // btr1(NS)
-    bool above = d3_above_tol(P[NSC + PO] - b1v, dmax(b1v, P[NSC + PO]) + real(1.0e-8));
-    Q[NSC + 1 + QO] = b1v;
-#pragma unroll
-    for (int nz = NSC; nz >= 2; --nz) {
-        const real xv = nz == 2 ? real(1.0) : Q[nz + QO];
-        const real yv = nz == 2 ? y2 : Y[nz];
-        const real ov = P[nz - 1 + PO];
-        b1v = b1v * xv + yv;  // btr1(nz-1)
-        Q[nz + QO] = b1v;
-        above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
-    }
-    return above;
-}
-
-// MINB resident blocks of 64 columns per SM: 6 (at most 168 registers) or
-// 8 (128 registers, a few spilled)
-template <int NSC, int MINB>
-__global__ void __launch_bounds__(64, MINB) k_d3end_sweep_reg(Dev d) {
-    pdl_enter();
-    const real t_inv = real(1.0) / d.dt;
-    const real cka = d.cka;
-    const real B1cka2 = real(16.6) * (cka * cka);
-    const size_t N = d.N;
-    constexpr int NS = NSC;
-    const int L = d.L;
-    GRID_LOOP(ii, (long long)d.N) {
-        const int node = (int)ii;
-        const real *bt = d.bt + (size_t)node * NS;
-        const real *Un = d.Unode + (size_t)node * L;
-        const real *Vn = d.Vnode + (size_t)node * L;
-        real *tke = d.tke_dissip + (size_t)node * NS;
-        auto SN = [&](int nz) { return __ldg(d.d3_sn + (size_t)(nz - 1) * N + node); };
-        real A[NSC + 2], B[NSC + 2], Y[NSC + 2];
-        const real dmean = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
-        const real dmean2 = dmean * dmean;
-        const real ajac = jac_a(d, d.eta_jac, node);
-#pragma unroll
-        for (int nz = 1; nz <= NS; ++nz) A[nz] = bt[nz - 1];
-        real y2;
-        {
-            const real d1 = real(0.5) * (__ldg(d.sig + NS - 2) - __ldg(d.sig + NS - 1));
-            const real wx = d.windx[node], wy = d.windy[node];
-            const real u_din_sur = real(0.05) * (wx * wx + wy * wy);
-            const real snu_m = real(0.5) * (SN(NS) + SN(NS - 1));
-            y2 = (real(0.4e-3) * (u_din_sur * u_din_sur * u_din_sur) * dmean * d1) / (snu_m * real(0.76));
-        }
-        const real delta_b = jc_of(d, ajac, NS - 2) + d.z0b_min;
-        const real lg = fesomc_log(delta_b / d.z0b_min);
-        const real bott_R = B1cka2 / (lg * lg);
-        const real ubt = Un[L - 1], vbt = Vn[L - 1];
-        const real bot = bott_R * (ubt * ubt + vbt * vbt);
-        // A ends as the final btr: the previous iterate when a sweep
-        // converges, the last sweep's result after 200 without convergence
-        bool converged = false;
-        int iters = 200;
-        for (int it = 1; it <= 200; ++it) {
-            if (!d3_sweep_reg<NSC>(d, N, node, A, B, Y, y2, bot, dmean2, t_inv, it == 200, tke)) {
-                converged = true;
-                iters = it;
-                break;
-            }
-#pragma unroll
-            for (int m = 1; m <= NS; ++m) A[m] = B[m + 1];
-        }
-        if (d.d3_iters) d.d3_iters[node] = iters;   // measurement only (fesomc_gpu_d3end_iterations)
-        if (converged) {
-#pragma unroll
-            for (int nz = 2; nz <= NS - 1; ++nz) tke[nz - 1] = real(0.046) * (A[nz] * A[nz]) / SN(nz);
-        } else {
-            atomicAdd(d.notconv, 1);
-        }
-        real *btw = d.bt + (size_t)node * NS;
-        real *snw = d.snu + (size_t)node * NS;
-        real *Kvw = d.Kv + (size_t)node * NS;
-#pragma unroll
-        for (int nz = 1; nz <= NS; ++nz) {
-            const real btn = dmax(A[nz], real(1.0e-8));
-            btw[nz - 1] = btn;
-            const real zt = __ldg(d.sig + nz - 1) * dmean;
-            const real Zh = zt + d.z0b_min;
-            const real Zd = fabs(dmean - zt) + d.z0s_min;
-            const real Z0 = real(1.0) - d.beta_scale * Zh * Zd / (dmean * dmean);
-            const real scale_t = cka * Zh * Zd * Z0 / dmean;
-            real s = scale_t * sqrt(btn) + d.snul;
-            if (s >= real(0.2)) s = real(0.2);
-            snw[nz - 1] = s;
-            Kvw[nz - 1] = d.Pr_num * s;
-        }
     }
 }
 
@@ -868,56 +427,50 @@ __global__ void k_av(Dev d) {
     }
 }
 
-static size_t d3end_smem(const Dev &d) { return (size_t)d3end_values(d.NS) * kD3Block * sizeof(real); }
-static size_t d3end_setup_smem(const Dev &d) { return ((size_t)8 * kD3Tile * d.NS + 2 * kD3Tile) * sizeof(real); }
-// the two-kernel form: up to 40 levels (its sweep's local arrays are sized
-// like k_d3end's)
-static bool d3end_split(const Dev &d) { return d.tune[TK_D3END] >= 3 && d.NS <= 40; }
-// the register sweep is compiled for these level counts; others take the
-// local-memory sweep
-static bool d3end_reg(const Dev &d) { return d.tune[TK_D3END] >= 5 && (d.NS == 11 || d.NS == 21); }
-static size_t d3end_sweep_smem(const Dev &d) { return (size_t)(4 * d.NS - 2) * kD3Block * sizeof(real); }
+// Which form: the tiles while three blocks of 16 columns fit an SM (FP64 up
+// to 61 interfaces, 40 k nodes: 0.49 against 0.53 ms; 81 interfaces, two
+// blocks: 0.92 against 0.72), else one thread per column (also with the
+// launch-shape knob "d3end_arrays" at 1).  FP32 always takes the tiles: half
+// the size (81 interfaces: 3.1 against 3.9 ms, 127: 16.1 against 18.6), and
+// the two forms' contracted arithmetic would not give the same bits.
+static bool d3end_tiled(const Dev &d) {
+    return FESOMC_FP32 || (d.tune[TK_D3END] != 1 && d3end_tile_smem(d, 16) <= 75 * 1024);
+}
+// columns per tile: 32; 16 where 32 would not leave an SM two blocks, and on
+// meshes whose 16-column tiles are at most two per SM (twice the blocks for
+// the same chains: 4.5 k nodes, 40 interfaces: 0.058 -> 0.050 ms)
+static int d3end_cols(const Dev &d) {
+    return d.N > 2 * 148 * 16 && d3end_tile_smem(d, 32) <= 113 * 1024 ? 32 : 16;
+}
 int config_d3end(const Dev &d) {
     if (d.NS > 127) return 1;
-    if (d.NS <= 40 && (raise_smem_limit(k_d3end_setup, d3end_setup_smem(d)) != cudaSuccess ||
-                       raise_smem_limit(k_d3end_sweep_sm, d3end_sweep_smem(d)) != cudaSuccess))
-        return 1;
-    return (raise_smem_limit(k_d3end_sm<false>, d3end_smem(d)) == cudaSuccess &&
-            raise_smem_limit(k_d3end_sm<true>, d3end_smem(d)) == cudaSuccess) ? 0 : 1;
+    const size_t t32 = d3end_tile_smem(d, 32), t16 = d3end_tile_smem(d, 16);
+    bool ok = true;
+    if (t32 <= 113 * 1024)
+        ok = raise_smem_limit(k_d3end_tile<32, false>, t32) == cudaSuccess &&
+             raise_smem_limit(k_d3end_tile<32, true>, t32) == cudaSuccess;
+    return ok && raise_smem_limit(k_d3end_tile<16, false>, t16) == cudaSuccess &&
+                   raise_smem_limit(k_d3end_tile<16, true>, t16) == cudaSuccess
+               ? 0 : 1;
 }
-static void launch_d3end_split(const Dev &d, cudaStream_t s) {
-    const int tiles = (d.N + kD3Tile - 1) / kD3Tile;
-    launch_k(k_d3end_setup, tiles < 148 * 16 ? tiles : 148 * 16, kD3SetupThreads, d3end_setup_smem(d), s, d);
-    if (d3end_reg(d)) {
-        const bool b8 = d.tune[TK_D3END] == 6;
-        if (d.NS == 11 && b8) launch_k(k_d3end_sweep_reg<11, 8>, grid_for(d.N, 64), 64, 0, s, d);
-        else if (d.NS == 11) launch_k(k_d3end_sweep_reg<11, 6>, grid_for(d.N, 64), 64, 0, s, d);
-        else if (b8) launch_k(k_d3end_sweep_reg<21, 8>, grid_for(d.N, 64), 64, 0, s, d);
-        else launch_k(k_d3end_sweep_reg<21, 6>, grid_for(d.N, 64), 64, 0, s, d);
+template <bool kList>
+static void launch_d3end_form(const Dev &d, const int *list, const unsigned long long *count, cudaStream_t s) {
+    if (d3end_tiled(d)) {
+        const int C = d3end_cols(d), tiles = (d.N + C - 1) / C;
+        if (C == 32) launch_k(k_d3end_tile<32, kList>, tiles, kT3Threads, d3end_tile_smem(d, 32), s, d, list, count);
+        else launch_k(k_d3end_tile<16, kList>, tiles, kT3Threads, d3end_tile_smem(d, 16), s, d, list, count);
     }
-    else if (d.tune[TK_D3END] == 4) launch_k(k_d3end_sweep_sm, grid_for(d.N, kD3Block), kD3Block, d3end_sweep_smem(d), s, d);
-    else if (d.NS <= 11) launch_k(k_d3end_sweep<12, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
-    else if (d.NS <= 21) launch_k(k_d3end_sweep<22, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
-    else launch_k(k_d3end_sweep<41, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
+#if !FESOMC_FP32
+    else if (d.NS <= 21) launch_k(k_d3end<22, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);
+    else if (d.NS <= 40) launch_k(k_d3end<41, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);
+    else launch_k(k_d3end<128, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);
+#endif
 }
-void launch_d3end(const Dev &d, cudaStream_t s) {
-    if (d3end_split(d)) launch_d3end_split(d, s);
-    else if (d.tune[TK_D3END] == 2) launch_k(k_d3end_sm<false>, grid_for(d.N, kD3Block), kD3Block, d3end_smem(d), s, d, nullptr, nullptr);
-    else if (d.NS <= 11) launch_k(k_d3end<12, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
-    else if (d.NS <= 21) launch_k(k_d3end<22, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
-    else if (d.NS <= 40) launch_k(k_d3end<41, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
-    else launch_k(k_d3end<128, false>, grid_for(d.N, 64), 64, 0, s, d, nullptr, nullptr);
-}
+void launch_d3end(const Dev &d, cudaStream_t s) { launch_d3end_form<false>(d, nullptr, nullptr, s); }
 // the plain closure on the listed columns (count read on the device, so the
-// launch covers every node and the grid-stride loop stops at the count)
-// (the two-kernel form sets up every column, so the listed columns take the
-// one-kernel forms, which leave the others' Ri alone)
+// launch covers every node and the loop over columns stops at the count)
 void launch_d3end_list(const Dev &d, const int *list, const unsigned long long *count, cudaStream_t s) {
-    if (d.tune[TK_D3END] == 2) launch_k(k_d3end_sm<true>, grid_for(d.N, kD3Block), kD3Block, d3end_smem(d), s, d, list, count);
-    else if (d.NS <= 11) launch_k(k_d3end<12, true>, grid_for(d.N, 64), 64, 0, s, d, list, count);
-    else if (d.NS <= 21) launch_k(k_d3end<22, true>, grid_for(d.N, 64), 64, 0, s, d, list, count);
-    else if (d.NS <= 40) launch_k(k_d3end<41, true>, grid_for(d.N, 64), 64, 0, s, d, list, count);
-    else launch_k(k_d3end<128, true>, grid_for(d.N, 64), 64, 0, s, d, list, count);
+    launch_d3end_form<true>(d, list, count, s);
 }
 void launch_av(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_AV, 256);

@@ -807,10 +807,6 @@ int alloc_3d(fesomc_model *m, D &d) {
     }
     decltype(&d.U_n) nsn[] = {&d.hpressure, &d.bt, &d.snu, &d.Kv, &d.Ri, &d.tke_dissip, &d.Wvel};
     for (auto p : nsn) if ((rc = dalloc(m, p, NS * N))) return rc;
-    if (m->p.ver_mix == 3) {
-        decltype(&d.U_n) d3s[] = {&d.d3_pb, &d.d3_qb, &d.d3_c2, &d.d3_sn};
-        for (auto p : d3s) if ((rc = dalloc(m, p, NS * N))) return rc;
-    }
     if ((rc = dalloc(m, &d.Av, NS * E))) return rc;
     const size_t nm = (size_t)m->n_members;
     if ((rc = dalloc(m, &d.mm_part, (size_t)4 * nm * fesomc::f64::minmax_parts((int)nm)))) return rc;
@@ -2045,7 +2041,7 @@ const KnobInfo kKnobs[fesomc::kTuneKnobs] = {
     {"muscl_egrad", "muscl_egrad", 256}, {"muscl_ngrad", "muscl_ngrad", 256}, {"muscl_edge", "muscl_edge", 256},
     {"muscl_h", "muscl_h", 128}, {"upwind_h", "upwind_h", 128}, {"av", "av", 256},
     {"columns", "pressure_col,bpg_elem,update3d,wvel", 0},
-    {"d3end_arrays", "d3end,d3end_list", 1},
+    {"d3end_arrays", "d3end,d3end_list", 2},
     {"vdiff_form", "vdiff_col", 3},
     {"implvisc_form", "implvisc", 2},
 };

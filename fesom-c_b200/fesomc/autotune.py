@@ -28,10 +28,8 @@ from . import abi, cases, model
 
 THREADS = (64, 128, 256, 512, 1024)
 COLUMNS = (1, 2, 4, 8, 16, 32)
-# d3_end: local-memory arrays, shared-memory arrays, set-up and sweep kernels
-# (the sweep's arrays in local memory, in shared memory, or in registers at
-# 6 or 8 resident blocks per SM)
-D3END_ARRAYS = (1, 2, 3, 4, 5, 6)
+# d3_end: one thread per column, or tiles of columns in shared memory
+D3END_ARRAYS = (1, 2)
 # tracer_impl_vert_diff: columns read directly, or tiles of 128 or 64 columns
 # staged in shared memory
 VDIFF_FORMS = (1, 2, 3)

@@ -452,9 +452,10 @@ int  fesomc_ensemble_run(fesomc_model *const *members, int32_t n_members, int32_
  * fesomc_gpu_tune_set takes one value per knob (0 = the default) and
  * returns FESOMC_EINVAL, changing nothing, when a thread count is not a
  * multiple of 32 or a value exceeds its limit ("d3end_arrays" takes 1 to 6:
- * d3_end's column arrays in local or in shared memory, or a set-up and a
- * sweep kernel with the sweep's arrays in local memory, in shared memory, or
- * (11 or 21 levels) in registers at 6 or 8 blocks of 64 columns per SM;
+ * d3_end with one thread per column, its arrays in local memory, or (2 to 6,
+ * the same form under every number, so that saved shapes stay valid) on
+ * tiles of columns in shared memory, the default up to 61 levels; the FP32
+ * form takes the tiles under every number;
  * "vdiff_form" 1 to 3: the tracers' implicit vertical diffusion with each
  * column read directly by its thread, or on tiles of 128 or 64 (the
  * default) columns staged in shared memory, for 10 or 20 layers;

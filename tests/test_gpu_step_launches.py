@@ -45,3 +45,12 @@ def test_sub_cycle_lengths(built, sub):
 
     assert case_of(None).params.Mt == sub
     _compare(case_of, 4)
+
+
+# d3_end on tiles of columns: ragged last tiles of 16 and 32 columns, the
+# smallest level count, and the level counts on both sides of the switches
+# from 32 to 16 columns (47 interfaces, FP64) and to one thread per column (61)
+@pytest.mark.parametrize("nx,ny,nsigma", [(9, 9, 5), (70, 69, 11), (71, 68, 47), (71, 68, 48), (12, 11, 61), (12, 11, 62)])
+def test_d3end_tiles(built, nx, ny, nsigma):
+    from fesomc import cases
+    _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib), 3)
