@@ -57,6 +57,63 @@ inline cudaError_t raise_smem_limit(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// ---- compensated sums of the energy diagnostic --------------------------------
+// running sum s with its rounding errors in c (Neumaier 1974)
+struct CompSum {
+    double s, c;
+    __device__ __forceinline__ void add(double x) {
+        const double t = s + x;
+        if (fabs(s) >= fabs(x)) c += (s - t) + x;
+        else c += (x - t) + s;
+        s = t;
+    }
+    __device__ __forceinline__ void merge(double os, double oc) {
+        add(os);
+        c += oc;
+    }
+};
+// The three compensated sums of a block of BLOCK threads, merged in a fixed
+// tree (lanes of a warp, then the warps), so that the result does not depend
+// on timing; thread k < 3 of the block returns sum k.  Bound by the latency
+// of dependent FP64 additions: with three threads adding the block's 256
+// values one after the other, and the grid's 592, fesomc_energy_device took
+// 74 us on 262 k nodes; the trees are 12 and 15 additions deep: 37 us, of
+// which the two kernels 10 + 4.5 us.
+template <int BLOCK>
+__device__ __forceinline__ double block_sum3(CompSum (&v)[3]) {
+    constexpr int W = BLOCK / 32;
+    __shared__ double sh[3][2][W];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double os = __shfl_down_sync(0xffffffffu, v[k].s, o), oc = __shfl_down_sync(0xffffffffu, v[k].c, o);
+            v[k].merge(os, oc);
+        }
+        if (lane == 0) {
+            sh[k][0][warp] = v[k].s;
+            sh[k][1][warp] = v[k].c;
+        }
+    }
+    __syncthreads();
+    CompSum t{0.0, 0.0};
+    if (threadIdx.x < 3) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) t.merge(sh[threadIdx.x][0][w], sh[threadIdx.x][1][w]);
+    }
+    return t.s + t.c;
+}
+// the sums of nparts triples, one block
+template <int BLOCK>
+__device__ __forceinline__ double block_total3(const double *part, int nparts) {
+    CompSum v[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    for (int b = threadIdx.x; b < nparts; b += BLOCK)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k].add(part[(size_t)b * 3 + k]);
+    return block_sum3<BLOCK>(v);
+}
+
 // ---- max/min exactly as the Fortran MAX/MIN of two values -------------------
 template <typename T>
 __device__ __forceinline__ T dmax(T a, T b) { return a > b ? a : b; }

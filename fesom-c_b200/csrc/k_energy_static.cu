@@ -42,25 +42,13 @@ static_assert(kEsDoubles * sizeof(double) == 14232, "documented scratch size");
 
 static __device__ __align__(256) double g_energy_scratch[kEsDoubles];
 
-// compensated (Neumaier) running sum
-struct NSum {
-    double s, c;
-    __device__ void add(double x) {
-        const double t = s + x;
-        if (fabs(s) >= fabs(x)) c += (s - t) + x;
-        else c += (x - t) + s;
-        s = t;
-    }
-    __device__ double value() const { return s + c; }
-};
-
 // Per-block partial sums of potential energy, kinetic energy and area;
 // element nodes are 1-based (4 per element, triangles repeat node 1).
 __global__ void k_energy_dev_part(int N, int E, double Dmin, const double *eta, const double *depth,
                                   const double *area, const int32_t *en4, const double *w4, const double *u2,
                                   const double *earea, double *scratch) {
-    __shared__ double sh[3][kEsBlock];
-    NSum pe{0.0, 0.0}, ke{0.0, 0.0}, ar{0.0, 0.0};
+    CompSum v[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    CompSum &pe = v[0], &ke = v[1], &ar = v[2];
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
         const double e = eta[i];
         pe.add(0.5 * kG * area[i] * (e * e));
@@ -74,23 +62,14 @@ __global__ void k_energy_dev_part(int N, int E, double Dmin, const double *eta, 
         const double ux = u2[2 * i], uy = u2[2 * i + 1];
         ke.add(0.5 * s * earea[i] * (ux * ux + uy * uy));
     }
-    sh[0][threadIdx.x] = pe.value();
-    sh[1][threadIdx.x] = ke.value();
-    sh[2][threadIdx.x] = ar.value();
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        NSum t{0.0, 0.0};
-        for (int k = 0; k < kEsBlock; ++k) t.add(sh[threadIdx.x][k]);
-        scratch[(size_t)blockIdx.x * 3 + threadIdx.x] = t.value();
-    }
+    const double t = block_sum3<kEsBlock>(v);
+    if (threadIdx.x < 3) scratch[(size_t)blockIdx.x * 3 + threadIdx.x] = t;
 }
 
-__global__ void k_energy_dev_final(double *scratch, int nparts) {
-    if (threadIdx.x < 3 && blockIdx.x == 0) {
-        NSum t{0.0, 0.0};
-        for (int b = 0; b < nparts; ++b) t.add(scratch[(size_t)b * 3 + threadIdx.x]);
-        scratch[(size_t)kEsParts * 3 + threadIdx.x] = t.value();
-    }
+__global__ void __launch_bounds__(kEsBlock) k_energy_dev_final(double *scratch, int nparts) {
+    pdl_enter();
+    const double t = block_total3<kEsBlock>(scratch, nparts);
+    if (threadIdx.x < 3) scratch[(size_t)kEsParts * 3 + threadIdx.x] = t;
 }
 
 std::mutex g_setup_mu;
@@ -125,7 +104,7 @@ extern "C" int fesomc_energy_device(int32_t nod2D, int32_t elem2D, double Dmin, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     k_energy_dev_part<<<nparts, kEsBlock, 0, s>>>(nod2D, elem2D, Dmin, eta_n, depth, area, elem2D_nodes, w_cv,
                                                   U_n_2D, elem_area, scratch);
-    k_energy_dev_final<<<1, 32, 0, s>>>(scratch, nparts);
+    launch_k(k_energy_dev_final, 1, kEsBlock, 0, s, scratch, nparts);
     if (cudaGetLastError() != cudaSuccess) return FESOMC_ECUDA;
     double h[3];
     if (cudaMemcpyAsync(h, scratch + (size_t)kEsParts * 3, 3 * sizeof(double), cudaMemcpyDeviceToHost, s) !=

@@ -1012,21 +1012,10 @@ __global__ void __launch_bounds__(kVdBlock) k_vdiff_col(Dev d) {
 // energy: compensated (Neumaier) partial sums per block, then one block.
 // FP64 accumulation in both precision forms.
 // ---------------------------------------------------------------------------
-struct KSum {
-    double s, c;
-    __device__ void add(double x) {
-        double t = s + x;
-        if (fabs(s) >= fabs(x)) c += (s - t) + x;
-        else c += (x - t) + s;
-        s = t;
-    }
-    __device__ double value() const { return s + c; }
-};
-
 __global__ void k_energy_part(Dev d, double *part) {
     pdl_enter();
-    __shared__ double sh[3][kRedBlock];
-    KSum pe{0.0, 0.0}, ke{0.0, 0.0}, ar{0.0, 0.0};
+    CompSum v[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    CompSum &pe = v[0], &ke = v[1], &ar = v[2];
     GRID_LOOP(i, d.N) {
         const double e = d.eta_n[i];
         const double a = d.area[i];
@@ -1044,24 +1033,14 @@ __global__ void k_energy_part(Dev d, double *part) {
         const double ux = u.x, uy = u.y;
         ke.add(0.5 * s * (double)d.elem_area[i] * (ux * ux + uy * uy));
     }
-    sh[0][threadIdx.x] = pe.value();
-    sh[1][threadIdx.x] = ke.value();
-    sh[2][threadIdx.x] = ar.value();
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        KSum t{0.0, 0.0};
-        for (int k = 0; k < kRedBlock; ++k) t.add(sh[threadIdx.x][k]);
-        part[(size_t)blockIdx.x * 3 + threadIdx.x] = t.value();
-    }
+    const double t = block_sum3<kRedBlock>(v);
+    if (threadIdx.x < 3) part[(size_t)blockIdx.x * 3 + threadIdx.x] = t;
 }
 
-__global__ void k_energy_final(const double *part, int nparts, double *out) {
+__global__ void __launch_bounds__(kRedBlock) k_energy_final(const double *part, int nparts, double *out) {
     pdl_enter();
-    if (threadIdx.x < 3 && blockIdx.x == 0) {
-        KSum t{0.0, 0.0};
-        for (int b = 0; b < nparts; ++b) t.add(part[(size_t)b * 3 + threadIdx.x]);
-        out[threadIdx.x] = t.value();
-    }
+    const double t = block_total3<kRedBlock>(part, nparts);
+    if (threadIdx.x < 3) out[threadIdx.x] = t;
 }
 
 // ---- launch wrappers --------------------------------------------------------
@@ -1453,7 +1432,7 @@ void launch_vdiff(const Dev &d, cudaStream_t s) {
 int energy_parts() { return kRedGrid; }
 void launch_energy(const Dev &d, double *part, double *out, cudaStream_t s) {
     launch_k(k_energy_part, kRedGrid, kRedBlock, 0, s, d, part);
-    launch_k(k_energy_final, 1, 32, 0, s, part, kRedGrid, out);
+    launch_k(k_energy_final, 1, kRedBlock, 0, s, part, kRedGrid, out);
 }
 
 
