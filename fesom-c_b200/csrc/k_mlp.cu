@@ -1,6 +1,6 @@
 // Learned vertical-mixing closure, the network side: FP32 training on the
 // GPU with hand-written kernels (tiled SGEMM with fused bias / SiLU / SiLU'
-// epilogues, squared-error loss, bias-gradient column sums, Adam), the FP32
+// epilogues, split weight and bias gradients, squared-error loss, Adam), the FP32
 // forward pass, and the training-set statistics (normalisation and the
 // envelope the plain closure takes over outside of).  No counterpart in the
 // reference; the network stands in for d3_end (src/fv_mixing.F90:73-347).
@@ -24,67 +24,106 @@ __device__ __forceinline__ float silu_grad_f(float z) {
     return s * (1.0f + z * (1.0f - s));
 }
 
-enum { EPI_STORE = 0, EPI_BIAS = 1, EPI_BIAS_SILU = 2, EPI_SILU_GRAD = 3, EPI_SILU_ONLY = 4 };
+enum { EPI_PART = 0, EPI_BIAS = 1, EPI_BIAS_SILU = 2, EPI_SILU_GRAD = 3, EPI_SILU_ONLY = 4 };
 
 // C[M x N] = op(A)[M x K] op(B)[K x N]: A(m,k) = TA ? A[k*lda+m] : A[m*lda+k],
-// B(k,n) = TB ? B[n*ldb+k] : B[k*ldb+n].  64 x 64 tiles, 16-deep k slices in
-// shared memory, 4 x 4 outputs per thread, FP32 with explicit fused
-// multiply-adds.  Epilogues: store; + bias[n]; + bias[n] and SiLU (Z to C,
-// SiLU(Z) to C2); times SiLU'(Zin[m,n]).
+// B(k,n) = TB ? B[n*ldb+k] : B[k*ldb+n].  128 x 64 tiles, 16-deep k slices in
+// two shared-memory buffers (the next slice's loads are in flight while this
+// one is multiplied), 8 x 4 outputs per thread, FP32 with explicit fused
+// multiply-adds in k order.  Epilogues: store; + bias[n]; + bias[n] and SiLU
+// (Z to C, SiLU(Z) to C2); times SiLU'(Zin[m,n]); EPI_PART, the weight
+// gradients: blockIdx.z takes kSplit of the k range and stores its partial
+// product, and the column sums of A (the bias gradients) behind it, at C +
+// blockIdx.z * (M N + M).
+// Bound by the latency of the slices' loads at two blocks per SM.  8192 x 256
+// x 256: 45 us (64 x 64 tiles of 4 x 4, no load in flight: 50 us; 128 x 128
+// of 8 x 8: 49).  The weight gradients of 8192 samples, 23-40 us and 5 us to
+// sum their parts, took 585 us each without the split, 16 blocks working
+// 8192 deep, and their column sums 43 us in two more launches.  256 samples
+// a part: 256 blocks for a 256 x 256 gradient, and a shorter FP32 sum (error
+// of the gradients against 64 bits 1.2e-6 -> 1.3e-7).
+constexpr int kBM = 128, kBN = 64, kBK = 16;
+constexpr int kSplit = 256;
 template <bool TA, bool TB, int EPI>
 __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float *__restrict__ A, int lda,
                                               const float *__restrict__ B, int ldb, float *__restrict__ C, int ldc,
                                               const float *__restrict__ bias, float *__restrict__ C2,
                                               const float *__restrict__ Zin) {
-    __shared__ __align__(16) float As[16][68];
-    __shared__ __align__(16) float Bs[16][68];
+    __shared__ __align__(16) float As[2][kBK][kBM + 4];
+    __shared__ __align__(16) float Bs[2][kBK][kBN + 4];
     const int tid = threadIdx.x;
     const int tx = tid % 16, ty = tid / 16;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    float acc[4][4];
+    const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
+    const int k_lo = EPI == EPI_PART ? blockIdx.z * kSplit : 0;
+    const int k_hi = EPI == EPI_PART ? min(K, k_lo + kSplit) : K;
+    const bool sums = EPI == EPI_PART && blockIdx.x == 0 && tid < kBM;
+    float colsum = 0.0f;
+    float acc[8][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-    for (int k0 = 0; k0 < K; k0 += 16) {
+    float ra[8], rb[4];
+    auto fetch = [&](int k0) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < 8; ++r) {
             const int e = tid + r * 256;
-            int mm, kk;
-            if (TA) { mm = e % 64; kk = e / 64; }
-            else { kk = e % 16; mm = e / 16; }
+            const int mm = TA ? e % kBM : e / kBK, kk = TA ? e / kBM : e % kBK;
             const int gm = m0 + mm, gk = k0 + kk;
-            float v = 0.0f;
-            if (gm < M && gk < K) v = TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-            As[kk][mm] = v;
+            ra[r] = gm < M && gk < k_hi ? (TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk]) : 0.0f;
         }
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int e = tid + r * 256;
-            int nn, kk;
-            if (TB) { kk = e % 16; nn = e / 16; }
-            else { nn = e % 64; kk = e / 64; }
+            const int nn = TB ? e / kBK : e % kBN, kk = TB ? e % kBK : e / kBN;
             const int gn = n0 + nn, gk = k0 + kk;
-            float v = 0.0f;
-            if (gn < N && gk < K) v = TB ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn];
-            Bs[kk][nn] = v;
+            rb[r] = gn < N && gk < k_hi ? (TB ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn]) : 0.0f;
         }
-        __syncthreads();
+    };
+    auto stage = [&](int buf) {
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            const float4 a = *reinterpret_cast<const float4 *>(&As[kk][ty * 4]);
-            const float4 b = *reinterpret_cast<const float4 *>(&Bs[kk][tx * 4]);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+        for (int r = 0; r < 8; ++r) {
+            const int e = tid + r * 256;
+            As[buf][TA ? e / kBM : e % kBK][TA ? e % kBM : e / kBK] = ra[r];
+        }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+        for (int r = 0; r < 4; ++r) {
+            const int e = tid + r * 256;
+            Bs[buf][TB ? e % kBK : e / kBN][TB ? e / kBK : e % kBN] = rb[r];
+        }
+    };
+    fetch(k_lo);
+    stage(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = k_lo; k0 < k_hi; k0 += kBK, buf ^= 1) {
+        const bool more = k0 + kBK < k_hi;
+        if (more) fetch(k0 + kBK);
+        if (sums) {
+#pragma unroll
+            for (int kk = 0; kk < kBK; ++kk) colsum += As[buf][kk][tid];
+        }
+#pragma unroll
+        for (int kk = 0; kk < kBK; ++kk) {
+            const float4 a0 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 8]);
+            const float4 a1 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 8 + 4]);
+            const float4 b = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
+            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
         }
+        if (more) stage(buf ^ 1);
         __syncthreads();
     }
+    if (EPI == EPI_PART) {
+        C += (size_t)blockIdx.z * ((size_t)M * N + M);
+        if (sums && m0 + tid < M) C[(size_t)M * N + m0 + tid] = colsum;
+    }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gm = m0 + ty * 4 + i;
+    for (int i = 0; i < 8; ++i) {
+        const int gm = m0 + ty * 8 + i;
         if (gm >= M) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -104,8 +143,18 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float 
 template <bool TA, bool TB, int EPI>
 void sgemm(cudaStream_t s, int M, int N, int K, const float *A, int lda, const float *B, int ldb, float *C, int ldc,
            const float *bias = nullptr, float *C2 = nullptr, const float *Zin = nullptr) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
+    dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, EPI == EPI_PART ? (K + kSplit - 1) / kSplit : 1);
     k_sgemm<TA, TB, EPI><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, C2, Zin);
+}
+
+// the parts of a split product summed in k order: out[i] = sum_c part[c*n + i]
+__global__ void k_sum_parts(int nparts, int n, const float *part, float *out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        float s = 0.0f;
+#pragma unroll 8
+        for (int c = 0; c < nparts; ++c) s += part[(size_t)c * n + i];
+        out[i] = s;
+    }
 }
 
 // delta = 2 (Y - T) / (B OUT) and the sum of squared residuals
@@ -125,26 +174,6 @@ __global__ void k_mse_delta(long long n, const float *Y, const float *T, float *
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
         atomicAdd(loss, t);
     }
-}
-
-// column sums of D[B x N] in row chunks (deterministic: partials, then an
-// ordered sum over the chunks)
-constexpr int kColChunk = 512;
-__global__ void k_colsum_part(int B, int N, const float *D, float *part) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
-    if (n >= N) return;
-    const int r0 = c * kColChunk, r1 = min(B, r0 + kColChunk);
-    float s = 0.0f;
-    for (int r = r0; r < r1; ++r) s += D[(size_t)r * N + n];
-    part[(size_t)c * N + n] = s;
-}
-__global__ void k_colsum_final(int nchunk, int N, const float *part, float *out) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.0f;
-    for (int c = 0; c < nchunk; ++c) s += part[(size_t)c * N + n];
-    out[n] = s;
 }
 
 __global__ void k_adam(long long n, float *p, const float *g, float *m, float *v, float lr, float c1, float c2) {
@@ -254,7 +283,7 @@ LcNet *lc_create(int NS, long long hcap, unsigned long long seed, int Bmax, cuda
         (r = lc_alloc(n, &n->mom, n->np)) || (r = lc_alloc(n, &n->var, n->np)) ||
         (r = lc_alloc(n, &n->stats, kLcStatRows * (size_t)std::max(n->IN, n->OUT))) || (r = lc_alloc(n, &n->dloss, 2)) ||
         (r = lc_alloc(n, &n->Xb, (size_t)Bmax * n->IN)) || (r = lc_alloc(n, &n->Tb, (size_t)Bmax * n->OUT)) ||
-        (r = lc_alloc(n, &n->part, (size_t)((Bmax + kColChunk - 1) / kColChunk) * kLcHidden)) ||
+        (r = lc_alloc(n, &n->part, (size_t)((Bmax + kSplit - 1) / kSplit) * (kLcHidden * kLcHidden + kLcHidden))) ||
         (r = lc_alloc(n, &n->hcount, 1)) || (hcap > 0 && ((r = lc_alloc(n, &n->hx, (size_t)hcap * n->IN)) ||
                                                           (r = lc_alloc(n, &n->hy, (size_t)hcap * n->OUT))))) {
         *rc = r;
@@ -348,16 +377,15 @@ static void grad_batch(LcNet *n, const float *X, const float *T, int B) {
     const long long ny = (long long)B * OUT;
     float *D = n->Dl[3];
     k_mse_delta<<<grid_of(ny, 256), 256, 0, s>>>(ny, Y, T, D, 1.0f / (float)ny, n->dloss);
-    const int nchunk = (B + kColChunk - 1) / kColChunk;
+    const int nparts = (B + kSplit - 1) / kSplit;
     for (int l = 3; l >= 0; --l) {
         const int ni = n->dims[l], no = n->dims[l + 1];
         const float *ain = (l == 0) ? X : n->A[l - 1];
-        float *gW = n->grads + n->off[l], *gb = gW + (long long)no * ni;
-        // gW = D^T A_in   (no x ni), gb = column sums of D
-        sgemm<true, false, EPI_STORE>(s, no, ni, B, D, no, ain, ni, gW, ni);
-        dim3 g((no + 255) / 256, nchunk);
-        k_colsum_part<<<g, 256, 0, s>>>(B, no, D, n->part);
-        k_colsum_final<<<(no + 255) / 256, 256, 0, s>>>(nchunk, no, n->part, gb);
+        // gW = D^T A_in (no x ni) and, behind it, gb = column sums of D
+        const int np = no * ni + no;
+        float *g = n->grads + n->off[l];
+        sgemm<true, false, EPI_PART>(s, no, ni, B, D, no, ain, ni, nparts > 1 ? n->part : g, ni);
+        if (nparts > 1) k_sum_parts<<<(np + 255) / 256, 256, 0, s>>>(nparts, np, n->part, g);
         if (l > 0) {
             // D_prev = (D W) * SiLU'(Z_{l-1})
             float *Dp = n->Dl[l - 1];
