@@ -896,136 +896,183 @@ __global__ void k_wvel(Dev d) {
 }
 
 // ---- momentum_vert_impl_visc_tmp on tiles of element columns --------------
-// (launch-shape knob "implvisc_form" 2, the default for 10 and 20 layers):
-// a block takes kIvCols consecutive elements, whose columns are one
-// contiguous range of U_rhs, V_rhs, Je and Av, stages them in shared memory
-// with coalesced loads (kIvBatch per thread in flight), solves each column
-// with one thread from shared memory (odd row strides: no bank conflicts),
-// the recurrences in registers (LC layers fixed at compile time), writes the
-// result over the staged U_rhs / V_rhs and stores it coalesced.  The
-// arithmetic and its order are k_implvisc's im_vert_visc_fic branch.
-constexpr int kIvCols = 64;
+// (fv_viscosity.F90:1374-1486, no ice.)  A block takes kIvCols consecutive
+// elements, whose columns are one contiguous range of U_rhs, V_rhs, Je and
+// Av.  All threads, one (element, layer) each: the staging, the coefficients a
+// and c with their three divisions, and at the end the masked result.  One thread per column, all of one warp, runs the
+// elimination (three divisions per layer, in parallel) and the back
+// substitution from shared memory, [array][layer][column] with an odd column
+// stride: free of bank conflicts both over the columns of a layer and over
+// the layers of a column.  c, U and V are overwritten by xx1, yu and yv, then
+// by the solution.
+// Bound by latency (the chains, the staged loads).  FP64 stages Je and Av
+// too (4 loads of each field in flight per thread); FP32 reads them from
+// global memory where they are used, for half the shared memory and more
+// blocks.  Against tiles of 64 columns solved from row-major tiles
+// with all three divisions of a and c in the chain (10 and 20 layers only)
+// and one thread per column reading global memory (other layer counts): 4.5
+// k nodes, 39 layers 0.033 -> 0.025 ms, 697, 10: 0.015 -> 0.013, 232 k, 20:
+// 0.165 -> 0.150, 1.05 M: 0.62 as before, 232 k FP32: 0.064 -> 0.060.
+constexpr int kIvCols = 32;
+constexpr int kIvThreads = 128;
 constexpr int kIvBatch = 4;
-__host__ __device__ __forceinline__ int iv_odd(int x) { return x | 1; }
 
-template <int LC>
-__global__ void __launch_bounds__(kIvCols) k_implvisc_fic_tile(Dev d) {
+__global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char iv_smem[];
-    constexpr int L = LC, LP = LC | 1;
-    const int NS = d.NS, KP = iv_odd(d.NS), E = d.E;
-    real *sU = reinterpret_cast<real *>(iv_smem);   // row j: element e0 + j
-    real *sV = sU + kIvCols * LP;
-    real *sJ = sV + kIvCols * LP;
-    real *sA = sJ + kIvCols * LP;                   // Av, stride KP
+    constexpr int CP = kIvCols + 1;
+    const int L = d.L, NS = d.NS, E = d.E;
+    const int A = L * CP;
+    real *const sa = reinterpret_cast<real *>(iv_smem);   // layer z of column j at [z * CP + j]
+    real *const sc = sa + A, *const sU = sa + 2 * A, *const sV = sa + 3 * A;
+#if !FESOMC_FP32
+    real *const sJ = sa + 4 * A, *const sA = sa + 5 * A;  // sA: NS rows
+#endif
     const real dt = d.dt;
-    for (long long e0 = (long long)blockIdx.x * kIvCols; e0 < E; e0 += (long long)gridDim.x * kIvCols) {
-        const int nt = (int)(E - e0 < kIvCols ? E - e0 : kIvCols);
-        for (int i0 = threadIdx.x; i0 < nt * NS; i0 += kIvBatch * kIvCols) {
-            real av[kIvBatch];
-#pragma unroll
-            for (int u = 0; u < kIvBatch; ++u) {
-                const int i = i0 + u * kIvCols;
-                av[u] = i < nt * NS ? d.Av[(size_t)e0 * NS + i] : real(0.0);
-            }
-#pragma unroll
-            for (int u = 0; u < kIvBatch; ++u) {
-                const int i = i0 + u * kIvCols, j = d.by_NS.div(i);
-                if (i < nt * NS) sA[j * KP + (i - j * NS)] = av[u];
-            }
-        }
-        for (int i0 = threadIdx.x; i0 < nt * L; i0 += kIvBatch * kIvCols) {
-            real ur[kIvBatch], vr[kIvBatch], jv[kIvBatch];
-#pragma unroll
-            for (int u = 0; u < kIvBatch; ++u) {
-                const int i = i0 + u * kIvCols;
-                const size_t g = (size_t)e0 * L + (i < nt * L ? i : 0);
-                ur[u] = d.U_rhs[g];
-                vr[u] = d.V_rhs[g];
-                jv[u] = d.Je[g];
-            }
-#pragma unroll
-            for (int u = 0; u < kIvBatch; ++u) {
-                const int i = i0 + u * kIvCols;
-                if (i >= nt * L) continue;
-                const int j = i / L, z = i - j * L;
-                sU[j * LP + z] = ur[u];
-                sV[j * LP + z] = vr[u];
-                sJ[j * LP + z] = jv[u];
-            }
+    // the warps of the recurrences alternate between the blocks of an SM
+    constexpr int kChains = kIvCols / 32, kWarps = kIvThreads / 32;
+    const int warp = (int)(threadIdx.x / 32 + kChains * (blockIdx.x / 148)) % kWarps;
+    const bool mine = warp < kChains;
+    const int lane = warp * 32 + (threadIdx.x & 31);   // column of a recurrence
+    for (int e0 = blockIdx.x * kIvCols; e0 < E; e0 += gridDim.x * kIvCols) {
+        const int nt = E - e0 < kIvCols ? E - e0 : kIvCols;
+#if FESOMC_FP32
+        for (int i = threadIdx.x; i < nt * L; i += kIvThreads) {
+            const int j = d.by_L.div(i), z = i - j * L, o = z * CP + j;
+            const size_t g = (size_t)e0 * L + i, ga = g + e0 + j;
+            const real jz = d.Je[g];
+            const real d1 = (z == 0) ? real(0.5) * jz : real(0.5) * (jz + d.Je[g - 1]);
+            const real d2 = (z == L - 1) ? real(0.5) * jz : real(0.5) * (jz + d.Je[g + 1]);
+            const real zt = dt / jz;
+            sa[o] = zt * d.Av[ga] / d1;
+            sc[o] = zt * d.Av[ga + 1] / d2;
+            sU[o] = d.U_rhs[g];
+            sV[o] = d.V_rhs[g];
         }
         __syncthreads();
-        if ((int)threadIdx.x < nt) {
-            const int j = threadIdx.x, e = (int)e0 + j;
-            real *U = sU + j * LP, *V = sV + j * LP;
-            const real *J = sJ + j * LP, *A = sA + j * KP;
+#else
+        // kIvBatch items per thread loaded before any is used
+        for (int i0 = threadIdx.x; i0 < nt * L; i0 += kIvBatch * kIvThreads) {
+            real ur[kIvBatch], vr[kIvBatch], jz[kIvBatch], av[kIvBatch];
+#pragma unroll
+            for (int u = 0; u < kIvBatch; ++u) {
+                const int i = i0 + u * kIvThreads < nt * L ? i0 + u * kIvThreads : i0;
+                const int j = d.by_L.div(i);
+                const size_t g = (size_t)e0 * L + i;
+                ur[u] = d.U_rhs[g];
+                vr[u] = d.V_rhs[g];
+                jz[u] = d.Je[g];
+                av[u] = d.Av[g + e0 + j];
+            }
+#pragma unroll
+            for (int u = 0; u < kIvBatch; ++u) {
+                const int i = i0 + u * kIvThreads;
+                if (i >= nt * L) break;
+                const int j = d.by_L.div(i), z = i - j * L, o = z * CP + j;
+                sU[o] = ur[u];
+                sV[o] = vr[u];
+                sJ[o] = jz[u];
+                sA[o] = av[u];
+            }
+        }
+        if ((int)threadIdx.x < nt) sA[L * CP + threadIdx.x] = d.Av[(size_t)(e0 + threadIdx.x) * NS + L];
+        __syncthreads();
+        for (int i = threadIdx.x; i < nt * L; i += kIvThreads) {
+            const int j = d.by_L.div(i), z = i - j * L, o = z * CP + j;
+            const real jz = sJ[o];
+            const real d1 = (z == 0) ? real(0.5) * jz : real(0.5) * (jz + sJ[o - CP]);
+            const real d2 = (z == L - 1) ? real(0.5) * jz : real(0.5) * (jz + sJ[o + CP]);
+            const real zt = dt / jz;
+            sa[o] = zt * sA[o] / d1;
+            sc[o] = zt * sA[o + CP] / d2;
+        }
+        __syncthreads();
+#endif
+        if (mine && lane < nt) {
+            const int e = e0 + lane;
             const real mwd = d.mask_wd[e];
+            real *a_ = sa + lane, *x_ = sc + lane, *u_ = sU + lane, *v_ = sV + lane;
             if (mwd != real(0.0)) {
+#if FESOMC_FP32
+                const real *J = d.Je + (size_t)e * L, *Av = d.Av + (size_t)e * NS;
+                constexpr int R = 1;    // from one layer to the next
+#else
+                const real *J = sJ + lane, *Av = sA + lane;
+                constexpr int R = CP;
+#endif
                 const real ub = d.U_n[(size_t)e * L + L - 1], vb = d.V_n[(size_t)e * L + L - 1];
                 const real a_Cd = d.C_d * ((real(1.0) - d.elem_acc[e]) * d.Cd_bz + real(1.0));
-                real xx1[LC + 1], yu[LC + 1], yv[LC + 1];
-                real de = J[0] / (A[0] + A[1]);
+                real de = J[0] / (Av[0] + Av[R]);
                 const real rw = de / d.density_0;
                 real xv = real(1.0), yuv = d.taux[e] * rw, yvv = d.tauy[e] * rw;
-                xx1[0] = xv;
-                yu[0] = yuv;
-                yv[0] = yvv;
-#pragma unroll
+                #if FESOMC_FP32
+                const real jb = J[L - 1], av0 = Av[NS - 1], av1 = Av[L - 1];   // loaded ahead of the sweep
+#endif
+                real an = a_[0], cn = x_[0], un = u_[0], vn = v_[0];
                 for (int z = 0; z < L; ++z) {
-                    const real jz = J[z];
-                    const real d1 = (z == 0) ? real(0.5) * jz : real(0.5) * (jz + J[z > 0 ? z - 1 : 0]);
-                    const real d2 = (z == L - 1) ? real(0.5) * jz : real(0.5) * (jz + J[z + 1 < L ? z + 1 : z]);
-                    const real zt = dt / jz;
-                    const real a = zt * A[z] / d1;
-                    const real c = zt * A[z + 1] / d2;
+                    const real a = an, c = cn, Fx = un, Fy = vn;
+                    const int zn = (z + 1 < L ? z + 1 : z) * CP;
+                    an = a_[zn]; cn = x_[zn]; un = u_[zn]; vn = v_[zn];
                     const real b = a + c + real(1.0);
                     const real dd = b - a * xv;
                     xv = c / dd;
-                    yuv = (a * yuv + U[z]) / dd;
-                    yvv = (a * yvv + V[z]) / dd;
-                    xx1[z + 1] = xv;
-                    yu[z + 1] = yuv;
-                    yv[z + 1] = yvv;
+                    yuv = (a * yuv + Fx) / dd;
+                    yvv = (a * yvv + Fy) / dd;
+                    x_[z * CP] = xv;
+                    u_[z * CP] = yuv;
+                    v_[z * CP] = yvv;
                 }
-                de = J[L - 1] / (A[NS - 1] + A[L - 1]);
+#if FESOMC_FP32
+                de = jb / (av0 + av1);
+#else
+                de = J[(L - 1) * R] / (Av[(NS - 1) * R] + Av[(L - 1) * R]);
+#endif
                 const real friction = de * a_Cd * sqrt(ub * ub + vb * vb);
                 real Ut, Vt;
                 if (d.fic_point == 0) { Ut = real(0.0); Vt = real(0.0); }
                 else if (d.fic_point == 1) {
-                    const real a = friction + real(1.0) - xx1[L];
-                    Ut = yu[L] / a; Vt = yv[L] / a;
+                    const real a = friction + real(1.0) - xv;
+                    Ut = yuv / a; Vt = yvv / a;
                 } else {
-                    const real a = real(1.0) / (real(1.0) - friction) - xx1[L];
-                    Ut = yu[L] / a; Vt = yv[L] / a;
+                    const real a = real(1.0) / (real(1.0) - friction) - xv;
+                    Ut = yuv / a; Vt = yvv / a;
                 }
-#pragma unroll
                 for (int z = L - 1; z >= 0; --z) {
-                    Ut = Ut * xx1[z + 1] + yu[z + 1];
-                    Vt = Vt * xx1[z + 1] + yv[z + 1];
-                    U[z] = Ut * mwd;
-                    V[z] = Vt * mwd;
+                    const real x = x_[z * CP];
+                    Ut = Ut * x + u_[z * CP];
+                    Vt = Vt * x + v_[z * CP];
+                    u_[z * CP] = Ut * mwd;
+                    v_[z * CP] = Vt * mwd;
                 }
             } else {
-#pragma unroll
-                for (int z = 0; z < L; ++z) { U[z] = real(0.0); V[z] = real(0.0); }
+                for (int z = 0; z < L; ++z) { u_[z * CP] = real(0.0); v_[z * CP] = real(0.0); }
             }
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < nt * L; i += kIvCols) {
-            const int j = i / L, z = i - j * L;
+        for (int i = threadIdx.x; i < nt * L; i += kIvThreads) {
+            const int j = d.by_L.div(i), z = i - j * L;
             const size_t g = (size_t)e0 * L + i;
-            d.U_rhs[g] = sU[j * LP + z];
-            d.V_rhs[g] = sV[j * LP + z];
+            d.U_rhs[g] = sU[z * CP + j];
+            d.V_rhs[g] = sV[z * CP + j];
         }
         __syncthreads();
     }
 }
-static size_t implvisc_tile_smem(const Dev &d) {
-    return (size_t)kIvCols * (3 * iv_odd(d.L) + iv_odd(d.NS)) * sizeof(real);
-}
-// the tiled form: the fic variant alone, 10 or 20 layers
+static size_t implvisc_tile_smem(const Dev &d) { return (FESOMC_FP32 ? (size_t)4 * d.L : (size_t)6 * d.L + 1) * (kIvCols + 1) * sizeof(real); }
+// The tiles do the fic variant alone.  Between one and four full waves of
+// them the last, partly empty wave costs more than they gain over one thread
+// per column, whose blocks are all resident at once (42 k nodes, 20 layers,
+// 1.7 waves: 0.040 against 0.034 ms; 40 k, 30 layers, 2.7: 0.064 / 0.048; 16
+// k, 30 layers, 1.1: 0.041 / 0.035); with one wave or many they win (16 k, 20
+// layers: 0.021 / 0.025; 232 k: 0.148 / 0.184).  FP32 always takes the tiles:
+// the two forms' contracted arithmetic would not give the same bits.
 static bool implvisc_tiled(const Dev &d) {
-    return d.tune[TK_IMPLVISC] != 1 && !d.im_vert_visc && d.im_vert_visc_fic && (d.L == 10 || d.L == 20);
+    if (d.im_vert_visc || !d.im_vert_visc_fic) return false;
+    if (FESOMC_FP32) return true;
+    if (d.tune[TK_IMPLVISC] == 1) return false;
+    const long long per_sm = 227 * 1024 / (long long)(implvisc_tile_smem(d) + 1024);
+    const long long wave = 148 * (per_sm < 7 ? per_sm : 7) * kIvCols;   // 7: its registers
+    return d.E <= wave || d.E >= 4 * wave;
 }
 
 // ---- launch wrappers --------------------------------------------------------
@@ -1046,8 +1093,7 @@ static size_t col_smem(const Dev &d, int rows, int scalars) {
 int config_columns(const Dev &d) {
     const size_t big = col_smem(d, 2, kU3Sc);
     cudaError_t e = cudaSuccess;
-    if (d.L == 10) e = raise_smem_limit(k_implvisc_fic_tile<10>, implvisc_tile_smem(d));
-    if (d.L == 20) e = raise_smem_limit(k_implvisc_fic_tile<20>, implvisc_tile_smem(d));
+    e = raise_smem_limit(k_implvisc_fic_tile, implvisc_tile_smem(d));
     if (e == cudaSuccess) e = raise_smem_limit(k_bpg_elem, big);
     if (e == cudaSuccess) e = raise_smem_limit(k_update3d, big);
     if (e == cudaSuccess) e = raise_smem_limit(k_pressure_col, big);
@@ -1098,10 +1144,8 @@ void launch_velrhs(const Dev &d, real ff, cudaStream_t s) {
     } while (0)
 void launch_implvisc(const Dev &d, cudaStream_t s) {
     if (implvisc_tiled(d)) {
-        const long long tiles = ((long long)d.E + kIvCols - 1) / kIvCols;
-        const int g = (int)(tiles < (1LL << 30) ? tiles : (1LL << 30));
-        if (d.L == 10) launch_k(k_implvisc_fic_tile<10>, g, kIvCols, implvisc_tile_smem(d), s, d);
-        else launch_k(k_implvisc_fic_tile<20>, g, kIvCols, implvisc_tile_smem(d), s, d);
+        const int tiles = (d.E + kIvCols - 1) / kIvCols;
+        launch_k(k_implvisc_fic_tile, tiles, kIvThreads, implvisc_tile_smem(d), s, d);
         return;
     }
     MAXL_DISPATCH(k_implvisc, grid_for(d.E, 128), 128, s, d);

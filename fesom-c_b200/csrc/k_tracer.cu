@@ -786,7 +786,7 @@ __global__ void __launch_bounds__(128, 8) k_miura_h(Dev d) {
 // Tracer after advection and the river source, minus its mean: T(k) / S(k)
 // of tracer_impl_vert_diff.  The river source (fv_main.F90:1804-1823) adds
 // its terms to S in river-list order.
-// S: SF_adv of (n, z); Sn: Sold_new of (n, z), read only at river nodes
+// S: SF_adv of (n, z); Sn: Sold_new of (n, z)
 __device__ __forceinline__ real vd_salt_of(const Dev &d, int n, int z, real aj, real S, real Sn, real S_aver) {
     if (d.key_rivers) {
         for (int p = d.node_rptr[n]; p < d.node_rptr[n + 1]; ++p) {
@@ -798,38 +798,26 @@ __device__ __forceinline__ real vd_salt_of(const Dev &d, int n, int z, real aj, 
     }
     return S - S_aver;
 }
-__device__ __forceinline__ real vd_salt(const Dev &d, int n, size_t base, int z, real aj, real S_aver) {
-    const bool river = d.key_rivers && d.node_rptr[n] < d.node_rptr[n + 1];
-    return vd_salt_of(d, n, z, aj, d.SF_adv[base + z], river ? d.Sold_new[base + z] : real(0.0), S_aver);
-}
-
-// Tridiagonal coefficients a(k), b(k), c(k) of layer k (0-based) of node
-// column n (fv_tracer.F90:1380-1420).
-__device__ __forceinline__ void vd_coef(const Dev &d, const real *Kv, real aj, int k, real &a, real &b,
-                                        real &c) {
+// Tridiagonal coefficients a(k), c(k) of layer k (0-based) of a node column
+// (fv_tracer.F90:1380-1420) from Kv(k+1) of the layer (the reference takes the
+// same one for both sides; the top layer's is the interface below); b(k) = -a
+// - c + 1 with the absent one left out.
+__device__ __forceinline__ void vd_coef(const Dev &d, real kv, real aj, int k, real &a, real &c) {
     const int L = d.L, NS = d.NS;
     const real dt = d.dt;
     auto Zc = [&](int m) { return z_of(d, aj, m); };
     auto ZBc = [&](int m) { return zbar_of(d, aj, m); };
+    a = c = real(0.0);
     if (k == 0) {
-        c = -dt * Kv[1] / ((Zc(0) - Zc(1)) * (ZBc(0) - ZBc(1)));
-        a = real(0.0);
-        b = -c + real(1.0);
+        c = -dt * kv / ((Zc(0) - Zc(1)) * (ZBc(0) - ZBc(1)));
     } else if (k == L - 1) {
-        a = -dt * Kv[L - 1] / ((Zc(L - 2) - Zc(L - 1)) * (ZBc(L - 1) - ZBc(NS - 1)));
-        b = -a + real(1.0);
-        c = real(0.0);
+        a = -dt * kv / ((Zc(L - 2) - Zc(L - 1)) * (ZBc(L - 1) - ZBc(NS - 1)));
     } else {
-        a = -dt * Kv[k] / ((Zc(k - 1) - Zc(k)) * (ZBc(k) - ZBc(k + 1)));
-        c = -dt * Kv[k] / ((Zc(k) - Zc(k + 1)) * (ZBc(k) - ZBc(k + 1)));
-        b = -a - c + real(1.0);
+        a = -dt * kv / ((Zc(k - 1) - Zc(k)) * (ZBc(k) - ZBc(k + 1)));
+        c = -dt * kv / ((Zc(k) - Zc(k + 1)) * (ZBc(k) - ZBc(k + 1)));
     }
 }
 
-// rivers + tracer_impl_vert_diff (fv_tracer.F90:1319-1494), one thread per
-// node column.  The sweep coefficients live in shared memory
-// ([array][level][thread]); T and S are re-read instead of stored.
-constexpr int kVdBlock = 128;
 // ---- atmospheric forcing of the column solve (key_atm) -------------------
 // sw_cp (fv_tracer.F90:1775-1908): heat capacity of sea water, UNESCO 1983
 // polynomial; literals without _WP in the Fortran are REAL(4) (R4).
@@ -921,91 +909,6 @@ __device__ real evap_precip(const Dev &d, int n, real aj, real T0, real S0, real
         if (S <= real(0.2) && frw < real(0.0)) frw = real(0.0);
     }
     return frw;
-}
-
-// kAtm: the atmospheric sources (key_atm) compiled in; the plain kernel keeps
-// its register count without them
-template <bool kAtm>
-__global__ void __launch_bounds__(kVdBlock) k_vdiff_col(Dev d) {
-    pdl_enter();
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-    real *sm = reinterpret_cast<real *>(sm_raw);
-    const int L = d.L, NS = d.NS;
-    real *col = sm + threadIdx.x;
-    const int bd = blockDim.x;
-    auto CP = [&](int k) -> real & { return col[((size_t)0 * L + k) * bd]; };
-    auto TP = [&](int k) -> real & { return col[((size_t)1 * L + k) * bd]; };
-    auto SP = [&](int k) -> real & { return col[((size_t)2 * L + k) * bd]; };
-    GRID_LOOP(ii, d.N) {
-        const int n = (int)ii;
-        const real T_aver = t_aver_of(d, n), S_aver = s_aver_of(d, n);
-        const size_t base = (size_t)n * L;
-        const real aj = jac_a(d, d.eta_jac, n);
-        const real *Kv = d.Kv + (size_t)n * NS;
-        auto Tz = [&](int z) { return d.TF_adv[base + z] - T_aver; };
-        auto Sz = [&](int z) { return vd_salt(d, n, base, z, aj, S_aver); };
-        // forward elimination; the right-hand side of layer k uses T(k-1..k+1)
-        real Tm = real(0.0), T0 = Tz(0), Tp = Tz(1);
-        real Sm = real(0.0), S0 = Sz(0), Sp = Sz(1);
-        real cpv = real(0.0), tpv = real(0.0), spv = real(0.0);  // the recurrences, in registers
-        // surface sources on wet nodes with atmospheric forcing (fv_tracer.F90:1376,1396-1418)
-        const bool atm = kAtm && d.mask_wd_node[n] != real(0.0);
-        const real frw = atm ? evap_precip(d, n, aj, T0, S0, T_aver, S_aver) : real(0.0);
-        for (int k = 0; k < L; ++k) {
-            real a, b, c, tr, sr;
-            vd_coef(d, Kv, aj, k, a, b, c);
-            if (k == 0) {
-                tr = c * (-Tp + T0);
-                sr = c * (-Sp + S0);
-            } else if (k == L - 1) {
-                tr = a * (T0 - Tm);
-                sr = a * (S0 - Sm);
-            } else {
-                tr = -a * Tm - c * Tp + (a + c) * T0;
-                sr = -a * Sm - c * Sp + (a + c) * S0;
-            }
-            if (atm) {
-                tr = tr + d.dt * heat_source(d, n, base, k, aj, T_aver, S_aver);
-                if (k == 0) sr = sr + d.dt * frw;
-            }
-            if (k == 0) {
-                cpv = c / b;
-                tpv = tr / b;
-                spv = sr / b;
-            } else {
-                const real m = real(1.0) / (b - cpv * a);
-                cpv = c * m;
-                tpv = (tr - tpv * a) * m;
-                spv = (sr - spv * a) * m;
-            }
-            CP(k) = cpv;
-            TP(k) = tpv;
-            SP(k) = spv;
-            Tm = T0; T0 = Tp;
-            Sm = S0; S0 = Sp;
-            if (k + 2 < L) { Tp = Tz(k + 2); Sp = Sz(k + 2); }
-        }
-        // back substitution and update, bottom to top
-        unsigned int st = 0;
-        real tr = real(0.0), sr = real(0.0);
-        for (int z = L - 1; z >= 0; --z) {
-            if (z == L - 1) { tr = TP(z); sr = SP(z); }
-            else { tr = TP(z) - CP(z) * tr; sr = SP(z) - CP(z) * sr; }
-            const size_t i = base + z;
-            real t = Tz(z) + tr + T_aver;
-            real s = Sz(z) + sr + S_aver;
-            if (fabs(s) < real(1.0e-12)) s = fabs(s);
-            if (s < real(0.0)) st |= 0x1u;
-            if (t < -real(3.0)) st |= 0x2u;
-            if (!isfinite(t) || !isfinite(s)) st |= 0x4u;
-            d.TF[i] = t;
-            d.SF[i] = s;
-            d.T_old[i] = d.Told_new[i];
-            d.S_old[i] = d.Sold_new[i];
-        }
-        if (!isfinite(d.eta_n[n])) st |= 0x4u;
-        if (st) atomicOr(d.status, st);
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1238,57 +1141,203 @@ void launch_muscl_h(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_MH, 128);
     launch_k(k_muscl_h, grid_for((long long)d.N * d.L, b), b, 0, s, d);
 }
-// ---- tracer_impl_vert_diff on tiles of columns (knob vdiff_form = 2) -------
-// k_vdiff_col reads each column with one thread, so a warp's loads of one
-// layer touch 32 rows L values apart.  Here a block takes kVtCols (128 or
-// 64)
-// consecutive nodes, whose columns are one contiguous range of every
-// [node][layer] field: it stages T - T_aver, the river-adjusted S - S_aver
-// and Kv in shared memory with coalesced loads (copying Told_new / Sold_new
-// to T_old / S_old on the way; each thread loads a batch of items before
-// storing any), solves each column with one thread from
-// shared memory (rows of odd stride: no bank conflicts) with the sweep's
-// recurrences in registers (the layer count LC is fixed at compile time),
-// writes the new tracers over the staged ones and stores them coalesced.
-// The arithmetic and its order are k_vdiff_col's.
-constexpr int kVtBatch = 4;
-__host__ __device__ __forceinline__ int vd_odd(int x) { return x | 1; }
+// ---- tracer_impl_vert_diff on tiles of columns ------------------------------
+// rivers + tracer_impl_vert_diff (fv_tracer.F90:1319-1494).  A block takes
+// kVtCols consecutive nodes, whose columns are one contiguous range of every
+// [node][layer] field.  All threads, one (node, layer) each: the staging
+// (T - T_aver, the river-adjusted S - S_aver; Told_new / Sold_new copied to
+// T_old / S_old on the way), then the coefficients with their two divisions,
+// the right-hand sides and the heat source (four exponentials and a seawater
+// heat capacity polynomial per layer with atmospheric forcing), and at the
+// end the update, its checks and the coalesced stores.  One thread per column,
+// all of one warp, runs the elimination (one division per layer) and the back
+// substitution from shared memory, [array][layer][column] with an odd column
+// stride: free of bank conflicts both over the columns of a layer and over
+// the layers of a column.  c, tr and sr are overwritten by the eliminated
+// ones.
+// Bound by latency (the chains, the staged loads).  Against one thread per
+// column with everything in its chain: 4.5 k nodes, 39 layers 0.076 -> 0.023
+// ms, 40 k nodes, 30 layers with atmospheric sources 0.305 -> 0.144 (the heat
+// source was formed in the column's thread); against 64-column tiles solved
+// in registers, 10 layers: 697 nodes 0.017 -> 0.013, 16 k 0.019 -> 0.015.
+constexpr int kVtCols = 32;
+constexpr int kVtThreads = 128;
+constexpr int kVtArrays = 6, kVtBatch = 4;
 
-template <bool kAtm, int LC, int kVtCols>
-__global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
+template <bool kAtm>
+__global__ void __launch_bounds__(kVtThreads) k_vdiff_tile(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char vt_smem[];
-    constexpr int L = LC, LP = LC | 1;
-    const int NS = d.NS, KP = vd_odd(d.NS), N = d.N;
+    __shared__ real s_aj[kVtCols], s_ta[kVtCols], s_sa[kVtCols];
+    __shared__ bool s_wet[kVtCols];
+    constexpr int CP = kVtCols + 1;
+    const int L = d.L, NS = d.NS, N = d.N;
+    const int A = L * CP;
+    real *const sT = reinterpret_cast<real *>(vt_smem);   // layer k of column j at [k * CP + j]
+    real *const sS = sT + A, *const sa = sT + 2 * A, *const sc = sT + 3 * A, *const st = sT + 4 * A, *const ss = sT + 5 * A;
+    // the warps of the recurrences alternate between the blocks of an SM
+    constexpr int kChains = kVtCols / 32, kWarps = kVtThreads / 32;
+    const int warp = (int)(threadIdx.x / 32 + kChains * (blockIdx.x / 148)) % kWarps;
+    const bool mine = warp < kChains;
+    const int lane = warp * 32 + (threadIdx.x & 31);   // column of a recurrence
+    for (int n0 = blockIdx.x * kVtCols; n0 < N; n0 += gridDim.x * kVtCols) {
+        const int nt = N - n0 < kVtCols ? N - n0 : kVtCols;
+        if ((int)threadIdx.x < nt) {
+            const int n = n0 + threadIdx.x;
+            s_aj[threadIdx.x] = jac_a(d, d.eta_jac, n);
+            s_ta[threadIdx.x] = t_aver_of(d, n);
+            s_sa[threadIdx.x] = s_aver_of(d, n);
+            s_wet[threadIdx.x] = kAtm && d.mask_wd_node[n] != real(0.0);
+        }
+        __syncthreads();
+        // kVtBatch items per thread loaded before any is used
+        for (int i0 = threadIdx.x; i0 < nt * L; i0 += kVtBatch * kVtThreads) {
+            real ta[kVtBatch], sl[kVtBatch], tn[kVtBatch], sn[kVtBatch], kv[kVtBatch];
+#pragma unroll
+            for (int u = 0; u < kVtBatch; ++u) {
+                const int i = i0 + u * kVtThreads < nt * L ? i0 + u * kVtThreads : i0;
+                const int j = d.by_L.div(i), k = i - j * L;
+                const size_t g = (size_t)n0 * L + i;
+                ta[u] = d.TF_adv[g];
+                sl[u] = d.SF_adv[g];
+                tn[u] = d.Told_new[g];
+                sn[u] = d.Sold_new[g];
+                kv[u] = d.Kv[(size_t)(n0 + j) * NS + (k == 0 ? 1 : k)];
+            }
+#pragma unroll
+            for (int u = 0; u < kVtBatch; ++u) {
+                const int i = i0 + u * kVtThreads;
+                if (i >= nt * L) break;
+                const int j = d.by_L.div(i), k = i - j * L;
+                const size_t g = (size_t)n0 * L + i;
+                const int o = k * CP + j;
+                sT[o] = ta[u] - s_ta[j];
+                sS[o] = vd_salt_of(d, n0 + j, k, s_aj[j], sl[u], sn[u], s_sa[j]);
+                sa[o] = kv[u];
+                d.T_old[g] = tn[u];
+                d.S_old[g] = sn[u];
+            }
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < nt * L; i += kVtThreads) {
+            const int j = d.by_L.div(i), k = i - j * L, n = n0 + j;
+            const int o = k * CP + j;
+            const real aj = s_aj[j];
+            real a, c, tr, sr;
+            vd_coef(d, sa[o], aj, k, a, c);
+            const real T0 = sT[o], S0 = sS[o];
+            if (k == 0) {
+                tr = c * (-sT[o + CP] + T0);
+                sr = c * (-sS[o + CP] + S0);
+            } else if (k == L - 1) {
+                tr = a * (T0 - sT[o - CP]);
+                sr = a * (S0 - sS[o - CP]);
+            } else {
+                tr = -a * sT[o - CP] - c * sT[o + CP] + (a + c) * T0;
+                sr = -a * sS[o - CP] - c * sS[o + CP] + (a + c) * S0;
+            }
+            // surface sources on wet nodes (fv_tracer.F90:1376,1396-1418)
+            if (kAtm && s_wet[j]) {
+                const real T_aver = s_ta[j], S_aver = s_sa[j];
+                tr = tr + d.dt * heat_source(d, n, (size_t)n * L, k, aj, T_aver, S_aver);
+                if (k == 0) sr = sr + d.dt * evap_precip(d, n, aj, T0, S0, T_aver, S_aver);
+            }
+            sa[o] = a;
+            sc[o] = c;
+            st[o] = tr;
+            ss[o] = sr;
+        }
+        __syncthreads();
+        if (mine && lane < nt) {
+            const real *a_ = sa + lane;
+            real *c_ = sc + lane, *t_ = st + lane, *s_ = ss + lane;
+            real cpv = real(0.0), tpv = real(0.0), spv = real(0.0);
+            real an = a_[0], cn = c_[0], tn = t_[0], sn = s_[0];
+            for (int k = 0; k < L; ++k) {
+                const real a = an, c = cn, tr = tn, sr = sn;
+                const int kn = (k + 1 < L ? k + 1 : k) * CP;
+                an = a_[kn]; cn = c_[kn]; tn = t_[kn]; sn = s_[kn];
+                if (k == 0) {
+                    const real b = -c + real(1.0);
+                    cpv = c / b;
+                    tpv = tr / b;
+                    spv = sr / b;
+                } else {
+                    const real b = k == L - 1 ? -a + real(1.0) : -a - c + real(1.0);
+                    const real m = real(1.0) / (b - cpv * a);
+                    cpv = c * m;
+                    tpv = (tr - tpv * a) * m;
+                    spv = (sr - spv * a) * m;
+                }
+                c_[k * CP] = cpv;
+                t_[k * CP] = tpv;
+                s_[k * CP] = spv;
+            }
+            real tr = tpv, sr = spv;
+            for (int k = L - 2; k >= 0; --k) {
+                const real cp = c_[k * CP];
+                tr = t_[k * CP] - cp * tr;
+                sr = s_[k * CP] - cp * sr;
+                t_[k * CP] = tr;
+                s_[k * CP] = sr;
+            }
+        }
+        __syncthreads();
+        unsigned int flags = 0;
+        for (int i = threadIdx.x; i < nt * L; i += kVtThreads) {
+            const int j = d.by_L.div(i), k = i - j * L, n = n0 + j;
+            const int o = k * CP + j;
+            const size_t g = (size_t)n0 * L + i;
+            const real t = sT[o] + st[o] + s_ta[j];
+            real s = sS[o] + ss[o] + s_sa[j];
+            if (fabs(s) < real(1.0e-12)) s = fabs(s);
+            if (s < real(0.0)) flags |= 0x1u;
+            if (t < -real(3.0)) flags |= 0x2u;
+            if (!isfinite(t) || !isfinite(s)) flags |= 0x4u;
+            if (k == 0 && !isfinite(d.eta_n[n])) flags |= 0x4u;
+            d.TF[g] = t;
+            d.SF[g] = s;
+        }
+        if (flags) atomicOr(d.status, flags);
+        __syncthreads();
+    }
+}
+// The same on tiles of 64 columns for 20 layers, fixed at compile time: one
+// thread per column solves with its recurrences in registers, from rows of
+// odd stride, and stages with batched loads.  Fewer shared-memory passes,
+// but only as many threads as columns, which pays on full-size grids.
+constexpr int kVrCols = 64;
+constexpr int kVrLayers = 20;
+__global__ void __launch_bounds__(kVrCols) k_vdiff_reg(Dev d) {
+    pdl_enter();
+    extern __shared__ __align__(16) unsigned char vt_smem[];
+    constexpr int L = kVrLayers, LP = L | 1;
+    const int NS = d.NS, KP = (d.NS | 1), N = d.N;
     real *sT = reinterpret_cast<real *>(vt_smem);  // row j: node n0 + j
-    real *sS = sT + kVtCols * LP;
-    real *sK = sS + kVtCols * LP;
-    // with the atmospheric sources: the heat source of every (node, layer),
-    // formed in the staging phase by all threads instead of in the serial
-    // column solve
-    real *sH = sK + kVtCols * KP;
-    for (long long n0 = (long long)blockIdx.x * kVtCols; n0 < N; n0 += (long long)gridDim.x * kVtCols) {
-        const int nt = (int)(N - n0 < kVtCols ? N - n0 : kVtCols);
+    real *sS = sT + kVrCols * LP;
+    real *sK = sS + kVrCols * LP;
+    for (long long n0 = (long long)blockIdx.x * kVrCols; n0 < N; n0 += (long long)gridDim.x * kVrCols) {
+        const int nt = (int)(N - n0 < kVrCols ? N - n0 : kVrCols);
         // staging: kVtBatch items per thread loaded before any is used, so
         // that each thread keeps several loads in flight
-        for (int i0 = threadIdx.x; i0 < nt * NS; i0 += kVtBatch * kVtCols) {
+        for (int i0 = threadIdx.x; i0 < nt * NS; i0 += kVtBatch * kVrCols) {
             real kv[kVtBatch];
 #pragma unroll
             for (int u = 0; u < kVtBatch; ++u) {
-                const int i = i0 + u * kVtCols;
+                const int i = i0 + u * kVrCols;
                 kv[u] = i < nt * NS ? d.Kv[(size_t)n0 * NS + i] : real(0.0);
             }
 #pragma unroll
             for (int u = 0; u < kVtBatch; ++u) {
-                const int i = i0 + u * kVtCols, j = d.by_NS.div(i);
+                const int i = i0 + u * kVrCols, j = d.by_NS.div(i);
                 if (i < nt * NS) sK[j * KP + (i - j * NS)] = kv[u];
             }
         }
-        for (int i0 = threadIdx.x; i0 < nt * L; i0 += kVtBatch * kVtCols) {
+        for (int i0 = threadIdx.x; i0 < nt * L; i0 += kVtBatch * kVrCols) {
             real ta[kVtBatch], sa[kVtBatch], tn[kVtBatch], sn[kVtBatch];
 #pragma unroll
             for (int u = 0; u < kVtBatch; ++u) {
-                const int i = i0 + u * kVtCols;
+                const int i = i0 + u * kVrCols;
                 const size_t g = (size_t)n0 * L + (i < nt * L ? i : 0);
                 ta[u] = d.TF_adv[g];
                 sa[u] = d.SF_adv[g];
@@ -1297,7 +1346,7 @@ __global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
             }
 #pragma unroll
             for (int u = 0; u < kVtBatch; ++u) {
-                const int i = i0 + u * kVtCols;
+                const int i = i0 + u * kVrCols;
                 if (i >= nt * L) continue;
                 const int j = i / L, z = i - j * L;
                 const int n = (int)n0 + j;
@@ -1305,10 +1354,6 @@ __global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
                 const real ajn = jac_a(d, d.eta_jac, n);
                 sT[j * LP + z] = ta[u] - t_aver_of(d, n);
                 sS[j * LP + z] = vd_salt_of(d, n, z, ajn, sa[u], sn[u], s_aver_of(d, n));
-                if (kAtm)
-                    sH[j * LP + z] = d.mask_wd_node[n] != real(0.0)
-                                         ? heat_source(d, n, (size_t)n * L, z, ajn, t_aver_of(d, n), s_aver_of(d, n))
-                                         : real(0.0);
                 d.T_old[g] = tn[u];
                 d.S_old[g] = sn[u];
             }
@@ -1317,18 +1362,16 @@ __global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
         if ((int)threadIdx.x < nt) {
             const int j = threadIdx.x, n = (int)n0 + j;
             const real T_aver = t_aver_of(d, n), S_aver = s_aver_of(d, n);
-            const size_t base = (size_t)n * L;
             const real aj = jac_a(d, d.eta_jac, n);
             const real *Kv = sK + j * KP;
             real *T = sT + j * LP, *S = sS + j * LP;
-            real CP[LC], TP[LC], SP[LC];
+            real CP[L], TP[L], SP[L];
             real cpv = real(0.0), tpv = real(0.0), spv = real(0.0);
-            const bool atm = kAtm && d.mask_wd_node[n] != real(0.0);
-            const real frw = atm ? evap_precip(d, n, aj, T[0], S[0], T_aver, S_aver) : real(0.0);
 #pragma unroll
             for (int k = 0; k < L; ++k) {
                 real a, b, c, tr, sr;
-                vd_coef(d, Kv, aj, k, a, b, c);
+                vd_coef(d, Kv[k == 0 ? 1 : k], aj, k, a, c);
+                b = k == 0 ? -c + real(1.0) : k == L - 1 ? -a + real(1.0) : -a - c + real(1.0);
                 const real T0 = T[k], S0 = S[k];
                 if (k == 0) {
                     tr = c * (-T[1] + T0);
@@ -1339,10 +1382,6 @@ __global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
                 } else {
                     tr = -a * T[k - 1] - c * T[k + 1] + (a + c) * T0;
                     sr = -a * S[k - 1] - c * S[k + 1] + (a + c) * S0;
-                }
-                if (atm) {
-                    tr = tr + d.dt * sH[j * LP + k];
-                    if (k == 0) sr = sr + d.dt * frw;
                 }
                 if (k == 0) {
                     cpv = c / b;
@@ -1377,7 +1416,7 @@ __global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
             if (st) atomicOr(d.status, st);
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < nt * L; i += kVtCols) {
+        for (int i = threadIdx.x; i < nt * L; i += kVrCols) {
             const int j = i / L, z = i - j * L;
             const size_t g = (size_t)n0 * L + i;
             d.TF[g] = sT[j * LP + z];
@@ -1387,47 +1426,30 @@ __global__ void __launch_bounds__(kVtCols) k_vdiff_tile(Dev d) {
     }
 }
 
-// columns per tile: 128 (vdiff_form 2) or 64 (3, the default)
-static int vdiff_cols(const Dev &d) { return d.tune[TK_VDIFF] == 2 ? 128 : 64; }
-static size_t vdiff_tile_smem(const Dev &d, int cols, bool atm) {
-    return (size_t)cols * ((atm ? 3 : 2) * vd_odd(d.L) + vd_odd(d.NS)) * sizeof(real);
+static size_t vdiff_smem(const Dev &d) { return (size_t)kVtArrays * d.L * (kVtCols + 1) * sizeof(real); }
+static size_t vdiff_reg_smem(const Dev &d) {
+    return (size_t)kVrCols * (2 * (d.L | 1) + (d.NS | 1)) * sizeof(real);
 }
-// the tiled form is compiled for 10 and 20 layers (11 and 21 sigma levels)
-static bool vdiff_tiled(const Dev &d) { return d.tune[TK_VDIFF] != 1 && (d.L == 10 || d.L == 20); }
-
-static int vdiff_block(const Dev &d) { return d.L <= 48 ? kVdBlock : 32; }
-static size_t vdiff_smem(const Dev &d) { return (size_t)3 * d.L * vdiff_block(d) * sizeof(real); }
-template <int LC, int C>
-static bool config_vdiff_tile(const Dev &d) {
-    return raise_smem_limit(k_vdiff_tile<false, LC, C>, vdiff_tile_smem(d, C, false)) == cudaSuccess &&
-           raise_smem_limit(k_vdiff_tile<true, LC, C>, vdiff_tile_smem(d, C, true)) == cudaSuccess;
+// 20 layers without atmospheric sources, from four tiles of 64 per SM on: 42 k
+// nodes 0.033 ms against 0.037, 1.05 M 0.526 against 0.65, 232 k FP32 0.070
+// against 0.080; below, and with the sources, the level-parallel tiles: 16 k
+// nodes 0.021 against 0.029, with sources 40 k 0.080 against 0.114.
+static bool vdiff_reg(const Dev &d) {
+    return d.L == kVrLayers && !d.key_atm && d.N >= 4 * 148 * kVrCols;
 }
 int config_vdiff(const Dev &d) {
-    if (raise_smem_limit(k_vdiff_col<false>, vdiff_smem(d)) != cudaSuccess ||
-        raise_smem_limit(k_vdiff_col<true>, vdiff_smem(d)) != cudaSuccess)
-        return 1;
-    if (d.L == 10) return config_vdiff_tile<10, 128>(d) && config_vdiff_tile<10, 64>(d) ? 0 : 1;
-    if (d.L == 20) return config_vdiff_tile<20, 128>(d) && config_vdiff_tile<20, 64>(d) ? 0 : 1;
-    return 0;
-}
-template <int LC, int C>
-static void launch_vdiff_tile(const Dev &d, cudaStream_t s) {
-    const long long tiles = ((long long)d.N + C - 1) / C;
-    const int g = (int)(tiles < (1LL << 30) ? tiles : (1LL << 30));
-    if (d.key_atm) launch_k(k_vdiff_tile<true, LC, C>, g, C, vdiff_tile_smem(d, C, true), s, d);
-    else launch_k(k_vdiff_tile<false, LC, C>, g, C, vdiff_tile_smem(d, C, false), s, d);
+    const size_t sm = vdiff_smem(d);
+    bool ok = d.key_atm ? raise_smem_limit(k_vdiff_tile<true>, sm) == cudaSuccess
+                        : raise_smem_limit(k_vdiff_tile<false>, sm) == cudaSuccess;
+    if (vdiff_reg(d))
+        ok = ok && raise_smem_limit(k_vdiff_reg, vdiff_reg_smem(d)) == cudaSuccess;
+    return ok ? 0 : 1;
 }
 void launch_vdiff(const Dev &d, cudaStream_t s) {
-    if (vdiff_tiled(d)) {
-        const bool c64 = vdiff_cols(d) == 64;
-        if (d.L == 10 && c64) launch_vdiff_tile<10, 64>(d, s);
-        else if (d.L == 10) launch_vdiff_tile<10, 128>(d, s);
-        else if (c64) launch_vdiff_tile<20, 64>(d, s);
-        else launch_vdiff_tile<20, 128>(d, s);
-        return;
-    }
-    if (d.key_atm) launch_k(k_vdiff_col<true>, grid_for(d.N, vdiff_block(d)), vdiff_block(d), vdiff_smem(d), s, d);
-    else launch_k(k_vdiff_col<false>, grid_for(d.N, vdiff_block(d)), vdiff_block(d), vdiff_smem(d), s, d);
+    const int C = vdiff_reg(d) ? kVrCols : kVtCols, tiles = (d.N + C - 1) / C;
+    if (vdiff_reg(d)) launch_k(k_vdiff_reg, tiles, kVrCols, vdiff_reg_smem(d), s, d);
+    else if (d.key_atm) launch_k(k_vdiff_tile<true>, tiles, kVtThreads, vdiff_smem(d), s, d);
+    else launch_k(k_vdiff_tile<false>, tiles, kVtThreads, vdiff_smem(d), s, d);
 }
 int energy_parts() { return kRedGrid; }
 void launch_energy(const Dev &d, double *part, double *out, cudaStream_t s) {

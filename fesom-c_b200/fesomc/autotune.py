@@ -30,11 +30,10 @@ THREADS = (64, 128, 256, 512, 1024)
 COLUMNS = (1, 2, 4, 8, 16, 32)
 # d3_end: one thread per column, or tiles of columns in shared memory
 D3END_ARRAYS = (1, 2)
-# tracer_impl_vert_diff: columns read directly, or tiles of 128 or 64 columns
-# staged in shared memory
-VDIFF_FORMS = (1, 2, 3)
 # the knobs that pick a form rather than a block size
-# momentum_vert_impl_visc_tmp: columns read directly, or tiles of 64 columns
+# tracer_impl_vert_diff: one form under every number
+VDIFF_FORMS = (3,)
+# momentum_vert_impl_visc_tmp: columns read directly, or tiles of columns
 IMPLVISC_FORMS = (1, 2)
 FORMS = {"columns": COLUMNS, "d3end_arrays": D3END_ARRAYS, "vdiff_form": VDIFF_FORMS,
          "implvisc_form": IMPLVISC_FORMS}

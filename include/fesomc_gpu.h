@@ -456,12 +456,12 @@ int  fesomc_ensemble_run(fesomc_model *const *members, int32_t n_members, int32_
  * the same form under every number, so that saved shapes stay valid) on
  * tiles of columns in shared memory, the default up to 61 levels; the FP32
  * form takes the tiles under every number;
- * "vdiff_form" 1 to 3: the tracers' implicit vertical diffusion with each
- * column read directly by its thread, or on tiles of 128 or 64 (the
- * default) columns staged in shared memory, for 10 or 20 layers;
+ * "vdiff_form" 1 to 3, the same under every number: the tracers' implicit
+ * vertical diffusion runs on tiles of columns in shared memory;
  * "implvisc_form" 1 or 2: the implicit vertical viscosity with each element
- * column read directly, or on tiles of 64 columns staged in shared memory,
- * the default for the fic variant at 10 or 20 layers); the next step
+ * column read directly, or (the default) on tiles of columns in shared
+ * memory for the fic variant, where their number fills the device's waves
+ * well; the FP32 form takes the tiles under both numbers); the next step
  * captures its
  * graph again.  The search over the knobs and its cache per mesh size and
  * level count live with the host driver (fesomc/autotune.py).  No

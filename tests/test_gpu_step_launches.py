@@ -54,3 +54,16 @@ def test_sub_cycle_lengths(built, sub):
 def test_d3end_tiles(built, nx, ny, nsigma):
     from fesomc import cases
     _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib), 3)
+
+
+# the column solvers on tiles of 32 columns: the smallest and largest layer
+# counts, ragged last tiles, more layers than threads of a batch, and the
+# element counts around one wave of the viscosity's tiles at 30 layers
+# (148 SMs x 4 tiles x 32 = 18,944), with the river's salinity source and,
+# in the third variant, the atmospheric sources
+@pytest.mark.parametrize("nx,ny,nsigma,atm", [(9, 9, 5, False), (13, 11, 127, False), (25, 17, 33, True),
+                                              (160, 89, 31, False), (160, 92, 31, False), (60, 40, 21, False)])
+def test_column_solver_tiles(built, nx, ny, nsigma, atm):
+    from fesomc import cases
+    kw = {"atm": {"qns": -80.0, "qsr": 120.0, "emp": 1e-7, "mslp": 101000.0}} if atm else {}
+    _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib, **kw), 3)
