@@ -216,6 +216,7 @@ int grid_for(long long n, int block);
 // every kernel started early; 42 k nodes: 1.65 -> 1.74 ms with up to four
 // blocks per SM, 1.63 ms with two).
 constexpr unsigned kPdlMaxBlocks = 2 * 148;
+inline bool early_grid(unsigned blocks) { return blocks <= kPdlMaxBlocks; }
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
@@ -231,7 +232,7 @@ inline void launch_k(void (*kernel)(P...), dim3 grid, int block, size_t smem, cu
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = grid.x * grid.y <= kPdlMaxBlocks ? 1 : 0;
+    cfg.numAttrs = early_grid(grid.x * grid.y) ? 1 : 0;
     (void)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 

@@ -77,8 +77,7 @@ __global__ void k_ab3_elem(Dev d) {
 }
 
 // edge flux c1 of compute_ssh_rhs_elem (fv_average_dynamic.F90:119-120, 152-153)
-__device__ __forceinline__ real ssh_edge_flux(const Dev &d, int ed) {
-    const int2 et = d.edge_tri[ed];
+__device__ __forceinline__ real ssh_edge_flux(const Dev &d, int ed, const int2 et) {
     const real4 X = d.edge_cross[ed];
     const real2 u1 = d.UAB[et.x];
     real c1 = (u1.y * X.x - u1.x * X.y) * d.aux_elem[et.x];
@@ -98,43 +97,70 @@ __device__ __forceinline__ real ssh_edge_flux(const Dev &d, int ed) {
 // fv_average_dynamic.F90:190-216), written before the step either by the host
 // (fesomc_gpu_set_forcing) or by k_forcing_values (device forcing).
 // ---------------------------------------------------------------------------
+// acc: ssh_rhs, the FP64 accumulation of the node's edge fluxes
+__device__ __forceinline__ void ssh_node(const Dev &d, int sub, int n, double acc) {
+    const double de = 0.614, ga = 0.088, ep = 0.013, fe = 1.0 - de - ga - ep;
+    if (d.key_rivers) {
+        for (int p = d.node_rptr[n]; p < d.node_rptr[n + 1]; ++p) acc = acc + d.runoff[d.node_ridx[p]];
+    }
+    const int q = d.obn_of_node[n];
+    if (d.TF_presence && q >= 0) acc = d.ob_val[(size_t)sub * d.nobn + q];
+    // the previous sub-step's rotation of the time levels
+    // (fv_main.F90:1547-1551)
+    const double en = sub > 0 ? d.eta_new[n] : d.eta_n[n];
+    const double em1 = sub > 0 ? d.eta_n[n] : d.eta_n_1[n];
+    const double em2 = sub > 0 ? d.eta_n_1[n] : d.eta_n_2[n];
+    if (sub > 0) {
+        d.eta_n[n] = en;
+        d.eta_n_1[n] = em1;
+        d.eta_n_2[n] = em2;
+    }
+    double enew = acc;
+    if (d.index_nod2D[n] < 2) enew = en + d.dt_2D_d * acc / (double)d.area[n];
+    d.eta_new[n] = enew;
+    const double eab = de * enew + fe * en + ga * em1 + ep * em2;
+    d.etaAB[n] = eab;
+    if (d.wet_dry_on) d.mask_wd_node[n] = ((double)d.depth[n] + eab > d.Dmin_d) ? real(1.0) : real(0.0);
+}
+__device__ __forceinline__ double ssh_add(const Dev &d, double acc, int code) {
+    const double c1 = (double)d.sshfl[code >> 1];
+    return (code & 1) ? acc - c1 : acc + c1;
+}
 // 40 registers: 6 resident blocks per SM instead of 5 (3 % faster).
 __global__ void __maxnreg__(40) k_ssh_node(Dev d, int sub) {
     pdl_enter();
-    const double de = 0.614, ga = 0.088, ep = 0.013, fe = 1.0 - de - ga - ep;
     GRID_LOOP(ii, d.N) {
         const int n = (int)ii;
-        double acc = 0.0;   // ssh_rhs: FP64 accumulation of the edge fluxes
+        double acc = 0.0;
         const int p0 = d.node_eptr[n], p1 = d.node_eptr[n + 1];
 #pragma unroll 4
-        for (int p = p0; p < p1; ++p) {
-            const int code = d.node_eidx[p];
-            const double c1 = (double)d.sshfl[code >> 1];
-            if (code & 1) acc = acc - c1;
-            else acc = acc + c1;
-        }
-        if (d.key_rivers) {
-            for (int p = d.node_rptr[n]; p < d.node_rptr[n + 1]; ++p) acc = acc + d.runoff[d.node_ridx[p]];
-        }
-        const int q = d.obn_of_node[n];
-        if (d.TF_presence && q >= 0) acc = d.ob_val[(size_t)sub * d.nobn + q];
-        // the previous sub-step's rotation of the time levels
-        // (fv_main.F90:1547-1551)
-        const double en = sub > 0 ? d.eta_new[n] : d.eta_n[n];
-        const double em1 = sub > 0 ? d.eta_n[n] : d.eta_n_1[n];
-        const double em2 = sub > 0 ? d.eta_n_1[n] : d.eta_n_2[n];
-        if (sub > 0) {
-            d.eta_n[n] = en;
-            d.eta_n_1[n] = em1;
-            d.eta_n_2[n] = em2;
-        }
-        double enew = acc;
-        if (d.index_nod2D[n] < 2) enew = en + d.dt_2D_d * acc / (double)d.area[n];
-        d.eta_new[n] = enew;
-        const double eab = de * enew + fe * en + ga * em1 + ep * em2;
-        d.etaAB[n] = eab;
-        if (d.wet_dry_on) d.mask_wd_node[n] = ((double)d.depth[n] + eab > d.Dmin_d) ? real(1.0) : real(0.0);
+        for (int p = p0; p < p1; ++p) acc = ssh_add(d, acc, d.node_eidx[p]);
+        ssh_node(d, sub, n, acc);
     }
+}
+// Small grids (kernels that start early): one item per thread, and what does
+// not change during a step, the connectivity, is loaded while the kernel
+// before still runs, so that the chain after the wait is one gather shorter
+// (here two: the edge list's bounds and its first 6 edges).  With the other
+// three kernels of the sub-cycle: 697 nodes 0.256 -> 0.243 ms per step, 4 k
+// 0.330 -> 0.299, 16 k 0.377 -> 0.353.  (On large grids the same loads held
+// registers for nothing: 16.7 -> 16.8 ms at 1.05 M.)
+__global__ void k_ssh_node_head(Dev d, int sub) {
+    constexpr int kHead = 6;
+    const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = n < (unsigned)d.N;
+    const int p0 = on ? d.node_eptr[n] : 0, p1 = on ? d.node_eptr[n + 1] : 0;
+    int head[kHead];
+#pragma unroll
+    for (int k = 0; k < kHead; ++k) head[k] = p0 + k < p1 ? d.node_eidx[p0 + k] : -1;
+    pdl_enter();
+    if (!on) return;
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < kHead; ++k)
+        if (head[k] >= 0) acc = ssh_add(d, acc, head[k]);
+    for (int p = p0 + kHead; p < p1; ++p) acc = ssh_add(d, acc, d.node_eidx[p]);
+    ssh_node(d, sub, (int)n, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -320,9 +346,7 @@ __global__ void k_p1_elem(Dev d) {
 }
 
 // One upwind edge flux of momentum_adv_upwind_2D (fv_advection.F90:589-643)
-__device__ __forceinline__ void adv2d_edge(const Dev &d, int ed, real &uu, real &vv) {
-    const int2 nn = d.edge_nodes[ed];
-    const int2 et = d.edge_tri[ed];
+__device__ __forceinline__ void adv2d_edge(const Dev &d, int ed, const int2 nn, const int2 et) {
     const real dmean = (real)dmax(d.Dmin_d, 0.5 * ((d.etaAB[nn.x] + (double)d.depth[nn.x]) +
                                                     (d.etaAB[nn.y] + (double)d.depth[nn.y])));
     const real acc = (d.ac[nn.x] + d.ac[nn.y]) * real(0.5);
@@ -336,18 +360,23 @@ __device__ __forceinline__ void adv2d_edge(const Dev &d, int ed, real &uu, real 
     const real2 dxy = d.edge_dxdy[ed];
     const real un = real(0.5) * kREarth * dmean *
                       ((u1 + u2) * dxy.y - (v1 * d.elem_cos[et.x] + v2 * d.elem_cos[et.y]) * dxy.x);
+    real uu, vv;
     if (un >= real(0.0)) { uu = un * U1.x * acc; vv = un * U1.y * acc; }
     else { uu = un * U2.x * acc; vv = un * U2.y * acc; }
+    d.adv2d[ed] = make_real2(uu, vv);
 }
 
 // momentum_adv_upwind_2D edge fluxes of the sub-step, once per internal edge
 __global__ void k_adv2d_edge(Dev d) {
     pdl_enter();
-    GRID_LOOP(ed, d.Ed_in) {
-        real uu, vv;
-        adv2d_edge(d, (int)ed, uu, vv);
-        d.adv2d[ed] = make_real2(uu, vv);
-    }
+    GRID_LOOP(ed, d.Ed_in) adv2d_edge(d, (int)ed, d.edge_nodes[ed], d.edge_tri[ed]);
+}
+__global__ void k_adv2d_edge_head(Dev d) {
+    const unsigned ed = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = ed < (unsigned)d.Ed_in;
+    const int2 nn = on ? d.edge_nodes[ed] : make_int2(0, 0), et = on ? d.edge_tri[ed] : make_int2(0, 0);
+    pdl_enter();
+    if (on) adv2d_edge(d, (int)ed, nn, et);
 }
 
 // biharmonic_2D (fv_viscosity.F90:338-568, free slip): two Laplacians of the
@@ -423,10 +452,8 @@ __global__ void k_bih2d_ul(Dev d) {
 
 // vel_gradients_2D (fv_gradients.F90:97-176, free slip) of U into vel_grad:
 // of UAB in every sub-step (sub_edge), of Ul in biharmonic_2D
-__device__ __forceinline__ void velgrad2d_elem(const Dev &d, const real2 *U, int e) {
+__device__ __forceinline__ void velgrad2d_elem(const Dev &d, const real2 *U, int e, const int4 en, const int4 nb) {
     {
-        const int4 en = d.elem_nodes[e];
-        const int4 nb = d.elem_nb[e];
         const int4 ee = d.elem_edges[e];
         const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
         const int eds[4] = {ee.x, ee.y, ee.z, ee.w};
@@ -460,7 +487,7 @@ __device__ __forceinline__ void velgrad2d_elem(const Dev &d, const real2 *U, int
 }
 __global__ void k_velgrad2d(Dev d, const real2 *U) {
     pdl_enter();
-    GRID_LOOP(ii, d.E) velgrad2d_elem(d, U, (int)ii);
+    GRID_LOOP(ii, d.E) velgrad2d_elem(d, U, (int)ii, d.elem_nodes[ii], d.elem_nb[ii]);
 }
 
 // sub_edge: the SSH flux of every edge, once, for both end nodes to gather
@@ -472,9 +499,23 @@ __global__ void k_sub_edge(Dev d) {
     pdl_enter();
     const long long Ed = d.Ed;
     GRID_LOOP(i, Ed + d.E) {
-        if (i < Ed) d.sshfl[i] = ssh_edge_flux(d, (int)i);
-        else velgrad2d_elem(d, d.UAB, (int)(i - Ed));
+        if (i < Ed) d.sshfl[i] = ssh_edge_flux(d, (int)i, d.edge_tri[i]);
+        else velgrad2d_elem(d, d.UAB, (int)(i - Ed), d.elem_nodes[i - Ed], d.elem_nb[i - Ed]);
     }
+}
+__global__ void k_sub_edge_head(Dev d) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x, Ed = d.Ed;
+    const bool edge = i < Ed, elem = !edge && i < Ed + d.E;
+    int2 et = make_int2(0, 0);
+    int4 en = make_int4(0, 0, 0, 0), nb = en;
+    if (edge) et = d.edge_tri[i];
+    if (elem) {
+        en = d.elem_nodes[i - Ed];
+        nb = d.elem_nb[i - Ed];
+    }
+    pdl_enter();
+    if (edge) d.sshfl[i] = ssh_edge_flux(d, (int)i, et);
+    if (elem) velgrad2d_elem(d, d.UAB, (int)(i - Ed), en, nb);
 }
 
 // viscosity_filt2x_2D (fv_viscosity.F90:672-767), first half: U_c of every
@@ -507,133 +548,139 @@ __global__ void k_filt2x_2d(Dev d) {
 // key_atm off) + rotation of U time levels + U_filt accumulation
 // (fv_main.F90:1568-1606).
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void u2d_elem(const Dev &d, int next, real d0inv, int e, const int4 en, const int4 il,
+                                         const int4 nb) {
+            const int nd[4] = {en.x, en.y, en.z, en.w};
+            // elevations and total depths in FP64 (the elevation gradient and
+            // the wet/dry test with them); the momentum terms in 'real'
+            double eab[4], dep[4], etag[4];
+            for (int k = 0; k < 4; ++k) {
+                eab[k] = d.etaAB[nd[k]];
+                dep[k] = d.depth[nd[k]];
+                if (d.key_atm) {
+                    // with atmospheric forcing: E - P and the sea-level pressure
+                    // anomaly (fv_average_dynamic.F90:278-286)
+                    const double d0i = 1.0 / d.density_0_d;
+                    etag[k] = kG64 * ((double)d.atp1[nd[k]] * eab[k] - d.emp[nd[k]] * d0i -
+                                      (double)d.atp2[nd[k]] * d.ssh_gp[nd[k]]) + (kPref - d.mslp[nd[k]]) * d0i;
+                } else {
+                    etag[k] = kG64 * ((double)d.atp1[nd[k]] * eab[k] - (double)d.atp2[nd[k]] * d.ssh_gp[nd[k]]);
+                }
+            }
+            real mwd = d.mask_wd[e];
+            if (d.wet_dry_on) {
+                const double dmin4 = dmin(dmin(dep[0], dep[1]), dmin(dep[2], dep[3]));
+                const double emax4 = dmax(dmax(eab[0], eab[1]), dmax(eab[2], eab[3]));
+                mwd = (dmin4 + emax4 > d.Dmin_d) ? real(1.0) : real(0.0);
+                d.mask_wd[e] = mwd;
+            }
+            const real4 w = d.w_cv[e];
+            const real ar = d.elem_area[e];
+            const real dmean = (real)dmax(d.Dmin_d, wexp_d(w, eab[0] + dep[0], eab[1] + dep[1], eab[2] + dep[2], eab[3] + dep[3]));
+            const real4 gx = d.gs_x[e], gy = d.gs_y[e];
+            const real gex = (real)((double)gx.x * etag[0] + (double)gx.y * etag[1] + (double)gx.z * etag[2] + (double)gx.w * etag[3]);
+            const real gey = (real)((double)gy.x * etag[0] + (double)gy.y * etag[1] + (double)gy.z * etag[2] + (double)gy.w * etag[3]);
+            const real2 uab = d.UAB[e];
+            const real cor = d.coriolis[e];
+            real rx = ar * (-dmean * gex + uab.y * dmean * cor + d.taux[e] * d0inv);
+            real ry = ar * (-dmean * gey - uab.x * dmean * cor + d.tauy[e] * d0inv);
+            if (d.mom_adv_2D == 2) {
+                const int codes[4] = {il.x, il.y, il.z, il.w};
+    #pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int code = codes[c];
+                    if (code < 0) break;
+                    const real2 f = d.adv2d[code >> 1];
+                    if (code & 1) { rx = rx + f.x; ry = ry + f.y; }
+                    else { rx = rx - f.x; ry = ry - f.y; }
+                }
+            }
+            if (d.filt_2D) {
+                const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
+                const int jend = (en.x == en.w) ? 3 : 4;
+                real u1 = real(0.0), u2 = real(0.0);
+                for (int j = 0; j < jend; ++j)
+                    if (nbs[j] >= 0) {
+                        const real2 un = d.UAB[nbs[j]];
+                        u1 = u1 + un.x - uab.x;
+                        u2 = u2 + un.y - uab.y;
+                    }
+                const real sd = (real)wsum_d(w, dep[0], dep[1], dep[2], dep[3]);
+                rx = rx + d.tau_inv_filt * u1 * ar * sd;
+                ry = ry + d.tau_inv_filt * u2 * ar * sd;
+            }
+            // biharmonic_2D: the second-pass edge fluxes in edge order
+            if (d.bih_2D) {
+                const int4 se = d.elem_sedges[e];
+                const int codes[4] = {se.x, se.y, se.z, se.w};
+                for (int c = 0; c < 4; ++c) {
+                    const int code = codes[c];
+                    if (code < 0) break;
+                    const real2 f = d.b2fl[code >> 1];
+                    if (code & 1) { rx = rx - f.x; ry = ry - f.y; }
+                    else { rx = rx + f.x; ry = ry + f.y; }
+                }
+            }
+            const real2 r3 = d.U_rhs_2D_3D[e];
+            rx = rx + r3.x;
+            ry = ry + r3.y;
+            // final update with implicit bottom drag
+            double eo[4], enw[4];
+            for (int k = 0; k < 4; ++k) { eo[k] = d.eta_n[nd[k]]; enw[k] = d.eta_new[nd[k]]; }
+            const real dmo = (real)dmax(d.Dmin_d, wsum_d(w, eo[0] + dep[0], eo[1] + dep[1], eo[2] + dep[2], eo[3] + dep[3]));
+            const real4 bf = d.bfric[e];
+            const real ub = bf.x, vb = bf.y, friction = bf.z;
+            const real ff = real(1.0) / ((real)dmax(d.Dmin_d, wsum_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]))
+                                     + friction * d.dt_2D);
+            const real dt2 = d.dt_2D;
+            const real2 u0 = d.U_n_2D[e];
+            const real2 bp = d.Bar_pr_2D[e];
+            // UV2_rhs of viscosity_filt2x_2D (zero when it is off)
+            real uvx = real(0.0), uvy = real(0.0);
+            if (d.filt_bi_2D) {
+                const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
+                const real2 c0 = d.f2uv2d[e];
+                for (int j = 0; j < 4; ++j) {
+                    const int ne = nbs[j];
+                    if (!(ne >= 0 && (j < 3 || ne != nbs[0]))) continue;
+                    const real2 c2 = d.f2uv2d[ne];
+                    if (j == 0) { uvx = -c0.x + c2.x; uvy = -c0.y + c2.y; }
+                    else { uvx = uvx - c0.x + c2.x; uvy = uvy - c0.y + c2.y; }
+                }
+            }
+            const real nx = mwd * ((dmo * u0.x - dt2 * friction * (ub - u0.x) + dt2 * bp.x + dt2 * rx / ar) * ff + uvx);
+            const real ny = mwd * ((dmo * u0.y - dt2 * friction * (vb - u0.y) + dt2 * bp.y + dt2 * ry / ar) * ff + uvy);
+            // rotate U_n_2 <- U_n_1 <- U_n_2D <- new (fv_main.F90:1569-1578)
+            const real2 u1 = d.U_n_1[e];
+            d.U_n_2[e] = u1;
+            d.U_n_1[e] = u0;
+            d.U_n_2D[e] = make_real2(nx, ny);
+            // U_filt accumulation with the new elevation (fv_main.F90:1596-1605)
+            const real dmn = (real)dmax(d.Dmin_d, wexp_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]));
+            d.U_filt_2D[e] = d.U_filt_2D[e] + nx * dmn;
+            d.V_filt_2D[e] = d.V_filt_2D[e] + ny * dmn;
+            // the next sub-step's AB3 velocity and mean total depth
+            if (next) {
+                d.UAB_next[e] = ab3v(d.beta, make_real2(nx, ny), u0, u1);
+                double em[4];
+                for (int k = 0; k < 4; ++k) em[k] = d.eta_n_1[nd[k]];
+                d.aux_elem[e] = aux_of(d, w, enw, eo, em, dep);
+            }
+}
 // FP32: 8 resident blocks (at most 64 registers); FP64: 6.
 __global__ void __launch_bounds__(128, FESOMC_FP32 ? 8 : 6) k_u2d_elem(Dev d, int next) {
     pdl_enter();
     const real d0inv = real(1.0) / d.density_0;
-    GRID_LOOP(ii, d.E) {
-        const int e = (int)ii;
-        const int4 en = d.elem_nodes[e];
-        const int nd[4] = {en.x, en.y, en.z, en.w};
-        // elevations and total depths in FP64 (the elevation gradient and
-        // the wet/dry test with them); the momentum terms in 'real'
-        double eab[4], dep[4], etag[4];
-        for (int k = 0; k < 4; ++k) {
-            eab[k] = d.etaAB[nd[k]];
-            dep[k] = d.depth[nd[k]];
-            if (d.key_atm) {
-                // with atmospheric forcing: E - P and the sea-level pressure
-                // anomaly (fv_average_dynamic.F90:278-286)
-                const double d0i = 1.0 / d.density_0_d;
-                etag[k] = kG64 * ((double)d.atp1[nd[k]] * eab[k] - d.emp[nd[k]] * d0i -
-                                  (double)d.atp2[nd[k]] * d.ssh_gp[nd[k]]) + (kPref - d.mslp[nd[k]]) * d0i;
-            } else {
-                etag[k] = kG64 * ((double)d.atp1[nd[k]] * eab[k] - (double)d.atp2[nd[k]] * d.ssh_gp[nd[k]]);
-            }
-        }
-        real mwd = d.mask_wd[e];
-        if (d.wet_dry_on) {
-            const double dmin4 = dmin(dmin(dep[0], dep[1]), dmin(dep[2], dep[3]));
-            const double emax4 = dmax(dmax(eab[0], eab[1]), dmax(eab[2], eab[3]));
-            mwd = (dmin4 + emax4 > d.Dmin_d) ? real(1.0) : real(0.0);
-            d.mask_wd[e] = mwd;
-        }
-        const real4 w = d.w_cv[e];
-        const real ar = d.elem_area[e];
-        const real dmean = (real)dmax(d.Dmin_d, wexp_d(w, eab[0] + dep[0], eab[1] + dep[1], eab[2] + dep[2], eab[3] + dep[3]));
-        const real4 gx = d.gs_x[e], gy = d.gs_y[e];
-        const real gex = (real)((double)gx.x * etag[0] + (double)gx.y * etag[1] + (double)gx.z * etag[2] + (double)gx.w * etag[3]);
-        const real gey = (real)((double)gy.x * etag[0] + (double)gy.y * etag[1] + (double)gy.z * etag[2] + (double)gy.w * etag[3]);
-        const real2 uab = d.UAB[e];
-        const real cor = d.coriolis[e];
-        real rx = ar * (-dmean * gex + uab.y * dmean * cor + d.taux[e] * d0inv);
-        real ry = ar * (-dmean * gey - uab.x * dmean * cor + d.tauy[e] * d0inv);
-        if (d.mom_adv_2D == 2) {
-            const int4 il = d.elem_iedges[e];
-            const int codes[4] = {il.x, il.y, il.z, il.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int code = codes[c];
-                if (code < 0) break;
-                const real2 f = d.adv2d[code >> 1];
-                if (code & 1) { rx = rx + f.x; ry = ry + f.y; }
-                else { rx = rx - f.x; ry = ry - f.y; }
-            }
-        }
-        if (d.filt_2D) {
-            const int4 nb = d.elem_nb[e];
-            const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
-            const int jend = (en.x == en.w) ? 3 : 4;
-            real u1 = real(0.0), u2 = real(0.0);
-            for (int j = 0; j < jend; ++j)
-                if (nbs[j] >= 0) {
-                    const real2 un = d.UAB[nbs[j]];
-                    u1 = u1 + un.x - uab.x;
-                    u2 = u2 + un.y - uab.y;
-                }
-            const real sd = (real)wsum_d(w, dep[0], dep[1], dep[2], dep[3]);
-            rx = rx + d.tau_inv_filt * u1 * ar * sd;
-            ry = ry + d.tau_inv_filt * u2 * ar * sd;
-        }
-        // biharmonic_2D: the second-pass edge fluxes in edge order
-        if (d.bih_2D) {
-            const int4 se = d.elem_sedges[e];
-            const int codes[4] = {se.x, se.y, se.z, se.w};
-            for (int c = 0; c < 4; ++c) {
-                const int code = codes[c];
-                if (code < 0) break;
-                const real2 f = d.b2fl[code >> 1];
-                if (code & 1) { rx = rx - f.x; ry = ry - f.y; }
-                else { rx = rx + f.x; ry = ry + f.y; }
-            }
-        }
-        const real2 r3 = d.U_rhs_2D_3D[e];
-        rx = rx + r3.x;
-        ry = ry + r3.y;
-        // final update with implicit bottom drag
-        double eo[4], enw[4];
-        for (int k = 0; k < 4; ++k) { eo[k] = d.eta_n[nd[k]]; enw[k] = d.eta_new[nd[k]]; }
-        const real dmo = (real)dmax(d.Dmin_d, wsum_d(w, eo[0] + dep[0], eo[1] + dep[1], eo[2] + dep[2], eo[3] + dep[3]));
-        const real4 bf = d.bfric[e];
-        const real ub = bf.x, vb = bf.y, friction = bf.z;
-        const real ff = real(1.0) / ((real)dmax(d.Dmin_d, wsum_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]))
-                                 + friction * d.dt_2D);
-        const real dt2 = d.dt_2D;
-        const real2 u0 = d.U_n_2D[e];
-        const real2 bp = d.Bar_pr_2D[e];
-        // UV2_rhs of viscosity_filt2x_2D (zero when it is off)
-        real uvx = real(0.0), uvy = real(0.0);
-        if (d.filt_bi_2D) {
-            const int4 nb = d.elem_nb[e];
-            const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
-            const real2 c0 = d.f2uv2d[e];
-            for (int j = 0; j < 4; ++j) {
-                const int ne = nbs[j];
-                if (!(ne >= 0 && (j < 3 || ne != nbs[0]))) continue;
-                const real2 c2 = d.f2uv2d[ne];
-                if (j == 0) { uvx = -c0.x + c2.x; uvy = -c0.y + c2.y; }
-                else { uvx = uvx - c0.x + c2.x; uvy = uvy - c0.y + c2.y; }
-            }
-        }
-        const real nx = mwd * ((dmo * u0.x - dt2 * friction * (ub - u0.x) + dt2 * bp.x + dt2 * rx / ar) * ff + uvx);
-        const real ny = mwd * ((dmo * u0.y - dt2 * friction * (vb - u0.y) + dt2 * bp.y + dt2 * ry / ar) * ff + uvy);
-        // rotate U_n_2 <- U_n_1 <- U_n_2D <- new (fv_main.F90:1569-1578)
-        const real2 u1 = d.U_n_1[e];
-        d.U_n_2[e] = u1;
-        d.U_n_1[e] = u0;
-        d.U_n_2D[e] = make_real2(nx, ny);
-        // U_filt accumulation with the new elevation (fv_main.F90:1596-1605)
-        const real dmn = (real)dmax(d.Dmin_d, wexp_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]));
-        d.U_filt_2D[e] = d.U_filt_2D[e] + nx * dmn;
-        d.V_filt_2D[e] = d.V_filt_2D[e] + ny * dmn;
-        // the next sub-step's AB3 velocity and mean total depth
-        if (next) {
-            d.UAB_next[e] = ab3v(d.beta, make_real2(nx, ny), u0, u1);
-            double em[4];
-            for (int k = 0; k < 4; ++k) em[k] = d.eta_n_1[nd[k]];
-            d.aux_elem[e] = aux_of(d, w, enw, eo, em, dep);
-        }
-    }
+    GRID_LOOP(ii, d.E) u2d_elem(d, next, d0inv, (int)ii, d.elem_nodes[ii], d.elem_iedges[ii], d.elem_nb[ii]);
+}
+__global__ void __launch_bounds__(128) k_u2d_elem_head(Dev d, int next) {
+    const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = e < (unsigned)d.E;
+    const int4 none = make_int4(0, 0, 0, 0);
+    const int4 en = on ? d.elem_nodes[e] : none, il = on ? d.elem_iedges[e] : none, nb = on ? d.elem_nb[e] : none;
+    const real d0inv = real(1.0) / d.density_0;
+    pdl_enter();
+    if (on) u2d_elem(d, next, d0inv, (int)e, en, il, nb);
 }
 
 // ---- launch wrappers --------------------------------------------------------
@@ -643,11 +690,15 @@ void launch_ab3_elem(const Dev &d, cudaStream_t s) {
 }
 void launch_sub_edge(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_SSHEDGE, 256);
-    launch_k(k_sub_edge, grid_for((long long)d.Ed + d.E, b), b, 0, s, d);
+    const int g = grid_for((long long)d.Ed + d.E, b);
+    if (early_grid(g)) launch_k(k_sub_edge_head, g, b, 0, s, d);
+    else launch_k(k_sub_edge, g, b, 0, s, d);
 }
 void launch_ssh_node(const Dev &d, int sub, cudaStream_t s) {
     const int b = tuned(d, TK_SSHNODE, 256);
-    launch_k(k_ssh_node, grid_for(d.N, b), b, 0, s, d, sub);
+    const int g = grid_for(d.N, b);
+    if (early_grid(g)) launch_k(k_ssh_node_head, g, b, 0, s, d, sub);
+    else launch_k(k_ssh_node, g, b, 0, s, d, sub);
 }
 void launch_puls_elem(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_PULS, 256);
@@ -679,7 +730,9 @@ void launch_p1_elem(const Dev &d, cudaStream_t s) {
 }
 void launch_adv2d_edge(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ADV2D, 256);
-    launch_k(k_adv2d_edge, grid_for(d.Ed_in, b), b, 0, s, d);
+    const int g = grid_for(d.Ed_in, b);
+    if (early_grid(g)) launch_k(k_adv2d_edge_head, g, b, 0, s, d);
+    else launch_k(k_adv2d_edge, g, b, 0, s, d);
 }
 void launch_filt2x_2d(const Dev &d, cudaStream_t s) { launch_k(k_filt2x_2d, grid_for(d.E, 256), 256, 0, s, d); }
 void launch_bih_2d(const Dev &d, cudaStream_t s) {
@@ -691,7 +744,9 @@ void launch_bih_2d(const Dev &d, cudaStream_t s) {
 }
 void launch_u2d_elem(const Dev &d, int next, cudaStream_t s) {
     const int b = tuned(d, TK_U2D, 128);
-    launch_k(k_u2d_elem, grid_for(d.E, b), b, 0, s, d, next);
+    const int g = grid_for(d.E, b);
+    if (early_grid(g)) launch_k(k_u2d_elem_head, g, b, 0, s, d, next);
+    else launch_k(k_u2d_elem, g, b, 0, s, d, next);
 }
 
 
@@ -705,12 +760,16 @@ void tune_limits_barotropic(int *lim) {
     tune_lower(lim, TK_AB3, (const void *)k_ab3_elem);
     tune_lower(lim, TK_VELGRAD2D, (const void *)k_velgrad2d);
     tune_lower(lim, TK_SSHEDGE, (const void *)k_sub_edge);
+    tune_lower(lim, TK_SSHEDGE, (const void *)k_sub_edge_head);
     tune_lower(lim, TK_SSHNODE, (const void *)k_ssh_node);
+    tune_lower(lim, TK_SSHNODE, (const void *)k_ssh_node_head);
     tune_lower(lim, TK_PULS, (const void *)k_puls_elem);
     tune_lower(lim, TK_EL2NODES, (const void *)k_el2nodes);
     tune_lower(lim, TK_P1EDGE, (const void *)k_p1_edge);
     tune_lower(lim, TK_ADV2D, (const void *)k_adv2d_edge);
+    tune_lower(lim, TK_ADV2D, (const void *)k_adv2d_edge_head);
     tune_lower(lim, TK_U2D, (const void *)k_u2d_elem);
+    tune_lower(lim, TK_U2D, (const void *)k_u2d_elem_head);
 }
 
 FESOMC_PREC_END
