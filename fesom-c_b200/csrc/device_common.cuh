@@ -199,6 +199,12 @@ constexpr unsigned kFull = 0xffffffffu;
 
 // launch helpers (implemented in model.cu)
 int grid_for(long long n, int block);
+// entities per block of the column kernels (pressure_col, bpg_elem, update3d,
+// wvel) where the knob "columns" does not set them
+inline int default_columns(int L) {
+    const int b = 160 / L;
+    return b > 16 ? 16 : b < 1 ? 1 : b;
+}
 
 // Programmatic dependent launch: a kernel started with launch_k may be
 // resident while the kernel before it on the stream still runs, so that its
@@ -236,6 +242,18 @@ inline void launch_k(void (*kernel)(P...), dim3 grid, int block, size_t smem, cu
     (void)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
+
+// Launches a kernel whose blocks of 'threads' take groups of 'per_block'
+// entities and stride over them: as many blocks as are resident at once (a
+// few more would make a second, mostly empty wave of all the work).
+template <typename... P, typename... A>
+inline void launch_resident(void (*kernel)(P...), long long count, int per_block, int threads, size_t smem,
+                            cudaStream_t s, A... args) {
+    const long long blocks = (count + per_block - 1) / per_block;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
+    launch_k(kernel, (unsigned)(blocks < 148LL * occ ? blocks : 148LL * occ), threads, smem, s, args...);
+}
 
 }  // namespace fesomc
 

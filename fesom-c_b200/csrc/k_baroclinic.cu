@@ -71,85 +71,137 @@ __global__ void __launch_bounds__(1024) k_pressure_col(Dev d) {
     }
 }
 
+// What the level threads of a column block need of their element, staged in
+// shared memory by four lanes per element, one per node, before the level
+// phase: the level threads otherwise load nodes, geometry and elevations (24
+// of bpg_elem's 33 loads, the same for all levels of an element) each for
+// itself.  kEsReals values per element.
+constexpr int kEsW = 0, kEsGx = 4, kEsGy = 8, kEsAn = 12, kEsA = 16, kEsX = 20, kEsReals = 24;
+// lanes of the caller's warp that take part in a phase of the block's first
+// 'count' threads
+__device__ __forceinline__ unsigned lanes_below(int count) {
+    const int n = count - (int)(threadIdx.x & ~31u);
+    return n >= 32 ? kFull : (1u << n) - 1u;
+}
+
 // baroclinic_pressure_gradient_3D (fv_pressure_new.F90:146-221) per
 // (element, level); Bar_pr_2D as a level-ordered sum per element.  Also the
 // element's surface pressure force of compute_vel_rhs (fv_3D_vel.F90:60-75),
 // the same for every level.  Column blocks reach 1024 threads (B * L), so
-// the kernel is bounded to 64 registers (unbounded it takes 96, which a
-// block of more than 682 threads, i.e. L >= 43, could not launch with).
-__global__ void __launch_bounds__(1024) k_bpg_elem(Dev d) {
+// the kernel is bounded to 64 registers.
+// Bound by the latency of its loads between barriers, by its loads' number
+// before the staging.  FP32 (48 registers, 8 blocks of 160 threads per SM)
+// has the level loads in flight during the staging; FP64 has no registers
+// for that.  1.05 M nodes FP64 0.838 -> 0.762 ms (with the early loads 0.85),
+// 232 k FP32 0.195 -> 0.109, 40 k, 30 layers 0.058 as before.
+#if FESOMC_FP32
+#define BPG_BOUNDS __maxnreg__(48)
+constexpr bool kBpgEarly = true;
+#else
+#define BPG_BOUNDS __launch_bounds__(1024)
+constexpr bool kBpgEarly = false;
+#endif
+__global__ void BPG_BOUNDS k_bpg_elem(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
-    real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L, NS = d.NS;
     const ColBlock cb(d);
-    const int S = 2 * L + 1;
-    for (long long eb = (long long)blockIdx.x * cb.B; eb < d.E; eb += (long long)gridDim.x * cb.B) {
+    const int S = 2 * L + 1, B = cb.B;
+    real *const es = reinterpret_cast<real *>(sm_raw);    // kEsReals per element
+    real *const ex = es + B * kEsReals;                   // 12 per element: dh, depth, pressure of its nodes
+    real *const sm = ex + B * 12;
+    for (long long eb = (long long)blockIdx.x * B; eb < d.E; eb += (long long)gridDim.x * B) {
+        // the level loads first: they are in flight during the staging
         const long long e_ = eb + cb.jl;
-        if (cb.jl < cb.B && e_ < d.E) {
-            const int e = (int)e_, z = cb.z;
-            const int4 en = d.elem_nodes[e];
-            const int nd[4] = {en.x, en.y, en.z, en.w};
-            const real4 gx = d.gs_x[e], gy = d.gs_y[e], w = d.w_cv[e];
-            real dh[4], de[4];
-            for (int k = 0; k < 4; ++k) { dh[k] = d.depth[nd[k]] + d.eta_n[nd[k]]; de[k] = d.depth[nd[k]]; }
-            const real Ax = wsum(gx, dh[0], dh[1], dh[2], dh[3]);
-            const real Ay = wsum(gy, dh[0], dh[1], dh[2], dh[3]);
-            const real Bx = wsum(gx, de[0], de[1], de[2], de[3]);
-            const real By = wsum(gy, de[0], de[1], de[2], de[3]);
-            const real fac = d.elem_bpfac[e];
-            const real4 ae = elem_jac_a(d, d.eta_jac, en);
-            const real an[4] = {ae.x, ae.y, ae.z, ae.w};
-            const real je = d.Je[(size_t)e * L + z];
-            const real accJe_inv = -fac / je;
-            real hu[4], hl[4], pre[4];
-            for (int k = 0; k < 4; ++k) {
-                hu[k] = d.hpressure[(size_t)nd[k] * NS + z];
-                hl[k] = d.hpressure[(size_t)nd[k] * NS + z + 1];
-                pre[k] = real(0.5) * (hu[k] + hl[k]) * jc_of(d, an[k], z);
+        const bool act = cb.jl < B && e_ < d.E;
+        real je = real(1.0), hu[4], hl[4];
+        if (kBpgEarly) {
+            if (act) {
+                const int4 en = d.elem_nodes[e_];
+                const int nd[4] = {en.x, en.y, en.z, en.w};
+                je = d.Je[(size_t)e_ * L + cb.z];
+                for (int k = 0; k < 4; ++k) {
+                    hu[k] = d.hpressure[(size_t)nd[k] * NS + cb.z];
+                    hl[k] = d.hpressure[(size_t)nd[k] * NS + cb.z + 1];
+                }
             }
+        }
+        if ((int)threadIdx.x < 4 * B) {
+            const int j = threadIdx.x >> 2, k = threadIdx.x & 3;
+            const int e = (int)(eb + j < d.E ? eb + j : d.E - 1);
+            const int nd = reinterpret_cast<const int *>(d.elem_nodes)[4 * (size_t)e + k];
+            const real4 g = (k & 1) ? d.gs_y[e] : d.gs_x[e];
+            real *const o = es + j * kEsReals, *const x = ex + j * 12;
+            x[k] = d.depth[nd] + d.eta_n[nd];
+            x[4 + k] = d.depth[nd];
+            x[8 + k] = -kG * (d.atp1[nd] * d.eta_n[nd] - d.atp2[nd] * d.ssh_gp[nd]);
+            o[kEsAn + k] = jac_a(d, d.eta_jac, nd);
+            const real4 w = d.w_cv[e];
+            if (k == 2) { o[kEsW] = w.x; o[kEsW + 1] = w.y; o[kEsW + 2] = w.z; o[kEsW + 3] = w.w; }
+            if (k < 2) {
+                real *const go = o + (k ? kEsGy : kEsGx);
+                go[0] = g.x; go[1] = g.y; go[2] = g.z; go[3] = g.w;
+            }
+            if (k == 3) o[kEsX] = d.elem_bpfac[e];
+            __syncwarp(lanes_below(4 * B));
+            // Ax, Ay, Bx, By: gradients of the total depth and of the depth
+            const real *v = x + (k < 2 ? 0 : 4);
+            o[kEsA + k] = wsum(g, v[0], v[1], v[2], v[3]);
+            if (k < 2) {
+                real pr[4] = {x[8], x[9], x[10], x[11]};
+                if (d.key_atm) {
+                    // sea-level pressure and E - P of the element (fv_3D_vel.F90:40-53)
+                    const int4 en = d.elem_nodes[e];
+                    const real d0i = real(1.0) / d.density_0;
+                    const real atm_mean = wsum(w, (real)d.mslp[en.x], (real)d.mslp[en.y], (real)d.mslp[en.z], (real)d.mslp[en.w]);
+                    const real emp_mean = wsum(w, (real)d.emp[en.x], (real)d.emp[en.y], (real)d.emp[en.z], (real)d.emp[en.w]);
+                    for (int q = 0; q < 4; ++q)
+                        pr[q] = pr[q] - (real(kPref) - atm_mean) * d0i + kG * emp_mean * d0i;
+                }
+                if (eb + j < d.E)
+                    reinterpret_cast<real *>(d.Fp)[2 * (size_t)e + k] = wsum(g, pr[0], pr[1], pr[2], pr[3]) * d.elem_area[e];
+            }
+        }
+        __syncthreads();
+        if (act) {
+            const int e = (int)e_, z = cb.z;
+            const real *const o = es + cb.jl * kEsReals;
+            real pre[4];
+            if (!kBpgEarly) {
+                const int4 en = d.elem_nodes[e_];
+                const int nd[4] = {en.x, en.y, en.z, en.w};
+                je = d.Je[(size_t)e_ * L + cb.z];
+                for (int k = 0; k < 4; ++k) {
+                    hu[k] = d.hpressure[(size_t)nd[k] * NS + cb.z];
+                    hl[k] = d.hpressure[(size_t)nd[k] * NS + cb.z + 1];
+                }
+            }
+            for (int k = 0; k < 4; ++k) pre[k] = real(0.5) * (hu[k] + hl[k]) * jc_of(d, o[kEsAn + k], z);
+            const real4 w = make_real4(o[kEsW], o[kEsW + 1], o[kEsW + 2], o[kEsW + 3]);
+            const real4 gx = make_real4(o[kEsGx], o[kEsGx + 1], o[kEsGx + 2], o[kEsGx + 3]);
+            const real4 gy = make_real4(o[kEsGy], o[kEsGy + 1], o[kEsGy + 2], o[kEsGy + 3]);
+            const real accJe_inv = -o[kEsX] / je;
             const real qd_up = wsum(w, hu[0], hu[1], hu[2], hu[3]);
             const real qd_low = wsum(w, hl[0], hl[1], hl[2], hl[3]);
             const real sx = wsum(gx, pre[0], pre[1], pre[2], pre[3]);
             const real sy = wsum(gy, pre[0], pre[1], pre[2], pre[3]);
             const real s0 = __ldg(d.sig + z), s1 = __ldg(d.sig + z + 1);
+            const real Ax = o[kEsA], Ay = o[kEsA + 1], Bx = o[kEsA + 2], By = o[kEsA + 3];
             const real bu = accJe_inv * (sx + qd_low * (s1 * Ax - Bx) - qd_up * (s0 * Ax - Bx));
             const real bv = accJe_inv * (sy + qd_low * (s1 * Ay - By) - qd_up * (s0 * Ay - By));
             d.Bar_pru[(size_t)e * L + z] = bu;
             d.Bar_prv[(size_t)e * L + z] = bv;
             sm[cb.jl * S + z] = bu * je;
             sm[cb.jl * S + L + z] = bv * je;
-            // surface pressure force of the element (independent of the
-            // level sums): in this phase, off the serial path
-            if (z == 0) {
-                real pr[4];
-                for (int k = 0; k < 4; ++k)
-                    pr[k] = -kG * (d.atp1[nd[k]] * d.eta_n[nd[k]] - d.atp2[nd[k]] * d.ssh_gp[nd[k]]);
-                if (d.key_atm) {
-                    // sea-level pressure and E - P of the element (fv_3D_vel.F90:40-53)
-                    const real d0i = real(1.0) / d.density_0;
-                    const real atm_mean = wsum(w, (real)d.mslp[nd[0]], (real)d.mslp[nd[1]], (real)d.mslp[nd[2]],
-                                               (real)d.mslp[nd[3]]);
-                    const real emp_mean = wsum(w, (real)d.emp[nd[0]], (real)d.emp[nd[1]], (real)d.emp[nd[2]],
-                                               (real)d.emp[nd[3]]);
-                    for (int k = 0; k < 4; ++k)
-                        pr[k] = pr[k] - (real(kPref) - atm_mean) * d0i + kG * emp_mean * d0i;
-                }
-                const real ar = d.elem_area[e];
-                d.Fp[e] = make_real2(wsum(gx, pr[0], pr[1], pr[2], pr[3]) * ar, wsum(gy, pr[0], pr[1], pr[2], pr[3]) * ar);
-            }
         }
         __syncthreads();
-        const long long es = eb + threadIdx.x;
-        if ((int)threadIdx.x < cb.B && es < d.E) {
-            const int e = (int)es;
-            const real *row = sm + threadIdx.x * S;
-            real b1 = real(0.0), b2 = real(0.0);
-            for (int k = 0; k < L; ++k) {
-                b1 = b1 + row[k];
-                b2 = b2 + row[L + k];
-            }
-            d.Bar_pr_2D[e] = make_real2(b1, b2);
+        // one thread per (element, component): the level sums in level order
+        if ((int)threadIdx.x < 2 * B && eb + (threadIdx.x >> 1) < d.E) {
+            const int j = threadIdx.x >> 1, c = threadIdx.x & 1;
+            const real *row = sm + j * S + c * L;
+            real b = real(0.0);
+            for (int k = 0; k < L; ++k) b = b + row[k];
+            reinterpret_cast<real *>(d.Bar_pr_2D)[2 * (eb + j) + c] = b;
         }
         __syncthreads();
     }
@@ -760,70 +812,73 @@ __global__ void k_je_elem(Dev d) {
 // per element.  Runs right after the jacobian call: the stored Je still holds
 // the previous jacobian (Jc_old), and is replaced here by the new Je / Ze /
 // ZBe.
-constexpr int kU3Sc = 14;  // per element: U2p, V2p, uf, vf, w_cv(4), a(4), U_n_2D(2)
 // 48 registers: 4 resident column blocks per SM instead of 3 (15 % faster).
+// The element's scalars are formed by four lanes per element, one per node.
+// Blocks of 160 threads: 1.05 M nodes 0.80 -> 0.60 ms, 232 k FP32 0.131 ->
+// 0.095, 40 k, 30 layers 0.059 -> 0.039 (one lane per element formed them, 320
+// threads).
+constexpr int kU3Sc = 16;  // per element: w_cv(4), a(4), U2p, V2p, uf, vf, U_n_2D(2), dmean_inv; then dh(4)
 __global__ void __maxnreg__(48) k_update3d(Dev d, real Mt_inv) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L;
     const ColBlock cb(d);
-    const int S = 2 * L + 1;
-    real *sc = sm + (size_t)cb.B * S;  // kU3Sc scalars per element
-    for (long long eb = (long long)blockIdx.x * cb.B; eb < d.E; eb += (long long)gridDim.x * cb.B) {
+    const int S = 2 * L + 1, B = cb.B;
+    real *const sc = sm + (size_t)B * S, *const dhs = sc + (size_t)B * kU3Sc;
+    for (long long eb = (long long)blockIdx.x * B; eb < d.E; eb += (long long)gridDim.x * B) {
         const long long e_ = eb + cb.jl;
-        const bool act = cb.jl < cb.B && e_ < d.E;
+        const bool act = cb.jl < B && e_ < d.E;
         const size_t i = (size_t)e_ * L + cb.z;
         real a_old = real(0.0), ur = real(0.0), vr = real(0.0);
         if (act) {
             a_old = d.Je[i];
             ur = d.U_rhs[i];
             vr = d.V_rhs[i];
-            sm[cb.jl * S + cb.z] = ur * a_old;
-            sm[cb.jl * S + L + cb.z] = vr * a_old;
-            // the element's scalars, here rather than in the serial sum or
-            // the level loop, so that both read shared memory only
-            if (cb.z == 0) {
-                const int e = (int)e_;
-                const int4 en = d.elem_nodes[e];
-                const real4 w = d.w_cv[e];
-                const real dmean_inv = real(1.0) / dmax(d.Dmin, wsum(w, d.depth[en.x] + d.eta_n[en.x], d.depth[en.y] + d.eta_n[en.y],
-                                                                d.depth[en.z] + d.eta_n[en.z], d.depth[en.w] + d.eta_n[en.w]));
-                const real uf = (d.U_filt_2D[e] * Mt_inv) * dmean_inv;
-                const real vf = (d.V_filt_2D[e] * Mt_inv) * dmean_inv;
-                d.U_filt_2D[e] = uf;
-                d.V_filt_2D[e] = vf;
-                const real4 an = elem_jac_a(d, d.eta_jac, en);
-                const real2 u2d = d.U_n_2D[e];
-                real *o = sc + kU3Sc * cb.jl;
-                o[0] = dmean_inv;
-                o[2] = uf; o[3] = vf;
-                o[4] = w.x; o[5] = w.y; o[6] = w.z; o[7] = w.w;
-                o[8] = an.x; o[9] = an.y; o[10] = an.z; o[11] = an.w;
-                o[12] = u2d.x; o[13] = u2d.y;
+        }
+        // the element's scalars, here rather than in the serial sum or the
+        // level loop, so that both read shared memory only
+        if ((int)threadIdx.x < 4 * B) {
+            const int j = threadIdx.x >> 2, k = threadIdx.x & 3;
+            const int e = (int)(eb + j < d.E ? eb + j : d.E - 1);
+            const int n = reinterpret_cast<const int *>(d.elem_nodes)[4 * (size_t)e + k];
+            real *o = sc + kU3Sc * j;
+            o[k] = reinterpret_cast<const real *>(d.w_cv)[4 * (size_t)e + k];
+            dhs[4 * j + k] = d.depth[n] + d.eta_n[n];
+            o[4 + k] = jac_a(d, d.eta_jac, n);
+            if (k < 2) o[12 + k] = reinterpret_cast<const real *>(d.U_n_2D)[2 * (size_t)e + k];
+            __syncwarp(lanes_below(4 * B));
+            if (k < 2 && eb + j < d.E) {
+                const real4 w = make_real4(o[0], o[1], o[2], o[3]);
+                const real dmean_inv = real(1.0) / dmax(d.Dmin, wsum(w, dhs[4 * j], dhs[4 * j + 1], dhs[4 * j + 2], dhs[4 * j + 3]));
+                real *const F = k ? d.V_filt_2D : d.U_filt_2D;
+                const real f = (F[e] * Mt_inv) * dmean_inv;
+                F[e] = f;
+                o[10 + k] = f;
+                if (k == 0) o[14] = dmean_inv;
             }
         }
+        if (act) {
+            sm[cb.jl * S + cb.z] = ur * a_old;
+            sm[cb.jl * S + L + cb.z] = vr * a_old;
+        }
         __syncthreads();
-        const long long es = eb + threadIdx.x;
-        if ((int)threadIdx.x < cb.B && es < d.E) {
-            const real *row = sm + threadIdx.x * S;
-            real su = real(0.0), sv = real(0.0);
-            for (int k = 0; k < L; ++k) {
-                su = su + row[k];
-                sv = sv + row[L + k];
-            }
-            real *o = sc + kU3Sc * threadIdx.x;
-            const real dmean_inv = o[0];
-            o[0] = su * dmean_inv;
-            o[1] = sv * dmean_inv;
+        // one thread per (element, component): the level sums in level order
+        if ((int)threadIdx.x < 2 * B && eb + (threadIdx.x >> 1) < d.E) {
+            const int j = threadIdx.x >> 1, c = threadIdx.x & 1;
+            const real *row = sm + j * S + c * L;
+            real su = real(0.0);
+            for (int k = 0; k < L; ++k) su = su + row[k];
+            real *o = sc + kU3Sc * j;
+            o[8 + c] = su * o[14];
         }
         __syncthreads();
         if (act) {
             const int z = cb.z;
             const real *o = sc + kU3Sc * cb.jl;
-            const real U2p = o[0], V2p = o[1], uf = o[2], vf = o[3];
-            const real4 w = make_real4(o[4], o[5], o[6], o[7]);
-            const real4 an = make_real4(o[8], o[9], o[10], o[11]);
+            const real U2p = o[8], V2p = o[9], uf = o[10], vf = o[11];
+            const real4 w = make_real4(o[0], o[1], o[2], o[3]);
+            const real4 an = make_real4(o[4], o[5], o[6], o[7]);
             const real jn = je_of(d, w, an, z);
             const real az = a_old / jn;
             d.U_n_filt[i] = az * ur + uf - U2p;
@@ -840,48 +895,81 @@ __global__ void __maxnreg__(48) k_update3d(Dev d, real Mt_inv) {
 
 // vert_vel_sigma (fv_3D_vel.F90:309-456): column block per node; the layer
 // transport divergence of (node, level) gathered over the node's edges in
-// edge order, then summed upward from the bottom per node.
+// edge order, then summed upward from the bottom per node.  The edge lists
+// of a block's consecutive nodes are one contiguous range: its entries (side,
+// elements, edge_cross, the elements' filtered 2D velocities; three dependent
+// loads, the same for all levels) are staged in shared memory, kWvEdges per
+// node on average; a block with more reads them where they are used.
+// Blocks of 160 threads: 1.05 M nodes 0.82 -> 0.69 ms, 232 k FP32 0.167 ->
+// 0.134, 40 k, 30 layers 0.070 -> 0.050.
+constexpr int kWvEdges = 8;
+struct WvEdge {
+    real X[4], uf1, vf1, uf2, vf2;
+    int code, e1, e2, pad;
+};
+__device__ __forceinline__ WvEdge wv_edge(const Dev &d, int p) {
+    WvEdge w;
+    w.code = d.node_eidx[p];
+    const int ed = w.code >> 1;
+    const int2 et = d.edge_tri[ed];
+    const real4 X = d.edge_cross[ed];
+    w.X[0] = X.x; w.X[1] = X.y; w.X[2] = X.z; w.X[3] = X.w;
+    w.e1 = et.x;
+    w.e2 = ed < d.Ed_in ? et.y : -1;
+    w.uf1 = d.U_filt_2D[et.x];
+    w.vf1 = d.V_filt_2D[et.x];
+    w.uf2 = w.e2 >= 0 ? d.U_filt_2D[et.y] : real(0.0);
+    w.vf2 = w.e2 >= 0 ? d.V_filt_2D[et.y] : real(0.0);
+    return w;
+}
+__device__ __forceinline__ real wv_add(const Dev &d, real W, const WvEdge &w, int z) {
+    const size_t i1 = (size_t)w.e1 * d.L + z;
+    real c1 = d.Je[i1] * ((d.V_n_filt[i1] - w.vf1) * w.X[0] - (d.U_n_filt[i1] - w.uf1) * w.X[1]);
+    if (w.e2 >= 0) {
+        const size_t i2 = (size_t)w.e2 * d.L + z;
+        c1 = c1 + d.Je[i2] * (-(d.V_n_filt[i2] - w.vf2) * w.X[2] + (d.U_n_filt[i2] - w.uf2) * w.X[3]);
+    }
+    return (w.code & 1) ? W - c1 : W + c1;
+}
 __global__ void k_wvel(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
-    real *sm = reinterpret_cast<real *>(sm_raw);
     const int L = d.L, NS = d.NS;
     const ColBlock cb(d);
-    const int S = L | 1;
-    real *sc = sm + (size_t)cb.B * S;  // per node: bottom Wvel, 1/area
-    for (long long nb = (long long)blockIdx.x * cb.B; nb < d.N; nb += (long long)gridDim.x * cb.B) {
+    const int S = L | 1, B = cb.B;
+    WvEdge *const ed = reinterpret_cast<WvEdge *>(sm_raw);   // kWvEdges * B entries
+    real *const sm = reinterpret_cast<real *>(ed + kWvEdges * B);
+    real *const sc = sm + (size_t)B * S;  // per node: bottom Wvel, 1/area
+    for (long long nb = (long long)blockIdx.x * B; nb < d.N; nb += (long long)gridDim.x * B) {
         const long long n_ = nb + cb.jl;
-        const bool act = cb.jl < cb.B && n_ < d.N;
+        const bool act = cb.jl < B && n_ < d.N;
+        const int q0 = d.node_eptr[nb], q1 = d.node_eptr[nb + B < d.N ? nb + B : d.N];
+        const bool staged = q1 - q0 <= kWvEdges * B;
+        if (staged)
+            for (int t = threadIdx.x; t < q1 - q0; t += blockDim.x) ed[t] = wv_edge(d, q0 + t);
+        if (act && cb.z == 0) {
+            sc[2 * cb.jl] = d.Wvel[(size_t)n_ * NS + NS - 1];
+            sc[2 * cb.jl + 1] = real(1.0) / d.area[n_];
+        }
+        int p0 = 0, p1 = 0;
         if (act) {
-            const int n = (int)n_, z = cb.z;
-            if (z == 0) {
-                sc[2 * cb.jl] = d.Wvel[(size_t)n * NS + NS - 1];
-                sc[2 * cb.jl + 1] = real(1.0) / d.area[n];
-            }
-            const int p0 = d.node_eptr[n], p1 = d.node_eptr[n + 1];
+            p0 = d.node_eptr[n_];
+            p1 = d.node_eptr[n_ + 1];
+        }
+        __syncthreads();
+        if (act) {
             real W = real(0.0);
+            if (staged) {
 #pragma unroll 4
-            for (int p = p0; p < p1; ++p) {
-                const int code = d.node_eidx[p];
-                const int ed = code >> 1;
-                const int2 et = d.edge_tri[ed];
-                const real4 X = d.edge_cross[ed];
-                const real uf1 = d.U_filt_2D[et.x], vf1 = d.V_filt_2D[et.x];
-                const size_t i1 = (size_t)et.x * L + z;
-                real c1 = d.Je[i1] * ((d.V_n_filt[i1] - vf1) * X.x - (d.U_n_filt[i1] - uf1) * X.y);
-                if (ed < d.Ed_in) {
-                    const real uf2 = d.U_filt_2D[et.y], vf2 = d.V_filt_2D[et.y];
-                    const size_t i2 = (size_t)et.y * L + z;
-                    c1 = c1 + d.Je[i2] * (-(d.V_n_filt[i2] - vf2) * X.z + (d.U_n_filt[i2] - uf2) * X.w);
-                }
-                if (code & 1) W = W - c1;
-                else W = W + c1;
+                for (int p = p0; p < p1; ++p) W = wv_add(d, W, ed[p - q0], cb.z);
+            } else {
+                for (int p = p0; p < p1; ++p) W = wv_add(d, W, wv_edge(d, p), cb.z);
             }
-            sm[cb.jl * S + z] = W;
+            sm[cb.jl * S + cb.z] = W;
         }
         __syncthreads();
         const long long ns = nb + threadIdx.x;
-        if ((int)threadIdx.x < cb.B && ns < d.N) {
+        if ((int)threadIdx.x < B && ns < d.N) {
             real *row = sm + threadIdx.x * S;
             real below = sc[2 * threadIdx.x];
             for (int k = L - 1; k >= 0; --k) {
@@ -1076,35 +1164,35 @@ static bool implvisc_tiled(const Dev &d) {
 }
 
 // ---- launch wrappers --------------------------------------------------------
-// column blocks: B = min(16, 1024 / L) entities, B * L threads
+// Column blocks: B entities, B * L threads, about 160 of them (at most 16
+// entities): the barriers between staging, levels and level sums then hold
+// up 5 warps of an SM's 40, not 10 of 30 (blocks of 320 threads, 1.05 M nodes:
+// update3d 0.63 against 0.60 ms, wvel 0.78 / 0.69).  The grid is the blocks
+// resident at once; they stride over the entities.
 static int col_b(const Dev &d) {
-    if (d.tune[TK_COLUMNS] > 0) return d.tune[TK_COLUMNS];
-    int b = 1024 / d.L;
-    return b > 16 ? 16 : b;
+    return d.tune[TK_COLUMNS] > 0 ? d.tune[TK_COLUMNS] : default_columns(d.L);
 }
-static int col_grid(const Dev &d, long long count) {
-    const long long blocks = (count + col_b(d) - 1) / col_b(d);
-    return (int)(blocks < 148LL * 8 ? blocks : 148LL * 8);
+static size_t pressure_smem(const Dev &d) { return (size_t)col_b(d) * (d.L | 1) * sizeof(real); }
+static size_t bpg_smem(const Dev &d) {
+    return (size_t)col_b(d) * (kEsReals + 12 + 2 * d.L + 1) * sizeof(real);
 }
-static size_t col_smem(const Dev &d, int rows, int scalars) {
-    const int S = rows == 1 ? (d.L | 1) : rows * d.L + 1;
-    return ((size_t)col_b(d) * S + (size_t)col_b(d) * scalars) * sizeof(real);
+static size_t update3d_smem(const Dev &d) { return (size_t)col_b(d) * (2 * d.L + 1 + kU3Sc + 4) * sizeof(real); }
+static size_t wvel_smem(const Dev &d) {
+    return (size_t)col_b(d) * (kWvEdges * sizeof(WvEdge) + ((d.L | 1) + 2) * sizeof(real));
 }
 int config_columns(const Dev &d) {
-    const size_t big = col_smem(d, 2, kU3Sc);
-    cudaError_t e = cudaSuccess;
-    e = raise_smem_limit(k_implvisc_fic_tile, implvisc_tile_smem(d));
-    if (e == cudaSuccess) e = raise_smem_limit(k_bpg_elem, big);
-    if (e == cudaSuccess) e = raise_smem_limit(k_update3d, big);
-    if (e == cudaSuccess) e = raise_smem_limit(k_pressure_col, big);
-    if (e == cudaSuccess) e = raise_smem_limit(k_wvel, big);
+    cudaError_t e = raise_smem_limit(k_implvisc_fic_tile, implvisc_tile_smem(d));
+    if (e == cudaSuccess) e = raise_smem_limit(k_bpg_elem, bpg_smem(d));
+    if (e == cudaSuccess) e = raise_smem_limit(k_update3d, update3d_smem(d));
+    if (e == cudaSuccess) e = raise_smem_limit(k_pressure_col, pressure_smem(d));
+    if (e == cudaSuccess) e = raise_smem_limit(k_wvel, wvel_smem(d));
     return e == cudaSuccess ? 0 : 1;
 }
 void launch_pressure_col(const Dev &d, cudaStream_t s) {
-    launch_k(k_pressure_col, col_grid(d, d.N), col_b(d) * d.L, col_smem(d, 1, 0), s, d);
+    launch_resident(k_pressure_col, d.N, col_b(d), col_b(d) * d.L, pressure_smem(d), s, d);
 }
 void launch_bpg_elem(const Dev &d, cudaStream_t s) {
-    launch_k(k_bpg_elem, col_grid(d, d.E), col_b(d) * d.L, col_smem(d, 2, 0), s, d);
+    launch_resident(k_bpg_elem, d.E, col_b(d), col_b(d) * d.L, bpg_smem(d), s, d);
 }
 void launch_velgrad3d(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_VELGRAD3D, 256);
@@ -1156,9 +1244,9 @@ void launch_jac_swap(const Dev &d, cudaStream_t s) {
 }
 void launch_je(const Dev &d, cudaStream_t s) { launch_k(k_je_elem, grid_for((long long)d.E * d.L, 256), 256, 0, s, d); }
 void launch_update3d(const Dev &d, real Mt_inv, cudaStream_t s) {
-    launch_k(k_update3d, col_grid(d, d.E), col_b(d) * d.L, col_smem(d, 2, kU3Sc), s, d, Mt_inv);
+    launch_resident(k_update3d, d.E, col_b(d), col_b(d) * d.L, update3d_smem(d), s, d, Mt_inv);
 }
-void launch_wvel(const Dev &d, cudaStream_t s) { launch_k(k_wvel, col_grid(d, d.N), col_b(d) * d.L, col_smem(d, 1, 2), s, d); }
+void launch_wvel(const Dev &d, cudaStream_t s) { launch_resident(k_wvel, d.N, col_b(d), col_b(d) * d.L, wvel_smem(d), s, d); }
 
 
 // Largest block (threads) each tunable kernel of this file can launch with

@@ -708,9 +708,10 @@ void launch_el2nodes(const Dev &d, const real *Ue, const real *Ve, real *Un, rea
     const int b = tuned(d, TK_EL2NODES, 256);
     launch_k(k_el2nodes, grid_for((long long)d.N * d.L, b), b, 0, s, d, Ue, Ve, Un, Vn);
 }
-// B elements per block: B*L threads, at most 1024 and at most 32 elements;
-// per element its slot tile, 8 slot sums, 4 acc, dmean_n and 4 edge codes
-static int p1_elems(const Dev &d) { int b = 1024 / d.L; return b > 32 ? 32 : b; }
+// B elements per block, B*L threads, about 160 of them like the other column
+// kernels (up to 1024 threads before: 1.05 M nodes 0.90 -> 0.70 ms, 40 k, 30
+// layers 0.082 -> 0.054, 232 k FP32 0.133 -> 0.117); per element its slot tile, 8 slot sums, 4 acc, dmean_n and 4 edge codes
+static int p1_elems(const Dev &d) { return default_columns(d.L); }
 static size_t p1_smem(const Dev &d) {
     return (size_t)p1_elems(d) * ((2 * (kP1Slots + (d.bih_3D ? 1 : 0)) * d.L + 1 + 13) * sizeof(real) +
                                   4 * sizeof(int));
@@ -725,8 +726,7 @@ void launch_p1_edge(const Dev &d, cudaStream_t s) {
 }
 void launch_p1_elem(const Dev &d, cudaStream_t s) {
     const int B = p1_elems(d);
-    const long long blocks = ((long long)d.E + B - 1) / B;
-    launch_k(k_p1_elem, (int)(blocks < 148LL * 16 ? blocks : 148LL * 16), B * d.L, p1_smem(d), s, d);
+    launch_resident(k_p1_elem, d.E, B, B * d.L, p1_smem(d), s, d);
 }
 void launch_adv2d_edge(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ADV2D, 256);

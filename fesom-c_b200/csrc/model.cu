@@ -2245,7 +2245,6 @@ const KnobInfo kKnobs[fesomc::kTuneKnobs] = {
     {"vdiff_form", "vdiff_col", 3},
     {"implvisc_form", "implvisc", 2},
 };
-int default_columns(int L) { const int b = 1024 / L; return b > 16 ? 16 : b; }
 // knobs that pick a form or a count rather than threads per block
 bool form_knob(int k) {
     return k == fesomc::TK_COLUMNS || k == fesomc::TK_D3END || k == fesomc::TK_VDIFF || k == fesomc::TK_IMPLVISC;
