@@ -857,6 +857,15 @@ int build_mesh(fesomc_model *m, const fesomc_mesh *msh) {
         nptr[ni + 1] = (int)nidx.size();
         tvol[ni] = sum;
     }
+    // nodes whose MUSCL gradients are used: those of edges without an up- or
+    // downwind element
+    std::vector<char> fallback(N, 0);
+    for (int di = 0; di < Ed; ++di)
+        if (eud[di].x < 0 || eud[di].y < 0) fallback[edn[di].x] = fallback[edn[di].y] = 1;
+    std::vector<int> ngrad;
+    for (int i = 0; i < N; ++i)
+        if (fallback[i]) ngrad.push_back(i);
+    d.n_ngrad = (int)ngrad.size();
     // rivers and open boundary
     std::vector<int> rcount(N + 1, 0);
     for (int i = 0; i < msh->n_rivers; ++i) {
@@ -886,6 +895,7 @@ int build_mesh(fesomc_model *m, const fesomc_mesh *msh) {
         (rc = upload(m, &d.elem_iedges, iel)) || (rc = upload(m, &d.elem_sedges, sel)) ||
         (rc = upload(m, &d.edge_nodes, edn)) ||
         (rc = upload(m, &d.edge_tri, edt)) || (rc = upload(m, &d.edge_updn, eud)) ||
+        (rc = upload(m, &d.ngrad_nodes, ngrad)) ||
         (rc = upload(m, &d.node_eptr, eptr)) || (rc = upload(m, &d.node_eidx, eidx)) ||
         (rc = upload(m, &d.node_nptr, nptr)) || (rc = upload(m, &d.node_nidx, nidx)) ||
         (rc = upload(m, &d.node_bptr, bptr)) || (rc = upload(m, &d.node_bidx, bidx)) ||
@@ -1035,6 +1045,7 @@ int setup_f32_view(fesomc_model *m) {
     b.elem_nodes = a.elem_nodes; b.elem_nb = a.elem_nb; b.elem_edges = a.elem_edges; b.elem_iedges = a.elem_iedges;
     b.elem_sedges = a.elem_sedges;
     b.edge_nodes = a.edge_nodes; b.edge_tri = a.edge_tri; b.edge_updn = a.edge_updn;
+    b.n_ngrad = a.n_ngrad; b.ngrad_nodes = a.ngrad_nodes;
     b.node_eptr = a.node_eptr; b.node_eidx = a.node_eidx; b.node_nptr = a.node_nptr; b.node_nidx = a.node_nidx;
     b.node_bptr = a.node_bptr; b.node_bidx = a.node_bidx; b.node_rptr = a.node_rptr; b.node_ridx = a.node_ridx;
     b.obn_of_node = a.obn_of_node; b.index_nod2D = a.index_nod2D;
@@ -1154,7 +1165,10 @@ double kernel_bytes_fp64(const fesomc_model *m, const std::string &k) {
     if (k == "upwind_h")
         return L * N * 16 + L * E * 24 + NS * N * 8 + L * N * 16 + N * 28 + 4 * nnz_ne + Ed * 48 + L * N * 32;
     if (k == "muscl_egrad") return L * N * 16 + E * 80 + L * E * 32;
-    if (k == "muscl_ngrad") return L * E * 32 + N * 4 + 4 * (4.0 * E) + E * 8 + L * N * 32;
+    if (k == "muscl_ngrad") {   // the listed nodes and, about four each, their elements
+        const double n = d.n_ngrad;
+        return n * (8 + 4 * 4 + 4 * 8) + L * n * 4 * 32 + L * n * 32;
+    }
     // edge pass: AB2 tracers of the 2 end nodes and gradients (up/down
     // elements or the node fallback), Je / transports of the 2 elements,
     // edge geometry; 3 flux pairs per (edge, level) written
