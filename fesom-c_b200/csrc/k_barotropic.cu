@@ -550,122 +550,122 @@ __global__ void k_filt2x_2d(Dev d) {
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void u2d_elem(const Dev &d, int next, real d0inv, int e, const int4 en, const int4 il,
                                          const int4 nb) {
-            const int nd[4] = {en.x, en.y, en.z, en.w};
-            // elevations and total depths in FP64 (the elevation gradient and
-            // the wet/dry test with them); the momentum terms in 'real'
-            double eab[4], dep[4], etag[4];
-            for (int k = 0; k < 4; ++k) {
-                eab[k] = d.etaAB[nd[k]];
-                dep[k] = d.depth[nd[k]];
-                if (d.key_atm) {
-                    // with atmospheric forcing: E - P and the sea-level pressure
-                    // anomaly (fv_average_dynamic.F90:278-286)
-                    const double d0i = 1.0 / d.density_0_d;
-                    etag[k] = kG64 * ((double)d.atp1[nd[k]] * eab[k] - d.emp[nd[k]] * d0i -
-                                      (double)d.atp2[nd[k]] * d.ssh_gp[nd[k]]) + (kPref - d.mslp[nd[k]]) * d0i;
-                } else {
-                    etag[k] = kG64 * ((double)d.atp1[nd[k]] * eab[k] - (double)d.atp2[nd[k]] * d.ssh_gp[nd[k]]);
-                }
+    const int nd[4] = {en.x, en.y, en.z, en.w};
+    // elevations and total depths in FP64 (the elevation gradient and
+    // the wet/dry test with them); the momentum terms in 'real'
+    double eab[4], dep[4], etag[4];
+    for (int k = 0; k < 4; ++k) {
+        eab[k] = d.etaAB[nd[k]];
+        dep[k] = d.depth[nd[k]];
+        if (d.key_atm) {
+            // with atmospheric forcing: E - P and the sea-level pressure
+            // anomaly (fv_average_dynamic.F90:278-286)
+            const double d0i = 1.0 / d.density_0_d;
+            etag[k] = kG64 * ((double)d.atp1[nd[k]] * eab[k] - d.emp[nd[k]] * d0i -
+                              (double)d.atp2[nd[k]] * d.ssh_gp[nd[k]]) + (kPref - d.mslp[nd[k]]) * d0i;
+        } else {
+            etag[k] = kG64 * ((double)d.atp1[nd[k]] * eab[k] - (double)d.atp2[nd[k]] * d.ssh_gp[nd[k]]);
+        }
+    }
+    real mwd = d.mask_wd[e];
+    if (d.wet_dry_on) {
+        const double dmin4 = dmin(dmin(dep[0], dep[1]), dmin(dep[2], dep[3]));
+        const double emax4 = dmax(dmax(eab[0], eab[1]), dmax(eab[2], eab[3]));
+        mwd = (dmin4 + emax4 > d.Dmin_d) ? real(1.0) : real(0.0);
+        d.mask_wd[e] = mwd;
+    }
+    const real4 w = d.w_cv[e];
+    const real ar = d.elem_area[e];
+    const real dmean = (real)dmax(d.Dmin_d, wexp_d(w, eab[0] + dep[0], eab[1] + dep[1], eab[2] + dep[2], eab[3] + dep[3]));
+    const real4 gx = d.gs_x[e], gy = d.gs_y[e];
+    const real gex = (real)((double)gx.x * etag[0] + (double)gx.y * etag[1] + (double)gx.z * etag[2] + (double)gx.w * etag[3]);
+    const real gey = (real)((double)gy.x * etag[0] + (double)gy.y * etag[1] + (double)gy.z * etag[2] + (double)gy.w * etag[3]);
+    const real2 uab = d.UAB[e];
+    const real cor = d.coriolis[e];
+    real rx = ar * (-dmean * gex + uab.y * dmean * cor + d.taux[e] * d0inv);
+    real ry = ar * (-dmean * gey - uab.x * dmean * cor + d.tauy[e] * d0inv);
+    if (d.mom_adv_2D == 2) {
+        const int codes[4] = {il.x, il.y, il.z, il.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int code = codes[c];
+            if (code < 0) break;
+            const real2 f = d.adv2d[code >> 1];
+            if (code & 1) { rx = rx + f.x; ry = ry + f.y; }
+            else { rx = rx - f.x; ry = ry - f.y; }
+        }
+    }
+    if (d.filt_2D) {
+        const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
+        const int jend = (en.x == en.w) ? 3 : 4;
+        real u1 = real(0.0), u2 = real(0.0);
+        for (int j = 0; j < jend; ++j)
+            if (nbs[j] >= 0) {
+                const real2 un = d.UAB[nbs[j]];
+                u1 = u1 + un.x - uab.x;
+                u2 = u2 + un.y - uab.y;
             }
-            real mwd = d.mask_wd[e];
-            if (d.wet_dry_on) {
-                const double dmin4 = dmin(dmin(dep[0], dep[1]), dmin(dep[2], dep[3]));
-                const double emax4 = dmax(dmax(eab[0], eab[1]), dmax(eab[2], eab[3]));
-                mwd = (dmin4 + emax4 > d.Dmin_d) ? real(1.0) : real(0.0);
-                d.mask_wd[e] = mwd;
-            }
-            const real4 w = d.w_cv[e];
-            const real ar = d.elem_area[e];
-            const real dmean = (real)dmax(d.Dmin_d, wexp_d(w, eab[0] + dep[0], eab[1] + dep[1], eab[2] + dep[2], eab[3] + dep[3]));
-            const real4 gx = d.gs_x[e], gy = d.gs_y[e];
-            const real gex = (real)((double)gx.x * etag[0] + (double)gx.y * etag[1] + (double)gx.z * etag[2] + (double)gx.w * etag[3]);
-            const real gey = (real)((double)gy.x * etag[0] + (double)gy.y * etag[1] + (double)gy.z * etag[2] + (double)gy.w * etag[3]);
-            const real2 uab = d.UAB[e];
-            const real cor = d.coriolis[e];
-            real rx = ar * (-dmean * gex + uab.y * dmean * cor + d.taux[e] * d0inv);
-            real ry = ar * (-dmean * gey - uab.x * dmean * cor + d.tauy[e] * d0inv);
-            if (d.mom_adv_2D == 2) {
-                const int codes[4] = {il.x, il.y, il.z, il.w};
-    #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int code = codes[c];
-                    if (code < 0) break;
-                    const real2 f = d.adv2d[code >> 1];
-                    if (code & 1) { rx = rx + f.x; ry = ry + f.y; }
-                    else { rx = rx - f.x; ry = ry - f.y; }
-                }
-            }
-            if (d.filt_2D) {
-                const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
-                const int jend = (en.x == en.w) ? 3 : 4;
-                real u1 = real(0.0), u2 = real(0.0);
-                for (int j = 0; j < jend; ++j)
-                    if (nbs[j] >= 0) {
-                        const real2 un = d.UAB[nbs[j]];
-                        u1 = u1 + un.x - uab.x;
-                        u2 = u2 + un.y - uab.y;
-                    }
-                const real sd = (real)wsum_d(w, dep[0], dep[1], dep[2], dep[3]);
-                rx = rx + d.tau_inv_filt * u1 * ar * sd;
-                ry = ry + d.tau_inv_filt * u2 * ar * sd;
-            }
-            // biharmonic_2D: the second-pass edge fluxes in edge order
-            if (d.bih_2D) {
-                const int4 se = d.elem_sedges[e];
-                const int codes[4] = {se.x, se.y, se.z, se.w};
-                for (int c = 0; c < 4; ++c) {
-                    const int code = codes[c];
-                    if (code < 0) break;
-                    const real2 f = d.b2fl[code >> 1];
-                    if (code & 1) { rx = rx - f.x; ry = ry - f.y; }
-                    else { rx = rx + f.x; ry = ry + f.y; }
-                }
-            }
-            const real2 r3 = d.U_rhs_2D_3D[e];
-            rx = rx + r3.x;
-            ry = ry + r3.y;
-            // final update with implicit bottom drag
-            double eo[4], enw[4];
-            for (int k = 0; k < 4; ++k) { eo[k] = d.eta_n[nd[k]]; enw[k] = d.eta_new[nd[k]]; }
-            const real dmo = (real)dmax(d.Dmin_d, wsum_d(w, eo[0] + dep[0], eo[1] + dep[1], eo[2] + dep[2], eo[3] + dep[3]));
-            const real4 bf = d.bfric[e];
-            const real ub = bf.x, vb = bf.y, friction = bf.z;
-            const real ff = real(1.0) / ((real)dmax(d.Dmin_d, wsum_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]))
-                                     + friction * d.dt_2D);
-            const real dt2 = d.dt_2D;
-            const real2 u0 = d.U_n_2D[e];
-            const real2 bp = d.Bar_pr_2D[e];
-            // UV2_rhs of viscosity_filt2x_2D (zero when it is off)
-            real uvx = real(0.0), uvy = real(0.0);
-            if (d.filt_bi_2D) {
-                const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
-                const real2 c0 = d.f2uv2d[e];
-                for (int j = 0; j < 4; ++j) {
-                    const int ne = nbs[j];
-                    if (!(ne >= 0 && (j < 3 || ne != nbs[0]))) continue;
-                    const real2 c2 = d.f2uv2d[ne];
-                    if (j == 0) { uvx = -c0.x + c2.x; uvy = -c0.y + c2.y; }
-                    else { uvx = uvx - c0.x + c2.x; uvy = uvy - c0.y + c2.y; }
-                }
-            }
-            const real nx = mwd * ((dmo * u0.x - dt2 * friction * (ub - u0.x) + dt2 * bp.x + dt2 * rx / ar) * ff + uvx);
-            const real ny = mwd * ((dmo * u0.y - dt2 * friction * (vb - u0.y) + dt2 * bp.y + dt2 * ry / ar) * ff + uvy);
-            // rotate U_n_2 <- U_n_1 <- U_n_2D <- new (fv_main.F90:1569-1578)
-            const real2 u1 = d.U_n_1[e];
-            d.U_n_2[e] = u1;
-            d.U_n_1[e] = u0;
-            d.U_n_2D[e] = make_real2(nx, ny);
-            // U_filt accumulation with the new elevation (fv_main.F90:1596-1605)
-            const real dmn = (real)dmax(d.Dmin_d, wexp_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]));
-            d.U_filt_2D[e] = d.U_filt_2D[e] + nx * dmn;
-            d.V_filt_2D[e] = d.V_filt_2D[e] + ny * dmn;
-            // the next sub-step's AB3 velocity and mean total depth
-            if (next) {
-                d.UAB_next[e] = ab3v(d.beta, make_real2(nx, ny), u0, u1);
-                double em[4];
-                for (int k = 0; k < 4; ++k) em[k] = d.eta_n_1[nd[k]];
-                d.aux_elem[e] = aux_of(d, w, enw, eo, em, dep);
-            }
+        const real sd = (real)wsum_d(w, dep[0], dep[1], dep[2], dep[3]);
+        rx = rx + d.tau_inv_filt * u1 * ar * sd;
+        ry = ry + d.tau_inv_filt * u2 * ar * sd;
+    }
+    // biharmonic_2D: the second-pass edge fluxes in edge order
+    if (d.bih_2D) {
+        const int4 se = d.elem_sedges[e];
+        const int codes[4] = {se.x, se.y, se.z, se.w};
+        for (int c = 0; c < 4; ++c) {
+            const int code = codes[c];
+            if (code < 0) break;
+            const real2 f = d.b2fl[code >> 1];
+            if (code & 1) { rx = rx - f.x; ry = ry - f.y; }
+            else { rx = rx + f.x; ry = ry + f.y; }
+        }
+    }
+    const real2 r3 = d.U_rhs_2D_3D[e];
+    rx = rx + r3.x;
+    ry = ry + r3.y;
+    // final update with implicit bottom drag
+    double eo[4], enw[4];
+    for (int k = 0; k < 4; ++k) { eo[k] = d.eta_n[nd[k]]; enw[k] = d.eta_new[nd[k]]; }
+    const real dmo = (real)dmax(d.Dmin_d, wsum_d(w, eo[0] + dep[0], eo[1] + dep[1], eo[2] + dep[2], eo[3] + dep[3]));
+    const real4 bf = d.bfric[e];
+    const real ub = bf.x, vb = bf.y, friction = bf.z;
+    const real ff = real(1.0) / ((real)dmax(d.Dmin_d, wsum_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]))
+                             + friction * d.dt_2D);
+    const real dt2 = d.dt_2D;
+    const real2 u0 = d.U_n_2D[e];
+    const real2 bp = d.Bar_pr_2D[e];
+    // UV2_rhs of viscosity_filt2x_2D (zero when it is off)
+    real uvx = real(0.0), uvy = real(0.0);
+    if (d.filt_bi_2D) {
+        const int nbs[4] = {nb.x, nb.y, nb.z, nb.w};
+        const real2 c0 = d.f2uv2d[e];
+        for (int j = 0; j < 4; ++j) {
+            const int ne = nbs[j];
+            if (!(ne >= 0 && (j < 3 || ne != nbs[0]))) continue;
+            const real2 c2 = d.f2uv2d[ne];
+            if (j == 0) { uvx = -c0.x + c2.x; uvy = -c0.y + c2.y; }
+            else { uvx = uvx - c0.x + c2.x; uvy = uvy - c0.y + c2.y; }
+        }
+    }
+    const real nx = mwd * ((dmo * u0.x - dt2 * friction * (ub - u0.x) + dt2 * bp.x + dt2 * rx / ar) * ff + uvx);
+    const real ny = mwd * ((dmo * u0.y - dt2 * friction * (vb - u0.y) + dt2 * bp.y + dt2 * ry / ar) * ff + uvy);
+    // rotate U_n_2 <- U_n_1 <- U_n_2D <- new (fv_main.F90:1569-1578)
+    const real2 u1 = d.U_n_1[e];
+    d.U_n_2[e] = u1;
+    d.U_n_1[e] = u0;
+    d.U_n_2D[e] = make_real2(nx, ny);
+    // U_filt accumulation with the new elevation (fv_main.F90:1596-1605)
+    const real dmn = (real)dmax(d.Dmin_d, wexp_d(w, enw[0] + dep[0], enw[1] + dep[1], enw[2] + dep[2], enw[3] + dep[3]));
+    d.U_filt_2D[e] = d.U_filt_2D[e] + nx * dmn;
+    d.V_filt_2D[e] = d.V_filt_2D[e] + ny * dmn;
+    // the next sub-step's AB3 velocity and mean total depth
+    if (next) {
+        d.UAB_next[e] = ab3v(d.beta, make_real2(nx, ny), u0, u1);
+        double em[4];
+        for (int k = 0; k < 4; ++k) em[k] = d.eta_n_1[nd[k]];
+        d.aux_elem[e] = aux_of(d, w, enw, eo, em, dep);
+    }
 }
 // FP32: 8 resident blocks (at most 64 registers); FP64: 6.
 __global__ void __launch_bounds__(128, FESOMC_FP32 ? 8 : 6) k_u2d_elem(Dev d, int next) {
@@ -745,7 +745,10 @@ void launch_bih_2d(const Dev &d, cudaStream_t s) {
 void launch_u2d_elem(const Dev &d, int next, cudaStream_t s) {
     const int b = tuned(d, TK_U2D, 128);
     const int g = grid_for(d.E, b);
-    if (early_grid(g)) launch_k(k_u2d_elem_head, g, b, 0, s, d, next);
+    // the form of one element per thread holds 102 registers instead of
+    // spilling at 80; it also wins while all of its blocks are resident (42 k
+    // nodes 0.177 -> 0.169 ms per step, 40 k 0.129 -> 0.117)
+    if (g <= 4 * 148 && (long long)g * b >= d.E) launch_k(k_u2d_elem_head, g, b, 0, s, d, next);
     else launch_k(k_u2d_elem, g, b, 0, s, d, next);
 }
 
