@@ -206,10 +206,10 @@ __global__ void k_d3end(Dev d, const int *list, const unsigned long long *count)
 // interface) each: the set-up (the two densityJM and the divisions of b1,
 // b2, c2, Ri: most of the FP64 work), the sweep-invariant am and cm, in
 // every sweep the divisions of c1 and bm, and the final bt, snu, Kv and
-// tke_dissip.  Only the recurrences of the sweep (two divisions per level,
-// in parallel) and the back substitution are left to one thread per column,
-// all of one warp; which warp alternates between the blocks of an SM, so
-// that their chains run on different schedulers.  The arithmetic and its
+// tke_dissip.  Only the recurrences of the sweep and the back substitution
+// are left to one or two lanes per column, all of one or two warps; which
+// ones alternates between the blocks of an SM, so that their chains run on
+// different schedulers.  The arithmetic and its
 // order are k_d3end's.
 //
 // Shared memory, [array][interface][column] with an odd column stride, so
@@ -220,17 +220,23 @@ __global__ void k_d3end(Dev d, const int *list, const unsigned long long *count)
 // m holds bm(m), then xx1(m+1), then btr1(m), each written when the one
 // before has been read.
 //
-// Bound by latency: the FP64 chains of the recurrences and of the set-up
-// (FP64 pipe 29 %, barrier and dependency waits) at the 4 blocks of 32
-// columns (21 interfaces, FP64) that shared memory holds per SM; 256 threads
-// and 64 registers for the most warps on the set-up.  FP32 tiles are half
-// the size: 128 threads, more blocks.  Against one thread per column with its arrays in
-// local memory (whose traffic streamed through DRAM): 1.05 M nodes FP64 2.71
-// -> 2.30 ms, 232 k FP32 0.31 -> 0.18, 40 k with 31 interfaces 0.23 -> 0.18,
-// 16 k with 11 0.046 -> 0.031, 4.5 k with 40 0.196 -> 0.050 ms.  A set-up
-// kernel and a sweep kernel with the sweep's arrays in local memory, shared
-// memory or registers took 2.32-2.54 ms, 0.25-0.30, 0.19, 0.046-0.055 and
-// 0.11 ms.  128 threads or tiles of 16 at 1.05 M nodes: 2.54 and 2.65 ms.
+// Bound by latency, the chains of the recurrences first (with one lane per
+// column and the convergence test in its loop they took 47 % of a block's
+// time, 640 cycles a level: an FP64 division is 114 cycles, and two of them
+// in one thread run one after the other), then the set-up's divisions.  In
+// FP64 a pair of lanes forms xx1 and yy1 of a column at the same time, the
+// test is done by all threads afterwards, and a layer's density at its two
+// interfaces shares the terms without the pressure; FP32, whose divisions are
+// short, keeps one lane and the test in its loop.  FP64: 256 threads and 64
+// registers, four blocks of 32 columns (21 interfaces) per SM by shared
+// memory; FP32 tiles are half the size: 128 threads, more blocks.
+// Against one thread per column with its arrays in local memory (whose
+// traffic streamed through DRAM): 1.05 M nodes FP64 2.71 -> 2.03 ms (2.31 with
+// one lane per column), 42 k 0.134 -> 0.107, 40 k with 31 interfaces 0.23 ->
+// 0.146, 16 k with 11 0.046 -> 0.028, 4.5 k with 40 0.196 -> 0.039, 232 k FP32
+// 0.31 -> 0.19 ms.  A set-up kernel and a sweep kernel with the sweep's arrays
+// in local memory, shared memory or registers took 2.32-2.54 ms at 1.05 M
+// nodes, 128 threads or tiles of 16 2.54 and 2.65.
 constexpr int kT3Arrays = 9;
 constexpr int kT3Threads = FESOMC_FP32 ? 128 : 256;
 #if FESOMC_FP32
@@ -239,7 +245,7 @@ constexpr int kT3Threads = FESOMC_FP32 ? 128 : 256;
 #define D3_TILE_BOUNDS __launch_bounds__(kT3Threads, 4)
 #endif
 static size_t d3end_tile_smem(const Dev &d, int cols) {
-    return ((size_t)kT3Arrays * d.NS * (cols + 1) + 2 * cols) * sizeof(real) + 3 * cols * sizeof(int);
+    return ((size_t)kT3Arrays * d.NS * (cols + 1) + 2 * cols) * sizeof(real) + 4 * cols * sizeof(int);
 }
 
 template <int C, bool kList>
@@ -254,13 +260,23 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
     real *const s_pb = s_sn + 3 * A, *const s_qb = s_sn + 4 * A, *const s_c2 = s_sn + 5 * A;
     real *const s_am = s_sn + 6 * A, *const s_cm = s_sn + 7 * A, *const s_fy = s_sn + 8 * A;
     real *const s_dm = s_sn + 9 * A, *const s_aj = s_dm + C;
-    int *const s_node = reinterpret_cast<int *>(s_aj + C), *const s_done = s_node + C, *const s_par = s_done + C;
+    int *const s_node = reinterpret_cast<int *>(s_aj + C), *const s_done = s_node + C, *const s_par = s_done + C, *const s_above = s_par + C;
     const real t_inv = real(1.0) / d.dt;
     const real cka = d.cka;
     const real B1cka2 = real(16.6) * (cka * cka);
     const int ncol = kList ? (int)*count : d.N;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool mine = warp == (int)((blockIdx.x / 148) % (kT3Threads / 32));   // the warp of the recurrences
+    // the warps of the recurrences: FP32 one lane, FP64 a pair of lanes per
+    // column
+#if FESOMC_FP32
+    const int lane = threadIdx.x & 31;
+    const bool mine = (int)(threadIdx.x >> 5) == (int)((blockIdx.x / 148) % (kT3Threads / 32));
+#else
+    constexpr int kChains = C / 16, kWarps = kT3Threads / 32;
+    static_assert(kWarps % kChains == 0, "the warps of the recurrences lie side by side");
+    const int w0 = (int)(kChains * (blockIdx.x / 148) % kWarps), cw = (int)(threadIdx.x >> 5) - w0;
+    const int lane = cw * 16 + (int)(threadIdx.x & 31) / 2;   // column
+    const bool mine = cw >= 0 && cw < kChains;
+#endif
     for (int n0 = blockIdx.x * C; n0 < ncol; n0 += gridDim.x * C) {
         const int nt = ncol - n0 < C ? ncol - n0 : C;
         if ((int)threadIdx.x < nt) {
@@ -271,6 +287,20 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
             s_done[threadIdx.x] = 0;
         }
         __syncthreads();
+#if !FESOMC_FP32
+        // each layer's density at its two interfaces, one (column, layer) per
+        // thread: the terms without the pressure serve both.  Layer m is below
+        // interface m (rho_dn of m, in s_qb) and above m + 1 (rho_up, in s_pb).
+        for (int i = threadIdx.x; i < nt * L; i += kT3Threads) {
+            const int j = d.by_L.div(i), m = i - j * L;
+            const size_t gl = (size_t)s_node[j] * L + m;
+            const DensityJM rho(d.TF[gl], d.SF[gl]);
+            const int o = m * CP + j;
+            if (m > 0) s_qb[o] = rho.at(-zbar_of(d, s_aj[j], m), d.density_0);
+            if (m < L - 1) s_pb[o + CP] = rho.at(-zbar_of(d, s_aj[j], m + 1), d.density_0);
+        }
+        __syncthreads();
+#endif
         // set-up, one (column, interface) per thread; k = nz - 1
         for (int i = threadIdx.x; i < nt * NS; i += kT3Threads) {
             const int j = d.by_NS.div(i), k = i - j * NS;
@@ -295,9 +325,13 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
             const real ap2 = d.Vnode[gl - 1] - d.Vnode[gl];
             real b1 = div_pos(sn_0 * (ap1 * ap1 + ap2 * ap2), dd * dd);
             b1 = div_pos(b1, dmean2);
+#if FESOMC_FP32
             const real zb = zbar_of(d, s_aj[j], k);
             const real rho_up = density_jm(d.TF[gl - 1], d.SF[gl - 1], -zb, d.density_0);
             const real rho_dn = density_jm(d.TF[gl], d.SF[gl], -zb, d.density_0);
+#else
+            const real rho_up = s_pb[o], rho_dn = s_qb[o];
+#endif
             ap1 = div_pos(rho_up - rho_dn, dd);
             const real b2 = div_pos(-real(0.5) * kG * d.Kv[g] * ap1, d.density_0 * dmean);
             const real snu_p = real(0.5) * (sn_m + sn_0);
@@ -345,6 +379,7 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
                 bx[o] = s_am[o] + s_cm[o] + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
             }
             __syncthreads();
+#if FESOMC_FP32
             if (open) {
                 const real *am_ = s_am + lane, *cm_ = s_cm + lane, *bo = bt + lane;
                 real *X = bx + lane, *Y = s_fy + lane;
@@ -385,6 +420,68 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
                     open = false;
                 }
             }
+#else
+            if (mine) {
+                // forward: the lanes of a pair form xx1 and yy1, one division
+                // each at the same time, and share xx1 (__shfl needs every
+                // lane: columns that have converged run along on lane 0's)
+                const int role = threadIdx.x & 1, c = lane < nt ? lane : 0;
+                const real *am_ = s_am + c, *bm_ = bx + c, *nu_ = (role ? s_fy : s_cm) + c;
+                real *const out = (role ? s_fy : bx) + c;
+                real x = real(1.0), y = y2;
+                real am_n = am_[CP], bm_n = bm_[CP], nu_n = nu_[CP];
+                for (int k = 1; k <= NS - 2; ++k) {
+                    const real am = am_n, bm = bm_n, nu = nu_n;
+                    const int kn = (k < NS - 2 ? k + 1 : k) * CP;
+                    am_n = am_[kn]; bm_n = bm_[kn]; nu_n = nu_[kn];
+                    const real a = bm - am * x;
+                    const real q = (role ? am * y - nu : nu) / a;
+                    x = __shfl_sync(kFull, q, threadIdx.x & 30);
+                    y = q;
+                    if (open) out[k * CP] = q;   // xx1(nz+1) and yy1(nz+1), nz = k + 1
+                }
+                __syncwarp();
+                if (open && !(threadIdx.x & 1)) {
+                    real *X = bx + lane;
+                    const real *Y = s_fy + lane;
+                    real b1v = bot;  // btr1(NS)
+                    X[(NS - 1) * CP] = b1v;
+                    real x_n = X[(NS - 2) * CP], y_n = Y[(NS - 2) * CP];
+                    for (int k = NS - 2; k >= 1; --k) {
+                        const real xv = x_n, yv = y_n;
+                        const int kn = (k > 1 ? k - 1 : k) * CP;
+                        x_n = X[kn]; y_n = Y[kn];
+                        b1v = b1v * xv + yv;  // btr1(k+1), into the slot of xx1(k+2)
+                        X[k * CP] = b1v;
+                    }
+                    X[0] = b1v * real(1.0) + y2;
+                    s_above[lane] = 0;
+                }
+            }
+            __syncthreads();
+            // the convergence test, one (column, interface) per thread
+            for (int i = threadIdx.x; i < C * NS; i += kT3Threads) {
+                const int j = i % C, k = i / C;
+                if (j >= nt || s_done[j]) continue;
+                const real ov = bt[k * CP + j], nv = bx[k * CP + j];
+                if (d3_above_tol(ov - nv, dmax(nv, ov) + real(1.0e-8))) s_above[j] = 1;
+            }
+            __syncthreads();
+            if (open) {
+                const bool above = s_above[lane] != 0;
+                if (!above || it == 200) {
+                    // the final btr: the previous iterate when the sweep
+                    // converges, else the last sweep's
+                    if (!(threadIdx.x & 1)) {
+                        s_par[lane] = above ? par ^ 1 : par;
+                        s_done[lane] = above ? 2 : 1;
+                        if (above) atomicAdd(d.notconv, 1);
+                        if (d.d3_iters) d.d3_iters[s_node[lane]] = it;   // measurement only (fesomc_gpu_d3end_iterations)
+                    }
+                    open = false;
+                }
+            }
+#endif
             par ^= 1;
             if (!__syncthreads_or(open)) break;
         }
