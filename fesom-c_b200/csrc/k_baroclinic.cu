@@ -645,8 +645,8 @@ __global__ void __launch_bounds__(256, 4) k_velrhs(Dev d, real ff) {
 }
 
 // ---------------------------------------------------------------------------
-// implvisc: momentum_vert_impl_visc_tmp (fv_viscosity.F90:1374-1486, no ice)
-// or momentum_vert_impl_visc (fv_viscosity.F90:1266-1371); thread per column.
+// implvisc: momentum_vert_impl_visc (fv_viscosity.F90:1266-1371), thread per
+// column; the fic variant is k_implvisc_fic_tile.
 // ---------------------------------------------------------------------------
 template <int MAXL>
 __global__ void k_implvisc(Dev d) {
@@ -662,117 +662,54 @@ __global__ void k_implvisc(Dev d) {
         const real ub = d.U_n[(size_t)e * L + L - 1], vb = d.V_n[(size_t)e * L + L - 1];
         const real a_Cd = d.C_d * ((real(1.0) - d.elem_acc[e]) * d.Cd_bz + real(1.0));
         const real *je = d.Je + (size_t)e * L;
-        if (d.im_vert_visc) {
-            real a[MAXL], b[MAXL], c[MAXL], cp[MAXL], up[MAXL], vp[MAXL], uu[MAXL], vv[MAXL];
-            const real *zc = d.Ze + (size_t)e * L;
-            for (int z = 1; z <= L - 2; ++z) {
-                const real zinv = dt / je[z];
-                a[z] = -Av[z] / (zc[z] - zc[z - 1]) * zinv;
-                c[z] = -Av[z + 1] / (zc[z + 1] - zc[z]) * zinv;
-                b[z] = -a[z] - c[z] + real(1.0);
-            }
-            real zinv = dt / je[L - 1];
-            a[L - 1] = -Av[L - 1] / (zc[L - 1] - zc[L - 2]) * zinv;
-            b[L - 1] = -a[L - 1] + real(1.0);
-            c[L - 1] = real(0.0);
-            zinv = dt / je[0];
-            c[0] = -Av[1] / (zc[1] - zc[0]) * zinv;
-            a[0] = real(0.0);
-            b[0] = -c[0] + real(1.0);
-            for (int z = 0; z < L; ++z) { uu[z] = ur[z]; vv[z] = vr[z]; }
-            uu[0] = uu[0] + zinv * d.taux[e] / d.density_0;
-            vv[0] = vv[0] + zinv * d.tauy[e] / d.density_0;
-            zinv = dt / je[L - 1];
-            const real friction = -a_Cd * sqrt(ub * ub + vb * vb);
-            uu[L - 1] = uu[L - 1] + zinv * friction * ub;
-            vv[L - 1] = vv[L - 1] + zinv * friction * vb;
-            // the recurrences carry their last value in registers
-            real cpv = c[0] / b[0], upv = uu[0] / b[0], vpv = vv[0] / b[0];
-            cp[0] = cpv;
-            up[0] = upv;
-            vp[0] = vpv;
-            for (int z = 1; z < L; ++z) {
-                const real az = a[z];
-                const real m = b[z] - cpv * az;
-                cpv = c[z] / m;
-                upv = (uu[z] - upv * az) / m;
-                vpv = (vv[z] - vpv * az) / m;
-                cp[z] = cpv;
-                up[z] = upv;
-                vp[z] = vpv;
-            }
-            real un = upv, vn = vpv;
-            uu[L - 1] = un;
-            vv[L - 1] = vn;
-            for (int z = L - 2; z >= 0; --z) {
-                un = up[z] - cp[z] * un;
-                vn = vp[z] - cp[z] * vn;
-                uu[z] = un;
-                vv[z] = vn;
-            }
-            for (int z = 0; z < L; ++z) { ur[z] = uu[z] * mwd; vr[z] = vv[z] * mwd; }
+        real a[MAXL], b[MAXL], c[MAXL], cp[MAXL], up[MAXL], vp[MAXL], uu[MAXL], vv[MAXL];
+        const real *zc = d.Ze + (size_t)e * L;
+        for (int z = 1; z <= L - 2; ++z) {
+            const real zinv = dt / je[z];
+            a[z] = -Av[z] / (zc[z] - zc[z - 1]) * zinv;
+            c[z] = -Av[z + 1] / (zc[z + 1] - zc[z]) * zinv;
+            b[z] = -a[z] - c[z] + real(1.0);
         }
-        if (d.im_vert_visc_fic) {
-            if (mwd != real(0.0)) {
-                real xx1[MAXL + 2], yu[MAXL + 2], yv[MAXL + 2];
-                xx1[0] = real(1.0);
-                real de = je[0] / (Av[0] + Av[1]);
-                const real rw = de / d.density_0;
-                yu[0] = d.taux[e] * rw;
-                yv[0] = d.tauy[e] * rw;
-                // the recurrences carry their last value in registers; the
-                // column values of the next level are loaded one level ahead
-                real xv = xx1[0], yuv = yu[0], yvv = yv[0];
-                real je_m = real(0.0), je_0 = je[0], je_p = L > 1 ? je[1] : real(0.0);
-                real av_0 = Av[0], av_p = Av[1];
-                real fx_n = ur[0], fy_n = vr[0];
-                for (int z = 0; z < L; ++z) {
-                    const real Fx = fx_n, Fy = fy_n;
-                    const real jz = je_0, jm = je_m, jp = je_p, a0 = av_0, a1 = av_p;
-                    if (z + 1 < L) {
-                        fx_n = ur[z + 1];
-                        fy_n = vr[z + 1];
-                        je_m = je_0;
-                        je_0 = je_p;
-                        if (z + 2 < L) je_p = je[z + 2];
-                        av_0 = av_p;
-                        av_p = Av[z + 2];
-                    }
-                    const real d1 = (z == 0) ? real(0.5) * jz : real(0.5) * (jz + jm);
-                    const real d2 = (z == L - 1) ? real(0.5) * jz : real(0.5) * (jz + jp);
-                    const real zt = dt / jz;
-                    const real a = zt * a0 / d1;
-                    const real c = zt * a1 / d2;
-                    const real b = a + c + real(1.0);
-                    const real dd = b - a * xv;
-                    xv = c / dd;
-                    yuv = (a * yuv + Fx) / dd;
-                    yvv = (a * yvv + Fy) / dd;
-                    xx1[z + 1] = xv;
-                    yu[z + 1] = yuv;
-                    yv[z + 1] = yvv;
-                }
-                de = je[L - 1] / (Av[NS - 1] + Av[L - 1]);
-                const real friction = de * a_Cd * sqrt(ub * ub + vb * vb);
-                real Ut, Vt;
-                if (d.fic_point == 0) { Ut = real(0.0); Vt = real(0.0); }
-                else if (d.fic_point == 1) {
-                    const real a = friction + real(1.0) - xx1[L];
-                    Ut = yu[L] / a; Vt = yv[L] / a;
-                } else {
-                    const real a = real(1.0) / (real(1.0) - friction) - xx1[L];
-                    Ut = yu[L] / a; Vt = yv[L] / a;
-                }
-                for (int z = L - 1; z >= 0; --z) {
-                    Ut = Ut * xx1[z + 1] + yu[z + 1];
-                    Vt = Vt * xx1[z + 1] + yv[z + 1];
-                    ur[z] = Ut * mwd;
-                    vr[z] = Vt * mwd;
-                }
-            } else {
-                for (int z = 0; z < L; ++z) { ur[z] = real(0.0); vr[z] = real(0.0); }
-            }
+        real zinv = dt / je[L - 1];
+        a[L - 1] = -Av[L - 1] / (zc[L - 1] - zc[L - 2]) * zinv;
+        b[L - 1] = -a[L - 1] + real(1.0);
+        c[L - 1] = real(0.0);
+        zinv = dt / je[0];
+        c[0] = -Av[1] / (zc[1] - zc[0]) * zinv;
+        a[0] = real(0.0);
+        b[0] = -c[0] + real(1.0);
+        for (int z = 0; z < L; ++z) { uu[z] = ur[z]; vv[z] = vr[z]; }
+        uu[0] = uu[0] + zinv * d.taux[e] / d.density_0;
+        vv[0] = vv[0] + zinv * d.tauy[e] / d.density_0;
+        zinv = dt / je[L - 1];
+        const real friction = -a_Cd * sqrt(ub * ub + vb * vb);
+        uu[L - 1] = uu[L - 1] + zinv * friction * ub;
+        vv[L - 1] = vv[L - 1] + zinv * friction * vb;
+        // the recurrences carry their last value in registers
+        real cpv = c[0] / b[0], upv = uu[0] / b[0], vpv = vv[0] / b[0];
+        cp[0] = cpv;
+        up[0] = upv;
+        vp[0] = vpv;
+        for (int z = 1; z < L; ++z) {
+            const real az = a[z];
+            const real m = b[z] - cpv * az;
+            cpv = c[z] / m;
+            upv = (uu[z] - upv * az) / m;
+            vpv = (vv[z] - vpv * az) / m;
+            cp[z] = cpv;
+            up[z] = upv;
+            vp[z] = vpv;
         }
+        real un = upv, vn = vpv;
+        uu[L - 1] = un;
+        vv[L - 1] = vn;
+        for (int z = L - 2; z >= 0; --z) {
+            un = up[z] - cp[z] * un;
+            vn = vp[z] - cp[z] * vn;
+            uu[z] = un;
+            vv[z] = vn;
+        }
+        for (int z = 0; z < L; ++z) { ur[z] = uu[z] * mwd; vr[z] = vv[z] * mwd; }
     }
 }
 
@@ -987,23 +924,27 @@ __global__ void k_wvel(Dev d) {
 // (fv_viscosity.F90:1374-1486, no ice.)  A block takes kIvCols consecutive
 // elements, whose columns are one contiguous range of U_rhs, V_rhs, Je and
 // Av.  All threads, one (element, layer) each: the staging, the coefficients a
-// and c with their three divisions, and at the end the masked result.  One thread per column, all of one warp, runs the
-// elimination (three divisions per layer, in parallel) and the back
-// substitution from shared memory, [array][layer][column] with an odd column
-// stride: free of bank conflicts both over the columns of a layer and over
-// the layers of a column.  c, U and V are overwritten by xx1, yu and yv, then
-// by the solution.
-// Bound by latency (the chains, the staged loads).  FP64 stages Je and Av
-// too (4 loads of each field in flight per thread); FP32 reads them from
-// global memory where they are used, for half the shared memory and more
-// blocks.  Against tiles of 64 columns solved from row-major tiles
-// with all three divisions of a and c in the chain (10 and 20 layers only)
-// and one thread per column reading global memory (other layer counts): 4.5
-// k nodes, 39 layers 0.033 -> 0.025 ms, 697, 10: 0.015 -> 0.013, 232 k, 20:
-// 0.165 -> 0.150, 1.05 M: 0.62 as before, 232 k FP32: 0.064 -> 0.060.
+// and c with their three divisions, and at the end the masked result.  The
+// elimination (three quotients per layer by the same denominator) and the back
+// substitution run from shared memory, [array][layer][column] with an odd
+// column stride: free of bank conflicts both over the columns of a layer and
+// over the layers of a column.  c, U and V are overwritten by xx1, yu and yv,
+// then by the solution.
+// Bound by latency: the chain of the elimination, whose FP64 divisions (114
+// cycles each) one thread runs one after the other.  So in FP64 four lanes per
+// column, all threads of the block, form the quotients of xx1, yu and yv at
+// the same time; FP32, whose divisions are short, takes one thread per column.
+// Staging (FP64): kIvBatch items per thread, the neighbour layers' Je and Av
+// again from L1 instead of staged, so that four arrays remain and more blocks
+// are resident; FP32 was slower with batches (0.060 -> 0.064 ms).
+// FP64, against one thread per column reading global memory, and against
+// tiles with one thread per column: 1.05 M nodes, 20 layers 0.68, 0.62 ->
+// 0.43 ms, 232 k 0.185, 0.148 -> 0.107, 42 k 0.035, 0.040 -> 0.029, 40 k, 30
+// layers 0.049, 0.064 -> 0.043, 16 k, 10 layers 0.017, 0.016 -> 0.013, 4.5 k,
+// 39 layers 0.032, 0.025 -> 0.019.
 constexpr int kIvCols = 32;
 constexpr int kIvThreads = 128;
-constexpr int kIvBatch = 4;
+constexpr int kIvBatch = 3;
 
 __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
     pdl_enter();
@@ -1013,15 +954,16 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
     const int A = L * CP;
     real *const sa = reinterpret_cast<real *>(iv_smem);   // layer z of column j at [z * CP + j]
     real *const sc = sa + A, *const sU = sa + 2 * A, *const sV = sa + 3 * A;
-#if !FESOMC_FP32
-    real *const sJ = sa + 4 * A, *const sA = sa + 5 * A;  // sA: NS rows
-#endif
     const real dt = d.dt;
+#if FESOMC_FP32
     // the warps of the recurrences alternate between the blocks of an SM
     constexpr int kChains = kIvCols / 32, kWarps = kIvThreads / 32;
     const int warp = (int)(threadIdx.x / 32 + kChains * (blockIdx.x / 148)) % kWarps;
     const bool mine = warp < kChains;
     const int lane = warp * 32 + (threadIdx.x & 31);   // column of a recurrence
+#else
+    static_assert(kIvThreads == 4 * kIvCols, "four lanes per column");
+#endif
     for (int e0 = blockIdx.x * kIvCols; e0 < E; e0 += gridDim.x * kIvCols) {
         const int nt = E - e0 < kIvCols ? E - e0 : kIvCols;
 #if FESOMC_FP32
@@ -1037,20 +979,22 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
             sU[o] = d.U_rhs[g];
             sV[o] = d.V_rhs[g];
         }
-        __syncthreads();
 #else
         // kIvBatch items per thread loaded before any is used
         for (int i0 = threadIdx.x; i0 < nt * L; i0 += kIvBatch * kIvThreads) {
-            real ur[kIvBatch], vr[kIvBatch], jz[kIvBatch], av[kIvBatch];
+            real ur[kIvBatch], vr[kIvBatch], j0[kIvBatch], jm[kIvBatch], jp[kIvBatch], a0[kIvBatch], a1[kIvBatch];
 #pragma unroll
             for (int u = 0; u < kIvBatch; ++u) {
                 const int i = i0 + u * kIvThreads < nt * L ? i0 + u * kIvThreads : i0;
-                const int j = d.by_L.div(i);
+                const int j = d.by_L.div(i), z = i - j * L;
                 const size_t g = (size_t)e0 * L + i;
                 ur[u] = d.U_rhs[g];
                 vr[u] = d.V_rhs[g];
-                jz[u] = d.Je[g];
-                av[u] = d.Av[g + e0 + j];
+                j0[u] = d.Je[g];
+                jm[u] = d.Je[z > 0 ? g - 1 : g];
+                jp[u] = d.Je[z < L - 1 ? g + 1 : g];
+                a0[u] = d.Av[g + e0 + j];
+                a1[u] = d.Av[g + e0 + j + 1];
             }
 #pragma unroll
             for (int u = 0; u < kIvBatch; ++u) {
@@ -1059,43 +1003,29 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
                 const int j = d.by_L.div(i), z = i - j * L, o = z * CP + j;
                 sU[o] = ur[u];
                 sV[o] = vr[u];
-                sJ[o] = jz[u];
-                sA[o] = av[u];
+                const real jz = j0[u];
+                const real d1 = (z == 0) ? real(0.5) * jz : real(0.5) * (jz + jm[u]);
+                const real d2 = (z == L - 1) ? real(0.5) * jz : real(0.5) * (jz + jp[u]);
+                const real zt = dt / jz;
+                sa[o] = zt * a0[u] / d1;
+                sc[o] = zt * a1[u] / d2;
             }
         }
-        if ((int)threadIdx.x < nt) sA[L * CP + threadIdx.x] = d.Av[(size_t)(e0 + threadIdx.x) * NS + L];
-        __syncthreads();
-        for (int i = threadIdx.x; i < nt * L; i += kIvThreads) {
-            const int j = d.by_L.div(i), z = i - j * L, o = z * CP + j;
-            const real jz = sJ[o];
-            const real d1 = (z == 0) ? real(0.5) * jz : real(0.5) * (jz + sJ[o - CP]);
-            const real d2 = (z == L - 1) ? real(0.5) * jz : real(0.5) * (jz + sJ[o + CP]);
-            const real zt = dt / jz;
-            sa[o] = zt * sA[o] / d1;
-            sc[o] = zt * sA[o + CP] / d2;
-        }
-        __syncthreads();
 #endif
+        __syncthreads();
+#if FESOMC_FP32
         if (mine && lane < nt) {
             const int e = e0 + lane;
             const real mwd = d.mask_wd[e];
             real *a_ = sa + lane, *x_ = sc + lane, *u_ = sU + lane, *v_ = sV + lane;
             if (mwd != real(0.0)) {
-#if FESOMC_FP32
                 const real *J = d.Je + (size_t)e * L, *Av = d.Av + (size_t)e * NS;
-                constexpr int R = 1;    // from one layer to the next
-#else
-                const real *J = sJ + lane, *Av = sA + lane;
-                constexpr int R = CP;
-#endif
                 const real ub = d.U_n[(size_t)e * L + L - 1], vb = d.V_n[(size_t)e * L + L - 1];
                 const real a_Cd = d.C_d * ((real(1.0) - d.elem_acc[e]) * d.Cd_bz + real(1.0));
-                real de = J[0] / (Av[0] + Av[R]);
+                real de = J[0] / (Av[0] + Av[1]);
                 const real rw = de / d.density_0;
                 real xv = real(1.0), yuv = d.taux[e] * rw, yvv = d.tauy[e] * rw;
-                #if FESOMC_FP32
                 const real jb = J[L - 1], av0 = Av[NS - 1], av1 = Av[L - 1];   // loaded ahead of the sweep
-#endif
                 real an = a_[0], cn = x_[0], un = u_[0], vn = v_[0];
                 for (int z = 0; z < L; ++z) {
                     const real a = an, c = cn, Fx = un, Fy = vn;
@@ -1110,11 +1040,7 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
                     u_[z * CP] = yuv;
                     v_[z * CP] = yvv;
                 }
-#if FESOMC_FP32
                 de = jb / (av0 + av1);
-#else
-                de = J[(L - 1) * R] / (Av[(NS - 1) * R] + Av[(L - 1) * R]);
-#endif
                 const real friction = de * a_Cd * sqrt(ub * ub + vb * vb);
                 real Ut, Vt;
                 if (d.fic_point == 0) { Ut = real(0.0); Vt = real(0.0); }
@@ -1136,6 +1062,53 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
                 for (int z = 0; z < L; ++z) { u_[z * CP] = real(0.0); v_[z * CP] = real(0.0); }
             }
         }
+#else
+        {
+            // four lanes per column: xx1, yu and yv form their quotient each
+            // at the same time and share xx1 (__shfl needs every lane: those
+            // past the last column run along on column 0, the fourth lane on
+            // yv; what they form is not used)
+            const int role = threadIdx.x & 3, col = threadIdx.x >> 2;
+            const bool in = col < nt;
+            const int c0 = in ? col : 0, e = e0 + c0;
+            const real mwd = d.mask_wd[e];
+            const real *a_ = sa + c0, *J = d.Je + (size_t)e * L, *Av = d.Av + (size_t)e * NS;
+            real *x_ = sc + c0, *const y_ = (role == 0 ? sc : role == 1 ? sU : sV) + c0;
+            const bool out = in && role < 3;
+            const real ub = d.U_n[(size_t)e * L + L - 1], vb = d.V_n[(size_t)e * L + L - 1];
+            const real a_Cd = d.C_d * ((real(1.0) - d.elem_acc[e]) * d.Cd_bz + real(1.0));
+            const real rw = J[0] / (Av[0] + Av[1]) / d.density_0;
+            const real jb = J[L - 1], av0 = Av[NS - 1], av1 = Av[L - 1];
+            real x = real(1.0), y = (role == 1 ? d.taux[e] : d.tauy[e]) * rw;
+            real an = a_[0], cn = x_[0], fn = y_[0];
+            for (int z = 0; z < L; ++z) {
+                const real a = an, c = cn, F = fn;
+                const int zn = (z + 1 < L ? z + 1 : z) * CP;
+                an = a_[zn]; cn = x_[zn]; fn = y_[zn];
+                const real b = a + c + real(1.0);
+                const real q = (role == 0 ? c : a * y + F) / (b - a * x);
+                x = __shfl_sync(kFull, q, threadIdx.x & 28);
+                y = q;
+                if (out) y_[z * CP] = q;
+            }
+            __syncwarp();
+            if (out && role > 0) {
+                const real de = jb / (av0 + av1);
+                const real friction = de * a_Cd * sqrt(ub * ub + vb * vb);
+                real W = real(0.0);
+                if (d.fic_point == 1) W = y / (friction + real(1.0) - x);
+                else if (d.fic_point != 0) W = y / (real(1.0) / (real(1.0) - friction) - x);
+                if (mwd != real(0.0)) {
+                    for (int z = L - 1; z >= 0; --z) {
+                        W = W * x_[z * CP] + y_[z * CP];
+                        y_[z * CP] = W * mwd;
+                    }
+                } else {
+                    for (int z = 0; z < L; ++z) y_[z * CP] = real(0.0);
+                }
+            }
+        }
+#endif
         __syncthreads();
         for (int i = threadIdx.x; i < nt * L; i += kIvThreads) {
             const int j = d.by_L.div(i), z = i - j * L;
@@ -1146,22 +1119,7 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
         __syncthreads();
     }
 }
-static size_t implvisc_tile_smem(const Dev &d) { return (FESOMC_FP32 ? (size_t)4 * d.L : (size_t)6 * d.L + 1) * (kIvCols + 1) * sizeof(real); }
-// The tiles do the fic variant alone.  Between one and four full waves of
-// them the last, partly empty wave costs more than they gain over one thread
-// per column, whose blocks are all resident at once (42 k nodes, 20 layers,
-// 1.7 waves: 0.040 against 0.034 ms; 40 k, 30 layers, 2.7: 0.064 / 0.048; 16
-// k, 30 layers, 1.1: 0.041 / 0.035); with one wave or many they win (16 k, 20
-// layers: 0.021 / 0.025; 232 k: 0.148 / 0.184).  FP32 always takes the tiles:
-// the two forms' contracted arithmetic would not give the same bits.
-static bool implvisc_tiled(const Dev &d) {
-    if (d.im_vert_visc || !d.im_vert_visc_fic) return false;
-    if (FESOMC_FP32) return true;
-    if (d.tune[TK_IMPLVISC] == 1) return false;
-    const long long per_sm = 227 * 1024 / (long long)(implvisc_tile_smem(d) + 1024);
-    const long long wave = 148 * (per_sm < 7 ? per_sm : 7) * kIvCols;   // 7: its registers
-    return d.E <= wave || d.E >= 4 * wave;
-}
+static size_t implvisc_tile_smem(const Dev &d) { return (size_t)4 * d.L * (kIvCols + 1) * sizeof(real); }
 
 // ---- launch wrappers --------------------------------------------------------
 // Column blocks: B entities, B * L threads, about 160 of them (at most 16
@@ -1231,12 +1189,8 @@ void launch_velrhs(const Dev &d, real ff, cudaStream_t s) {
         else launch_k(KERNEL<128>, GRID, BLOCK, 0, STREAM, __VA_ARGS__);                         \
     } while (0)
 void launch_implvisc(const Dev &d, cudaStream_t s) {
-    if (implvisc_tiled(d)) {
-        const int tiles = (d.E + kIvCols - 1) / kIvCols;
-        launch_k(k_implvisc_fic_tile, tiles, kIvThreads, implvisc_tile_smem(d), s, d);
-        return;
-    }
-    MAXL_DISPATCH(k_implvisc, grid_for(d.E, 128), 128, s, d);
+    if (d.im_vert_visc) MAXL_DISPATCH(k_implvisc, grid_for(d.E, 128), 128, s, d);
+    if (d.im_vert_visc_fic) launch_k(k_implvisc_fic_tile, (d.E + kIvCols - 1) / kIvCols, kIvThreads, implvisc_tile_smem(d), s, d);
 }
 void launch_jac_swap(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ROT, 256);

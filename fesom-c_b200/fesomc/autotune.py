@@ -33,8 +33,8 @@ D3END_ARRAYS = (1, 2)
 # the knobs that pick a form rather than a block size
 # tracer_impl_vert_diff: one form under every number
 VDIFF_FORMS = (3,)
-# momentum_vert_impl_visc_tmp: columns read directly, or tiles of columns
-IMPLVISC_FORMS = (1, 2)
+# momentum_vert_impl_visc_tmp: one form under both numbers
+IMPLVISC_FORMS = (2,)
 FORMS = {"columns": COLUMNS, "d3end_arrays": D3END_ARRAYS, "vdiff_form": VDIFF_FORMS,
          "implvisc_form": IMPLVISC_FORMS}
 SHIPPED = os.path.join(os.path.dirname(os.path.abspath(__file__)), "launch_shapes_b200.json")

@@ -458,14 +458,11 @@ int  fesomc_ensemble_run(fesomc_model *const *members, int32_t n_members, int32_
  * form takes the tiles under every number;
  * "vdiff_form" 1 to 3, the same under every number: the tracers' implicit
  * vertical diffusion runs on tiles of columns in shared memory;
- * "implvisc_form" 1 or 2: the implicit vertical viscosity with each element
- * column read directly, or (the default) on tiles of columns in shared
- * memory for the fic variant, where their number fills the device's waves
- * well; the FP32 form takes the tiles under both numbers); the next step
- * captures its
- * graph again.  The search over the knobs and its cache per mesh size and
- * level count live with the host driver (fesomc/autotune.py).  No
- * counterpart in the reference. */
+ * "implvisc_form" 1 or 2, the same under both numbers: the implicit vertical
+ * viscosity's fic variant runs on tiles of columns in shared memory); the
+ * next step captures its graph again.  The search over the knobs and its
+ * cache per mesh size and level count live with the host driver
+ * (fesomc/autotune.py).  No counterpart in the reference. */
 int  fesomc_gpu_tune_knobs(void);
 int  fesomc_gpu_tune_knob(int32_t k, char *name, int32_t name_len, char *records, int32_t records_len);
 int  fesomc_gpu_tune_get(fesomc_model *m, int32_t *values, int32_t *limits);
