@@ -879,8 +879,8 @@ __device__ __forceinline__ real swr_frac(const Dev &d, int n, real z) {
 // As in the reference: T and S are T_old + T_aver and S_old + S_aver (the
 // tracers of the previous step, which are not shifted by their means at
 // this point), and sw_cp receives them in the order (T, S) against its
-// (S, T) arguments.
-__device__ real heat_source(const Dev &d, int n, size_t base, int z, real aj, real T_aver, real S_aver) {
+// (S, T) arguments.  swr1, swr2: swr_frac at the layer's two interfaces.
+__device__ real heat_source(const Dev &d, int n, size_t base, int z, real aj, real T_aver, real S_aver, real swr1, real swr2) {
     const real d1 = zbar_of(d, aj, z), d2 = zbar_of(d, aj, z + 1);
     const real T = d.Told_new[base + z] + T_aver;
     const real S = d.Sold_new[base + z] + S_aver;
@@ -889,7 +889,6 @@ __device__ real heat_source(const Dev &d, int n, size_t base, int z, real aj, re
     const real ms = (real)d.mslp[n];
     const real P = (ms == real(0.0)) ? (rho * kG * aux + real(kPref)) * real(10.0e-5) : (rho * kG * aux + ms) * real(10.0e-5);
     const real c_p = sw_cp(T, S, P);
-    const real swr1 = swr_frac(d, n, -d1), swr2 = swr_frac(d, n, -d2);
     const real jc = jc_of(d, aj, z);
     const real qsr = (real)d.qsr[n];
     real src;
@@ -1159,17 +1158,22 @@ void launch_muscl_h(const Dev &d, cudaStream_t s) {
 // stride: free of bank conflicts both over the columns of a layer and over
 // the layers of a column.  c, tr and sr are overwritten by the eliminated
 // ones.
-// Bound by latency (the chains, the staged loads).  Against one thread per
-// column with everything in its chain: 4.5 k nodes, 39 layers 0.076 -> 0.023
-// ms, 40 k nodes, 30 layers with atmospheric sources 0.305 -> 0.144 (the heat
-// source was formed in the column's thread); against 64-column tiles solved
-// in registers, 10 layers: 697 nodes 0.017 -> 0.013, 16 k 0.019 -> 0.015.
+// Bound by latency (the chains, the staged loads).  FP64: 192 threads and five
+// blocks per SM (64 registers); with atmospheric sources 256 threads and
+// four, and the shortwave fraction (two exponentials and two divisions) formed
+// once per interface instead of by both layers.  Against 128 threads without
+// a register cap: 4.5 k nodes, 39 layers 0.023 -> 0.021 ms, 16 k, 30 layers
+// 0.027 -> 0.024, 1.05 M, 20 layers 0.75 -> 0.58; with sources 40 k, 30 layers
+// 0.144 -> 0.097, 40 k, 20 layers 0.080 -> 0.073, 232 k 0.39 -> 0.33.  One thread
+// per column with everything in its chain: 0.076 ms at 4.5 k, 0.305 with
+// sources at 40 k.
 constexpr int kVtCols = 32;
-constexpr int kVtThreads = 128;
+constexpr int kVtThreads = FESOMC_FP32 ? 128 : 192;
+constexpr int kVtAtmThreads = FESOMC_FP32 ? 128 : 256;
 constexpr int kVtArrays = 6, kVtBatch = 4;
 
 template <bool kAtm>
-__global__ void __launch_bounds__(kVtThreads) k_vdiff_tile(Dev d) {
+__global__ void __launch_bounds__(kAtm ? kVtAtmThreads : kVtThreads, FESOMC_FP32 ? 1 : kAtm ? 4 : 5) k_vdiff_tile(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char vt_smem[];
     __shared__ real s_aj[kVtCols], s_ta[kVtCols], s_sa[kVtCols];
@@ -1178,9 +1182,10 @@ __global__ void __launch_bounds__(kVtThreads) k_vdiff_tile(Dev d) {
     const int L = d.L, NS = d.NS, N = d.N;
     const int A = L * CP;
     real *const sT = reinterpret_cast<real *>(vt_smem);   // layer k of column j at [k * CP + j]
-    real *const sS = sT + A, *const sa = sT + 2 * A, *const sc = sT + 3 * A, *const st = sT + 4 * A, *const ss = sT + 5 * A;
+    real *const sS = sT + A, *const sa = sT + 2 * A, *const sc = sT + 3 * A, *const st = sT + 4 * A, *const ss = st + A + (kAtm ? CP : 0);
+    constexpr int kThreads = kAtm ? kVtAtmThreads : kVtThreads;
     // the warps of the recurrences alternate between the blocks of an SM
-    constexpr int kChains = kVtCols / 32, kWarps = kVtThreads / 32;
+    constexpr int kChains = kVtCols / 32, kWarps = kThreads / 32;
     const int warp = (int)(threadIdx.x / 32 + kChains * (blockIdx.x / 148)) % kWarps;
     const bool mine = warp < kChains;
     const int lane = warp * 32 + (threadIdx.x & 31);   // column of a recurrence
@@ -1194,12 +1199,19 @@ __global__ void __launch_bounds__(kVtThreads) k_vdiff_tile(Dev d) {
             s_wet[threadIdx.x] = kAtm && d.mask_wd_node[n] != real(0.0);
         }
         __syncthreads();
+        // the shortwave fraction at each interface, once for its two layers
+        // (st has a row more for it)
+        if (kAtm)
+            for (int i = threadIdx.x; i < nt * NS; i += kThreads) {
+                const int j = d.by_NS.div(i), k = i - j * NS;
+                if (s_wet[j]) st[k * CP + j] = swr_frac(d, n0 + j, -zbar_of(d, s_aj[j], k));
+            }
         // kVtBatch items per thread loaded before any is used
-        for (int i0 = threadIdx.x; i0 < nt * L; i0 += kVtBatch * kVtThreads) {
+        for (int i0 = threadIdx.x; i0 < nt * L; i0 += kVtBatch * kThreads) {
             real ta[kVtBatch], sl[kVtBatch], tn[kVtBatch], sn[kVtBatch], kv[kVtBatch];
 #pragma unroll
             for (int u = 0; u < kVtBatch; ++u) {
-                const int i = i0 + u * kVtThreads < nt * L ? i0 + u * kVtThreads : i0;
+                const int i = i0 + u * kThreads < nt * L ? i0 + u * kThreads : i0;
                 const int j = d.by_L.div(i), k = i - j * L;
                 const size_t g = (size_t)n0 * L + i;
                 ta[u] = d.TF_adv[g];
@@ -1210,7 +1222,7 @@ __global__ void __launch_bounds__(kVtThreads) k_vdiff_tile(Dev d) {
             }
 #pragma unroll
             for (int u = 0; u < kVtBatch; ++u) {
-                const int i = i0 + u * kVtThreads;
+                const int i = i0 + u * kThreads;
                 if (i >= nt * L) break;
                 const int j = d.by_L.div(i), k = i - j * L;
                 const size_t g = (size_t)n0 * L + i;
@@ -1223,7 +1235,16 @@ __global__ void __launch_bounds__(kVtThreads) k_vdiff_tile(Dev d) {
             }
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < nt * L; i += kVtThreads) {
+        // the heat source of wet nodes' layers, in ss
+        if (kAtm) {
+            for (int i = threadIdx.x; i < nt * L; i += kThreads) {
+                const int j = d.by_L.div(i), k = i - j * L, n = n0 + j;
+                const int o = k * CP + j;
+                if (s_wet[j]) ss[o] = heat_source(d, n, (size_t)n * L, k, s_aj[j], s_ta[j], s_sa[j], st[o], st[o + CP]);
+            }
+            __syncthreads();
+        }
+        for (int i = threadIdx.x; i < nt * L; i += kThreads) {
             const int j = d.by_L.div(i), k = i - j * L, n = n0 + j;
             const int o = k * CP + j;
             const real aj = s_aj[j];
@@ -1243,7 +1264,7 @@ __global__ void __launch_bounds__(kVtThreads) k_vdiff_tile(Dev d) {
             // surface sources on wet nodes (fv_tracer.F90:1376,1396-1418)
             if (kAtm && s_wet[j]) {
                 const real T_aver = s_ta[j], S_aver = s_sa[j];
-                tr = tr + d.dt * heat_source(d, n, (size_t)n * L, k, aj, T_aver, S_aver);
+                tr = tr + d.dt * ss[o];
                 if (k == 0) sr = sr + d.dt * evap_precip(d, n, aj, T0, S0, T_aver, S_aver);
             }
             sa[o] = a;
@@ -1288,7 +1309,7 @@ __global__ void __launch_bounds__(kVtThreads) k_vdiff_tile(Dev d) {
         }
         __syncthreads();
         unsigned int flags = 0;
-        for (int i = threadIdx.x; i < nt * L; i += kVtThreads) {
+        for (int i = threadIdx.x; i < nt * L; i += kThreads) {
             const int j = d.by_L.div(i), k = i - j * L, n = n0 + j;
             const int o = k * CP + j;
             const size_t g = (size_t)n0 * L + i;
@@ -1430,14 +1451,14 @@ __global__ void __launch_bounds__(kVrCols) k_vdiff_reg(Dev d) {
     }
 }
 
-static size_t vdiff_smem(const Dev &d) { return (size_t)kVtArrays * d.L * (kVtCols + 1) * sizeof(real); }
+static size_t vdiff_smem(const Dev &d) { return ((size_t)kVtArrays * d.L + (d.key_atm ? 1 : 0)) * (kVtCols + 1) * sizeof(real); }
 static size_t vdiff_reg_smem(const Dev &d) {
     return (size_t)kVrCols * (2 * (d.L | 1) + (d.NS | 1)) * sizeof(real);
 }
 // 20 layers without atmospheric sources, from four tiles of 64 per SM on: 42 k
-// nodes 0.033 ms against 0.037, 1.05 M 0.526 against 0.65, 232 k FP32 0.070
-// against 0.080; below, and with the sources, the level-parallel tiles: 16 k
-// nodes 0.021 against 0.029, with sources 40 k 0.080 against 0.114.
+// nodes 0.034 ms against 0.035, 1.05 M 0.563 against 0.583, 232 k FP32 0.072
+// against 0.086; below, and with the sources, the level-parallel tiles: 16 k
+// nodes 0.019 against 0.029, with sources 40 k 0.073 against 0.114.
 static bool vdiff_reg(const Dev &d) {
     return d.L == kVrLayers && !d.key_atm && d.N >= 4 * 148 * kVrCols;
 }
@@ -1452,7 +1473,7 @@ int config_vdiff(const Dev &d) {
 void launch_vdiff(const Dev &d, cudaStream_t s) {
     const int C = vdiff_reg(d) ? kVrCols : kVtCols, tiles = (d.N + C - 1) / C;
     if (vdiff_reg(d)) launch_k(k_vdiff_reg, tiles, kVrCols, vdiff_reg_smem(d), s, d);
-    else if (d.key_atm) launch_k(k_vdiff_tile<true>, tiles, kVtThreads, vdiff_smem(d), s, d);
+    else if (d.key_atm) launch_k(k_vdiff_tile<true>, tiles, kVtAtmThreads, vdiff_smem(d), s, d);
     else launch_k(k_vdiff_tile<false>, tiles, kVtThreads, vdiff_smem(d), s, d);
 }
 int energy_parts() { return kRedGrid; }
