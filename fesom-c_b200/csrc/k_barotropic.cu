@@ -194,7 +194,8 @@ __global__ void k_el2nodes(Dev d, const real *Ue, const real *Ve, real *Un, real
         const int z = (int)ii - n * d.L;
         const real tvol_inv = real(1.0) / d.node_tvol[n];
         real su = real(0.0), sv = real(0.0);
-        for (int p = d.node_nptr[n]; p < d.node_nptr[n + 1]; ++p) {
+        const int p0 = d.node_nptr[n], p1 = d.node_nptr[n + 1];
+        for (int p = p0; p < p1; ++p) {
             const int el = d.node_nidx[p];
             const real ar = d.elem_area[el];
             su = su + Ue[(size_t)el * d.L + z] * ar;
@@ -366,10 +367,67 @@ __device__ __forceinline__ void adv2d_edge(const Dev &d, int ed, const int2 nn, 
     d.adv2d[ed] = make_real2(uu, vv);
 }
 
+// biharmonic_2D (fv_viscosity.F90:338-568, free slip): two Laplacians of the
+// 2D velocity.  bih2d_flux: the flux of an edge from U and the gradients in
+// vel_grad (boundary edges with the free-slip projection, whose v uses the
+// projected u, as the reference); bih2d_ul: Ul = Ah acc sum of the fluxes;
+// bih2d_grad: vel_gradients_2D(Ul) into vel_grad (adv2d_edge has used the
+// gradients of UAB by then).  The first fluxes share a pass with adv2d_edge,
+// which reads the same fields; u2d_elem gathers the second.  Bound by the
+// passes' chains of dependent loads (42 k nodes, 20 sub-steps: bih_2d and
+// adv2d_edge 0.335 -> 0.309 ms);
+// Ul of the neighbours formed again in bih2d_grad instead of in its own
+// pass made those chains longer: 0.055 ms slower.
+__device__ __forceinline__ void bih2d_flux(const Dev &d, const real2 *U, int ed, const int2 et) {
+    real u1, v1;
+    if (ed < d.Ed_in) {
+        const real4 G = d.bih_dir[ed];
+        const real xe = G.x, ye = G.y, tx = G.z, ty = G.w, tl = d.bih_len[ed];
+        const real4 a = d.vel_grad[et.x], b = d.vel_grad[et.y];
+        const real2 U1 = U[et.x], U2 = U[et.y];
+        real g1 = real(0.5) * (a.x + b.x);
+        real g2 = real(0.5) * (a.y + b.y);
+        real tt = g1 * tx + g2 * ty - (U2.x - U1.x) / tl;
+        g1 = g1 - tx * tt;
+        g2 = g2 - ty * tt;
+        u1 = (g1 * ye - g2 * xe);
+        g1 = real(0.5) * (a.z + b.z);
+        g2 = real(0.5) * (a.w + b.w);
+        tt = g1 * tx + g2 * ty - (U2.y - U1.y) / tl;
+        g1 = g1 - tx * tt;
+        g2 = g2 - ty * tt;
+        v1 = (g1 * ye - g2 * xe);
+    } else {
+        const real2 dxy = d.edge_dxdy[ed];
+        const real xe = dxy.x * kREarth;
+        const real xed = xe * d.elem_cos[et.x];
+        const real ye = dxy.y * kREarth;
+        const real4 a = d.vel_grad[et.x];
+        u1 = (a.x) * ye - (a.y) * xed;
+        v1 = (a.z) * ye - (a.w) * xed;
+        u1 = ye * (u1 * ye - v1 * xe) / (xe * xe + ye * ye);
+        v1 = -xe * (u1 * ye - v1 * xe) / (xe * xe + ye * ye);
+    }
+    d.b2fl[ed] = make_real2(u1, v1);
+}
+
 // momentum_adv_upwind_2D edge fluxes of the sub-step, once per internal edge
 __global__ void k_adv2d_edge(Dev d) {
     pdl_enter();
     GRID_LOOP(ed, d.Ed_in) adv2d_edge(d, (int)ed, d.edge_nodes[ed], d.edge_tri[ed]);
+}
+__global__ void k_adv2d_bih_edge(Dev d) {
+    pdl_enter();
+    GRID_LOOP(ii, d.Ed) {
+        const int ed = (int)ii;
+        const int2 et = d.edge_tri[ed];
+        if (ed < d.Ed_in) adv2d_edge(d, ed, d.edge_nodes[ed], et);
+        bih2d_flux(d, d.UAB, ed, et);
+    }
+}
+__global__ void k_bih2d_edge(Dev d, const real2 *U) {
+    pdl_enter();
+    GRID_LOOP(ed, d.Ed) bih2d_flux(d, U, (int)ed, d.edge_tri[ed]);
 }
 __global__ void k_adv2d_edge_head(Dev d) {
     const unsigned ed = blockIdx.x * blockDim.x + threadIdx.x;
@@ -379,72 +437,23 @@ __global__ void k_adv2d_edge_head(Dev d) {
     if (on) adv2d_edge(d, (int)ed, nn, et);
 }
 
-// biharmonic_2D (fv_viscosity.F90:338-568, free slip): two Laplacians of the
-// 2D velocity.  bih2d_edge: the flux of every edge from U and the gradients
-// in vel_grad (boundary edges with the free-slip projection, whose v uses
-// the projected u, as the reference); bih2d_ul: Ul = Ah acc sum of the
-// fluxes; bih2d_grad: vel_gradients_2D(Ul) into vel_grad (adv2d_edge has
-// used the gradients of UAB by then).  u2d_elem gathers the second pass.
-__global__ void k_bih2d_edge(Dev d, const real2 *U) {
-    pdl_enter();
-    GRID_LOOP(ii, d.Ed) {
-        const int ed = (int)ii;
-        const int2 et = d.edge_tri[ed];
-        const real2 dxy = d.edge_dxdy[ed];
-        real u1, v1;
-        if (ed < d.Ed_in) {
-            const real4 X = d.edge_cross[ed];
-            const real xe = dxy.x * kREarth * real(0.5) * (d.elem_cos[et.x] + d.elem_cos[et.y]);
-            const real ye = dxy.y * kREarth;
-            real tx = -X.x + X.z;
-            real ty = -X.y + X.w;
-            const real tl = sqrt(tx * tx + ty * ty);
-            tx = tx / tl;
-            ty = ty / tl;
-            const real4 a = d.vel_grad[et.x], b = d.vel_grad[et.y];
-            const real2 U1 = U[et.x], U2 = U[et.y];
-            real g1 = real(0.5) * (a.x + b.x);
-            real g2 = real(0.5) * (a.y + b.y);
-            real tt = g1 * tx + g2 * ty - (U2.x - U1.x) / tl;
-            g1 = g1 - tx * tt;
-            g2 = g2 - ty * tt;
-            u1 = (g1 * ye - g2 * xe);
-            g1 = real(0.5) * (a.z + b.z);
-            g2 = real(0.5) * (a.w + b.w);
-            tt = g1 * tx + g2 * ty - (U2.y - U1.y) / tl;
-            g1 = g1 - tx * tt;
-            g2 = g2 - ty * tt;
-            v1 = (g1 * ye - g2 * xe);
-        } else {
-            const real xe = dxy.x * kREarth;
-            const real xed = xe * d.elem_cos[et.x];
-            const real ye = dxy.y * kREarth;
-            const real4 a = d.vel_grad[et.x];
-            u1 = (a.x) * ye - (a.y) * xed;
-            v1 = (a.z) * ye - (a.w) * xed;
-            u1 = ye * (u1 * ye - v1 * xe) / (xe * xe + ye * ye);
-            v1 = -xe * (u1 * ye - v1 * xe) / (xe * xe + ye * ye);
-        }
-        d.b2fl[ed] = make_real2(u1, v1);
-    }
-}
-
 __global__ void k_bih2d_ul(Dev d) {
     pdl_enter();
     GRID_LOOP(ii, d.E) {
         const int e = (int)ii;
         const int4 se = d.elem_sedges[e];
-        const int codes[4] = {se.x, se.y, se.z, se.w};
+        const int codes[4] = {se.x, se.y, se.z, se.w};   // absent ones (-1) last
+        real2 f[4];   // loaded together, not one after the other behind the tests
+#pragma unroll
+        for (int c = 0; c < 4; ++c) f[c] = codes[c] >= 0 ? d.b2fl[codes[c] >> 1] : make_real2(real(0.0), real(0.0));
         real ux = real(0.0), uy = real(0.0);
+#pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int code = codes[c];
-            if (code < 0) break;
-            const real2 f = d.b2fl[code >> 1];
-            if (code & 1) { ux = ux - f.x; uy = uy - f.y; }
-            else { ux = ux + f.x; uy = uy + f.y; }
+            if (codes[c] < 0) continue;
+            if (codes[c] & 1) { ux = ux - f[c].x; uy = uy - f[c].y; }
+            else { ux = ux + f[c].x; uy = uy + f[c].y; }
         }
-        const real sa = scale_area_of(d, e);
-        const real Ah = -d.Abh0 * sqrt(d.elem_area[e] / sa) / sa;
+        const real Ah = d.bih_ah[e].x;
         const real acc = d.elem_acc[e];
         d.b2ul[e] = make_real2(ux * (Ah) * acc, uy * (Ah) * acc);
     }
@@ -485,9 +494,9 @@ __device__ __forceinline__ void velgrad2d_elem(const Dev &d, const real2 *U, int
         d.vel_grad[e] = make_real4(g1, g2, g3, g4);
     }
 }
-__global__ void k_velgrad2d(Dev d, const real2 *U) {
+__global__ void k_bih2d_grad(Dev d) {
     pdl_enter();
-    GRID_LOOP(ii, d.E) velgrad2d_elem(d, U, (int)ii, d.elem_nodes[ii], d.elem_nb[ii]);
+    GRID_LOOP(e, d.E) velgrad2d_elem(d, d.b2ul, (int)e, d.elem_nodes[e], d.elem_nb[e]);
 }
 
 // sub_edge: the SSH flux of every edge, once, for both end nodes to gather
@@ -731,15 +740,17 @@ void launch_p1_elem(const Dev &d, cudaStream_t s) {
 void launch_adv2d_edge(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ADV2D, 256);
     const int g = grid_for(d.Ed_in, b);
-    if (early_grid(g)) launch_k(k_adv2d_edge_head, g, b, 0, s, d);
+    if (d.bih_2D) launch_k(k_adv2d_bih_edge, grid_for(d.Ed, b), b, 0, s, d);
+    else if (early_grid(g)) launch_k(k_adv2d_edge_head, g, b, 0, s, d);
     else launch_k(k_adv2d_edge, g, b, 0, s, d);
 }
 void launch_filt2x_2d(const Dev &d, cudaStream_t s) { launch_k(k_filt2x_2d, grid_for(d.E, 256), 256, 0, s, d); }
+// the first fluxes come with launch_adv2d_edge where that runs
 void launch_bih_2d(const Dev &d, cudaStream_t s) {
     const int bg = tuned(d, TK_VELGRAD2D, 256);
-    launch_k(k_bih2d_edge, grid_for(d.Ed, 256), 256, 0, s, d, d.UAB);
+    if (d.mom_adv_2D != 2) launch_k(k_bih2d_edge, grid_for(d.Ed, 256), 256, 0, s, d, d.UAB);
     launch_k(k_bih2d_ul, grid_for(d.E, 256), 256, 0, s, d);
-    launch_k(k_velgrad2d, grid_for(d.E, bg), bg, 0, s, d, d.b2ul);
+    launch_k(k_bih2d_grad, grid_for(d.E, bg), bg, 0, s, d);
     launch_k(k_bih2d_edge, grid_for(d.Ed, 256), 256, 0, s, d, d.b2ul);
 }
 void launch_u2d_elem(const Dev &d, int next, cudaStream_t s) {
@@ -761,7 +772,7 @@ static void tune_lower(int *lim, int knob, const void *k) {
 }
 void tune_limits_barotropic(int *lim) {
     tune_lower(lim, TK_AB3, (const void *)k_ab3_elem);
-    tune_lower(lim, TK_VELGRAD2D, (const void *)k_velgrad2d);
+    tune_lower(lim, TK_VELGRAD2D, (const void *)k_bih2d_grad);
     tune_lower(lim, TK_SSHEDGE, (const void *)k_sub_edge);
     tune_lower(lim, TK_SSHEDGE, (const void *)k_sub_edge_head);
     tune_lower(lim, TK_SSHNODE, (const void *)k_ssh_node);

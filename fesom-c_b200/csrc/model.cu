@@ -38,6 +38,7 @@ namespace fesomc {
     void launch_adv3_edge(const Dev &, cudaStream_t); \
     void launch_velrhs(const Dev &, real, cudaStream_t); \
     void launch_bih(const Dev &, cudaStream_t); \
+    void launch_bih_geom(const Dev &, cudaStream_t); \
     void launch_filt2x(const Dev &, cudaStream_t); \
     void launch_filt2x_2d(const Dev &, cudaStream_t); \
     void launch_bih_2d(const Dev &, cudaStream_t); \
@@ -982,6 +983,9 @@ int alloc_3d(fesomc_model *m, D &d) {
     if (m->p.bih_3D && ((rc = dalloc(m, &d.bihfl, L * (size_t)d.Ed)) || (rc = dalloc(m, &d.bihU, L * E)) ||
                         (rc = dalloc(m, &d.bihV, L * E))))
         return rc;
+    if ((m->p.bih_3D || m->p.bih_2D) && ((rc = dalloc(m, &d.bih_dir, (size_t)d.Ed)) || (rc = dalloc(m, &d.bih_len, (size_t)d.Ed)) ||
+                                         (rc = dalloc(m, &d.bih_ah, E))))
+        return rc;
     if (m->p.filt_bi_3D && ((rc = dalloc(m, &d.f2U, L * E)) || (rc = dalloc(m, &d.f2V, L * E)))) return rc;
     decltype(&d.U_n) le[] = {&d.U_n, &d.V_n, &d.U_rhsAB, &d.V_rhsAB, &d.U_n_filt, &d.V_n_filt, &d.U_rhs, &d.V_rhs,
                              &d.U_puls, &d.V_puls, &d.vgux, &d.vguy, &d.vgvx, &d.vgvy, &d.Bar_pru, &d.Bar_prv,
@@ -1106,15 +1110,15 @@ double kernel_bytes_fp64(const fesomc_model *m, const std::string &k) {
     const double N = d.N, E = d.E, Ed = d.Ed, Ei = d.Ed_in, L = d.L, NS = d.NS;
     const double nnz_ne = (double)(2 * d.Ed);  // node->edge incidences
     if (k == "biharmonic")   // two edge passes, U_c, its gradients
-        return 2 * (L * Ed * 16 + Ed * (8 + 8 + 16 + 32 + 16) + L * E * 32 + L * E * 16) + L * E * (16 + 16) +
-               E * 16 + L * E * (16 + 32) + E * (16 + 16 + 64) + N * 16;
+        return 2 * (L * Ed * 16 + Ed * (8 + 8 + 32 + 8) + L * E * 32 + L * E * 16) + L * E * (16 + 16) +
+               E * 32 + L * E * (16 + 32) + E * (16 + 16 + 64) + N * 16;
     if (k == "biharmonic_2d")   // pulsation gradients, two edge passes, U_c, its gradients
         return L * E * (16 + 32) + E * (16 + 16 + 64 + 16) + 2 * (L * Ed * 16 + Ed * 48 + L * E * 48) +
-               L * E * (16 + 16) + E * 16 + L * E * (16 + 32);
+               L * E * (16 + 16) + E * 32 + L * E * (16 + 32);
     if (k == "filt2x") return L * E * (16 + 16 + 8 * 4) + E * (16 + 8) + L * E * 16;
     if (k == "filt2x_2d") return E * (16 + 16 + 8 + 16);
     if (k == "potential") return N * (16 + 8);   // coordinates in, ssh_gp out
-    if (k == "bih_2d") return 2 * (Ed * (16 + 8 + 32 + 8 + 16) + E * 32 + Ed * 16) + E * (16 + 16 + 8 + 8 + 16) +
+    if (k == "bih_2d") return 2 * (Ed * (8 + 32 + 8) + E * 48 + Ed * 16) + E * (16 + 16 + 8 + 16 + 16) +
                               E * (16 + 16 + 64 + 16 + 32);
     if (k == "forcing") return (double)d.nobn * (m->p.Mt * 8 + 12 * 16) + 36 * 8 + d.n_rivers * 16.0 + 16;
     // AB3 levels, w_cv, nodes; eta levels and depth; UAB, aux out; bottom
@@ -1342,7 +1346,7 @@ int enqueue_step(fesomc_model *m, double ff) {
         }
         if (d.mom_adv_2D == 2) { rec(m, "adv2d_edge", [&] { K3(launch_adv2d_edge, s); }); n += 1; }
         if (d.filt_bi_2D) { rec(m, "filt2x_2d", [&] { K3(launch_filt2x_2d, s); }); n += 1; }
-        if (d.bih_2D) { rec(m, "bih_2d", [&] { K3(launch_bih_2d, s); }); n += 4; }
+        if (d.bih_2D) { rec(m, "bih_2d", [&] { K3(launch_bih_2d, s); }); n += d.mom_adv_2D == 2 ? 3 : 4; }
         rec(m, "u2d_elem", [&] { K3(launch_u2d_elem, sub + 1 < d0.Mt, s); });
         n += 1;
     }
@@ -1678,6 +1682,10 @@ int fesomc_gpu_init_packed(const fesomc_mesh *mesh, const fesomc_params *par, co
         return fail(FESOMC_ECUDA);
     if (m->fp32) fesomc::f32::launch_je(m->d32, m->stream);
     else launch_je(m->d, m->stream);
+    if (par->bih_3D || par->bih_2D) {
+        if (m->fp32) fesomc::f32::launch_bih_geom(m->d32, m->stream);
+        else launch_bih_geom(m->d, m->stream);
+    }
     if (cudaGetLastError() != cudaSuccess) return fail(FESOMC_ECUDA);
     m->lfirst = st->lfirst;
     m->time_jd = st->time_jd;

@@ -67,3 +67,15 @@ def test_column_solver_tiles(built, nx, ny, nsigma, atm):
     from fesomc import cases
     kw = {"atm": {"qns": -80.0, "qsr": 120.0, "emp": 1e-7, "mslp": 101000.0}} if atm else {}
     _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib, **kw), 3)
+
+
+# biharmonic_2D's first edge pass runs inside adv2d_edge, or on its own
+# without the 2D advection; with biharmonic_viscosity the two operators share
+# the mesh's coefficients
+@pytest.mark.parametrize("params", [{"bih_2D": 1, "mom_adv_2D": 0}, {"bih_2D": 1}, {"bih_3D": 1},
+                                    {"bih_2D": 1, "bih_3D": 1, "mom_adv_2D": 0}])
+@pytest.mark.parametrize("nx,ny", [(7, 6), (23, 14)])
+def test_biharmonic_passes(built, params, nx, ny):
+    from fesomc import cases
+    _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, 11, 2.0, 25.0, stress=(0.0, 0.05), Abh0=1e4, lib=lib,
+                                            **params), 4)
