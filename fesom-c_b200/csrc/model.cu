@@ -979,7 +979,7 @@ int alloc_3d(fesomc_model *m, D &d) {
     const size_t N = d.N, E = d.E, L = d.L, NS = d.NS;
     int rc = 0;
     if ((rc = dalloc(m, &d.Fp, E))) return rc;
-    if ((rc = dalloc(m, &d.adv3, L * (size_t)d.Ed_in))) return rc;
+    if ((rc = dalloc(m, &d.adv3, L * (size_t)std::max(d.Ed_in, 1)))) return rc;
     if (m->p.bih_3D && ((rc = dalloc(m, &d.bihfl, L * (size_t)d.Ed)) || (rc = dalloc(m, &d.bihU, L * E)) ||
                         (rc = dalloc(m, &d.bihV, L * E))))
         return rc;
