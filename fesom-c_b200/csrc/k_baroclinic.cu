@@ -208,8 +208,10 @@ __global__ void BPG_BOUNDS k_bpg_elem(Dev d) {
 }
 
 // vel_gradients (fv_gradients.F90:2-93), one thread per (element, level).
-// 64 registers: 32 resident warps per SM instead of 24 (11 % faster).
-__global__ void __maxnreg__(64) k_velgrad3d(Dev d) {
+// FP64: 64 registers: 32 resident warps per SM instead of 24 (11 % faster; 48:
+// 0.380 against 0.373 ms at 1.05 M nodes).  FP32: 32 registers, 232 k nodes
+// 0.074 -> 0.052 ms.
+__global__ void __maxnreg__(FESOMC_FP32 ? 32 : 64) k_velgrad3d(Dev d) {
     pdl_enter();
     const unsigned total = (unsigned)d.E * d.L;
     GRID_LOOP(ii, total) {
@@ -564,10 +566,12 @@ __global__ void k_filt2x_uc(Dev d) {
 // other: 1.05 M nodes 1.36 -> 1.27 ms, 232 k FP32 0.257 -> 0.230, 42 k 0.098 ->
 // 0.091.
 // ---------------------------------------------------------------------------
-// 4 resident blocks (at most 64 registers) in both forms: in FP64 the few
-// spilled registers cost less than the lost warps (11 % faster than 3
-// blocks at 80 registers).
-__global__ void __launch_bounds__(256, 4) k_velrhs(Dev d, real ff) {
+// FP64: 4 resident blocks (at most 64 registers): the few spilled registers
+// cost less than the lost warps (11 % faster than 3 blocks at 80 registers; 5
+// blocks: 1.25 ms at 1.05 M nodes against 1.27, but 0.021 against 0.019 at 16
+// k).  FP32: 8 blocks (32 registers), 232 k nodes 0.230 -> 0.160 ms; its
+// latency is hidden by warps alone.
+__global__ void __launch_bounds__(256, FESOMC_FP32 ? 8 : 4) k_velrhs(Dev d, real ff) {
     pdl_enter();
     const unsigned total = (unsigned)d.E * d.L;
     const int lane = threadIdx.x & 31;
@@ -795,13 +799,14 @@ __global__ void k_je_elem(Dev d) {
 // per element.  Runs right after the jacobian call: the stored Je still holds
 // the previous jacobian (Jc_old), and is replaced here by the new Je / Ze /
 // ZBe.
-// 48 registers: 4 resident column blocks per SM instead of 3 (15 % faster).
+// FP64: 48 registers (40: 0.62 ms, 32: 0.70 against 0.60 at 1.05 M nodes); FP32:
+// 32, 232 k nodes 0.095 -> 0.087.
 // The element's scalars are formed by four lanes per element, one per node.
 // Blocks of 160 threads: 1.05 M nodes 0.80 -> 0.60 ms, 232 k FP32 0.131 ->
 // 0.095, 40 k, 30 layers 0.059 -> 0.039 (one lane per element formed them, 320
 // threads).
 constexpr int kU3Sc = 16;  // per element: w_cv(4), a(4), U2p, V2p, uf, vf, U_n_2D(2), dmean_inv; then dh(4)
-__global__ void __maxnreg__(48) k_update3d(Dev d, real Mt_inv) {
+__global__ void __maxnreg__(FESOMC_FP32 ? 32 : 48) k_update3d(Dev d, real Mt_inv) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     real *sm = reinterpret_cast<real *>(sm_raw);

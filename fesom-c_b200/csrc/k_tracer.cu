@@ -202,7 +202,12 @@ __global__ void k_ab2_node(Dev d) {
 // solve_tracer_upwind: one thread per (node, level), levels on consecutive
 // lanes of a flat index (no lane idles when L < 32); level data coalesced.
 // ---------------------------------------------------------------------------
-__global__ void k_upwind_h(Dev d) {
+#if FESOMC_FP32
+#define UPWIND_BOUNDS
+#else   // 56 registers instead of 62, for a block more: 40 k nodes 0.0885 -> 0.0845 ms
+#define UPWIND_BOUNDS __maxnreg__(56)
+#endif
+__global__ void UPWIND_BOUNDS k_upwind_h(Dev d) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int L = d.L, NS = d.NS;
@@ -446,9 +451,12 @@ __device__ __forceinline__ real muscl_mean(bool upw2, real Tm1, real Tm2) {
 // MUSCL segment fluxes of one (edge, level) (fv_tracer.F90:59-170 for T and
 // S, :172-209 for the continuity term); thread per (edge, level), levels on
 // consecutive threads.  Each flux is computed once here and gathered by both
-// end nodes below.  64 registers: 32 resident warps per SM instead of 24
-// (17 % faster).
-__global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
+// end nodes below.  The elements' fields are loaded before the gradients'
+// branch and the first segment's divisions (an edge without a second element
+// loads the first's again): 1.05 M nodes 1.28 -> 1.21 ms, 232 k FP32 0.213 ->
+// 0.166.  Registers for the most resident warps: FP64 64 (48: 1.69 ms, 72:
+// 1.41), FP32 48 (0.143 ms; 40: 0.157, 56: 0.151).
+__global__ void __maxnreg__(FESOMC_FP32 ? 48 : 64) k_muscl_edge(Dev d) {
     pdl_enter();
     const unsigned total = (unsigned)d.Ed * d.L;
     const int L = d.L;
@@ -464,6 +472,9 @@ __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
         const real T1 = d.ttfold[i1], T2 = d.ttfold[i2];
         const real S1 = d.stfold[i1], S2 = d.stfold[i2];
         real g1, g2, g3, g4, h1, h2, h3, h4;
+        const size_t e1 = (size_t)et.x * L + z, e2 = et.y >= 0 ? (size_t)et.y * L + z : e1;
+        const real J1 = d.Je[e1], U1 = d.U_n_filt[e1], V1 = d.V_n_filt[e1];
+        const real J2 = d.Je[e2], U2f = d.U_n_filt[e2], V2f = d.V_n_filt[e2], Un2 = d.U_n[e2], Vn2 = d.V_n[e2];
         if (ud.x >= 0 && ud.y >= 0) {
             const size_t u = (size_t)ud.x * L + z, w = (size_t)ud.y * L + z;
             g1 = d.ttx[u]; g2 = d.ttx[w]; g3 = d.tty[u]; g4 = d.tty[w];
@@ -475,9 +486,6 @@ __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
         real2 fT, fS, fC;
         {
             const real a = kREarth * d.elem_cos[et.x];
-            const size_t e1 = (size_t)et.x * L + z;
-            const real J1 = d.Je[e1];
-            const real U1 = d.U_n_filt[e1], V1 = d.V_n_filt[e1];
             const bool up1 = V1 * X.x - U1 * X.y > 0;
             const real Tm2 = T2 - (real(2.0) * (T2 - T1) + exy.x * a * g2 + exy.y * kREarth * g4) / real(6.0);
             const real Tm1 = T1 + (real(2.0) * (T2 - T1) + exy.x * a * g1 + exy.y * kREarth * g3) / real(6.0);
@@ -491,9 +499,6 @@ __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
         }
         if (et.y >= 0) {
             const real b = kREarth * d.elem_cos[et.y];
-            const size_t e2 = (size_t)et.y * L + z;
-            const real J2 = d.Je[e2];
-            const real U2f = d.U_n_filt[e2], V2f = d.V_n_filt[e2];
             const bool up2 = V2f * X.z - U2f * X.w < 0;
             const real Tm2 = T2 - (real(2.0) * (T2 - T1) + exy.x * b * g2 + exy.y * kREarth * g4) / real(6.0);
             const real Tm1 = T1 + (real(2.0) * (T2 - T1) + exy.x * b * g1 + exy.y * kREarth * g3) / real(6.0);
@@ -502,7 +507,6 @@ __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
             const real Sm1 = S1 + (real(2.0) * (S2 - S1) + exy.x * b * h1 + exy.y * kREarth * h3) / real(6.0);
             const real Sm = muscl_mean(up2, Sm1, Sm2);
             // second segment uses U_n / V_n (fv_tracer.F90:158-159)
-            const real Un2 = d.U_n[e2], Vn2 = d.V_n[e2];
             fT.y = -(J2 * Vn2 * Tm) * X.z + (J2 * Un2 * Tm) * X.w;
             fS.y = -(J2 * Vn2 * Sm) * X.z + (J2 * Un2 * Sm) * X.w;
             fC.y = -J2 * V2f * X.z + J2 * U2f * X.w;
@@ -521,7 +525,9 @@ __global__ void __maxnreg__(64) k_muscl_edge(Dev d) {
 // loop is unrolled so the flux loads of several edges are in flight
 // together; the sums stay in edge order.  The vertical flux at interface
 // z+1 comes from the next lane when that lane holds the same node.
-__global__ void __launch_bounds__(128, 8) k_muscl_h(Dev d) {
+// FP64: 8 blocks per SM (12: 1.164 against 1.172 ms at 1.05 M nodes, but 0.024
+// against 0.021 at 16 k); FP32: 14, 232 k nodes 0.190 -> 0.134 ms.
+__global__ void __launch_bounds__(128, FESOMC_FP32 ? 14 : 8) k_muscl_h(Dev d) {
     pdl_enter();
     const unsigned total = (unsigned)d.N * d.L;
     const int lane = threadIdx.x & 31;
@@ -657,8 +663,9 @@ __global__ void k_miura_ngrad(Dev d) {
 }
 
 // Miura segment fluxes of one (edge, level) (fv_tracer.F90:1010-1140) and the
-// continuity terms (:1141-1168); thread per (edge, level)
-__global__ void k_miura_edge(Dev d) {
+// continuity terms (:1141-1168); thread per (edge, level).  48 registers, with
+// 12 blocks of miura_h: 42 k nodes 0.163 -> 0.154 ms (64 and 8 before).
+__global__ void __maxnreg__(48) k_miura_edge(Dev d) {
     pdl_enter();
     const unsigned total = (unsigned)d.Ed * d.L;
     const int L = d.L;
@@ -725,7 +732,7 @@ __global__ void k_miura_edge(Dev d) {
 // node gather of the Miura fluxes in edge order + vertical + update (T),
 // salinity passed through; one thread per (node, level), levels on
 // consecutive lanes of a flat index
-__global__ void __launch_bounds__(128, 8) k_miura_h(Dev d) {
+__global__ void __launch_bounds__(128, 12) k_miura_h(Dev d) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int L = d.L, NS = d.NS;
@@ -1173,7 +1180,7 @@ constexpr int kVtAtmThreads = FESOMC_FP32 ? 128 : 256;
 constexpr int kVtArrays = 6, kVtBatch = 4;
 
 template <bool kAtm>
-__global__ void __launch_bounds__(kAtm ? kVtAtmThreads : kVtThreads, FESOMC_FP32 ? 1 : kAtm ? 4 : 5) k_vdiff_tile(Dev d) {
+__global__ void __launch_bounds__(kAtm ? kVtAtmThreads : kVtThreads, FESOMC_FP32 ? 8 : kAtm ? 4 : 5) k_vdiff_tile(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char vt_smem[];
     __shared__ real s_aj[kVtCols], s_ta[kVtCols], s_sa[kVtCols];
@@ -1331,9 +1338,10 @@ __global__ void __launch_bounds__(kAtm ? kVtAtmThreads : kVtThreads, FESOMC_FP32
 // thread per column solves with its recurrences in registers, from rows of
 // odd stride, and stages with batched loads.  Fewer shared-memory passes,
 // but only as many threads as columns, which pays on full-size grids.
+// FP32: at least 14 blocks (72 registers), 232 k nodes 0.070 -> 0.062 ms.
 constexpr int kVrCols = 64;
 constexpr int kVrLayers = 20;
-__global__ void __launch_bounds__(kVrCols) k_vdiff_reg(Dev d) {
+__global__ void __launch_bounds__(kVrCols, FESOMC_FP32 ? 14 : 1) k_vdiff_reg(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char vt_smem[];
     constexpr int L = kVrLayers, LP = L | 1;
