@@ -995,7 +995,9 @@ __global__ void k_wvel(Dev d) {
 // 39 layers 0.032, 0.025 -> 0.019.
 constexpr int kIvCols = 32;
 constexpr int kIvThreads = 128;
+#if !FESOMC_FP32
 constexpr int kIvBatch = 3;
+#endif
 
 __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
     pdl_enter();

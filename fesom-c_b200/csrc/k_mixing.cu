@@ -32,7 +32,6 @@ __device__ __forceinline__ real div_pos(real x, real d) {
     return x == real(0.0) ? x : q;
 }
 
-#if !FESOMC_FP32
 // d3_end per node column (local-memory arrays indexed 1..NS like the Fortran
 // ones, ARR >= NS + 1 entries each).  The kernel is bound by the traffic of
 // those arrays: the working set of the resident columns does not fit in L2,
@@ -50,7 +49,8 @@ __device__ __forceinline__ real div_pos(real x, real d) {
 //   * both sweeps load the next level's array values one level ahead, so
 //     that their latency overlaps the current level's division chain (3 %
 //     faster; unrolling by 4 instead was 9 % slower).
-// The form for level counts whose tiles (below) do not fit well.
+// The form of FP32, and in FP64 for level counts whose tiles (below) do not
+// fit well.
 //
 // kList: the columns are list[0 .. *count) instead of every node (the
 // columns the learned closure hands back to the plain one).
@@ -197,7 +197,6 @@ __global__ void k_d3end(Dev d, const int *list, const unsigned long long *count)
         }
     }
 }
-#endif
 
 // ---- d3_end on tiles of columns in shared memory ----------------------------
 // A block takes kT3Cols consecutive (or listed) node columns and keeps all
@@ -207,7 +206,7 @@ __global__ void k_d3end(Dev d, const int *list, const unsigned long long *count)
 // b2, c2, Ri: most of the FP64 work), the sweep-invariant am and cm, in
 // every sweep the divisions of c1 and bm, and the final bt, snu, Kv and
 // tke_dissip.  Only the recurrences of the sweep and the back substitution
-// are left to one or two lanes per column, all of one or two warps; which
+// are left to a pair of lanes per column, all of one or two warps; which
 // ones alternates between the blocks of an SM, so that their chains run on
 // different schedulers.  The arithmetic and its
 // order are k_d3end's.
@@ -223,33 +222,28 @@ __global__ void k_d3end(Dev d, const int *list, const unsigned long long *count)
 // Bound by latency, the chains of the recurrences first (with one lane per
 // column and the convergence test in its loop they took 47 % of a block's
 // time, 640 cycles a level: an FP64 division is 114 cycles, and two of them
-// in one thread run one after the other), then the set-up's divisions.  In
-// FP64 a pair of lanes forms xx1 and yy1 of a column at the same time, the
-// test is done by all threads afterwards, and a layer's density at its two
-// interfaces shares the terms without the pressure; FP32, whose divisions are
-// short, keeps one lane and the test in its loop.  FP64: 256 threads and 64
+// in one thread run one after the other), then the set-up's divisions.  So
+// a pair of lanes forms xx1 and yy1 of a column at the same time, the test is
+// done by all threads afterwards, and a layer's density at its two
+// interfaces shares the terms without the pressure.  256 threads and 64
 // registers, four blocks of 32 columns (21 interfaces) per SM by shared
-// memory; FP32 tiles are half the size: 128 threads, more blocks.
+// memory.
 // Against one thread per column with its arrays in local memory (whose
-// traffic streamed through DRAM): 1.05 M nodes FP64 2.71 -> 2.03 ms (2.31 with
-// one lane per column), 42 k 0.134 -> 0.107, 40 k with 31 interfaces 0.23 ->
-// 0.146, 16 k with 11 0.046 -> 0.028, 4.5 k with 40 0.196 -> 0.039, 232 k FP32
-// 0.31 -> 0.19 ms.  A set-up kernel and a sweep kernel with the sweep's arrays
-// in local memory, shared memory or registers took 2.32-2.54 ms at 1.05 M
-// nodes, 128 threads or tiles of 16 2.54 and 2.65.
+// traffic streamed through DRAM): 1.05 M nodes 2.71 -> 2.05 ms (2.31 with one
+// lane per column), 42 k 0.134 -> 0.107, 40 k with 31 interfaces 0.23 -> 0.146,
+// 16 k with 11 0.046 -> 0.028, 4.5 k with 40 0.196 -> 0.039.  A set-up kernel and
+// a sweep kernel with the sweep's arrays in local memory, shared memory or
+// registers took 2.32-2.54 ms at 1.05 M nodes, 128 threads or tiles of 16 2.54
+// and 2.65.
+#if !FESOMC_FP32
 constexpr int kT3Arrays = 9;
-constexpr int kT3Threads = FESOMC_FP32 ? 128 : 256;
-#if FESOMC_FP32
-#define D3_TILE_BOUNDS __launch_bounds__(kT3Threads)
-#else
-#define D3_TILE_BOUNDS __launch_bounds__(kT3Threads, 4)
-#endif
+constexpr int kT3Threads = 256;
 static size_t d3end_tile_smem(const Dev &d, int cols) {
     return ((size_t)kT3Arrays * d.NS * (cols + 1) + 2 * cols) * sizeof(real) + 4 * cols * sizeof(int);
 }
 
 template <int C, bool kList>
-__global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsigned long long *count) {
+__global__ void __launch_bounds__(kT3Threads, 4) k_d3end_tile(Dev d, const int *list, const unsigned long long *count) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char d3t_smem[];
     constexpr int CP = C + 1;
@@ -265,18 +259,12 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
     const real cka = d.cka;
     const real B1cka2 = real(16.6) * (cka * cka);
     const int ncol = kList ? (int)*count : d.N;
-    // the warps of the recurrences: FP32 one lane, FP64 a pair of lanes per
-    // column
-#if FESOMC_FP32
-    const int lane = threadIdx.x & 31;
-    const bool mine = (int)(threadIdx.x >> 5) == (int)((blockIdx.x / 148) % (kT3Threads / 32));
-#else
+    // the warps of the recurrences: a pair of lanes per column
     constexpr int kChains = C / 16, kWarps = kT3Threads / 32;
     static_assert(kWarps % kChains == 0, "the warps of the recurrences lie side by side");
     const int w0 = (int)(kChains * (blockIdx.x / 148) % kWarps), cw = (int)(threadIdx.x >> 5) - w0;
     const int lane = cw * 16 + (int)(threadIdx.x & 31) / 2;   // column
     const bool mine = cw >= 0 && cw < kChains;
-#endif
     for (int n0 = blockIdx.x * C; n0 < ncol; n0 += gridDim.x * C) {
         const int nt = ncol - n0 < C ? ncol - n0 : C;
         if ((int)threadIdx.x < nt) {
@@ -287,7 +275,6 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
             s_done[threadIdx.x] = 0;
         }
         __syncthreads();
-#if !FESOMC_FP32
         // each layer's density at its two interfaces, one (column, layer) per
         // thread: the terms without the pressure serve both.  Layer m is below
         // interface m (rho_dn of m, in s_qb) and above m + 1 (rho_up, in s_pb).
@@ -300,7 +287,6 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
             if (m < L - 1) s_pb[o + CP] = rho.at(-zbar_of(d, s_aj[j], m + 1), d.density_0);
         }
         __syncthreads();
-#endif
         // set-up, one (column, interface) per thread; k = nz - 1
         for (int i = threadIdx.x; i < nt * NS; i += kT3Threads) {
             const int j = d.by_NS.div(i), k = i - j * NS;
@@ -325,13 +311,7 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
             const real ap2 = d.Vnode[gl - 1] - d.Vnode[gl];
             real b1 = div_pos(sn_0 * (ap1 * ap1 + ap2 * ap2), dd * dd);
             b1 = div_pos(b1, dmean2);
-#if FESOMC_FP32
-            const real zb = zbar_of(d, s_aj[j], k);
-            const real rho_up = density_jm(d.TF[gl - 1], d.SF[gl - 1], -zb, d.density_0);
-            const real rho_dn = density_jm(d.TF[gl], d.SF[gl], -zb, d.density_0);
-#else
             const real rho_up = s_pb[o], rho_dn = s_qb[o];
-#endif
             ap1 = div_pos(rho_up - rho_dn, dd);
             const real b2 = div_pos(-real(0.5) * kG * d.Kv[g] * ap1, d.density_0 * dmean);
             const real snu_p = real(0.5) * (sn_m + sn_0);
@@ -379,48 +359,6 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
                 bx[o] = s_am[o] + s_cm[o] + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
             }
             __syncthreads();
-#if FESOMC_FP32
-            if (open) {
-                const real *am_ = s_am + lane, *cm_ = s_cm + lane, *bo = bt + lane;
-                real *X = bx + lane, *Y = s_fy + lane;
-                real x = real(1.0), y = y2;
-                real am_n = am_[CP], cm_n = cm_[CP], bm_n = X[CP], fr_n = Y[CP];
-                for (int k = 1; k <= NS - 2; ++k) {
-                    const real am = am_n, cm = cm_n, bm = bm_n, fr = fr_n;
-                    const int kn = (k < NS - 2 ? k + 1 : k) * CP;
-                    am_n = am_[kn]; cm_n = cm_[kn]; bm_n = X[kn]; fr_n = Y[kn];
-                    const real a = bm - am * x;
-                    const real xn = cm / a;
-                    const real yn = (am * y - fr) / a;
-                    X[k * CP] = xn;   // xx1(nz+1), nz = k + 1
-                    Y[k * CP] = yn;
-                    x = xn;
-                    y = yn;
-                }
-                real b1v = bot;  // btr1(NS)
-                const real top = bo[(NS - 1) * CP];
-                bool above = d3_above_tol(top - b1v, dmax(b1v, top) + real(1.0e-8));
-                X[(NS - 1) * CP] = b1v;
-                for (int k = NS - 2; k >= 1; --k) {
-                    const real xv = X[k * CP], yv = Y[k * CP], ov = bo[k * CP];
-                    b1v = b1v * xv + yv;  // btr1(k+1), into the slot of xx1(k+2)
-                    X[k * CP] = b1v;
-                    above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
-                }
-                b1v = b1v * real(1.0) + y2;
-                X[0] = b1v;
-                above |= d3_above_tol(bo[0] - b1v, dmax(b1v, bo[0]) + real(1.0e-8));
-                if (!above || it == 200) {
-                    // the final btr: the previous iterate when the sweep
-                    // converges, else the last sweep's
-                    s_par[lane] = above ? par ^ 1 : par;
-                    s_done[lane] = above ? 2 : 1;
-                    if (above) atomicAdd(d.notconv, 1);
-                    if (d.d3_iters) d.d3_iters[s_node[lane]] = it;   // measurement only (fesomc_gpu_d3end_iterations)
-                    open = false;
-                }
-            }
-#else
             if (mine) {
                 // forward: the lanes of a pair form xx1 and yy1, one division
                 // each at the same time, and share xx1 (__shfl needs every
@@ -481,7 +419,6 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
                     open = false;
                 }
             }
-#endif
             par ^= 1;
             if (!__syncthreads_or(open)) break;
         }
@@ -508,6 +445,7 @@ __global__ void D3_TILE_BOUNDS k_d3end_tile(Dev d, const int *list, const unsign
         __syncthreads();
     }
 }
+#endif
 
 // Av(nz,elem) = sum(w_cv*snu(nz,nodes)) (fv_mixing.F90:308-313)
 __global__ void k_av(Dev d) {
@@ -527,11 +465,13 @@ __global__ void k_av(Dev d) {
 // Which form: the tiles while three blocks of 16 columns fit an SM (FP64 up
 // to 61 interfaces, 40 k nodes: 0.49 against 0.53 ms; 81 interfaces, two
 // blocks: 0.92 against 0.72), else one thread per column (also with the
-// launch-shape knob "d3end_arrays" at 1).  FP32 always takes the tiles: half
-// the size (81 interfaces: 3.1 against 3.9 ms, 127: 16.1 against 18.6), and
-// the two forms' contracted arithmetic would not give the same bits.
+// launch-shape knob "d3end_arrays" at 1).  FP32 takes one thread per column
+// alone: the tiles were faster (232 k nodes 0.32 -> 0.20 ms), but their
+// contracted arithmetic rounds otherwise, and the elevation, held in FP64,
+// shows it (1.8e-6 relative after 78 steps).
+#if !FESOMC_FP32
 static bool d3end_tiled(const Dev &d) {
-    return FESOMC_FP32 || (d.tune[TK_D3END] != 1 && d3end_tile_smem(d, 16) <= 75 * 1024);
+    return d.tune[TK_D3END] != 1 && d3end_tile_smem(d, 16) <= 75 * 1024;
 }
 // columns per tile: 32; 16 where 32 would not leave an SM two blocks, and on
 // meshes whose 16-column tiles are at most two per SM (twice the blocks for
@@ -539,8 +479,12 @@ static bool d3end_tiled(const Dev &d) {
 static int d3end_cols(const Dev &d) {
     return d.N > 2 * 148 * 16 && d3end_tile_smem(d, 32) <= 113 * 1024 ? 32 : 16;
 }
+#endif
 int config_d3end(const Dev &d) {
     if (d.NS > 127) return 1;
+#if FESOMC_FP32
+    return 0;
+#else
     const size_t t32 = d3end_tile_smem(d, 32), t16 = d3end_tile_smem(d, 16);
     bool ok = true;
     if (t32 <= 113 * 1024)
@@ -549,19 +493,22 @@ int config_d3end(const Dev &d) {
     return ok && raise_smem_limit(k_d3end_tile<16, false>, t16) == cudaSuccess &&
                    raise_smem_limit(k_d3end_tile<16, true>, t16) == cudaSuccess
                ? 0 : 1;
+#endif
 }
 template <bool kList>
 static void launch_d3end_form(const Dev &d, const int *list, const unsigned long long *count, cudaStream_t s) {
+#if !FESOMC_FP32
     if (d3end_tiled(d)) {
         const int C = d3end_cols(d), tiles = (d.N + C - 1) / C;
         if (C == 32) launch_k(k_d3end_tile<32, kList>, tiles, kT3Threads, d3end_tile_smem(d, 32), s, d, list, count);
         else launch_k(k_d3end_tile<16, kList>, tiles, kT3Threads, d3end_tile_smem(d, 16), s, d, list, count);
+        return;
     }
-#if !FESOMC_FP32
+#endif
+    if (d.NS <= 11) launch_k(k_d3end<12, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);
     else if (d.NS <= 21) launch_k(k_d3end<22, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);
     else if (d.NS <= 40) launch_k(k_d3end<41, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);
     else launch_k(k_d3end<128, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);
-#endif
 }
 void launch_d3end(const Dev &d, cudaStream_t s) { launch_d3end_form<false>(d, nullptr, nullptr, s); }
 // the plain closure on the listed columns (count read on the device, so the

@@ -455,7 +455,7 @@ int  fesomc_ensemble_run(fesomc_model *const *members, int32_t n_members, int32_
  * d3_end with one thread per column, its arrays in local memory, or (2 to 6,
  * the same form under every number, so that saved shapes stay valid) on
  * tiles of columns in shared memory, the default up to 61 levels; the FP32
- * form takes the tiles under every number;
+ * form has one thread per column under every number;
  * "vdiff_form" 1 to 3, the same under every number: the tracers' implicit
  * vertical diffusion runs on tiles of columns in shared memory;
  * "implvisc_form" 1 or 2, the same under both numbers: the implicit vertical
