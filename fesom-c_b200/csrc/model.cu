@@ -501,26 +501,25 @@ struct FieldOut {
     FieldRef f;
     double *h;
 };
-// all fields through the staging slots; g_staging.in_use is held
-int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields, unsigned char *buf) {
-    size_t total = 0;
-    for (const FieldOut &o : fields) total += (o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double)) + 15) & ~(size_t)15;
-    if (total <= kSlots * kSlotBytes / 4) {
-        std::vector<StagedPiece> out;
-        size_t off = 0;
-        for (const FieldOut &o : fields) {
-            const size_t bytes = o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double));
-            const unsigned char *src;
-            const int rc = field_source(m, o.f, &src);
-            if (rc) return rc;
-            CK(cudaMemcpyAsync(buf + off, src, bytes, cudaMemcpyDeviceToHost, m->stream));
-            out.push_back({buf + off, o.h, bytes, o.f.f32});
-            off += (bytes + 15) & ~(size_t)15;
-        }
-        CK(cudaStreamSynchronize(m->stream));
-        for (const StagedPiece &p : out) piece_out(p);
-        return FESOMC_OK;
+// all fields, enqueued at once
+int fields_at_once(fesomc_model *m, const std::vector<FieldOut> &fields, unsigned char *buf) {
+    std::vector<StagedPiece> out;
+    size_t off = 0;
+    for (const FieldOut &o : fields) {
+        const size_t bytes = o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double));
+        const unsigned char *src;
+        const int rc = field_source(m, o.f, &src);
+        if (rc) return rc;
+        CK(cudaMemcpyAsync(buf + off, src, bytes, cudaMemcpyDeviceToHost, m->stream));
+        out.push_back({buf + off, o.h, bytes, o.f.f32});
+        off += (bytes + 15) & ~(size_t)15;
     }
+    CK(cudaStreamSynchronize(m->stream));
+    for (const StagedPiece &p : out) piece_out(p);
+    return FESOMC_OK;
+}
+// all fields, slot after slot with worker threads
+int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, unsigned char *buf) {
     int dev = 0;
     CK(cudaGetDevice(&dev));
     std::mutex mu;
@@ -592,6 +591,16 @@ int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields, 
     for (std::thread &t : pool) t.join();
     CK(cudaStreamSynchronize(m->stream));
     return rc ? rc : (bad ? FESOMC_ECUDA : FESOMC_OK);
+}
+// all fields through the staging slots; g_staging.in_use is held
+int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields, unsigned char *buf) {
+    size_t total = 0;
+    for (const FieldOut &o : fields) total += (o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double)) + 15) & ~(size_t)15;
+    const int rc = total <= kSlots * kSlotBytes / 4 ? fields_at_once(m, fields, buf) : fields_by_slots(m, fields, buf);
+    // after a failure too, no copy may still be on its way to the slots when
+    // another model's read-back takes them
+    if (rc) (void)cudaStreamSynchronize(m->stream);
+    return rc;
 }
 
 // host double <-> device field (converting for FP32 level fields, and
