@@ -213,8 +213,10 @@ inline int default_columns(int L) {
 // completed and its writes are visible, and only then lets the one after be
 // launched: at most one kernel waits at a time, and when a kernel passes its
 // wait, every earlier kernel of the stream has completed (each of them
-// passed its own first).  The first kernel after a memset or copy on the
-// stream is launched plainly.
+// passed its own first).  That rests on the work before being a kernel: the
+// first kernel of a step and every other one behind a memset, a copy or a
+// graph on its stream is launched plainly (launch_plain; a captured step
+// loses nothing by it, its first kernel has none before it).
 // Only grids of at most two blocks per SM are started early.  Steps of small
 // meshes are bound by launches (697 nodes: 0.353 -> 0.328 ms per step, 16 k
 // nodes: 0.488 -> 0.440 ms); the waiting blocks of a large grid take slots
@@ -228,7 +230,7 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;");
 }
 template <typename... P, typename... A>
-inline void launch_k(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
+inline void launch_as(bool early, void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
@@ -238,21 +240,33 @@ inline void launch_k(void (*kernel)(P...), dim3 grid, int block, size_t smem, cu
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = early_grid(grid.x * grid.y) ? 1 : 0;
+    cfg.numAttrs = early && early_grid(grid.x * grid.y) ? 1 : 0;
     (void)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
-
+template <typename... P, typename... A>
+inline void launch_k(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
+    launch_as(true, kernel, grid, block, smem, s, args...);
+}
+template <typename... P, typename... A>
+inline void launch_plain(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
+    launch_as(false, kernel, grid, block, smem, s, args...);
+}
 
 // Launches a kernel whose blocks of 'threads' take groups of 'per_block'
 // entities and stride over them: as many blocks as are resident at once (a
 // few more would make a second, mostly empty wave of all the work).
 template <typename... P, typename... A>
-inline void launch_resident(void (*kernel)(P...), long long count, int per_block, int threads, size_t smem,
-                            cudaStream_t s, A... args) {
+inline void launch_resident_as(bool early, void (*kernel)(P...), long long count, int per_block, int threads,
+                               size_t smem, cudaStream_t s, A... args) {
     const long long blocks = (count + per_block - 1) / per_block;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
-    launch_k(kernel, (unsigned)(blocks < 148LL * occ ? blocks : 148LL * occ), threads, smem, s, args...);
+    launch_as(early, kernel, (unsigned)(blocks < 148LL * occ ? blocks : 148LL * occ), threads, smem, s, args...);
+}
+template <typename... P, typename... A>
+inline void launch_resident(void (*kernel)(P...), long long count, int per_block, int threads, size_t smem,
+                            cudaStream_t s, A... args) {
+    launch_resident_as(true, kernel, count, per_block, threads, smem, s, args...);
 }
 
 }  // namespace fesomc

@@ -35,6 +35,6 @@ struct PotentialDev {
     double *ssh_gp;
 };
 
-void launch_potential(const PotentialDev &p, cudaStream_t s);
+void launch_potential(const PotentialDev &p, bool first, cudaStream_t s);
 
 }  // namespace fesomc

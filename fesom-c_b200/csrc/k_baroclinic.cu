@@ -1199,8 +1199,9 @@ int config_columns(const Dev &d) {
     if (e == cudaSuccess) e = raise_smem_limit(k_wvel, wvel_smem(d));
     return e == cudaSuccess ? 0 : 1;
 }
-void launch_pressure_col(const Dev &d, cudaStream_t s) {
-    launch_resident(k_pressure_col, d.N, col_b(d), col_b(d) * d.L, pressure_smem(d), s, d);
+// first: nothing but copies, fills or graphs before it on the stream
+void launch_pressure_col(const Dev &d, bool first, cudaStream_t s) {
+    launch_resident_as(!first, k_pressure_col, d.N, col_b(d), col_b(d) * d.L, pressure_smem(d), s, d);
 }
 void launch_bpg_elem(const Dev &d, cudaStream_t s) {
     launch_resident(k_bpg_elem, d.E, col_b(d), col_b(d) * d.L, bpg_smem(d), s, d);
@@ -1250,7 +1251,8 @@ void launch_jac_swap(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ROT, 256);
     launch_k(k_jac_swap, grid_for(d.N, b), b, 0, s, d);
 }
-void launch_je(const Dev &d, cudaStream_t s) { launch_k(k_je_elem, grid_for((long long)d.E * d.L, 256), 256, 0, s, d); }
+// after an upload or a copy of the elevation
+void launch_je(const Dev &d, cudaStream_t s) { launch_plain(k_je_elem, grid_for((long long)d.E * d.L, 256), 256, 0, s, d); }
 void launch_update3d(const Dev &d, real Mt_inv, cudaStream_t s) {
     launch_resident(k_update3d, d.E, col_b(d), col_b(d) * d.L, update3d_smem(d), s, d, Mt_inv);
 }

@@ -236,7 +236,7 @@ __global__ void k_lc_judge(Dev d, LcView c) {
 }
 
 void launch_lc_features(const Dev &d, const LcView &c, cudaStream_t s) {
-    k_lc_features<<<grid_for(d.N, 128), 128, 0, s>>>(d, c);   // follows a memset
+    launch_plain(k_lc_features, grid_for(d.N, 128), 128, 0, s, d, c);   // follows a memset
 }
 void launch_lc_apply(const Dev &d, const LcView &c, cudaStream_t s) {
     launch_k(k_lc_apply, grid_for(d.N, 128), 128, 0, s, d, c);

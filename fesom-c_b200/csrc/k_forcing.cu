@@ -106,16 +106,17 @@ __global__ void k_potential(PotentialDev p) {
     }
 }
 
-void launch_potential(const PotentialDev &p, cudaStream_t s) {
+void launch_potential(const PotentialDev &p, bool first, cudaStream_t s) {
     const int block = 256;
     long long g = ((long long)p.N + block - 1) / block;
     if (g < 1) g = 1;
     if (g > 148 * 8) g = 148 * 8;
-    launch_k(k_potential, (int)g, block, 0, s, p);
+    launch_as(!first, k_potential, (int)g, block, 0, s, p);
 }
 
+// the first kernels of a step with device forcing
 void launch_forcing(const ForcingDev &f, cudaStream_t s) {
-    launch_k(k_forcing_clock, 1, 32, 0, s, f);
+    launch_plain(k_forcing_clock, 1, 32, 0, s, f);
     const long long n = (f.tides_on ? (long long)f.Mt * f.nobn : 0) + (f.rivers_on ? f.n_rivers : 0);
     const int block = 128;
     long long g = (n + block - 1) / block;

@@ -1102,8 +1102,8 @@ __global__ void k_atm_stress(Dev d, AtmDev a) {
         d.tauy[e] = (real)sy;
     }
 }
-void launch_atm(const Dev &d, const AtmDev &a, cudaStream_t s) {
-    launch_k(k_atm_nodes, grid_for(d.N, 128), 128, 0, s, d, a);
+void launch_atm(const Dev &d, const AtmDev &a, bool first, cudaStream_t s) {
+    launch_as(!first, k_atm_nodes, grid_for(d.N, 128), 128, 0, s, d, a);
     launch_k(k_atm_stress, grid_for(d.E, 256), 256, 0, s, d, a);
 }
 

@@ -32,7 +32,7 @@ namespace fesomc {
     void launch_adv2d_edge(const Dev &, cudaStream_t); \
     void launch_sub_edge(const Dev &, cudaStream_t); \
     void launch_u2d_elem(const Dev &, int, cudaStream_t); \
-    void launch_pressure_col(const Dev &, cudaStream_t); \
+    void launch_pressure_col(const Dev &, bool, cudaStream_t); \
     void launch_bpg_elem(const Dev &, cudaStream_t); \
     void launch_velgrad3d(const Dev &, cudaStream_t); \
     void launch_adv3_edge(const Dev &, cudaStream_t); \
@@ -57,7 +57,7 @@ namespace fesomc {
     void launch_av(const Dev &, cudaStream_t); \
     void launch_minmax(const Dev &, cudaStream_t); \
     void launch_aver_from_range(const Dev &, const double *, cudaStream_t); \
-    void launch_atm(const Dev &, const AtmDev &, cudaStream_t); \
+    void launch_atm(const Dev &, const AtmDev &, bool, cudaStream_t); \
     void launch_upwind(const Dev &, cudaStream_t); \
     void launch_muscl_egrad(const Dev &, cudaStream_t); \
     void launch_muscl_ngrad(const Dev &, cudaStream_t); \
@@ -1278,7 +1278,7 @@ int enqueue_step(fesomc_model *m, double ff) {
         // sbc_do (fv_main.F90:419), before the step, from the previous
         // step's surface velocity and temperature
         const AtmDev a{m->d_atm_a, m->d_atm_b, m->d_clock, m->d_tau_node, m->atm_net_flux, m->atm_prec_coef};
-        rec(m, "atm_fluxes", [&] { fesomc::f64::launch_atm(d, a, s); });
+        rec(m, "atm_fluxes", [&] { fesomc::f64::launch_atm(d, a, n == 0, s); });
         n += 2;
     }
     if (m->p.T_potential) {
@@ -1291,10 +1291,10 @@ int enqueue_step(fesomc_model *m, double ff) {
         pd.clock = m->d_clock;
         pd.coord = m->d_coord;
         pd.ssh_gp = f ? q.ssh_gp : d.ssh_gp;
-        rec(m, "potential", [&] { launch_potential(pd, s); });
+        rec(m, "potential", [&] { launch_potential(pd, n == 0, s); });
         n += 1;
     }
-    rec(m, "pressure_col", [&] { K3(launch_pressure_col, s); });
+    rec(m, "pressure_col", [&] { K3(launch_pressure_col, n == 0, s); });
     rec(m, "bpg_elem", [&] { K3(launch_bpg_elem, s); });
     n += 2;
     rec(m, "el2nodes", [&] { K3E2N(U_n, V_n, Unode, Vnode); });

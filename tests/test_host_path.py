@@ -52,3 +52,57 @@ def test_failed_readback_leaves_no_copy_pending(fake, fp32, sfc):
         fake.lib.fake_fail_copy(-1)
         a.close()
         b.close()
+
+
+def _check_starts(fake):
+    """Every kernel started early directly follows a kernel on its stream (or
+    opens a captured step, which as a graph waits for all before it)."""
+    before, early = {}, 0
+    for o in fake.ops():
+        if o.early:
+            early += 1
+            prev = before.get((o.stream, o.captured), "k" if o.captured else "")
+            assert prev == "k", (o.name, prev)
+        before[(o.stream, o.captured)] = o.kind
+    return early
+
+
+@pytest.mark.parametrize("kw", [{}, {"fp32_form": 1, "sfc_order": 1}, {"T_potential": 1}, {"atm": {"qns": -50.0}},
+                                {"bih_3D": 1, "bih_2D": 1, "Abh0": 1e4}])
+@pytest.mark.parametrize("device_forcing", [False, True])
+def test_early_starts_follow_kernels(fake, kw, device_forcing):
+    """What makes an early start safe is the kernel before it; behind a copy
+    or a fill (the forcing's upload, a snapshot, a halo, the status) a kernel
+    is launched plainly: in first, captured, replayed and harvesting steps."""
+    from fesomc import abi, cases, closure
+    fake.clear()
+    g = _model(**kw)
+    c = closure.Closure(g.case.mesh.NS, capacity=4096)
+    try:
+        if "atm" in kw and not device_forcing:
+            g.set_atm_fields(*cases.atm_coefficients(g.case.mesh, g.case.params.time_jd0))
+        if device_forcing:
+            f = g.case.forcing_fn(1, g.case.params.time_jd0 + 20.0)
+            g.set_forcing(f)
+            base = np.ascontiguousarray(f["runoff_rivers"])
+            abi.check(g.lib.fesomc_gpu_set_device_forcing(g.h, abi.dptr(base), 1))
+        g.snapshot_begin()            # its copies on the step's stream are not waited for
+        g.step(1)
+        g.snapshot_end()
+        g.step(2)
+        g.snapshot_begin()
+        c.harvest(g, 2)
+        g.snapshot_end()
+        g.energy()
+        n = np.arange(1, 40, dtype=np.int32)
+        h, m = C.c_void_p(), C.c_int64()
+        abi.check(g.lib.fesomc_gpu_halo_plan(g.h, len(n), abi.iptr(n), len(n), abi.iptr(n), C.byref(h)))
+        abi.check(g.lib.fesomc_gpu_halo_size(h, C.byref(m)))
+        buf = np.zeros(m.value)
+        abi.check(g.lib.fesomc_gpu_halo_pack(g.h, h, buf.ctypes.data))
+        abi.check(g.lib.fesomc_gpu_halo_unpack(g.h, h, buf.ctypes.data))
+        g.lib.fesomc_gpu_halo_free(h)
+        assert _check_starts(fake) > 50
+    finally:
+        c.close()
+        g.close()
