@@ -1332,7 +1332,7 @@ int enqueue_step(fesomc_model *m, double ff) {
     if (d.bih_3D) { rec(m, "biharmonic", [&] { K3(launch_bih, s); }); n += 4; }
     rec(m, "velrhs", [&] { K3(launch_velrhs, ff, s); });
     n += 1;
-    if (d.im_vert_visc || d.im_vert_visc_fic) { rec(m, "implvisc", [&] { K3(launch_implvisc, s); }); n += 1; }
+    if (d.im_vert_visc || d.im_vert_visc_fic) { rec(m, "implvisc", [&] { K3(launch_implvisc, s); }); n += (d.im_vert_visc != 0) + (d.im_vert_visc_fic != 0); }
     // the AB3 velocity of a sub-step is formed by the u2d_elem of the one
     // before (its neighbours still read this sub-step's: two buffers in turn)
     rec(m, "ab3_elem", [&] { K3(launch_ab3_elem, s); });

@@ -106,3 +106,31 @@ def test_early_starts_follow_kernels(fake, kw, device_forcing):
     finally:
         c.close()
         g.close()
+
+
+def _kernels(fake):
+    return sum(o.kind == "k" for o in fake.ops())
+
+
+@pytest.mark.parametrize("kw", [{}, {"fp32_form": 1}, {"tracer_adv": 1}, {"tracer_adv": 4}, {"T_potential": 1},
+                                {"atm": {"qns": -50.0}}, {"bih_3D": 1, "Abh0": 1e4}, {"bih_2D": 1, "Abh0": 1e4},
+                                {"bih_2D": 1, "mom_adv_2D": 0, "Abh0": 1e4}, {"mom_adv_3D": 0},
+                                {"filt_bi_3D": 1, "filt_bi_2D": 1}, {"im_vert_visc": 1, "im_vert_visc_fic": 0},
+                                {"im_vert_visc": 1, "im_vert_visc_fic": 1}, {"im_vert_visc_fic": 0}])
+def test_counted_launches_are_the_launches(fake, kw):
+    """fesomc_gpu_kernel_launches against the launches made: the first step
+    and the captured one."""
+    from fesomc import cases
+    g = _model(**kw)
+    try:
+        if "atm" in kw:
+            g.set_atm_fields(*cases.atm_coefficients(g.case.mesh, g.case.params.time_jd0))
+        for _ in range(2):
+            f = g.case.forcing_fn(1, g.time_jd)
+            g.set_forcing(f)
+            fake.clear()
+            n0 = g.kernel_launches()
+            assert g.lib.fesomc_gpu_step(g.h, 1) == 0
+            assert g.kernel_launches() - n0 == _kernels(fake)
+    finally:
+        g.close()
