@@ -603,6 +603,15 @@ int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields, 
     return rc;
 }
 
+// whether a field's array in the caller's memory is page-locked
+bool page_locked(const double *h, size_t count) {
+    cudaPointerAttributes a, b;
+    if (cudaPointerGetAttributes(&a, h) == cudaSuccess && cudaPointerGetAttributes(&b, h + count - 1) == cudaSuccess)
+        return a.type == cudaMemoryTypeHost && b.type == cudaMemoryTypeHost;
+    (void)cudaGetLastError();
+    return false;
+}
+
 // host double <-> device field (converting for FP32 level fields, and
 // between the reference and the storage order)
 int field_to_host(fesomc_model *m, const FieldRef &f, double *h) {
@@ -1820,20 +1829,37 @@ int fesomc_gpu_sync_to_host(fesomc_model *m, uint32_t mask, fesomc_state *st) {
     if (!m || !st) return FESOMC_EINVAL;
     CK(cudaStreamSynchronize(m->stream));
     std::vector<FieldOut> fields;
+    int rc = FESOMC_OK;
+    bool direct = false;
     for (const FieldRef &f : field_table(m)) {
         double *h = st->*(f.host);
-        if ((f.group & mask) && h) fields.push_back({f, h});
+        if (rc || !(f.group & mask) || !h) continue;
+        if (f.f32 || !page_locked(h, f.count)) {
+            fields.push_back({f, h});
+            continue;
+        }
+        // a page-locked array receives the copy directly
+        const unsigned char *src;
+        rc = field_source(m, f, &src);
+        if (!rc && cudaMemcpyAsync(h, src, f.count * sizeof(double), cudaMemcpyDeviceToHost, m->stream) != cudaSuccess)
+            rc = FESOMC_ECUDA;
+        direct = true;
     }
-    int rc = FESOMC_ENOMEM;   // the staging could not be had: field by field
-    {
+    if (direct && (rc || fields.empty()) && cudaStreamSynchronize(m->stream) != cudaSuccess) rc = FESOMC_ECUDA;
+    if (rc) return rc;
+    rc = fields.empty() ? FESOMC_OK : FESOMC_ENOMEM;   // ENOMEM: the staging could not be had: field by field
+    if (!fields.empty()) {
         std::unique_lock<std::mutex> lk(g_staging.in_use, std::try_to_lock);
-        unsigned char *buf = lk.owns_lock() && !fields.empty() ? staging_for(m) : nullptr;
+        unsigned char *buf = lk.owns_lock() ? staging_for(m) : nullptr;
         if (buf) rc = fields_to_host_staged(m, fields, buf);
     }
-    if (rc != FESOMC_OK && rc != FESOMC_ENOMEM) return rc;
-    for (size_t k = 0; rc != FESOMC_OK && k < fields.size(); ++k) {
-        const int r = field_to_host(m, fields[k].f, fields[k].h);
-        if (r) return r;
+    if (rc == FESOMC_ENOMEM) {
+        rc = FESOMC_OK;
+        for (size_t k = 0; !rc && k < fields.size(); ++k) rc = field_to_host(m, fields[k].f, fields[k].h);
+    }
+    if (rc) {
+        if (direct) (void)cudaStreamSynchronize(m->stream);   // no copy to the caller's memory outlives the call
+        return rc;
     }
     st->lfirst = m->lfirst;
     st->time_jd = m->time_jd;

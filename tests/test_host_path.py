@@ -134,3 +134,33 @@ def test_counted_launches_are_the_launches(fake, kw):
             assert g.kernel_launches() - n0 == _kernels(fake)
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+def test_page_locked_arrays_receive_the_copy_directly(fake, fp32):
+    """A read-back into page-locked arrays (here the ones a snapshot locked)
+    copies its FP64 fields straight into them; the FP32 fields, which are
+    widened on the host, and pageable arrays go through the staging slots."""
+    from fesomc import abi
+    g = _model(fp32_form=fp32)
+    try:
+        want = g.state()
+        g.snapshot_begin()
+        g.snapshot_end()
+        arrays, st = g._snap
+        fp64 = {"eta_n", "eta_n_1", "eta_n_2", "etaAB", "ssh_gp"} if fp32 else set(arrays)
+        for pageable in (False, True):
+            if pageable:
+                arrays = {k: np.empty_like(v) for k, v in arrays.items()}
+                st = g.case.state_struct(arrays, 0.0)
+            for v in arrays.values():
+                v[...] = -1.0
+            fake.clear()
+            abi.check(g.lib.fesomc_gpu_sync_to_host(g.h, abi.F_ALL, C.byref(st)))
+            assert fake.lib.fake_pending() == 0
+            to = {o.dst for o in fake.ops() if o.kind == "h"}
+            for k, v in arrays.items():
+                assert np.array_equal(v, want[k]), k
+                assert (v.ctypes.data in to) == (k in fp64 and not pageable), k
+    finally:
+        g.close()
