@@ -409,51 +409,70 @@ std::vector<FieldRef> field_table(fesomc_model *m) {
 }
 
 // ---- state read-back ----------------------------------------------------------
-// The fields of a read-back go through page-locked staging slots of 1 MB:
-// the calling thread enqueues the device copies slot after slot, worker
-// threads wait for a slot's copy and move it to the caller's array (widening
-// FP32), so that the caller's page faults, the conversion and the transfer
-// overlap.  A read-back that fits the slots whole is enqueued at once and
-// waited for once, without workers: up to 4 MB in all, where starting
-// threads costs more than they save.  Against copying each field to pageable
+// A field whose array is page-locked is copied straight into it.  The others
+// go through page-locked staging slots of 1 MB: the calling thread enqueues
+// the device copies slot after slot, worker threads wait for a slot's copy and
+// move it to the caller's array (widening FP32), so that the caller's page
+// faults, the conversion and the transfer overlap.  Read-backs of up to 4 MB
+// fill and empty one slot in turn, without workers: starting threads costs
+// more than they save there.  Against copying each field to pageable
 // memory and waiting for it: 803 MB into fresh arrays 166 -> 35 ms (the page
 // faults of one thread were most of it), 148 MB of FP32 fields 37 -> 8.7 ms,
 // 90 MB 40 -> 8 ms, 10 MB 2.2 -> 1.4 ms, 1.2 MB in 25 fields 0.44 -> 0.18 ms.
-// The slots (16 MB) are shared by the process's models: made by the first
-// read-back, freed with the last model.  A read-back that finds them in use
-// by another thread takes the plain path.
+// Page-locking is slow (1 to 2.5 ms per 2 MB), so the slots are made as the
+// volume read so far justifies them: the first at once (2 us: it comes out of
+// what the runtime holds for a model's small buffers), then one for every 8
+// MB, and no more than one for every 2 MB of a read-back.  First read-back of
+// a process's only model with all 16 made at once, and so: 0.3 MB 8.8 -> 0.6 ms,
+// 1.4 MB 12 -> 0.7, 8.5 MB 17 -> 2.6 (2.6 field by field), 34 MB 13 -> 10 (10).
+// The slots are shared by the process's models and freed with the last of
+// them.  A read-back that finds them in use by another thread takes the plain
+// path.
 constexpr size_t kSlotBytes = 1 << 20;
 constexpr int kSlots = 16;
+constexpr size_t kSlotsAlone = 4 * kSlotBytes;   // read-backs that need no workers
+constexpr size_t kBytesPerSlot = 8 * kSlotBytes; // volume that justifies a slot more
 struct StagingPool {
     std::mutex in_use;                // held for the length of a read-back
-    std::mutex mu;                    // guards the two below
+    std::mutex mu;                    // guards the rest
     int users = 0;
-    unsigned char *buf = nullptr;
+    int n = 0;                        // slots made
+    size_t volume = 0;                // of the larger read-backs
+    unsigned char *slot[kSlots] = {};
 };
 StagingPool g_staging;
 
-// the pool's buffer (null: page-locked memory could not be had), and the
-// model's events, made on first use
-unsigned char *staging_for(fesomc_model *m) {
-    while ((int)m->stage_done.size() < kSlots) {
-        cudaEvent_t e;
-        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return nullptr;
-        m->stage_done.push_back(e);
-    }
+// the slots of a read-back of 'total' bytes (0: page-locked memory could not
+// be had), and the model's events for them
+int staging_for(fesomc_model *m, size_t total) {
     std::lock_guard<std::mutex> lk(g_staging.mu);
     if (!m->stage_ref) {
         g_staging.users += 1;
         m->stage_ref = true;
     }
-    if (!g_staging.buf) {
-        void *q = nullptr;
-        if (cudaMallocHost(&q, kSlots * kSlotBytes) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return nullptr;
-        }
-        g_staging.buf = static_cast<unsigned char *>(q);
+    size_t want = 1;
+    if (total > kSlotsAlone) {
+        g_staging.volume += total;
+        want = std::max<size_t>(1, std::min({(size_t)kSlots, g_staging.volume / kBytesPerSlot, total / (2 * kSlotBytes)}));
     }
-    return g_staging.buf;
+    while (g_staging.n < (int)want) {
+        void *q = nullptr;
+        if (cudaMallocHost(&q, kSlotBytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            break;
+        }
+        g_staging.slot[g_staging.n++] = static_cast<unsigned char *>(q);
+    }
+    const int ns = total <= kSlotsAlone ? std::min(g_staging.n, 1) : std::min<int>(g_staging.n, total / (2 * kSlotBytes));
+    while ((int)m->stage_done.size() < ns && ns > 1) {
+        cudaEvent_t e;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            (void)cudaGetLastError();
+            break;
+        }
+        m->stage_done.push_back(e);
+    }
+    return ns > 1 ? std::max(1, (int)std::min<size_t>(ns, m->stage_done.size())) : ns;
 }
 void staging_release(fesomc_model *m) {
     for (cudaEvent_t e : m->stage_done) cudaEventDestroy(e);
@@ -461,10 +480,10 @@ void staging_release(fesomc_model *m) {
     if (!m->stage_ref) return;
     std::lock_guard<std::mutex> lk(g_staging.mu);
     m->stage_ref = false;
-    if (--g_staging.users == 0 && g_staging.buf) {
-        cudaFreeHost(g_staging.buf);
-        g_staging.buf = nullptr;
-    }
+    if (--g_staging.users > 0) return;
+    for (int i = 0; i < g_staging.n; ++i) cudaFreeHost(g_staging.slot[i]);
+    g_staging.n = 0;
+    g_staging.volume = 0;
 }
 
 // one staged piece of a field: 'bytes' device bytes at slot memory 'src' to
@@ -501,25 +520,36 @@ struct FieldOut {
     FieldRef f;
     double *h;
 };
-// all fields, enqueued at once
-int fields_at_once(fesomc_model *m, const std::vector<FieldOut> &fields, unsigned char *buf) {
+// all fields through one slot, filled and emptied in turn
+int fields_in_rounds(fesomc_model *m, const std::vector<FieldOut> &fields) {
+    unsigned char *const buf = g_staging.slot[0];
     std::vector<StagedPiece> out;
     size_t off = 0;
+    auto empty = [&]() -> int {
+        CK(cudaStreamSynchronize(m->stream));
+        for (const StagedPiece &p : out) piece_out(p);
+        out.clear();
+        off = 0;
+        return FESOMC_OK;
+    };
     for (const FieldOut &o : fields) {
-        const size_t bytes = o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double));
+        const size_t value = o.f.f32 ? sizeof(float) : sizeof(double), bytes = o.f.count * value;
         const unsigned char *src;
-        const int rc = field_source(m, o.f, &src);
+        int rc = field_source(m, o.f, &src);
         if (rc) return rc;
-        CK(cudaMemcpyAsync(buf + off, src, bytes, cudaMemcpyDeviceToHost, m->stream));
-        out.push_back({buf + off, o.h, bytes, o.f.f32});
-        off += (bytes + 15) & ~(size_t)15;
+        for (size_t at = 0; at < bytes;) {
+            if (off == kSlotBytes && (rc = empty())) return rc;
+            const size_t n = std::min(kSlotBytes - off, bytes - at);
+            CK(cudaMemcpyAsync(buf + off, src + at, n, cudaMemcpyDeviceToHost, m->stream));
+            out.push_back({buf + off, o.h + at / value, n, o.f.f32});
+            at += n;
+            off += (n + 15) & ~(size_t)15;   // the slot's size is a multiple of 16
+        }
     }
-    CK(cudaStreamSynchronize(m->stream));
-    for (const StagedPiece &p : out) piece_out(p);
-    return FESOMC_OK;
+    return empty();
 }
-// all fields, slot after slot with worker threads
-int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, unsigned char *buf) {
+// all fields, slot after slot of the first ns with worker threads
+int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, int ns) {
     int dev = 0;
     CK(cudaGetDevice(&dev));
     std::mutex mu;
@@ -537,7 +567,7 @@ int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, unsign
                 std::unique_lock<std::mutex> lk(mu);
                 cv.wait(lk, [&] { return taken < queued || closed; });
                 if (taken == queued) return;
-                i = (int)(taken++ % kSlots);
+                i = (int)(taken++ % ns);
             }
             if (cudaEventSynchronize(m->stage_done[i]) != cudaSuccess) bad = 1;
             else piece_out(slot[i]);
@@ -548,8 +578,8 @@ int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, unsign
             cv.notify_all();
         }
     };
-    // half the host's threads, at most 8
-    const int want = (int)std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency() / 2));
+    // half the host's threads, at most 8, and no more than slots
+    const int want = std::min(ns, (int)std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency() / 2)));
     std::vector<std::thread> pool;
     try {
         for (int w = 0; w < want; ++w) pool.emplace_back(work);
@@ -564,13 +594,13 @@ int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, unsign
         if (r) return r;
         for (size_t at = 0; at < bytes; at += kSlotBytes) {
             const size_t n = std::min(kSlotBytes, bytes - at);
-            const int i = (int)(queued % kSlots);
+            const int i = (int)(queued % ns);
             {
                 std::unique_lock<std::mutex> lk(mu);
                 cv.wait(lk, [&] { return free_slot[i]; });
                 free_slot[i] = false;
             }
-            unsigned char *s = buf + (size_t)i * kSlotBytes;
+            unsigned char *s = g_staging.slot[i];
             CK(cudaMemcpyAsync(s, src + at, n, cudaMemcpyDeviceToHost, m->stream));
             CK(cudaEventRecord(m->stage_done[i], m->stream));
             {
@@ -593,10 +623,12 @@ int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, unsign
     return rc ? rc : (bad ? FESOMC_ECUDA : FESOMC_OK);
 }
 // all fields through the staging slots; g_staging.in_use is held
-int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields, unsigned char *buf) {
+int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields) {
     size_t total = 0;
-    for (const FieldOut &o : fields) total += (o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double)) + 15) & ~(size_t)15;
-    const int rc = total <= kSlots * kSlotBytes / 4 ? fields_at_once(m, fields, buf) : fields_by_slots(m, fields, buf);
+    for (const FieldOut &o : fields) total += o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double));
+    const int ns = staging_for(m, total);
+    if (ns < 1) return FESOMC_ENOMEM;
+    const int rc = ns == 1 ? fields_in_rounds(m, fields) : fields_by_slots(m, fields, ns);
     // after a failure too, no copy may still be on its way to the slots when
     // another model's read-back takes them
     if (rc) (void)cudaStreamSynchronize(m->stream);
@@ -1850,8 +1882,7 @@ int fesomc_gpu_sync_to_host(fesomc_model *m, uint32_t mask, fesomc_state *st) {
     rc = fields.empty() ? FESOMC_OK : FESOMC_ENOMEM;   // ENOMEM: the staging could not be had: field by field
     if (!fields.empty()) {
         std::unique_lock<std::mutex> lk(g_staging.in_use, std::try_to_lock);
-        unsigned char *buf = lk.owns_lock() ? staging_for(m) : nullptr;
-        if (buf) rc = fields_to_host_staged(m, fields, buf);
+        if (lk.owns_lock()) rc = fields_to_host_staged(m, fields);
     }
     if (rc == FESOMC_ENOMEM) {
         rc = FESOMC_OK;

@@ -164,3 +164,39 @@ def test_page_locked_arrays_receive_the_copy_directly(fake, fp32):
                 assert (v.ctypes.data in to) == (k in fp64 and not pageable), k
     finally:
         g.close()
+
+
+def test_staging_memory_grows_with_use_and_is_given_back(fake):
+    """The page-locked slots are made as read-backs justify them (1 MB for
+    small ones, more with the volume of larger ones, 16 MB at most), shared by
+    the process's models and freed with the last of them; the values are the
+    same at every stage."""
+    from fesomc import cases, model
+    MB = 1 << 20
+    base = fake.lib.fake_pinned_bytes()
+    events = fake.lib.fake_live_events()
+    a = _model()
+    held = fake.lib.fake_pinned_bytes()          # a model's own small buffers
+    try:
+        want = a.state()
+        assert fake.lib.fake_pinned_bytes() - held == MB
+        case = cases.estuary_case("e", 200, 100, 300.0, 11, 2.0, 25.0)
+        b = model.GpuModel(case)
+        held = fake.lib.fake_pinned_bytes() - MB
+        sizes = []
+        first = b.state()
+        device = sum(v.nbytes for k, v in first.items() if k != "_time_jd")
+        assert 32 * MB < device < 64 * MB
+        for _ in range(12):
+            sizes.append((fake.lib.fake_pinned_bytes() - held) // MB)
+            got = b.state()
+            for k, v in got.items():
+                assert np.array_equal(v, first[k]) and np.array_equal(v, case.state0[k] if k in case.state0 else v), k
+        assert sizes[0] < 8 and sizes == sorted(sizes) and sizes[-1] == 16
+        got = a.state()
+        assert all(np.array_equal(got[k], v) for k, v in want.items())
+        b.close()
+        assert fake.lib.fake_pinned_bytes() - base >= 16 * MB
+    finally:
+        a.close()
+    assert fake.lib.fake_pinned_bytes() == base and fake.lib.fake_live_events() == events
