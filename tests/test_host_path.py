@@ -200,3 +200,19 @@ def test_staging_memory_grows_with_use_and_is_given_back(fake):
     finally:
         a.close()
     assert fake.lib.fake_pinned_bytes() == base and fake.lib.fake_live_events() == events
+
+
+@pytest.mark.parametrize("fp32,nsigma,early", [(1, 40, True), (1, 41, False), (1, 127, False), (0, 63, False), (0, 127, False)])
+def test_column_kernel_with_large_local_arrays_is_not_started_early(fake, fp32, nsigma, early):
+    """d3_end with one thread per column and local arrays for more than 40
+    levels: started early its few blocks crowd the first SMs that have room,
+    and their arrays leave the cache."""
+    from fesomc import cases, model
+    g = model.GpuModel(cases.estuary_case("e", 20, 10, 300.0, nsigma, 2.0, 25.0, fp32_form=fp32))
+    try:
+        fake.clear()
+        g.step(2)
+        got = {o.early for o in fake.ops() if "k_d3endILi" in o.name}
+        assert got == {early}
+    finally:
+        g.close()
