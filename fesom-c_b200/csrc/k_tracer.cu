@@ -1334,17 +1334,18 @@ __global__ void __launch_bounds__(kAtm ? kVtAtmThreads : kVtThreads, FESOMC_FP32
         __syncthreads();
     }
 }
-// The same on tiles of 64 columns for 20 layers, fixed at compile time: one
-// thread per column solves with its recurrences in registers, from rows of
-// odd stride, and stages with batched loads.  Fewer shared-memory passes,
-// but only as many threads as columns, which pays on full-size grids.
-// FP32: at least 14 blocks (72 registers), 232 k nodes 0.070 -> 0.062 ms.
+// The same on tiles of 64 columns with the layer count LC fixed at compile
+// time (4 to 10, and 20): one thread per column solves with its recurrences in
+// registers, from rows of odd stride, and stages with batched loads.  Fewer
+// shared-memory passes, but only as many threads as columns, which pays on
+// full-size grids.  FP32, 20 layers: at least 14 blocks (72 registers), 232 k
+// nodes 0.070 -> 0.062 ms.
 constexpr int kVrCols = 64;
-constexpr int kVrLayers = 20;
-__global__ void __launch_bounds__(kVrCols, FESOMC_FP32 ? 14 : 1) k_vdiff_reg(Dev d) {
+template <int LC>
+__global__ void __launch_bounds__(kVrCols, FESOMC_FP32 && LC == 20 ? 14 : 1) k_vdiff_reg(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char vt_smem[];
-    constexpr int L = kVrLayers, LP = L | 1;
+    constexpr int L = LC, LP = L | 1;
     const int NS = d.NS, KP = (d.NS | 1), N = d.N;
     real *sT = reinterpret_cast<real *>(vt_smem);  // row j: node n0 + j
     real *sS = sT + kVrCols * LP;
@@ -1467,20 +1468,38 @@ static size_t vdiff_reg_smem(const Dev &d) {
 // nodes 0.034 ms against 0.035, 1.05 M 0.563 against 0.583, 232 k FP32 0.072
 // against 0.086; below, and with the sources, the level-parallel tiles: 16 k
 // nodes 0.019 against 0.029, with sources 40 k 0.073 against 0.114.
+// 4 to 10 layers, whose tiles are more barriers than chains, from four tiles
+// per SM on in FP64 and five in FP32 (ms, register tiles / level-parallel):
+// 10 layers 40 k nodes 0.0207 / 0.0229, 100 k 0.0351 / 0.0453, 1.0 M 0.213 /
+// 0.347, FP32 53 k 0.0181 / 0.0205 (40 k 0.0182 / 0.0167), 1.0 M 0.105 / 0.190;
+// 8 layers 1.0 M 0.158 / 0.318; 5 layers 1.0 M 0.132 / 0.244.
 static bool vdiff_reg(const Dev &d) {
-    return d.L == kVrLayers && !d.key_atm && d.N >= 4 * 148 * kVrCols;
+    if (d.key_atm) return false;
+    if (d.L == 20) return d.N >= 4 * 148 * kVrCols;
+    return d.L >= 4 && d.L <= 10 && d.N >= (FESOMC_FP32 ? 5 : 4) * 148 * kVrCols;
+}
+static void (*vdiff_reg_kernel(const Dev &d))(Dev) {
+    switch (d.L) {
+        case 4: return k_vdiff_reg<4>;
+        case 5: return k_vdiff_reg<5>;
+        case 6: return k_vdiff_reg<6>;
+        case 7: return k_vdiff_reg<7>;
+        case 8: return k_vdiff_reg<8>;
+        case 9: return k_vdiff_reg<9>;
+        case 10: return k_vdiff_reg<10>;
+        default: return k_vdiff_reg<20>;
+    }
 }
 int config_vdiff(const Dev &d) {
     const size_t sm = vdiff_smem(d);
     bool ok = d.key_atm ? raise_smem_limit(k_vdiff_tile<true>, sm) == cudaSuccess
                         : raise_smem_limit(k_vdiff_tile<false>, sm) == cudaSuccess;
-    if (vdiff_reg(d))
-        ok = ok && raise_smem_limit(k_vdiff_reg, vdiff_reg_smem(d)) == cudaSuccess;
+    if (vdiff_reg(d)) ok = ok && raise_smem_limit(vdiff_reg_kernel(d), vdiff_reg_smem(d)) == cudaSuccess;
     return ok ? 0 : 1;
 }
 void launch_vdiff(const Dev &d, cudaStream_t s) {
     const int C = vdiff_reg(d) ? kVrCols : kVtCols, tiles = (d.N + C - 1) / C;
-    if (vdiff_reg(d)) launch_k(k_vdiff_reg, tiles, kVrCols, vdiff_reg_smem(d), s, d);
+    if (vdiff_reg(d)) launch_k(vdiff_reg_kernel(d), tiles, kVrCols, vdiff_reg_smem(d), s, d);
     else if (d.key_atm) launch_k(k_vdiff_tile<true>, tiles, kVtAtmThreads, vdiff_smem(d), s, d);
     else launch_k(k_vdiff_tile<false>, tiles, kVtThreads, vdiff_smem(d), s, d);
 }

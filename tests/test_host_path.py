@@ -216,3 +216,25 @@ def test_column_kernel_with_large_local_arrays_is_not_started_early(fake, fp32, 
         assert got == {early}
     finally:
         g.close()
+
+
+def _launched(fake, nx, ny, nsigma, fp32, **kw):
+    """Names of the kernels of a step."""
+    from fesomc import cases, model
+    g = model.GpuModel(cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, fp32_form=fp32, **kw))
+    try:
+        fake.clear()
+        g.step(1)
+        return " ".join(o.name for o in fake.ops() if o.kind == "k")
+    finally:
+        g.close()
+
+
+# 160x100: 16,261 nodes; 280x150: 42,431; 310x160: 50,071
+@pytest.mark.parametrize("nx,ny,nsigma,fp32,reg", [(160, 100, 11, 0, False), (280, 150, 11, 0, True), (280, 150, 11, 1, False),
+                                                   (310, 160, 11, 1, True), (310, 160, 5, 1, True), (280, 150, 9, 0, True),
+                                                   (310, 160, 12, 0, False), (280, 150, 21, 1, True), (160, 100, 21, 0, False)])
+def test_vertical_diffusion_form(fake, nx, ny, nsigma, fp32, reg):
+    """Register tiles for few layers (and 20) on grids that fill the device."""
+    names = _launched(fake, nx, ny, nsigma, fp32)
+    assert ("k_vdiff_regILi%dE" % (nsigma - 1) in names) == reg and ("k_vdiff_tile" in names) != reg
