@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(256, FESOMC_FP32 ? 8 : 4) k_velrhs(Dev d, real
 
 // ---------------------------------------------------------------------------
 // implvisc: momentum_vert_impl_visc (fv_viscosity.F90:1266-1371), thread per
-// column; the fic variant is k_implvisc_fic_tile.
+// column; the fic variant is k_implvisc_fic_tile or k_implvisc_fic_reg.
 // ---------------------------------------------------------------------------
 template <int MAXL>
 __global__ void k_implvisc(Dev d) {
@@ -1172,6 +1172,141 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
         __syncthreads();
     }
 }
+// The fic variant on tiles of 64 element columns with the layer count LC fixed
+// at compile time (4 to 10): all threads stage U_rhs, V_rhs, Je and Av of the
+// block's consecutive elements with batched loads, one thread per column
+// solves with its recurrences in registers, from rows of odd stride.  The
+// arithmetic and its order are k_implvisc_fic_tile's.
+constexpr int kIrCols = 64;
+template <int LC>
+__global__ void __launch_bounds__(kIrCols) k_implvisc_fic_reg(Dev d) {
+    pdl_enter();
+    extern __shared__ __align__(16) unsigned char iv_smem[];
+    constexpr int L = LC, LP = LC | 1, NS = LC + 1, KP = NS | 1, C = kIrCols, kB = 4;
+    const int E = d.E;
+    real *sU = reinterpret_cast<real *>(iv_smem);   // row j: element e0 + j
+    real *sV = sU + C * LP, *sJ = sV + C * LP, *sA = sJ + C * LP;
+    const real dt = d.dt;
+    for (int e0 = blockIdx.x * C; e0 < E; e0 += gridDim.x * C) {
+        const int nt = E - e0 < C ? E - e0 : C;
+        for (int i0 = threadIdx.x; i0 < nt * NS; i0 += kB * C) {
+            real av[kB];
+#pragma unroll
+            for (int u = 0; u < kB; ++u) {
+                const int i = i0 + u * C;
+                av[u] = i < nt * NS ? d.Av[(size_t)e0 * NS + i] : real(0.0);
+            }
+#pragma unroll
+            for (int u = 0; u < kB; ++u) {
+                const int i = i0 + u * C, j = i / NS;
+                if (i < nt * NS) sA[j * KP + (i - j * NS)] = av[u];
+            }
+        }
+        for (int i0 = threadIdx.x; i0 < nt * L; i0 += kB * C) {
+            real ur[kB], vr[kB], jv[kB];
+#pragma unroll
+            for (int u = 0; u < kB; ++u) {
+                const int i = i0 + u * C;
+                const size_t g = (size_t)e0 * L + (i < nt * L ? i : 0);
+                ur[u] = d.U_rhs[g];
+                vr[u] = d.V_rhs[g];
+                jv[u] = d.Je[g];
+            }
+#pragma unroll
+            for (int u = 0; u < kB; ++u) {
+                const int i = i0 + u * C;
+                if (i >= nt * L) continue;
+                const int j = i / L, z = i - j * L;
+                sU[j * LP + z] = ur[u];
+                sV[j * LP + z] = vr[u];
+                sJ[j * LP + z] = jv[u];
+            }
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < nt) {
+            const int j = threadIdx.x, e = e0 + j;
+            real *U = sU + j * LP, *V = sV + j * LP;
+            const real *J = sJ + j * LP, *A = sA + j * KP;
+            const real mwd = d.mask_wd[e];
+            if (mwd != real(0.0)) {
+                const real ub = d.U_n[(size_t)e * L + L - 1], vb = d.V_n[(size_t)e * L + L - 1];
+                const real a_Cd = d.C_d * ((real(1.0) - d.elem_acc[e]) * d.Cd_bz + real(1.0));
+                real xx1[LC + 1], yu[LC + 1], yv[LC + 1];
+                real de = J[0] / (A[0] + A[1]);
+                const real rw = de / d.density_0;
+                real xv = real(1.0), yuv = d.taux[e] * rw, yvv = d.tauy[e] * rw;
+                xx1[0] = xv;
+                yu[0] = yuv;
+                yv[0] = yvv;
+#pragma unroll
+                for (int z = 0; z < L; ++z) {
+                    const real jz = J[z];
+                    const real d1 = (z == 0) ? real(0.5) * jz : real(0.5) * (jz + J[z > 0 ? z - 1 : 0]);
+                    const real d2 = (z == L - 1) ? real(0.5) * jz : real(0.5) * (jz + J[z + 1 < L ? z + 1 : z]);
+                    const real zt = dt / jz;
+                    const real a = zt * A[z] / d1;
+                    const real c = zt * A[z + 1] / d2;
+                    const real b = a + c + real(1.0);
+                    const real dd = b - a * xv;
+                    xv = c / dd;
+                    yuv = (a * yuv + U[z]) / dd;
+                    yvv = (a * yvv + V[z]) / dd;
+                    xx1[z + 1] = xv;
+                    yu[z + 1] = yuv;
+                    yv[z + 1] = yvv;
+                }
+                de = J[L - 1] / (A[NS - 1] + A[L - 1]);
+                const real friction = de * a_Cd * sqrt(ub * ub + vb * vb);
+                real Ut, Vt;
+                if (d.fic_point == 0) { Ut = real(0.0); Vt = real(0.0); }
+                else if (d.fic_point == 1) {
+                    const real a = friction + real(1.0) - xx1[L];
+                    Ut = yu[L] / a; Vt = yv[L] / a;
+                } else {
+                    const real a = real(1.0) / (real(1.0) - friction) - xx1[L];
+                    Ut = yu[L] / a; Vt = yv[L] / a;
+                }
+#pragma unroll
+                for (int z = L - 1; z >= 0; --z) {
+                    Ut = Ut * xx1[z + 1] + yu[z + 1];
+                    Vt = Vt * xx1[z + 1] + yv[z + 1];
+                    U[z] = Ut * mwd;
+                    V[z] = Vt * mwd;
+                }
+            } else {
+#pragma unroll
+                for (int z = 0; z < L; ++z) { U[z] = real(0.0); V[z] = real(0.0); }
+            }
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < nt * L; i += C) {
+            const int j = i / L, z = i - j * L;
+            const size_t g = (size_t)e0 * L + i;
+            d.U_rhs[g] = sU[j * LP + z];
+            d.V_rhs[g] = sV[j * LP + z];
+        }
+        __syncthreads();
+    }
+}
+static void (*implvisc_reg_kernel(const Dev &d))(Dev) {
+    switch (d.L) {
+        case 4: return k_implvisc_fic_reg<4>;
+        case 5: return k_implvisc_fic_reg<5>;
+        case 6: return k_implvisc_fic_reg<6>;
+        case 7: return k_implvisc_fic_reg<7>;
+        case 8: return k_implvisc_fic_reg<8>;
+        case 9: return k_implvisc_fic_reg<9>;
+        default: return k_implvisc_fic_reg<10>;
+    }
+}
+static size_t implvisc_reg_smem(const Dev &d) { return (size_t)kIrCols * (3 * (d.L | 1) + (d.NS | 1)) * sizeof(real); }
+// Few layers leave the level-parallel tiles little to share between their
+// barriers: the register tiles from five of them per SM on (elements; ms at
+// nodes, register / level-parallel tiles): 10 layers 40 k nodes 0.0183 /
+// 0.0198, 1.0 M 0.229 / 0.251, FP32 40 k 0.0126 / 0.0138, 100 k 0.0164 / 0.0228,
+// 1.0 M 0.095 / 0.127; 5 layers 1.0 M 0.101 / 0.176, FP32 0.054 / 0.088; 24 k
+// nodes 0.0166 / 0.0149.
+static bool implvisc_reg(const Dev &d) { return d.L >= 4 && d.L <= 10 && d.E >= 5 * 148 * kIrCols; }
 static size_t implvisc_tile_smem(const Dev &d) { return (size_t)4 * d.L * (kIvCols + 1) * sizeof(real); }
 
 // ---- launch wrappers --------------------------------------------------------
@@ -1245,7 +1380,9 @@ void launch_velrhs(const Dev &d, real ff, cudaStream_t s) {
     } while (0)
 void launch_implvisc(const Dev &d, cudaStream_t s) {
     if (d.im_vert_visc) MAXL_DISPATCH(k_implvisc, grid_for(d.E, 128), 128, s, d);
-    if (d.im_vert_visc_fic) launch_k(k_implvisc_fic_tile, (d.E + kIvCols - 1) / kIvCols, kIvThreads, implvisc_tile_smem(d), s, d);
+    if (!d.im_vert_visc_fic) return;
+    if (implvisc_reg(d)) launch_k(implvisc_reg_kernel(d), (d.E + kIrCols - 1) / kIrCols, kIrCols, implvisc_reg_smem(d), s, d);
+    else launch_k(k_implvisc_fic_tile, (d.E + kIvCols - 1) / kIvCols, kIvThreads, implvisc_tile_smem(d), s, d);
 }
 void launch_jac_swap(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ROT, 256);

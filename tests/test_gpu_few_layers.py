@@ -11,13 +11,13 @@ FIELDS = ("eta_n", "U_n_2D", "U_n", "V_n", "TF", "SF", "T_old", "S_old", "bt", "
 
 
 # 48,461 nodes, about 63 k elements: not a multiple of the tiles' 64 columns
-@pytest.mark.parametrize("nsigma", [5, 6, 7, 8, 9, 10, 11])
-def test_large_grid_bit_exact(built, nsigma):
+@pytest.mark.parametrize("nsigma,kw", [(n, {}) for n in range(5, 12)] + [(11, {"fic_point": 0}), (6, {"fic_point": 2})])
+def test_large_grid_bit_exact(built, nsigma, kw):
     import pyoracle
     from fesomc import abi, cases, model
 
     def case_of(lib):
-        return cases.estuary_case("e", 300, 160, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib)
+        return cases.estuary_case("e", 300, 160, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib, **kw)
 
     g = model.GpuModel(case_of(None))
     o = pyoracle.Oracle(case_of(pyoracle.MeshLib(abi)), abi, cases)

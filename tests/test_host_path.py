@@ -238,3 +238,12 @@ def test_vertical_diffusion_form(fake, nx, ny, nsigma, fp32, reg):
     """Register tiles for few layers (and 20) on grids that fill the device."""
     names = _launched(fake, nx, ny, nsigma, fp32)
     assert ("k_vdiff_regILi%dE" % (nsigma - 1) in names) == reg and ("k_vdiff_tile" in names) != reg
+
+
+# 160x100: about 21 k elements; 280x150: 55 k
+@pytest.mark.parametrize("nx,ny,nsigma,fp32,reg", [(160, 100, 11, 0, False), (280, 150, 11, 0, True), (280, 150, 11, 1, True),
+                                                   (280, 150, 5, 1, True), (280, 150, 12, 0, False), (280, 150, 21, 1, False)])
+def test_implicit_viscosity_form(fake, nx, ny, nsigma, fp32, reg):
+    """Register tiles for few layers on grids that fill the device."""
+    names = _launched(fake, nx, ny, nsigma, fp32)
+    assert ("k_implvisc_fic_regILi%dE" % (nsigma - 1) in names) == reg and ("k_implvisc_fic_tile" in names) != reg
