@@ -469,9 +469,16 @@ __global__ void k_av(Dev d) {
 // alone: the tiles were faster (232 k nodes 0.32 -> 0.20 ms), but their
 // contracted arithmetic rounds otherwise, and the elevation, held in FP64,
 // shows it (1.8e-6 relative after 78 steps).
+// Up to 11 interfaces on grids of more than eight tiles per SM the one thread
+// per column wins again: its arrays are short and the tiles' barriers come
+// every few divisions (ms, thread / tiles: 11 interfaces 1.0 M nodes 0.957 /
+// 1.164, 100 k 0.116 / 0.130, 40 k 0.059 / 0.062, 35 k 0.055 / 0.049; 6
+// interfaces 1.0 M 0.373 / 0.599, 35 k 0.0291 / 0.0290; 14 interfaces 1.0 M
+// 1.363 / 1.334).  Not for the listed columns, of which there are few.
 #if !FESOMC_FP32
-static bool d3end_tiled(const Dev &d) {
-    return d.tune[TK_D3END] != 1 && d3end_tile_smem(d, 16) <= 75 * 1024;
+static bool d3end_tiled(const Dev &d, bool list) {
+    if (d.tune[TK_D3END] == 1 || d3end_tile_smem(d, 16) > 75 * 1024) return false;
+    return list || d.tune[TK_D3END] != 0 || d.NS > 11 || d.N < 8 * 148 * 32;
 }
 // columns per tile: 32; 16 where 32 would not leave an SM two blocks, and on
 // meshes whose 16-column tiles are at most two per SM (twice the blocks for
@@ -480,6 +487,17 @@ static int d3end_cols(const Dev &d) {
     return d.N > 2 * 148 * 16 && d3end_tile_smem(d, 32) <= 113 * 1024 ? 32 : 16;
 }
 #endif
+// the knob's number for the form that the sizes choose
+int d3end_default(const Dev &d) {
+#if FESOMC_FP32
+    (void)d;
+    return 1;
+#else
+    Dev q = d;
+    q.tune[TK_D3END] = 0;
+    return d3end_tiled(q, false) ? 2 : 1;
+#endif
+}
 int config_d3end(const Dev &d) {
     if (d.NS > 127) return 1;
 #if FESOMC_FP32
@@ -498,7 +516,7 @@ int config_d3end(const Dev &d) {
 template <bool kList>
 static void launch_d3end_form(const Dev &d, const int *list, const unsigned long long *count, cudaStream_t s) {
 #if !FESOMC_FP32
-    if (d3end_tiled(d)) {
+    if (d3end_tiled(d, kList)) {
         const int C = d3end_cols(d), tiles = (d.N + C - 1) / C;
         if (C == 32) launch_k(k_d3end_tile<32, kList>, tiles, kT3Threads, d3end_tile_smem(d, 32), s, d, list, count);
         else launch_k(k_d3end_tile<16, kList>, tiles, kT3Threads, d3end_tile_smem(d, 16), s, d, list, count);

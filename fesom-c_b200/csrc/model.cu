@@ -46,6 +46,7 @@ namespace fesomc {
     void launch_implvisc(const Dev &, cudaStream_t); \
     void launch_jac_swap(const Dev &, cudaStream_t); \
     void launch_je(const Dev &, cudaStream_t); \
+    int d3end_default(const Dev &); \
     int config_d3end(const Dev &); \
     int config_vdiff(const Dev &); \
     int config_p1(const Dev &); \
@@ -2318,7 +2319,7 @@ namespace {
 struct KnobInfo {
     const char *name;      // the kernel (or kernel group) the knob shapes
     const char *records;   // the fesomc_gpu_profile records that time it
-    int def;               // default threads per block (0: column entities per block)
+    int def;               // default threads per block or form (0: by the mesh's sizes)
 };
 const KnobInfo kKnobs[fesomc::kTuneKnobs] = {
     {"velrhs", "velrhs", 256}, {"velgrad3d", "velgrad3d", 256}, {"adv3_edge", "adv3_edge", 256},
@@ -2329,7 +2330,7 @@ const KnobInfo kKnobs[fesomc::kTuneKnobs] = {
     {"muscl_egrad", "muscl_egrad", 256}, {"muscl_ngrad", "muscl_ngrad", 256}, {"muscl_edge", "muscl_edge", 256},
     {"muscl_h", "muscl_h", 128}, {"upwind_h", "upwind_h", 128}, {"av", "av", 256},
     {"columns", "pressure_col,bpg_elem,update3d,wvel", 0},
-    {"d3end_arrays", "d3end,d3end_list", 2},
+    {"d3end_arrays", "d3end,d3end_list", 0},
     {"vdiff_form", "vdiff_col", 3},
     {"implvisc_form", "implvisc", 2},
 };
@@ -2421,7 +2422,11 @@ int fesomc_gpu_tune_get(fesomc_model *m, int32_t *values, int32_t *limits) {
     for (int k = 0; k < fesomc::kTuneKnobs; ++k) {
         if (values) {
             const int v = m->d.tune[k];
-            values[k] = v > 0 ? v : (kKnobs[k].def > 0 ? kKnobs[k].def : default_columns(m->d.L));
+            const int def = k == fesomc::TK_COLUMNS ? default_columns(m->d.L)
+                            : k != fesomc::TK_D3END ? kKnobs[k].def
+                            : m->fp32               ? fesomc::f32::d3end_default(m->d32)
+                                                    : fesomc::f64::d3end_default(m->d);
+            values[k] = v > 0 ? v : def;
         }
         if (limits)
             limits[k] = form_knob(k) ? lim[k] : (lim[k] / 32) * 32;

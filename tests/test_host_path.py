@@ -247,3 +247,26 @@ def test_implicit_viscosity_form(fake, nx, ny, nsigma, fp32, reg):
     """Register tiles for few layers on grids that fill the device."""
     names = _launched(fake, nx, ny, nsigma, fp32)
     assert ("k_implvisc_fic_regILi%dE" % (nsigma - 1) in names) == reg and ("k_implvisc_fic_tile" in names) != reg
+
+
+@pytest.mark.parametrize("nx,ny,nsigma,fp32,tiles", [(160, 100, 11, 0, True), (280, 150, 11, 0, False), (280, 150, 5, 0, False),
+                                                     (280, 150, 12, 0, True), (280, 150, 11, 1, False), (160, 100, 21, 1, False)])
+def test_d3end_form(fake, nx, ny, nsigma, fp32, tiles):
+    """Tiles of columns, or one thread per column: FP32, and few levels on
+    grids that fill the device; the knob reports the form."""
+    from fesomc import autotune, cases, model
+    case = cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, fp32_form=fp32)
+    g = model.GpuModel(case)
+    try:
+        for form in (None, 1, 2):
+            if form:
+                autotune.apply(g, {"d3end_arrays": form})
+            else:
+                assert autotune.get(g)[0]["d3end_arrays"] == (2 if tiles else 1)
+            fake.clear()
+            g.step(1)
+            names = " ".join(o.name for o in fake.ops() if o.kind == "k")
+            want = tiles if form is None else form == 2 and not fp32
+            assert ("k_d3end_tileILi" in names) == want and ("k_d3endILi" in names) != want
+    finally:
+        g.close()
