@@ -972,7 +972,7 @@ __global__ void k_wvel(Dev d) {
 }
 
 // ---- momentum_vert_impl_visc_tmp on tiles of element columns --------------
-// (fv_viscosity.F90:1374-1486, no ice.)  A block takes kIvCols consecutive
+// (fv_viscosity.F90:1374-1486, no ice.)  A block takes kIvCols (32) consecutive
 // elements, whose columns are one contiguous range of U_rhs, V_rhs, Je and
 // Av.  All threads, one (element, layer) each: the staging, the coefficients a
 // and c with their three divisions, and at the end the masked result.  The
@@ -983,7 +983,7 @@ __global__ void k_wvel(Dev d) {
 // then by the solution.
 // Bound by latency: the chain of the elimination, whose FP64 divisions (114
 // cycles each) one thread runs one after the other.  So in FP64 four lanes per
-// column, all threads of the block, form the quotients of xx1, yu and yv at
+// column form the quotients of xx1, yu and yv at
 // the same time; FP32, whose divisions are short, takes one thread per column.
 // Staging (FP64): kIvBatch items per thread, the neighbour layers' Je and Av
 // again from L1 instead of staged, so that four arrays remain and more blocks
@@ -993,12 +993,18 @@ __global__ void k_wvel(Dev d) {
 // 0.43 ms, 232 k 0.185, 0.148 -> 0.107, 42 k 0.035, 0.040 -> 0.029, 40 k, 30
 // layers 0.049, 0.064 -> 0.043, 16 k, 10 layers 0.017, 0.016 -> 0.013, 4.5 k,
 // 39 layers 0.032, 0.025 -> 0.019.
-constexpr int kIvCols = 32;
-constexpr int kIvThreads = 128;
+// A column takes 32 B of shared memory per layer (FP64): where 32 of them
+// would leave an SM fewer than three blocks (73 layers on), a block takes 16,
+// and 256 threads, four times as many as its recurrences need, for the staging
+// and its divisions.  16 k nodes, 80 layers 0.091 -> 0.051 ms, 126 layers 0.222 ->
+// 0.097, 100 k nodes 0.429 -> 0.260 and 1.235 -> 0.562 (one thread per column:
+// 0.103, 0.142, 0.416, 0.710; 16 columns with 64 threads 0.354 and 0.849, with 128
+// 0.288 and 0.660).
 #if !FESOMC_FP32
 constexpr int kIvBatch = 3;
 #endif
 
+template <int kIvCols, int kIvThreads>
 __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char iv_smem[];
@@ -1015,7 +1021,7 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
     const bool mine = warp < kChains;
     const int lane = warp * 32 + (threadIdx.x & 31);   // column of a recurrence
 #else
-    static_assert(kIvThreads == 4 * kIvCols, "four lanes per column");
+    static_assert(kIvThreads >= 4 * kIvCols && kIvCols % 8 == 0, "four lanes per column, all of a warp");
 #endif
     for (int e0 = blockIdx.x * kIvCols; e0 < E; e0 += gridDim.x * kIvCols) {
         const int nt = E - e0 < kIvCols ? E - e0 : kIvCols;
@@ -1116,7 +1122,7 @@ __global__ void __launch_bounds__(kIvThreads) k_implvisc_fic_tile(Dev d) {
             }
         }
 #else
-        {
+        if (threadIdx.x < 4 * kIvCols) {
             // four lanes per column: xx1, yu and yv form their quotient each
             // at the same time and share xx1 (__shfl needs every lane: those
             // past the last column run along on column 0, the fourth lane on
@@ -1307,7 +1313,10 @@ static size_t implvisc_reg_smem(const Dev &d) { return (size_t)kIrCols * (3 * (d
 // 1.0 M 0.095 / 0.127; 5 layers 1.0 M 0.101 / 0.176, FP32 0.054 / 0.088; 24 k
 // nodes 0.0166 / 0.0149.
 static bool implvisc_reg(const Dev &d) { return d.L >= 4 && d.L <= 10 && d.E >= 5 * 148 * kIrCols; }
-static size_t implvisc_tile_smem(const Dev &d) { return (size_t)4 * d.L * (kIvCols + 1) * sizeof(real); }
+static size_t implvisc_tile_smem(const Dev &d, int cols) { return (size_t)4 * d.L * (cols + 1) * sizeof(real); }
+#if !FESOMC_FP32
+static bool implvisc_narrow(const Dev &d) { return implvisc_tile_smem(d, 32) > 75 * 1024; }
+#endif
 
 // ---- launch wrappers --------------------------------------------------------
 // Column blocks: B entities, B * L threads, about 160 of them (at most 16
@@ -1327,7 +1336,12 @@ static size_t wvel_smem(const Dev &d) {
     return (size_t)col_b(d) * (kWvEdges * sizeof(WvEdge) + ((d.L | 1) + 2) * sizeof(real));
 }
 int config_columns(const Dev &d) {
-    cudaError_t e = raise_smem_limit(k_implvisc_fic_tile, implvisc_tile_smem(d));
+    cudaError_t e = cudaSuccess;
+#if !FESOMC_FP32
+    if (implvisc_narrow(d)) e = raise_smem_limit(k_implvisc_fic_tile<16, 256>, implvisc_tile_smem(d, 16));
+    else
+#endif
+        e = raise_smem_limit(k_implvisc_fic_tile<32, 128>, implvisc_tile_smem(d, 32));
     if (e == cudaSuccess) e = raise_smem_limit(k_bpg_elem, bpg_smem(d));
     if (e == cudaSuccess) e = raise_smem_limit(k_update3d, update3d_smem(d));
     if (e == cudaSuccess) e = raise_smem_limit(k_pressure_col, pressure_smem(d));
@@ -1382,7 +1396,10 @@ void launch_implvisc(const Dev &d, cudaStream_t s) {
     if (d.im_vert_visc) MAXL_DISPATCH(k_implvisc, grid_for(d.E, 128), 128, s, d);
     if (!d.im_vert_visc_fic) return;
     if (implvisc_reg(d)) launch_k(implvisc_reg_kernel(d), (d.E + kIrCols - 1) / kIrCols, kIrCols, implvisc_reg_smem(d), s, d);
-    else launch_k(k_implvisc_fic_tile, (d.E + kIvCols - 1) / kIvCols, kIvThreads, implvisc_tile_smem(d), s, d);
+#if !FESOMC_FP32
+    else if (implvisc_narrow(d)) launch_k(k_implvisc_fic_tile<16, 256>, (d.E + 15) / 16, 256, implvisc_tile_smem(d, 16), s, d);
+#endif
+    else launch_k(k_implvisc_fic_tile<32, 128>, (d.E + 31) / 32, 128, implvisc_tile_smem(d, 32), s, d);
 }
 void launch_jac_swap(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ROT, 256);

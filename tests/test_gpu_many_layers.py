@@ -1,0 +1,31 @@
+"""Kernel forms of meshes with many layers against the oracle, bit for bit:
+the implicit viscosity's tiles of 32 and 16 columns on both sides of their
+choice (72 and 73 layers) with whole and ragged last tiles."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _compare(case_of, steps):
+    import pyoracle
+    from fesomc import abi, cases, model
+    g = model.GpuModel(case_of(None))
+    o = pyoracle.Oracle(case_of(pyoracle.MeshLib(abi)), abi, cases)
+    try:
+        g.step(steps)
+        o.step(steps)
+        sg, so = g.state(), o.state()
+        for f in ("eta_n", "U_n_2D", "U_n", "V_n", "U_n_filt", "TF", "SF", "bt", "snu", "Kv", "Ri", "tke_dissip", "Av", "Wvel",
+                  "rho_c", "hpressure", "Bar_pr_2D"):
+            assert np.array_equal(sg[f], so[f]), f
+    finally:
+        g.close()
+        o.close()
+
+
+@pytest.mark.parametrize("nx,ny,nsigma,kw", [(12, 11, 73, {}), (12, 11, 74, {}), (19, 13, 91, {"fic_point": 0}),
+                                             (21, 12, 102, {"fic_point": 2}), (33, 17, 127, {})])
+def test_implicit_viscosity_tiles(built, nx, ny, nsigma, kw):
+    from fesomc import cases
+    _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib, **kw), 3)

@@ -270,3 +270,9 @@ def test_d3end_form(fake, nx, ny, nsigma, fp32, tiles):
             assert ("k_d3end_tileILi" in names) == want and ("k_d3endILi" in names) != want
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("nsigma,fp32,cols", [(73, 0, 32), (74, 0, 16), (127, 0, 16), (127, 1, 32)])
+def test_implicit_viscosity_tile(fake, nsigma, fp32, cols):
+    """FP64 tiles of 16 columns where 32 would leave an SM fewer than three."""
+    assert "k_implvisc_fic_tileILi%dE" % cols in _launched(fake, 20, 10, nsigma, fp32)
