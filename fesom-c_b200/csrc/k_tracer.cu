@@ -35,7 +35,14 @@ __global__ void k_minmax_part(Dev d) {
     const long long n1 = d.member_node_off ? d.member_node_off[mb + 1] : d.N;
     const long long first = n0 * d.L, total = (n1 - n0) * d.L;
     real tmin = d.TF[first], tmax = d.TF[first], smin = d.SF[first], smax = d.SF[first];
+    // FP32: a 64-bit loop, whose loads the compiler has in flight together;
+    // with the 32-bit one 1.0 M nodes, 20 layers take 0.086 instead of 0.045 ms
+    // (FP64: 0.094 both ways)
+#if FESOMC_FP32
+    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < total; j += (long long)gridDim.x * blockDim.x) {
+#else
     GRID_LOOP(j, total) {
+#endif
         const long long i = first + j;
         const real t = d.TF[i], x = d.SF[i];
         tmin = dmin(tmin, t); tmax = dmax(tmax, t);
