@@ -1327,7 +1327,12 @@ static bool implvisc_narrow(const Dev &d) { return implvisc_tile_smem(d, 32) > 7
 static int col_b(const Dev &d) {
     return d.tune[TK_COLUMNS] > 0 ? d.tune[TK_COLUMNS] : default_columns(d.L);
 }
-static size_t pressure_smem(const Dev &d) { return (size_t)col_b(d) * (d.L | 1) * sizeof(real); }
+// pressure_col's level sums take one lane per column, and its blocks do little
+// else: four columns where the others take one or two.  100 k nodes, FP32: 54
+// layers 0.064 -> 0.054 ms, 100 layers 0.144 -> 0.103, 126 layers 0.161 -> 0.126,
+// FP64 0.100 -> 0.091, 0.222 -> 0.168, 0.251 -> 0.249.
+static int pressure_b(const Dev &d) { return d.tune[TK_COLUMNS] == 0 && d.L > 53 ? 4 : col_b(d); }
+static size_t pressure_smem(const Dev &d) { return (size_t)pressure_b(d) * (d.L | 1) * sizeof(real); }
 static size_t bpg_smem(const Dev &d) {
     return (size_t)col_b(d) * (kEsReals + 12 + 2 * d.L + 1) * sizeof(real);
 }
@@ -1350,7 +1355,7 @@ int config_columns(const Dev &d) {
 }
 // first: nothing but copies, fills or graphs before it on the stream
 void launch_pressure_col(const Dev &d, bool first, cudaStream_t s) {
-    launch_resident_as(!first, k_pressure_col, d.N, col_b(d), col_b(d) * d.L, pressure_smem(d), s, d);
+    launch_resident_as(!first, k_pressure_col, d.N, pressure_b(d), pressure_b(d) * d.L, pressure_smem(d), s, d);
 }
 void launch_bpg_elem(const Dev &d, cudaStream_t s) {
     launch_resident(k_bpg_elem, d.E, col_b(d), col_b(d) * d.L, bpg_smem(d), s, d);

@@ -1,6 +1,7 @@
 """Kernel forms of meshes with many layers against the oracle, bit for bit:
 the implicit viscosity's tiles of 32 and 16 columns on both sides of their
-choice (72 and 73 layers) with whole and ragged last tiles."""
+choice (72 and 73 layers) with whole and ragged last tiles, and the column
+kernels' entities per block, which change with the level count."""
 import numpy as np
 import pytest
 
@@ -29,3 +30,9 @@ def _compare(case_of, steps):
 def test_implicit_viscosity_tiles(built, nx, ny, nsigma, kw):
     from fesomc import cases
     _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib, **kw), 3)
+
+
+@pytest.mark.parametrize("nsigma", [54, 55, 84, 97, 101, 106, 108, 120, 121])
+def test_columns_per_block(built, nsigma):
+    from fesomc import cases
+    _compare(lambda lib: cases.estuary_case("e", 13, 11, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib), 3)

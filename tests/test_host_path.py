@@ -276,3 +276,21 @@ def test_d3end_form(fake, nx, ny, nsigma, fp32, tiles):
 def test_implicit_viscosity_tile(fake, nsigma, fp32, cols):
     """FP64 tiles of 16 columns where 32 would leave an SM fewer than three."""
     assert "k_implvisc_fic_tileILi%dE" % cols in _launched(fake, 20, 10, nsigma, fp32)
+
+
+@pytest.mark.parametrize("nsigma,columns,pressure,p1", [(21, 8, 8, 8), (54, 3, 3, 3), (55, 2, 4, 2), (81, 2, 4, 2), (84, 3, 4, 3),
+                                                        (97, 1, 4, 2), (106, 3, 4, 3), (108, 1, 4, 2), (120, 1, 4, 2),
+                                                        (121, 1, 4, 1), (127, 1, 4, 1)])
+def test_columns_per_block(fake, nsigma, columns, pressure, p1):
+    """Entities per block of the column kernels, by the level count."""
+    from fesomc import cases, model
+    g = model.GpuModel(cases.estuary_case("e", 20, 10, 300.0, nsigma, 2.0, 25.0))
+    try:
+        fake.clear()
+        g.step(1)
+        block = {o.name: o.block for o in fake.ops() if o.kind == "k"}
+        for k, b in (("k_pressure_col", pressure), ("k_bpg_elem", columns), ("k_update3d", columns), ("k_wvel", columns),
+                     ("k_p1_elem", p1)):
+            assert {v for n, v in block.items() if k in n} == {b * (nsigma - 1)}, k
+    finally:
+        g.close()
