@@ -133,8 +133,9 @@ __host__ __device__ __forceinline__ float4 make_real4(float x, float y, float z,
 // whose results do not depend on the block shape (one thread per entity or
 // per (entity, level), grid-stride, no block-level reduction), and entities
 // per block of the column kernels (pressure_col, bpg_elem, update3d, wvel),
-// and the form of d3_end (1 one thread per column, 2 to 6 tiles of columns
-// in shared memory), and the form of the tracers'
+// and the form of d3_end (1 one thread per column; FP64 2 to 6 tiles of columns
+// in shared memory; FP32 2 one thread per column with its arrays in shared
+// memory, 3 to 6 a set-up and a sweep kernel), and the form of the tracers'
 // implicit vertical diffusion (1 to 3, the same under every number: the sizes
 // decide), and the form of the implicit vertical viscosity (1 one thread per
 // element column reading the fields directly, 2 tiles of columns in shared

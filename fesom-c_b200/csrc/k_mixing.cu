@@ -24,6 +24,7 @@ __device__ __forceinline__ bool d3_above_tol(real a, real b) {
     return fabs(a / b) >= real(1.0e-6);
 }
 
+#if !FESOMC_FP32
 // x / d for d > 0: a zero x gives itself (the quotient's sign is x's).  The
 // division routine leaves its short path for a zero numerator; x is
 // replaced by 1 before the division instead.
@@ -31,6 +32,7 @@ __device__ __forceinline__ real div_pos(real x, real d) {
     const real q = (x == real(0.0) ? real(1.0) : x) / d;
     return x == real(0.0) ? x : q;
 }
+#endif
 
 // d3_end per node column (local-memory arrays indexed 1..NS like the Fortran
 // ones, ARR >= NS + 1 entries each).  The kernel is bound by the traffic of
@@ -447,6 +449,553 @@ __global__ void __launch_bounds__(kT3Threads, 4) k_d3end_tile(Dev d, const int *
 }
 #endif
 
+#if FESOMC_FP32
+// ---- further forms of d3_end in FP32 ------------------------------------------
+// Chosen by the launch-shape knob "d3end_arrays", for the meshes where the
+// search finds them faster than one thread per column (FP32 divisions are
+// short, so here the traffic of the local arrays counts for more); the same
+// bits as k_d3end.
+//
+// 2: the same closure with the column arrays in shared memory, laid out
+// [array][level][thread] so that a warp's access to one level is 32
+// consecutive words (697 nodes, 11 levels 0.0186 -> 0.0166 ms, 16 k nodes with
+// 127 levels 14.1 -> 8.8):
+//   sn        snu(nz), nz = 1..NS                 (constant over the iteration)
+//   bA, bB    btr / btr1 / xx1, nz = 1..NS        (alternating; the back
+//             substitution writes btr1(k) into the xx1(k) slot it has just
+//             read, xx1(2) = 1 and yy1(2) = y2 being constants)
+//   yy1       yy1(nz), nz = 3..NS
+//   pb, qb, c2  -b1-b2, t_inv*bt and c2, nz = 2..NS-1 (constant)
+// i.e. 7*NS - 8 values per column.  The same arithmetic as k_d3end, in the
+// same order.
+constexpr int kD3Block = 32;
+
+static int d3end_values(int NS) { return 7 * NS - 8; }
+
+__global__ void __launch_bounds__(kD3Block, 6) k_d3end_sm(Dev d) {
+    pdl_enter();
+    extern __shared__ __align__(16) unsigned char d3_smem[];
+    constexpr int B = kD3Block;
+    const int NS = d.NS, L = d.L;
+    real *const base = reinterpret_cast<real *>(d3_smem) + threadIdx.x;
+    // per-array views: element nz of an array at [(nz - first) * B]
+    real *const s_sn = base - 1 * B;                     // nz = 1..NS
+    real *const s_bA = base + (NS - 1) * B;              // nz = 1..NS
+    real *const s_bB = base + (2 * NS - 1) * B;          // nz = 1..NS
+    real *const s_yy = base + (3 * NS - 3) * B;          // nz = 3..NS
+    real *const s_pb = base + (4 * NS - 4) * B;          // nz = 2..NS-1
+    real *const s_qb = base + (5 * NS - 6) * B;          // nz = 2..NS-1
+    real *const s_c2 = base + (6 * NS - 8) * B;          // nz = 2..NS-1
+#define D3(a, nz) a[(size_t)(nz) * B]
+    const real t_inv = real(1.0) / d.dt;
+    const real cka = d.cka;
+    const real B1cka2 = real(16.6) * (cka * cka);
+    GRID_LOOP(ii, d.N) {
+        const int node = (int)ii;
+        const real *bt = d.bt + (size_t)node * NS;
+        const real *snu = d.snu + (size_t)node * NS;
+        const real *Kv = d.Kv + (size_t)node * NS;
+        const real *Un = d.Unode + (size_t)node * L;
+        const real *Vn = d.Vnode + (size_t)node * L;
+        const real *T = d.TF + (size_t)node * L;
+        const real *S = d.SF + (size_t)node * L;
+        real *Ri = d.Ri + (size_t)node * NS;
+        real *tke = d.tke_dissip + (size_t)node * NS;
+        const real dmean = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
+        const real dmean2 = dmean * dmean;
+        const real ajac = jac_a(d, d.eta_jac, node);
+        for (int nz = 1; nz <= NS; ++nz) {
+            D3(s_bA, nz) = bt[nz - 1];
+            D3(s_sn, nz) = snu[nz - 1];
+        }
+        Ri[0] = real(0.0);
+        Ri[NS - 1] = real(0.0);
+#pragma unroll 4
+        for (int nz = 2; nz <= NS - 1; ++nz) {
+            const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
+            const real d1 = s_m - s_0;
+            const real d2 = s_0 - s_p;
+            const real dd = real(0.5) * (d1 + d2);
+            real ap1 = Un[nz - 2] - Un[nz - 1];
+            const real ap2 = Vn[nz - 2] - Vn[nz - 1];
+            const real sn_m = snu[nz - 2], sn_0 = snu[nz - 1], sn_p = snu[nz];
+            real b1 = sn_0 * (ap1 * ap1 + ap2 * ap2) / (dd * dd);
+            b1 = b1 / dmean2;
+            const real zb = zbar_of(d, ajac, nz - 1);
+            const real rho_up = density_jm(T[nz - 2], S[nz - 2], -zb, d.density_0);
+            const real rho_dn = density_jm(T[nz - 1], S[nz - 1], -zb, d.density_0);
+            ap1 = (rho_up - rho_dn) / dd;
+            const real b2 = -real(0.5) * kG * Kv[nz - 1] * ap1 / (d.density_0 * dmean);
+            const real snu_p = real(0.5) * (sn_m + sn_0);
+            const real snu_m = real(0.5) * (sn_0 + sn_p);
+            const real cc = real(0.5) * real(0.73) * (snu_p * (bt[nz - 2] - bt[nz - 1]) / d1 - snu_m * (bt[nz - 1] - bt[nz]) / d2) / dd;
+            D3(s_c2, nz) = cc / dmean2;
+            if (b1 > real(0.0)) Ri[nz - 1] = -kG * ap1 / (d.density_0 * dmean) / b1 * sn_0;
+            else Ri[nz - 1] = real(10000.0);
+            D3(s_pb, nz) = -b1 - b2;
+            D3(s_qb, nz) = t_inv * bt[nz - 1];
+        }
+        real y2;
+        {
+            const real d1 = real(0.5) * (__ldg(d.sig + NS - 2) - __ldg(d.sig + NS - 1));
+            const real wx = d.windx[node], wy = d.windy[node];
+            const real u_din_sur = real(0.05) * (wx * wx + wy * wy);
+            const real snu_m = real(0.5) * (snu[NS - 1] + snu[NS - 2]);
+            y2 = (real(0.4e-3) * (u_din_sur * u_din_sur * u_din_sur) * dmean * d1) / (snu_m * real(0.76));
+        }
+        // bottom boundary value (independent of the iteration)
+        const real delta_b = jc_of(d, ajac, NS - 2) + d.z0b_min;
+        const real lg = fesomc_log(delta_b / d.z0b_min);
+        const real bott_R = B1cka2 / (lg * lg);
+        const real ubt = Un[L - 1], vbt = Vn[L - 1];
+        const real bot = bott_R * (ubt * ubt + vbt * vbt);
+        real *btr = s_bA, *xq = s_bB;   // xq: this iteration's xx1, then its btr1
+        bool converged = false;
+        int iters = 200;
+        for (int it = 1; it <= 200; ++it) {
+            real x = real(1.0), y = y2;
+            real s_lo = D3(s_sn, 1), s_mid = D3(s_sn, 2);
+            real b_n = D3(btr, 2), pb_n = D3(s_pb, 2), qb_n = D3(s_qb, 2), c2_n = D3(s_c2, 2), sh_n = D3(s_sn, 3);
+            for (int nz = 2; nz <= NS - 1; ++nz) {
+                const real s_hi = sh_n;
+                const real b = b_n, pbv = pb_n, qbv = qb_n, c2v = c2_n;
+                if (nz + 1 <= NS - 1) {
+                    b_n = D3(btr, nz + 1); pb_n = D3(s_pb, nz + 1); qb_n = D3(s_qb, nz + 1);
+                    c2_n = D3(s_c2, nz + 1); sh_n = D3(s_sn, nz + 2);
+                }
+                const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
+                const real dd1 = s_m - s_0;
+                const real dd2 = s_0 - s_p;
+                const real dd = real(0.5) * (dd1 + dd2);
+                const real c1 = real(0.046) * (b * b) / s_mid;
+                if (it == 200) tke[nz - 1] = c1;
+                const real fr = pbv - c1 - qbv - c2v;
+                const real snu_p = real(0.5) * (s_lo + s_mid);
+                const real snu_mm = real(0.5) * (s_mid + s_hi);
+                const real am = real(0.5) * (snu_p * real(0.73)) / (dmean2 * dd1 * dd);
+                const real cm = real(0.5) * (snu_mm * real(0.73)) / (dmean2 * dd2 * dd);
+                const real bm = am + cm + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
+                const real a = bm - am * x;
+                const real xn = cm / a;
+                const real yn = (am * y - fr) / a;
+                D3(xq, nz + 1) = xn;
+                D3(s_yy, nz + 1) = yn;
+                x = xn;
+                y = yn;
+                s_lo = s_mid;
+                s_mid = s_hi;
+            }
+            real b1v = bot;  // btr1(NS)
+            real x_n = D3(xq, NS), y_n = D3(s_yy, NS), o_n = D3(btr, NS - 1);
+            const real top = D3(btr, NS);
+            D3(xq, NS) = b1v;
+            bool above = d3_above_tol(top - b1v, dmax(b1v, top) + real(1.0e-8));
+            for (int nz = NS; nz >= 2; --nz) {
+                const real xv = x_n, yv = y_n, ov = o_n;
+                if (nz - 1 >= 3) { x_n = D3(xq, nz - 1); y_n = D3(s_yy, nz - 1); o_n = D3(btr, nz - 2); }
+                else if (nz - 1 == 2) { x_n = real(1.0); y_n = y2; o_n = D3(btr, nz - 2); }
+                b1v = b1v * xv + yv;  // btr1(nz-1), into the xx1(nz-1) slot already read
+                D3(xq, nz - 1) = b1v;
+                above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
+            }
+            if (!above) { converged = true; iters = it; break; }
+            real *t = btr;
+            btr = xq;
+            xq = t;
+        }
+        if (d.d3_iters) d.d3_iters[node] = iters;   // measurement only (fesomc_gpu_d3end_iterations)
+        if (converged) {
+            for (int nz = 2; nz <= NS - 1; ++nz) {
+                const real b = D3(btr, nz);
+                tke[nz - 1] = real(0.046) * (b * b) / D3(s_sn, nz);
+            }
+        } else {
+            atomicAdd(d.notconv, 1);
+        }
+        real *btw = d.bt + (size_t)node * NS;
+        real *snw = d.snu + (size_t)node * NS;
+        real *Kvw = d.Kv + (size_t)node * NS;
+#pragma unroll 4
+        for (int nz = 1; nz <= NS; ++nz) {
+            const real btn = dmax(D3(btr, nz), real(1.0e-8));
+            btw[nz - 1] = btn;
+            const real zt = __ldg(d.sig + nz - 1) * dmean;
+            const real Zh = zt + d.z0b_min;
+            const real Zd = fabs(dmean - zt) + d.z0s_min;
+            const real Z0 = real(1.0) - d.beta_scale * Zh * Zd / (dmean * dmean);
+            const real scale_t = cka * Zh * Zd * Z0 / dmean;
+            real s = scale_t * sqrt(btn) + d.snul;
+            if (s >= real(0.2)) s = real(0.2);
+            snw[nz - 1] = s;
+            Kvw[nz - 1] = d.Pr_num * s;
+        }
+    }
+#undef D3
+}
+
+// 3 to 6: d3_end in two kernels, up to 40 levels.  The set-up of a column (its per-interface constants: two
+// densityJM per interface and the divisions of b1, b2, c2, Ri) does not depend on the sweep, and its interfaces are independent.  The
+// set-up kernel takes blocks of kD3Tile consecutive nodes, stages their
+// columns in shared memory with coalesced loads, forms the constants with
+// one thread per (node, interface) exactly as k_d3end's first loop does, and
+// writes -b1-b2, t_inv*bt, c2 and snu level-major ([interface][node]: a warp
+// of 32 consecutive nodes reads contiguous bytes of one interface) and Ri in
+// the column layout.  The sweep kernels keep only xx1, yy1 and the btr pair per
+// column and read the constants level-major.
+constexpr int kD3Tile = 32;
+constexpr int kD3SetupThreads = 256;
+
+__global__ void __launch_bounds__(kD3SetupThreads) k_d3end_setup(Dev d) {
+    pdl_enter();
+    extern __shared__ __align__(16) unsigned char d3s_smem[];
+    const int NS = d.NS, L = d.L, N = d.N;
+    real *sm = reinterpret_cast<real *>(d3s_smem);
+    // per node j of the tile, stride NS: U, V, T, S (L levels), bt, snu, Kv, Ri (NS)
+    real *sU = sm, *sV = sm + 1 * kD3Tile * NS, *sT = sm + 2 * kD3Tile * NS, *sS = sm + 3 * kD3Tile * NS;
+    real *sB = sm + 4 * kD3Tile * NS, *sN = sm + 5 * kD3Tile * NS, *sK = sm + 6 * kD3Tile * NS;
+    real *sR = sm + 7 * kD3Tile * NS;
+    real *sDm = sm + 8 * kD3Tile * NS, *sAj = sDm + kD3Tile;
+    const real t_inv = real(1.0) / d.dt;
+    for (long long n0 = (long long)blockIdx.x * kD3Tile; n0 < N; n0 += (long long)gridDim.x * kD3Tile) {
+        const int nt = (int)(N - n0 < kD3Tile ? N - n0 : kD3Tile);
+        for (int i = threadIdx.x; i < nt * L; i += blockDim.x) {
+            const int j = d.by_L.div(i), k = i - j * L;
+            const size_t g = (size_t)n0 * L + i;
+            sU[j * NS + k] = d.Unode[g];
+            sV[j * NS + k] = d.Vnode[g];
+            sT[j * NS + k] = d.TF[g];
+            sS[j * NS + k] = d.SF[g];
+        }
+        for (int i = threadIdx.x; i < nt * NS; i += blockDim.x) {
+            const size_t g = (size_t)n0 * NS + i;
+            sB[i] = d.bt[g];
+            sN[i] = d.snu[g];
+            sK[i] = d.Kv[g];
+        }
+        if ((int)threadIdx.x < nt) {
+            const int node = (int)n0 + threadIdx.x;
+            sDm[threadIdx.x] = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
+            sAj[threadIdx.x] = jac_a(d, d.eta_jac, node);
+        }
+        __syncthreads();
+        // snu level-major, and Ri(1) = Ri(NS) = 0
+        for (int i = threadIdx.x; i < kD3Tile * NS; i += blockDim.x) {
+            const int j = i % kD3Tile, k = i / kD3Tile;   // node fastest
+            if (j < nt) d.d3_sn[(size_t)k * N + n0 + j] = sN[j * NS + k];
+        }
+        for (int j = threadIdx.x; j < nt; j += blockDim.x) {
+            sR[j * NS] = real(0.0);
+            sR[j * NS + NS - 1] = real(0.0);
+        }
+        // the interfaces nz = 2..NS-1, node fastest (k_d3end's first loop)
+        for (int i = threadIdx.x; i < kD3Tile * (NS - 2); i += blockDim.x) {
+            const int j = i % kD3Tile, nz = 2 + i / kD3Tile;
+            if (j >= nt) continue;
+            const real *Un = sU + j * NS, *Vn = sV + j * NS, *T = sT + j * NS, *S = sS + j * NS;
+            const real *bt = sB + j * NS, *Kv = sK + j * NS, *snc = sN + j * NS;
+            const real dmean = sDm[j], dmean2 = dmean * dmean, ajac = sAj[j];
+            const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
+            const real d1 = s_m - s_0;
+            const real d2 = s_0 - s_p;
+            const real dd = real(0.5) * (d1 + d2);
+            real ap1 = Un[nz - 2] - Un[nz - 1];
+            const real ap2 = Vn[nz - 2] - Vn[nz - 1];
+            const real sn_m = snc[nz - 2], sn_0 = snc[nz - 1], sn_p = snc[nz];
+            real b1 = sn_0 * (ap1 * ap1 + ap2 * ap2) / (dd * dd);
+            b1 = b1 / dmean2;
+            const real zb = zbar_of(d, ajac, nz - 1);
+            const real rho_up = density_jm(T[nz - 2], S[nz - 2], -zb, d.density_0);
+            const real rho_dn = density_jm(T[nz - 1], S[nz - 1], -zb, d.density_0);
+            ap1 = (rho_up - rho_dn) / dd;
+            const real b2 = -real(0.5) * kG * Kv[nz - 1] * ap1 / (d.density_0 * dmean);
+            const real snu_p = real(0.5) * (sn_m + sn_0);
+            const real snu_m = real(0.5) * (sn_0 + sn_p);
+            const real cc = real(0.5) * real(0.73) * (snu_p * (bt[nz - 2] - bt[nz - 1]) / d1 - snu_m * (bt[nz - 1] - bt[nz]) / d2) / dd;
+            const size_t o = (size_t)(nz - 2) * N + n0 + j;
+            d.d3_c2[o] = cc / dmean2;
+            if (b1 > real(0.0)) sR[j * NS + nz - 1] = -kG * ap1 / (d.density_0 * dmean) / b1 * sn_0;
+            else sR[j * NS + nz - 1] = real(10000.0);
+            d.d3_pb[o] = -b1 - b2;
+            d.d3_qb[o] = t_inv * bt[nz - 1];
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < nt * NS; i += blockDim.x) d.Ri[(size_t)n0 * NS + i] = sR[i];
+        __syncthreads();
+    }
+}
+
+// The sweeps with xx1, yy1 and the btr pair in shared memory, [array][level]
+// [thread] (3, 4, and 5, 6 for other level counts than 21): no local memory at
+// all, 4*NS - 2 values per column, blocks of kD3Block columns.  100 k nodes, 31
+// levels 0.255 -> 0.192 ms (one thread per column -> this), 40 levels 0.388 ->
+// 0.318.
+__global__ void __launch_bounds__(kD3Block) k_d3end_sweep_sm(Dev d) {
+    pdl_enter();
+    extern __shared__ __align__(16) unsigned char d3w_smem[];
+    constexpr int B = kD3Block;
+    const real t_inv = real(1.0) / d.dt;
+    const real cka = d.cka;
+    const real B1cka2 = real(16.6) * (cka * cka);
+    const size_t N = d.N;
+    const int NS = d.NS, L = d.L;
+    real *const base = reinterpret_cast<real *>(d3w_smem) + threadIdx.x;
+    // element nz of an array at [(nz - first) * B]
+    real *const s_x = base - 2 * B;                      // xx1, nz = 2..NS
+    real *const s_y = base + (NS - 1 - 2) * B;           // yy1, nz = 2..NS
+    real *const s_bA = base + (2 * NS - 2 - 1) * B;      // nz = 1..NS
+    real *const s_bB = base + (3 * NS - 2 - 1) * B;      // nz = 1..NS
+#define W3(a, nz) a[(size_t)(nz) * B]
+    GRID_LOOP(ii, d.N) {
+        const int node = (int)ii;
+        const real *bt = d.bt + (size_t)node * NS;
+        const real *Un = d.Unode + (size_t)node * L;
+        const real *Vn = d.Vnode + (size_t)node * L;
+        real *tke = d.tke_dissip + (size_t)node * NS;
+        // constants of interface nz (2..NS-1) and snu(nz) (1..NS), level-major
+        auto PB = [&](int nz) { return d.d3_pb[(size_t)(nz - 2) * N + node]; };
+        auto QB = [&](int nz) { return d.d3_qb[(size_t)(nz - 2) * N + node]; };
+        auto C2 = [&](int nz) { return d.d3_c2[(size_t)(nz - 2) * N + node]; };
+        auto SN = [&](int nz) { return d.d3_sn[(size_t)(nz - 1) * N + node]; };
+        const real dmean = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
+        const real dmean2 = dmean * dmean;
+        const real ajac = jac_a(d, d.eta_jac, node);
+        for (int nz = 1; nz <= NS; ++nz) W3(s_bA, nz) = bt[nz - 1];
+        real y2;
+        {
+            const real d1 = real(0.5) * (__ldg(d.sig + NS - 2) - __ldg(d.sig + NS - 1));
+            const real wx = d.windx[node], wy = d.windy[node];
+            const real u_din_sur = real(0.05) * (wx * wx + wy * wy);
+            const real snu_m = real(0.5) * (SN(NS) + SN(NS - 1));
+            y2 = (real(0.4e-3) * (u_din_sur * u_din_sur * u_din_sur) * dmean * d1) / (snu_m * real(0.76));
+        }
+        W3(s_x, 2) = real(1.0);
+        W3(s_y, 2) = y2;
+        const real delta_b = jc_of(d, ajac, NS - 2) + d.z0b_min;
+        const real lg = fesomc_log(delta_b / d.z0b_min);
+        const real bott_R = B1cka2 / (lg * lg);
+        const real ubt = Un[L - 1], vbt = Vn[L - 1];
+        const real bot = bott_R * (ubt * ubt + vbt * vbt);
+        real *btr = s_bA, *btr1 = s_bB;
+        bool converged = false;
+        int iters = 200;
+        for (int it = 1; it <= 200; ++it) {
+            real x = real(1.0), y = y2;
+            real s_lo = SN(1), s_mid = SN(2);
+            real b_n = W3(btr, 2), pb_n = PB(2), qb_n = QB(2), c2_n = C2(2), sh_n = SN(3);
+            for (int nz = 2; nz <= NS - 1; ++nz) {
+                const real s_hi = sh_n;
+                const real b = b_n, pbv = pb_n, qbv = qb_n, c2v = c2_n;
+                if (nz + 1 <= NS - 1) {
+                    b_n = W3(btr, nz + 1); pb_n = PB(nz + 1); qb_n = QB(nz + 1); c2_n = C2(nz + 1); sh_n = SN(nz + 2);
+                }
+                const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
+                const real dd1 = s_m - s_0;
+                const real dd2 = s_0 - s_p;
+                const real dd = real(0.5) * (dd1 + dd2);
+                const real c1 = real(0.046) * (b * b) / s_mid;
+                if (it == 200) tke[nz - 1] = c1;
+                const real fr = pbv - c1 - qbv - c2v;
+                const real snu_p = real(0.5) * (s_lo + s_mid);
+                const real snu_mm = real(0.5) * (s_mid + s_hi);
+                const real am = real(0.5) * (snu_p * real(0.73)) / (dmean2 * dd1 * dd);
+                const real cm = real(0.5) * (snu_mm * real(0.73)) / (dmean2 * dd2 * dd);
+                const real bm = am + cm + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
+                const real a = bm - am * x;
+                const real xn = cm / a;
+                const real yn = (am * y - fr) / a;
+                W3(s_x, nz + 1) = xn;
+                W3(s_y, nz + 1) = yn;
+                x = xn;
+                y = yn;
+                s_lo = s_mid;
+                s_mid = s_hi;
+            }
+            real b1v = bot;  // btr1(NS)
+            const real top = W3(btr, NS);
+            W3(btr1, NS) = b1v;
+            bool above = d3_above_tol(top - b1v, dmax(b1v, top) + real(1.0e-8));
+            real x_n = W3(s_x, NS), y_n = W3(s_y, NS), o_n = W3(btr, NS - 1);
+            for (int nz = NS; nz >= 2; --nz) {
+                const real xv = x_n, yv = y_n, ov = o_n;
+                if (nz - 1 >= 2) { x_n = W3(s_x, nz - 1); y_n = W3(s_y, nz - 1); o_n = W3(btr, nz - 2); }
+                b1v = b1v * xv + yv;  // btr1(nz-1)
+                W3(btr1, nz - 1) = b1v;
+                above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
+            }
+            if (!above) { converged = true; iters = it; break; }
+            real *t = btr;
+            btr = btr1;
+            btr1 = t;
+        }
+        if (d.d3_iters) d.d3_iters[node] = iters;   // measurement only (fesomc_gpu_d3end_iterations)
+        if (converged) {
+            for (int nz = 2; nz <= NS - 1; ++nz) {
+                const real b = W3(btr, nz);
+                tke[nz - 1] = real(0.046) * (b * b) / SN(nz);
+            }
+        } else {
+            atomicAdd(d.notconv, 1);
+        }
+        real *btw = d.bt + (size_t)node * NS;
+        real *snw = d.snu + (size_t)node * NS;
+        real *Kvw = d.Kv + (size_t)node * NS;
+        for (int nz = 1; nz <= NS; ++nz) {
+            const real btn = dmax(W3(btr, nz), real(1.0e-8));
+            btw[nz - 1] = btn;
+            const real zt = __ldg(d.sig + nz - 1) * dmean;
+            const real Zh = zt + d.z0b_min;
+            const real Zd = fabs(dmean - zt) + d.z0s_min;
+            const real Z0 = real(1.0) - d.beta_scale * Zh * Zd / (dmean * dmean);
+            const real scale_t = cka * Zh * Zd * Z0 / dmean;
+            real s = scale_t * sqrt(btn) + d.snul;
+            if (s >= real(0.2)) s = real(0.2);
+            snw[nz - 1] = s;
+            Kvw[nz - 1] = d.Pr_num * s;
+        }
+    }
+#undef W3
+}
+
+
+// The sweeps in registers (5 and 6, 21 levels: 6 or 8 resident blocks of 64
+// columns per SM): 1.0 M nodes 1.06 -> 0.93 and 0.90 ms, 100 k 0.125 -> 0.108 and
+// 0.106.  For a level count fixed at compile time (NSC) every loop over the levels
+// unrolls, so the column arrays live in registers and the sweep touches no
+// local memory.  Three arrays instead of four: the back substitution writes
+// btr1(m) into the slot of xx1(m + 1) it has just read (xx1(2) = 1 is a
+// constant), so with btr(m) = P[m] the sweep leaves btr1(m) in Q[m + 1],
+// copied back into P when the column has not converged.  yy1 keeps its own
+// array (yy1(2) = y2 a constant).  The arithmetic is k_d3end's, in the same
+// order; the constants are read level-major through the
+// read-only path.
+template <int NSC>
+__device__ __forceinline__ bool d3_sweep_reg(const Dev &d, size_t N, int node, const real (&P)[NSC + 2],
+                                             real (&Q)[NSC + 2], real (&Y)[NSC + 2], real y2, real bot, real dmean2,
+                                             real t_inv, bool last, real *tke) {
+    const real *pb = d.d3_pb + node, *qb = d.d3_qb + node, *c2 = d.d3_c2 + node, *sn = d.d3_sn + node;
+    real x = real(1.0), y = y2;
+    real s_lo = __ldg(sn), s_mid = __ldg(sn + N);
+#pragma unroll
+    for (int nz = 2; nz <= NSC - 1; ++nz) {
+        const real s_hi = __ldg(sn + (size_t)nz * N);
+        const real b = P[nz];
+        const real pbv = __ldg(pb + (size_t)(nz - 2) * N), qbv = __ldg(qb + (size_t)(nz - 2) * N);
+        const real c2v = __ldg(c2 + (size_t)(nz - 2) * N);
+        const real s_m = __ldg(d.sig + nz - 2), s_0 = __ldg(d.sig + nz - 1), s_p = __ldg(d.sig + nz);
+        const real dd1 = s_m - s_0;
+        const real dd2 = s_0 - s_p;
+        const real dd = real(0.5) * (dd1 + dd2);
+        const real c1 = real(0.046) * (b * b) / s_mid;
+        if (last) tke[nz - 1] = c1;
+        const real fr = pbv - c1 - qbv - c2v;
+        const real snu_p = real(0.5) * (s_lo + s_mid);
+        const real snu_mm = real(0.5) * (s_mid + s_hi);
+        const real am = real(0.5) * (snu_p * real(0.73)) / (dmean2 * dd1 * dd);
+        const real cm = real(0.5) * (snu_mm * real(0.73)) / (dmean2 * dd2 * dd);
+        const real bm = am + cm + (real(2.0) * real(0.046) * b) / s_mid + t_inv;
+        const real a = bm - am * x;
+        const real xn = cm / a;
+        const real yn = (am * y - fr) / a;
+        Q[nz + 1] = xn;
+        Y[nz + 1] = yn;
+        x = xn;
+        y = yn;
+        s_lo = s_mid;
+        s_mid = s_hi;
+    }
+    real b1v = bot;  // btr1(NS)
+    bool above = d3_above_tol(P[NSC] - b1v, dmax(b1v, P[NSC]) + real(1.0e-8));
+    Q[NSC + 1] = b1v;
+#pragma unroll
+    for (int nz = NSC; nz >= 2; --nz) {
+        const real xv = nz == 2 ? real(1.0) : Q[nz];
+        const real yv = nz == 2 ? y2 : Y[nz];
+        const real ov = P[nz - 1];
+        b1v = b1v * xv + yv;  // btr1(nz-1)
+        Q[nz] = b1v;
+        above |= d3_above_tol(ov - b1v, dmax(b1v, ov) + real(1.0e-8));
+    }
+    return above;
+}
+
+template <int NSC, int MINB>
+__global__ void __launch_bounds__(64, MINB) k_d3end_sweep_reg(Dev d) {
+    pdl_enter();
+    const real t_inv = real(1.0) / d.dt;
+    const real cka = d.cka;
+    const real B1cka2 = real(16.6) * (cka * cka);
+    const size_t N = d.N;
+    constexpr int NS = NSC;
+    const int L = d.L;
+    // 64-bit: with the 32-bit loop the 8-block variant spills more (1.0 M nodes
+    // 0.896 -> 0.962 ms)
+    for (long long ii = (long long)blockIdx.x * blockDim.x + threadIdx.x; ii < (long long)d.N; ii += (long long)gridDim.x * blockDim.x) {
+        const int node = (int)ii;
+        const real *bt = d.bt + (size_t)node * NS;
+        const real *Un = d.Unode + (size_t)node * L;
+        const real *Vn = d.Vnode + (size_t)node * L;
+        real *tke = d.tke_dissip + (size_t)node * NS;
+        auto SN = [&](int nz) { return __ldg(d.d3_sn + (size_t)(nz - 1) * N + node); };
+        real A[NSC + 2], B[NSC + 2], Y[NSC + 2];
+        const real dmean = dmax<real>(d.Dmin, d.depth[node] + d.eta_n[node]);
+        const real dmean2 = dmean * dmean;
+        const real ajac = jac_a(d, d.eta_jac, node);
+#pragma unroll
+        for (int nz = 1; nz <= NS; ++nz) A[nz] = bt[nz - 1];
+        real y2;
+        {
+            const real d1 = real(0.5) * (__ldg(d.sig + NS - 2) - __ldg(d.sig + NS - 1));
+            const real wx = d.windx[node], wy = d.windy[node];
+            const real u_din_sur = real(0.05) * (wx * wx + wy * wy);
+            const real snu_m = real(0.5) * (SN(NS) + SN(NS - 1));
+            y2 = (real(0.4e-3) * (u_din_sur * u_din_sur * u_din_sur) * dmean * d1) / (snu_m * real(0.76));
+        }
+        const real delta_b = jc_of(d, ajac, NS - 2) + d.z0b_min;
+        const real lg = fesomc_log(delta_b / d.z0b_min);
+        const real bott_R = B1cka2 / (lg * lg);
+        const real ubt = Un[L - 1], vbt = Vn[L - 1];
+        const real bot = bott_R * (ubt * ubt + vbt * vbt);
+        // A ends as the final btr: the previous iterate when a sweep
+        // converges, the last sweep's result after 200 without convergence
+        bool converged = false;
+        int iters = 200;
+        for (int it = 1; it <= 200; ++it) {
+            if (!d3_sweep_reg<NSC>(d, N, node, A, B, Y, y2, bot, dmean2, t_inv, it == 200, tke)) {
+                converged = true;
+                iters = it;
+                break;
+            }
+#pragma unroll
+            for (int m = 1; m <= NS; ++m) A[m] = B[m + 1];
+        }
+        if (d.d3_iters) d.d3_iters[node] = iters;   // measurement only (fesomc_gpu_d3end_iterations)
+        if (converged) {
+#pragma unroll
+            for (int nz = 2; nz <= NS - 1; ++nz) tke[nz - 1] = real(0.046) * (A[nz] * A[nz]) / SN(nz);
+        } else {
+            atomicAdd(d.notconv, 1);
+        }
+        real *btw = d.bt + (size_t)node * NS;
+        real *snw = d.snu + (size_t)node * NS;
+        real *Kvw = d.Kv + (size_t)node * NS;
+#pragma unroll
+        for (int nz = 1; nz <= NS; ++nz) {
+            const real btn = dmax(A[nz], real(1.0e-8));
+            btw[nz - 1] = btn;
+            const real zt = __ldg(d.sig + nz - 1) * dmean;
+            const real Zh = zt + d.z0b_min;
+            const real Zd = fabs(dmean - zt) + d.z0s_min;
+            const real Z0 = real(1.0) - d.beta_scale * Zh * Zd / (dmean * dmean);
+            const real scale_t = cka * Zh * Zd * Z0 / dmean;
+            real s = scale_t * sqrt(btn) + d.snul;
+            if (s >= real(0.2)) s = real(0.2);
+            snw[nz - 1] = s;
+            Kvw[nz - 1] = d.Pr_num * s;
+        }
+    }
+}
+#endif
+
 // Av(nz,elem) = sum(w_cv*snu(nz,nodes)) (fv_mixing.F90:308-313)
 __global__ void k_av(Dev d) {
     pdl_enter();
@@ -465,8 +1014,8 @@ __global__ void k_av(Dev d) {
 // Which form: the tiles while three blocks of 16 columns fit an SM (FP64 up
 // to 61 interfaces, 40 k nodes: 0.49 against 0.53 ms; 81 interfaces, two
 // blocks: 0.92 against 0.72), else one thread per column (also with the
-// launch-shape knob "d3end_arrays" at 1).  FP32 takes one thread per column
-// alone: the tiles were faster (232 k nodes 0.32 -> 0.20 ms), but their
+// launch-shape knob "d3end_arrays" at 1).  FP32 takes one thread per column,
+// or what the knob says: the tiles were faster (232 k nodes 0.32 -> 0.20 ms), but their
 // contracted arithmetic rounds otherwise, and the elevation, held in FP64,
 // shows it (1.8e-6 relative after 78 steps).
 // Up to 11 interfaces on grids of more than eight tiles per SM the one thread
@@ -487,6 +1036,21 @@ static int d3end_cols(const Dev &d) {
     return d.N > 2 * 148 * 16 && d3end_tile_smem(d, 32) <= 113 * 1024 ? 32 : 16;
 }
 #endif
+// the forms of FP32 beside one thread per column
+#if FESOMC_FP32
+static size_t d3end_sm_smem(const Dev &d) { return (size_t)d3end_values(d.NS) * kD3Block * sizeof(real); }
+static size_t d3end_setup_smem(const Dev &d) { return ((size_t)8 * kD3Tile * d.NS + 2 * kD3Tile) * sizeof(real); }
+static size_t d3end_sweep_smem(const Dev &d) { return (size_t)(4 * d.NS - 2) * kD3Block * sizeof(real); }
+bool d3end_split(const Dev &d, int form) { return form >= 3 && d.NS <= 40; }
+static void launch_d3end_split(const Dev &d, cudaStream_t s) {
+    const int tiles = (d.N + kD3Tile - 1) / kD3Tile, form = d.tune[TK_D3END];
+    launch_k(k_d3end_setup, tiles < 148 * 16 ? tiles : 148 * 16, kD3SetupThreads, d3end_setup_smem(d), s, d);
+    if (form >= 5 && d.NS == 21) launch_plain(form == 6 ? k_d3end_sweep_reg<21, 8> : k_d3end_sweep_reg<21, 6>, grid_for(d.N, 64), 64, 0, s, d);
+    else launch_plain(k_d3end_sweep_sm, grid_for(d.N, kD3Block), kD3Block, d3end_sweep_smem(d), s, d);
+}
+#else
+bool d3end_split(const Dev &, int) { return false; }
+#endif
 // the knob's number for the form that the sizes choose
 int d3end_default(const Dev &d) {
 #if FESOMC_FP32
@@ -501,7 +1065,10 @@ int d3end_default(const Dev &d) {
 int config_d3end(const Dev &d) {
     if (d.NS > 127) return 1;
 #if FESOMC_FP32
-    return 0;
+    if (d.NS <= 40 && (raise_smem_limit(k_d3end_setup, d3end_setup_smem(d)) != cudaSuccess ||
+                       raise_smem_limit(k_d3end_sweep_sm, d3end_sweep_smem(d)) != cudaSuccess))
+        return 1;
+    return raise_smem_limit(k_d3end_sm, d3end_sm_smem(d)) == cudaSuccess ? 0 : 1;
 #else
     const size_t t32 = d3end_tile_smem(d, 32), t16 = d3end_tile_smem(d, 16);
     bool ok = true;
@@ -522,6 +1089,12 @@ static void launch_d3end_form(const Dev &d, const int *list, const unsigned long
         else launch_k(k_d3end_tile<16, kList>, tiles, kT3Threads, d3end_tile_smem(d, 16), s, d, list, count);
         return;
     }
+#else
+    // the two-kernel forms set up every column and would overwrite the others'
+    // Ri: listed columns take k_d3end
+    if (!kList && d3end_split(d, d.tune[TK_D3END])) return launch_d3end_split(d, s);
+    if (!kList && d.tune[TK_D3END] == 2)
+        return launch_plain(k_d3end_sm, grid_for(d.N, kD3Block), kD3Block, d3end_sm_smem(d), s, d);
 #endif
     if (d.NS <= 11) launch_k(k_d3end<12, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);
     else if (d.NS <= 21) launch_k(k_d3end<22, kList>, grid_for(d.N, 64), 64, 0, s, d, list, count);

@@ -47,6 +47,7 @@ namespace fesomc {
     void launch_jac_swap(const Dev &, cudaStream_t); \
     void launch_je(const Dev &, cudaStream_t); \
     int d3end_default(const Dev &); \
+    bool d3end_split(const Dev &, int); \
     int config_d3end(const Dev &); \
     int config_vdiff(const Dev &); \
     int config_p1(const Dev &); \
@@ -234,7 +235,10 @@ template <typename T>
 int dalloc(fesomc_model *m, T **p, size_t n) {
     void *q = nullptr;
     cudaError_t e = cudaMalloc(&q, (n ? n : 1) * sizeof(T));
-    if (e != cudaSuccess) return FESOMC_ENOMEM;
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();   // the caller's refusal, not the next launch's error
+        return FESOMC_ENOMEM;
+    }
     // the zero fill runs on the legacy default stream, which the model's
     // non-blocking streams do not wait for: let it land before anything
     // is enqueued on them (an upload into a buffer allocated just before
@@ -1341,6 +1345,7 @@ int enqueue_step(fesomc_model *m, double ff) {
     n += 2;
     rec(m, "el2nodes", [&] { K3E2N(U_n, V_n, Unode, Vnode); });
     n += 1;
+    const int split = K3(d3end_split, d.tune[fesomc::TK_D3END]);   // d3_end in two kernels
     if (d.ver_mix == 3 && m->lc_on) {
         // learned closure: inputs, envelope test and fallback list; the
         // network on every column; its viscosity where it applies and the
@@ -1354,6 +1359,7 @@ int enqueue_step(fesomc_model *m, double ff) {
         n += 5;
         if (m->lc_judge_now) {
             rec(m, "d3end", [&] { K3(launch_d3end, s); });
+            n += split;
             rec(m, "lc_judge", [&] { K3(launch_lc_judge, c, s); });
         } else {
             rec(m, "lc_apply", [&] { K3(launch_lc_apply, c, s); });
@@ -1363,6 +1369,7 @@ int enqueue_step(fesomc_model *m, double ff) {
         n += 3;
     } else if (d.ver_mix == 3) {
         rec(m, "d3end", [&] { K3(launch_d3end, s); });
+        n += split;
         if (m->lc_harvest_now) { rec(m, "lc_harvest", [&] { K3(launch_lc_harvest, m->lcv, s); }); n += 3; }
         rec(m, "av", [&] { K3(launch_av, s); });
         n += 2;
@@ -2443,6 +2450,12 @@ int fesomc_gpu_tune_set(fesomc_model *m, const int32_t *values) {
         const int v = values[k];
         if (v < 0 || v > lim[k]) return FESOMC_EINVAL;
         if (!form_knob(k) && v != 0 && (v < 32 || v % 32 != 0)) return FESOMC_EINVAL;
+    }
+    // the arrays between the two kernels of d3_end, where a form first asks for them
+    if (m->fp32 && fesomc::f32::d3end_split(m->d32, values[fesomc::TK_D3END]) && m->p.ver_mix == 3) {
+        float **arr[] = {&m->d32.d3_pb, &m->d32.d3_qb, &m->d32.d3_c2, &m->d32.d3_sn};
+        for (float **p : arr)
+            if (!*p && (rc = dalloc(m, p, (size_t)m->d.NS * m->d.N))) return rc;
     }
     drop_graph(m);   // the captured step holds the old launch shapes
     for (int k = 0; k < fesomc::kTuneKnobs; ++k) m->d.tune[k] = m->d32.tune[k] = values[k];

@@ -28,8 +28,12 @@ from . import abi, cases, model
 
 THREADS = (64, 128, 256, 512, 1024)
 COLUMNS = (1, 2, 4, 8, 16, 32)
-# d3_end: one thread per column, or tiles of columns in shared memory
+# d3_end, FP64: one thread per column, or tiles of columns in shared memory;
+# FP32: one thread per column with its arrays in local or in shared memory, or
+# a set-up and a sweep kernel (the sweep's arrays in shared memory, or for 21
+# levels in registers at 6 or 8 blocks per SM)
 D3END_ARRAYS = (1, 2)
+D3END_ARRAYS_FP32 = (1, 2, 4, 5, 6)
 # the knobs that pick a form rather than a block size
 # tracer_impl_vert_diff: one form under every number
 VDIFF_FORMS = (3,)
@@ -139,6 +143,8 @@ def search(case, steps=3, warmup=2, margin=0.02, log=None):
         trials = 0
         for name, recs in ks:
             cands = FORMS.get(name, THREADS)
+            if name == "d3end_arrays" and case.params.fp32_form:
+                cands = D3END_ARRAYS_FP32
             cands = [c for c in cands if c <= lim[name]]
 
             def t_of(v):

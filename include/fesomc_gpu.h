@@ -452,10 +452,14 @@ int  fesomc_ensemble_run(fesomc_model *const *members, int32_t n_members, int32_
  * fesomc_gpu_tune_set takes one value per knob (0 = the default) and
  * returns FESOMC_EINVAL, changing nothing, when a thread count is not a
  * multiple of 32 or a value exceeds its limit ("d3end_arrays" takes 1 to 6:
- * d3_end with one thread per column, its arrays in local memory, or (2 to 6,
- * the same form under every number, so that saved shapes stay valid) on
- * tiles of columns in shared memory, the default up to 61 levels; the FP32
- * form has one thread per column under every number;
+ * d3_end with one thread per column, its arrays in local memory, or in FP64
+ * (2 to 6, the same form under every number, so that saved shapes stay
+ * valid) on tiles of columns in shared memory, the default up to 62 levels
+ * except for up to 11 levels on large grids; in FP32 2 holds the arrays in
+ * shared memory, 3 to 6 (up to 40 levels) are a set-up and a sweep kernel,
+ * the sweep's arrays in shared memory or (5 and 6, 21 levels) in registers
+ * at 6 or 8 blocks of 64 columns per SM; the forms from 3 on take device
+ * memory of 4 * levels * nodes floats, FESOMC_ENOMEM when it cannot be had;
  * "vdiff_form" 1 to 3, the same under every number: the tracers' implicit
  * vertical diffusion runs on tiles of columns in shared memory;
  * "implvisc_form" 1 or 2, the same under both numbers: the implicit vertical

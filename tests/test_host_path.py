@@ -258,7 +258,7 @@ def test_d3end_form(fake, nx, ny, nsigma, fp32, tiles):
     case = cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, fp32_form=fp32)
     g = model.GpuModel(case)
     try:
-        for form in (None, 1, 2):
+        for form in (None, 1) if fp32 else (None, 1, 2):
             if form:
                 autotune.apply(g, {"d3end_arrays": form})
             else:
@@ -266,7 +266,7 @@ def test_d3end_form(fake, nx, ny, nsigma, fp32, tiles):
             fake.clear()
             g.step(1)
             names = " ".join(o.name for o in fake.ops() if o.kind == "k")
-            want = tiles if form is None else form == 2 and not fp32
+            want = tiles if form is None else form == 2
             assert ("k_d3end_tileILi" in names) == want and ("k_d3endILi" in names) != want
     finally:
         g.close()
@@ -293,4 +293,37 @@ def test_columns_per_block(fake, nsigma, columns, pressure, p1):
                      ("k_p1_elem", p1)):
             assert {v for n, v in block.items() if k in n} == {b * (nsigma - 1)}, k
     finally:
+        g.close()
+
+
+@pytest.mark.parametrize("nsigma", [11, 21, 40, 41])
+@pytest.mark.parametrize("form", [2, 3, 4, 5, 6])
+def test_d3end_forms_of_fp32(fake, nsigma, form):
+    """The knob's forms of FP32: arrays in shared memory, a set-up and a sweep
+    kernel up to 40 levels (in registers for 21), all counted; the arrays
+    between the two kernels are made when a form asks for them, and a refusal
+    changes nothing."""
+    from fesomc import autotune, cases, model
+    g = model.GpuModel(cases.estuary_case("e", 20, 10, 300.0, nsigma, 2.0, 25.0, fp32_form=1))
+    try:
+        split = form >= 3 and nsigma <= 40
+        fake.lib.fake_fail_malloc(2)
+        if split:
+            with pytest.raises(RuntimeError):
+                autotune.apply(g, {"d3end_arrays": form})
+            assert autotune.get(g)[0]["d3end_arrays"] == 1
+        fake.lib.fake_fail_malloc(-1)
+        autotune.apply(g, {"d3end_arrays": form})
+        fake.clear()
+        n0 = g.kernel_launches()
+        g.step(1)
+        assert g.kernel_launches() - n0 == _kernels(fake)
+        names = " ".join(o.name for o in fake.ops() if o.kind == "k")
+        assert ("k_d3end_setup" in names) == split
+        assert ("k_d3end_sweep_regILi21ELi%dE" % (8 if form == 6 else 6) in names) == (form >= 5 and nsigma == 21)
+        assert ("k_d3end_sweep_sm" in names) == (split and not (form >= 5 and nsigma == 21))
+        assert ("k_d3end_sm" in names) == (form == 2)
+        assert ("k_d3endILi" in names) == (form >= 3 and not split)
+    finally:
+        fake.lib.fake_fail_malloc(-1)
         g.close()
