@@ -135,11 +135,9 @@ __host__ __device__ __forceinline__ float4 make_real4(float x, float y, float z,
 // per block of the column kernels (pressure_col, bpg_elem, update3d, wvel),
 // and the form of d3_end (1 one thread per column; FP64 2 to 6 tiles of columns
 // in shared memory; FP32 2 one thread per column with its arrays in shared
-// memory, 3 to 6 a set-up and a sweep kernel), and the form of the tracers'
-// implicit vertical diffusion (1 to 3, the same under every number: the sizes
-// decide), and the form of the implicit vertical viscosity (1 one thread per
-// element column reading the fields directly, 2 tiles of columns in shared
-// memory where they pay: the fic variant).  A value of 0 selects the built-in default.
+// memory, 3 to 6 a set-up and a sweep kernel).  A value of 0 selects the
+// built-in default.  TK_ZEROFILT, TK_VDIFF and TK_IMPLVISC are accepted and
+// read by no launch: the kernel is gone, and the sizes choose the forms.
 enum TuneKnob : int {
     TK_VELRHS, TK_VELGRAD3D, TK_ADV3, TK_PULS, TK_EL2NODES, TK_P1EDGE, TK_AB3, TK_VELGRAD2D, TK_SSHEDGE,
     TK_SSHNODE, TK_ADV2D, TK_U2D, TK_ROT, TK_ZEROFILT, TK_AB2, TK_MEGRAD, TK_MNGRAD, TK_MEDGE, TK_MH,

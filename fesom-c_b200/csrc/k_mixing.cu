@@ -1012,7 +1012,7 @@ __global__ void k_av(Dev d) {
 }
 
 // Which form: the tiles while three blocks of 16 columns fit an SM (FP64 up
-// to 61 interfaces, 40 k nodes: 0.49 against 0.53 ms; 81 interfaces, two
+// to 62 interfaces; 61 at 40 k nodes: 0.49 against 0.53 ms; 81 interfaces, two
 // blocks: 0.92 against 0.72), else one thread per column (also with the
 // launch-shape knob "d3end_arrays" at 1).  FP32 takes one thread per column,
 // or what the knob says: the tiles were faster (232 k nodes 0.32 -> 0.20 ms), but their

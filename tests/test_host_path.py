@@ -327,3 +327,16 @@ def test_d3end_forms_of_fp32(fake, nsigma, form):
     finally:
         fake.lib.fake_fail_malloc(-1)
         g.close()
+
+
+def test_search_leaves_out_what_nothing_reads(fake, monkeypatch):
+    """The autotuner's search tries no knob that no launch reads, or whose
+    kernels the case does not run; the shapes name every knob all the same."""
+    from fesomc import autotune, cases
+    tried = set()
+    apply = autotune.apply
+    monkeypatch.setattr(autotune, "apply", lambda g, shapes: (tried.update(shapes), apply(g, shapes)))
+    shapes, report = autotune.search(cases.estuary("small"), steps=1, warmup=1)
+    assert set(shapes) == {n for n, _ in autotune.knobs(fake.lib)} and all(v > 0 for v in shapes.values())
+    assert not tried & {"zero_filt", "vdiff_form", "implvisc_form", "upwind_h", "velgrad2d"}
+    assert {"velrhs", "columns", "d3end_arrays", "muscl_h"} <= tried and report["trials"] > 0
