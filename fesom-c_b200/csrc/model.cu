@@ -202,6 +202,7 @@ struct fesomc_model {
     // graph
     cudaGraphExec_t graph = nullptr;
     bool use_graph = true;
+    int device = 0;                   // the device the model was made on
     // state read-back: one event per slot of the staging pool
     std::vector<cudaEvent_t> stage_done;
     bool stage_ref = false;           // this model counts among the pool's users
@@ -555,8 +556,6 @@ int fields_in_rounds(fesomc_model *m, const std::vector<FieldOut> &fields) {
 }
 // all fields, slot after slot of the first ns with worker threads
 int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, int ns) {
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
     std::mutex mu;
     std::condition_variable cv;
     StagedPiece slot[kSlots];
@@ -565,7 +564,7 @@ int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, int ns
     for (bool &b : free_slot) b = true;
     std::atomic<int> bad{0};
     auto work = [&] {
-        cudaSetDevice(dev);
+        cudaSetDevice(m->device);
         for (;;) {
             int i;
             {
@@ -627,8 +626,19 @@ int fields_by_slots(fesomc_model *m, const std::vector<FieldOut> &fields, int ns
     CK(cudaStreamSynchronize(m->stream));
     return rc ? rc : (bad ? FESOMC_ECUDA : FESOMC_OK);
 }
+// the model's device current for a while: its events are made and recorded there
+struct OnDevice {
+    int was = 0;
+    explicit OnDevice(int device) {
+        if (cudaGetDevice(&was) != cudaSuccess || was == device || cudaSetDevice(device) != cudaSuccess) was = -1;
+    }
+    ~OnDevice() {
+        if (was >= 0) (void)cudaSetDevice(was);
+    }
+};
 // all fields through the staging slots; g_staging.in_use is held
 int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields) {
+    const OnDevice on(m->device);
     size_t total = 0;
     for (const FieldOut &o : fields) total += o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double));
     const int ns = staging_for(m, total);
@@ -1681,7 +1691,9 @@ int fesomc_gpu_init_packed(const fesomc_mesh *mesh, const fesomc_params *par, co
     // the launch checks below read the thread's last CUDA error: start from
     // a clean one (a non-sticky error of an earlier, unrelated call is not ours)
     (void)cudaGetLastError();
-    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(FESOMC_ECUDA);
+    if (cudaGetDevice(&m->device) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
+        return fail(FESOMC_ECUDA);
     if ((rc = build_mesh(m, mesh))) return fail(rc);
     if (m->fp32 && (rc = setup_f32_view(m))) return fail(rc);
     if ((rc = alloc_state(m))) return fail(rc);

@@ -37,7 +37,10 @@ std::vector<Pending> pending;
 void *capturing = nullptr;
 long long copies_left = -1, mallocs_left = -1;   // calls until one fails; -1: none fails
 cudaError_t last = cudaSuccess;
-int events = 0, pinned_calls = 0;
+int events = 0;
+thread_local int current = 0;                    // device
+std::map<void *, int> device_of;                 // of streams and events
+std::map<void *, void *> recorded;               // event: the stream it was recorded on
 dim3 cfg_grid, cfg_block;
 size_t cfg_smem;
 cudaStream_t cfg_stream;
@@ -209,25 +212,48 @@ cudaError_t cudaGetSymbolAddress(void **p, const void *) {
 }
 
 // ---- devices, streams, events, graphs ----
-cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
-cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int *n) { *n = 2; return cudaSuccess; }
+cudaError_t cudaGetDevice(int *d) { *d = current; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { current = d; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
     *v = a == cudaDevAttrMultiProcessorCount ? 148 : 10;
     return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize() { std::lock_guard<std::recursive_mutex> l(mu); land(nullptr, true); return cudaSuccess; }
-cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = (cudaStream_t)std::malloc(8); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+    std::lock_guard<std::recursive_mutex> l(mu);
+    *s = (cudaStream_t)std::malloc(8);
+    device_of[*s] = current;
+    return cudaSuccess;
+}
 cudaError_t cudaStreamDestroy(cudaStream_t s) { std::free(s); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { std::lock_guard<std::recursive_mutex> l(mu); land(s, false); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
-cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { ++events; *e = (cudaEvent_t)std::calloc(1, sizeof(void *)); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+    std::lock_guard<std::recursive_mutex> l(mu);
+    ++events;
+    *e = (cudaEvent_t)std::malloc(8);
+    device_of[*e] = current;
+    recorded.erase(*e);
+    return cudaSuccess;
+}
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return cudaEventCreateWithFlags(e, 0); }
-cudaError_t cudaEventDestroy(cudaEvent_t e) { --events; std::free(e); return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { *(void **)e = s; return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+    std::lock_guard<std::recursive_mutex> l(mu);
+    --events;
+    std::free(e);
+    return cudaSuccess;
+}
+// an event is recorded on streams of its own device
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    std::lock_guard<std::recursive_mutex> l(mu);
+    if (device_of[e] != (s ? device_of[s] : current)) return fail(cudaErrorInvalidResourceHandle);
+    recorded[e] = s;
+    return cudaSuccess;
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t e) {
     std::lock_guard<std::recursive_mutex> l(mu);
-    land(*(void **)e, false);
+    if (recorded.count(e)) land(recorded[e], false);
     return cudaSuccess;
 }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }

@@ -340,3 +340,21 @@ def test_search_leaves_out_what_nothing_reads(fake, monkeypatch):
     assert set(shapes) == {n for n, _ in autotune.knobs(fake.lib)} and all(v > 0 for v in shapes.values())
     assert not tried & {"zero_filt", "vdiff_form", "implvisc_form", "upwind_h", "velgrad2d"}
     assert {"velrhs", "columns", "d3end_arrays", "muscl_h"} <= tried and report["trials"] > 0
+
+
+def test_readback_with_another_device_current(fake):
+    """A model is read back on its own device's events whatever device is
+    current in the calling thread, which stays current."""
+    from fesomc import cases, model
+    rt = fake.lib
+    g = model.GpuModel(cases.estuary_case("e", 200, 100, 300.0, 11, 2.0, 25.0))
+    try:
+        assert rt.fesomc_gpu_set_device(1) == 0
+        got = g.state()
+        now = C.c_int(-1)
+        rt.cudaGetDevice(C.byref(now))
+        assert now.value == 1
+        assert all(np.array_equal(got[k], v) for k, v in g.case.state0.items())
+    finally:
+        rt.fesomc_gpu_set_device(0)
+        g.close()
