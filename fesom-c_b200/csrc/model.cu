@@ -419,49 +419,58 @@ std::vector<FieldRef> field_table(fesomc_model *m) {
 // go through page-locked staging slots of 1 MB: the calling thread enqueues
 // the device copies slot after slot, worker threads wait for a slot's copy and
 // move it to the caller's array (widening FP32), so that the caller's page
-// faults, the conversion and the transfer overlap.  Read-backs of up to 4 MB
+// faults, the conversion and the transfer overlap.  Read-backs of up to 6 MB
 // fill and empty one slot in turn, without workers: starting threads costs
-// more than they save there.  Against copying each field to pageable
-// memory and waiting for it: 803 MB into fresh arrays 166 -> 35 ms (the page
-// faults of one thread were most of it), 148 MB of FP32 fields 37 -> 8.7 ms,
-// 90 MB 40 -> 8 ms, 10 MB 2.2 -> 1.4 ms, 1.2 MB in 25 fields 0.44 -> 0.18 ms.
+// more than they save there.  Against copying each field to pageable memory
+// and waiting for it: 803 MB into fresh arrays 166 -> 35 ms (the page faults of
+// one thread were most of it), 148 MB of FP32 fields 37 -> 8.7 ms, 90 MB 40 -> 8
+// ms, 1.4 MB in 25 fields 0.62 -> 0.33 ms.
 // Page-locking is slow (1 to 2.5 ms per 2 MB), so the slots are made as the
 // volume read so far justifies them: the first at once (2 us: it comes out of
-// what the runtime holds for a model's small buffers), then one for every 8
-// MB, and no more than one for every 2 MB of a read-back.  First read-back of
-// a process's only model with all 16 made at once, and so: 0.3 MB 8.8 -> 0.6 ms,
-// 1.4 MB 12 -> 0.7, 8.5 MB 17 -> 2.6 (2.6 field by field), 34 MB 13 -> 10 (10).
+// what the runtime holds for a model's small buffers), then one for every 32
+// MB, which save as much as a slot costs (8 MB of FP32 fields, whose widening
+// gains more), and no more than one for every 4 MB of a read-back.  Until there
+// are two, FP64 fields of more than 16 MB are copied one by one.  First
+// read-back of a process's only model with all 16 made at once, so, and field
+// by field: 1.4 MB 14, 0.4, 0.6 ms; 8.5 MB 18, 1.3, 1.2; 34 MB 22, 3.6, 2.9;
+// 88 MB 23, 9.9, 5.5; FP32 24, 10.6, 13.5.
 // The slots are shared by the process's models and freed with the last of
 // them.  A read-back that finds them in use by another thread takes the plain
 // path.
 constexpr size_t kSlotBytes = 1 << 20;
 constexpr int kSlots = 16;
-constexpr size_t kSlotsAlone = 4 * kSlotBytes;   // read-backs that need no workers
-constexpr size_t kBytesPerSlot = 8 * kSlotBytes; // volume that justifies a slot more
+constexpr size_t kSlotsAlone = 6 * kSlotBytes;    // device bytes that need no workers
+constexpr size_t kRoundsMost = 16 * kSlotBytes;   // FP64 bytes worth one slot in turn
+constexpr size_t kBytesPerSlot = 32 * kSlotBytes; // volume that justifies a slot more
+constexpr size_t kSlotShare = 4 * kSlotBytes;     // of a read-back, for each slot it takes
 struct StagingPool {
     std::mutex in_use;                // held for the length of a read-back
     std::mutex mu;                    // guards the rest
     int users = 0;
     int n = 0;                        // slots made
-    size_t volume = 0;                // of the larger read-backs
+    size_t volume = 0;                // of the larger read-backs, FP32 fields counted four times
     unsigned char *slot[kSlots] = {};
 };
 StagingPool g_staging;
 
-// the slots of a read-back of 'total' bytes (0: page-locked memory could not
-// be had), and the model's events for them
-int staging_for(fesomc_model *m, size_t total) {
+// what a read-back moves: bytes on the device, in the caller's arrays, and
+// what they count towards a slot
+struct ReadBytes {
+    size_t dev = 0, out = 0, weight = 0;
+};
+// the slots of a read-back (0: page-locked memory could not be had), and the
+// model's events for them
+int staging_for(fesomc_model *m, const ReadBytes &b) {
     std::lock_guard<std::mutex> lk(g_staging.mu);
     if (!m->stage_ref) {
         g_staging.users += 1;
         m->stage_ref = true;
     }
-    size_t want = 1;
-    if (total > kSlotsAlone) {
-        g_staging.volume += total;
-        want = std::max<size_t>(1, std::min({(size_t)kSlots, g_staging.volume / kBytesPerSlot, total / (2 * kSlotBytes)}));
-    }
-    while (g_staging.n < (int)want) {
+    const bool alone = b.dev <= kSlotsAlone;
+    const int most = alone ? 1 : (int)std::min<size_t>(kSlots, std::max<size_t>(1, b.out / kSlotShare));
+    if (!alone) g_staging.volume += b.weight;
+    const int want = std::max(1, (int)std::min<size_t>(most, g_staging.volume / kBytesPerSlot));
+    while (g_staging.n < want) {
         void *q = nullptr;
         if (cudaMallocHost(&q, kSlotBytes) != cudaSuccess) {
             (void)cudaGetLastError();
@@ -469,8 +478,8 @@ int staging_for(fesomc_model *m, size_t total) {
         }
         g_staging.slot[g_staging.n++] = static_cast<unsigned char *>(q);
     }
-    const int ns = total <= kSlotsAlone ? std::min(g_staging.n, 1) : std::min<int>(g_staging.n, total / (2 * kSlotBytes));
-    while ((int)m->stage_done.size() < ns && ns > 1) {
+    const int ns = std::min(g_staging.n, most);
+    while (ns > 1 && (int)m->stage_done.size() < ns) {
         cudaEvent_t e;
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
             (void)cudaGetLastError();
@@ -639,10 +648,14 @@ struct OnDevice {
 // all fields through the staging slots; g_staging.in_use is held
 int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields) {
     const OnDevice on(m->device);
-    size_t total = 0;
-    for (const FieldOut &o : fields) total += o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double));
-    const int ns = staging_for(m, total);
-    if (ns < 1) return FESOMC_ENOMEM;
+    ReadBytes b;
+    for (const FieldOut &o : fields) {
+        b.dev += o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double));
+        b.out += o.f.count * sizeof(double);
+        b.weight += o.f.count * (o.f.f32 ? 4 * sizeof(float) : sizeof(double));
+    }
+    const int ns = staging_for(m, b);
+    if (ns < 1 || (ns == 1 && !m->fp32 && b.dev > kRoundsMost)) return FESOMC_ENOMEM;
     const int rc = ns == 1 ? fields_in_rounds(m, fields) : fields_by_slots(m, fields, ns);
     // after a failure too, no copy may still be on its way to the slots when
     // another model's read-back takes them
