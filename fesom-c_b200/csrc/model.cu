@@ -427,13 +427,15 @@ std::vector<FieldRef> field_table(fesomc_model *m) {
 // ms, 1.4 MB in 25 fields 0.62 -> 0.33 ms.
 // Page-locking is slow (1 to 2.5 ms per 2 MB), so the slots are made as the
 // volume read so far justifies them: the first at once (2 us: it comes out of
-// what the runtime holds for a model's small buffers), then one for every 32
-// MB, which save as much as a slot costs (8 MB of FP32 fields, whose widening
-// gains more), and no more than one for every 4 MB of a read-back.  Until there
-// are two, FP64 fields of more than 16 MB are copied one by one.  First
-// read-back of a process's only model with all 16 made at once, so, and field
-// by field: 1.4 MB 14, 0.4, 0.6 ms; 8.5 MB 18, 1.3, 1.2; 34 MB 22, 3.6, 2.9;
-// 88 MB 23, 9.9, 5.5; FP32 24, 10.6, 13.5.
+// what the runtime holds for a model's small buffers), then one for every 16
+// MB (8 MB of FP32 fields, whose widening gains more), and no more than one for
+// every 2 MB of a read-back.  A slot saves its cost on 8 MB where the caller's
+// pages are fresh (a page fault is the dearest part) and on 35 MB where they
+// are warm.  Until there are two, FP64 fields of more than 16 MB are copied one
+// by one.  First read-back of a process's only model with all 16 made at once,
+// so, and field by field: 1.4 MB 14, 0.4, 0.6 ms; 8.5 MB 18, 1.4, 1.1; 34 MB 22,
+// 5, 2.8 (fresh pages 13, 8, 10); 88 MB 22, 10, 5.5; FP32 24, 11, 13.5; 166 MB,
+// fresh pages 27, 19, 33.
 // The slots are shared by the process's models and freed with the last of
 // them.  A read-back that finds them in use by another thread takes the plain
 // path.
@@ -441,14 +443,14 @@ constexpr size_t kSlotBytes = 1 << 20;
 constexpr int kSlots = 16;
 constexpr size_t kSlotsAlone = 6 * kSlotBytes;    // device bytes that need no workers
 constexpr size_t kRoundsMost = 16 * kSlotBytes;   // FP64 bytes worth one slot in turn
-constexpr size_t kBytesPerSlot = 32 * kSlotBytes; // volume that justifies a slot more
-constexpr size_t kSlotShare = 4 * kSlotBytes;     // of a read-back, for each slot it takes
+constexpr size_t kBytesPerSlot = 16 * kSlotBytes; // volume that justifies a slot more
+constexpr size_t kSlotShare = 2 * kSlotBytes;     // of a read-back, for each slot it takes
 struct StagingPool {
     std::mutex in_use;                // held for the length of a read-back
     std::mutex mu;                    // guards the rest
     int users = 0;
     int n = 0;                        // slots made
-    size_t volume = 0;                // of the larger read-backs, FP32 fields counted four times
+    size_t volume = 0;                // of the larger read-backs, FP32 fields counted twice
     unsigned char *slot[kSlots] = {};
 };
 StagingPool g_staging;
@@ -652,7 +654,7 @@ int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields) 
     for (const FieldOut &o : fields) {
         b.dev += o.f.count * (o.f.f32 ? sizeof(float) : sizeof(double));
         b.out += o.f.count * sizeof(double);
-        b.weight += o.f.count * (o.f.f32 ? 4 * sizeof(float) : sizeof(double));
+        b.weight += o.f.count * (o.f.f32 ? 2 * sizeof(float) : sizeof(double));
     }
     const int ns = staging_for(m, b);
     if (ns < 1 || (ns == 1 && !m->fp32 && b.dev > kRoundsMost)) return FESOMC_ENOMEM;

@@ -192,7 +192,7 @@ def test_staging_memory_grows_with_use_and_is_given_back(fake, fp32):
             got = b.state()
             for k, v in got.items():
                 assert np.array_equal(v, first[k]), k
-        assert sizes[0] == (4 if fp32 else 2) and sizes == sorted(sizes) and sizes[-1] == 16
+        assert sizes[0] == 4 and sizes == sorted(sizes) and sizes[-1] == 16
         got = a.state()
         assert all(np.array_equal(got[k], v) for k, v in want.items())
         b.close()
