@@ -52,7 +52,7 @@ __device__ __forceinline__ real div_pos(real x, real d) {
 //     that their latency overlaps the current level's division chain (3 %
 //     faster; unrolling by 4 instead was 9 % slower).
 // The form of FP32, and in FP64 for level counts whose tiles (below) do not
-// fit well.
+// fit well and for few levels on large grids.
 //
 // kList: the columns are list[0 .. *count) instead of every node (the
 // columns the learned closure hands back to the plain one).
