@@ -27,9 +27,10 @@ __device__ __forceinline__ float silu_grad_f(float z) {
 enum { EPI_PART = 0, EPI_BIAS = 1, EPI_BIAS_SILU = 2, EPI_SILU_GRAD = 3, EPI_SILU_ONLY = 4 };
 
 // C[M x N] = op(A)[M x K] op(B)[K x N]: A(m,k) = TA ? A[k*lda+m] : A[m*lda+k],
-// B(k,n) = TB ? B[n*ldb+k] : B[k*ldb+n].  128 x 64 tiles, 16-deep k slices in
-// two shared-memory buffers (the next slice's loads are in flight while this
-// one is multiplied), 8 x 4 outputs per thread, FP32 with explicit fused
+// B(k,n) = TB ? B[n*ldb+k] : B[k*ldb+n].  BM x 64 tiles (BM 128, or 64 where
+// 128 would leave SMs without one), 16-deep k slices in two shared-memory
+// buffers (the next slice's loads are in flight while this one is
+// multiplied), BM / 16 x 4 outputs per thread, FP32 with explicit fused
 // multiply-adds in k order.  Epilogues: store; + bias[n]; + bias[n] and SiLU
 // (Z to C, SiLU(Z) to C2); times SiLU'(Zin[m,n]); EPI_PART, the weight
 // gradients: blockIdx.z takes kSplit of the k range and stores its partial
@@ -42,9 +43,12 @@ enum { EPI_PART = 0, EPI_BIAS = 1, EPI_BIAS_SILU = 2, EPI_SILU_GRAD = 3, EPI_SIL
 // 8192 deep, and their column sums 43 us in two more launches.  256 samples
 // a part: 256 blocks for a 256 x 256 gradient, and a shorter FP32 sum (error
 // of the gradients against 64 bits 1.2e-6 -> 1.3e-7).
-constexpr int kBM = 128, kBN = 64, kBK = 16;
+// With 128 rows always, a forward pass of 700 columns had 24 blocks and took 92
+// us on the device; with 64 where 128 give fewer than 148 blocks 66 us (64 x 64
+// without a load in flight 86), the gradients of 512 samples 385 -> 335 us.
+constexpr int kBN = 64, kBK = 16;
 constexpr int kSplit = 256;
-template <bool TA, bool TB, int EPI>
+template <bool TA, bool TB, int EPI, int kBM>
 __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float *__restrict__ A, int lda,
                                               const float *__restrict__ B, int ldb, float *__restrict__ C, int ldc,
                                               const float *__restrict__ bias, float *__restrict__ C2,
@@ -58,15 +62,16 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float 
     const int k_hi = EPI == EPI_PART ? min(K, k_lo + kSplit) : K;
     const bool sums = EPI == EPI_PART && blockIdx.x == 0 && tid < kBM;
     float colsum = 0.0f;
-    float acc[8][4];
+    constexpr int RM = kBM / 16;   // rows per thread
+    float acc[RM][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < RM; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-    float ra[8], rb[4];
+    float ra[RM], rb[4];
     auto fetch = [&](int k0) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
+        for (int r = 0; r < RM; ++r) {
             const int e = tid + r * 256;
             const int mm = TA ? e % kBM : e / kBK, kk = TA ? e / kBM : e % kBK;
             const int gm = m0 + mm, gk = k0 + kk;
@@ -82,7 +87,7 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float 
     };
     auto stage = [&](int buf) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
+        for (int r = 0; r < RM; ++r) {
             const int e = tid + r * 256;
             As[buf][TA ? e / kBM : e % kBK][TA ? e % kBM : e / kBK] = ra[r];
         }
@@ -105,12 +110,16 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float 
         }
 #pragma unroll
         for (int kk = 0; kk < kBK; ++kk) {
-            const float4 a0 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 8]);
-            const float4 a1 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 8 + 4]);
-            const float4 b = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b.x, b.y, b.z, b.w};
+            float av[RM];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < RM; i += 4) {
+                const float4 a = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * RM + i]);
+                av[i] = a.x; av[i + 1] = a.y; av[i + 2] = a.z; av[i + 3] = a.w;
+            }
+            const float4 b = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
+            const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < RM; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
         }
@@ -122,8 +131,8 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float 
         if (sums && m0 + tid < M) C[(size_t)M * N + m0 + tid] = colsum;
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int gm = m0 + ty * 8 + i;
+    for (int i = 0; i < RM; ++i) {
+        const int gm = m0 + ty * RM + i;
         if (gm >= M) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -143,8 +152,14 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float 
 template <bool TA, bool TB, int EPI>
 void sgemm(cudaStream_t s, int M, int N, int K, const float *A, int lda, const float *B, int ldb, float *C, int ldc,
            const float *bias = nullptr, float *C2 = nullptr, const float *Zin = nullptr) {
-    dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, EPI == EPI_PART ? (K + kSplit - 1) / kSplit : 1);
-    k_sgemm<TA, TB, EPI><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, C2, Zin);
+    const unsigned nb = (N + kBN - 1) / kBN, mb = (M + 127) / 128;
+    if (EPI == EPI_PART || nb * mb >= 148) {
+        const dim3 grid(nb, mb, EPI == EPI_PART ? (K + kSplit - 1) / kSplit : 1);
+        k_sgemm<TA, TB, EPI, 128><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, C2, Zin);
+    } else {
+        const dim3 grid(nb, (M + 63) / 64);
+        k_sgemm<TA, TB, EPI, 64><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, C2, Zin);
+    }
 }
 
 // the parts of a split product summed in k order: out[i] = sum_c part[c*n + i]

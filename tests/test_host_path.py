@@ -360,3 +360,22 @@ def test_readback_with_another_device_current(fake):
     finally:
         rt.fesomc_gpu_set_device(0)
         g.close()
+
+
+@pytest.mark.parametrize("batch,rows", [(1, 64), (4608, 64), (4609, 128), (8192, 128)])
+def test_network_tile(fake, batch, rows):
+    """The FP32 network's products (256 hidden units): tiles of 128 rows where
+    they give every SM a block, else of 64; the weight gradients, split over
+    the batch, of 128."""
+    from fesomc import closure
+    c = closure.Closure(21)
+    try:
+        fake.clear()
+        c.grad(np.zeros((batch, c.n_in), dtype=np.float32), np.zeros((batch, c.n_out), dtype=np.float32))
+        hidden = [o for o in fake.ops() if "k_sgemmILb0ELb1ELi2E" in o.name]
+        parts = [o for o in fake.ops() if "k_sgemmILb1ELb0ELi0E" in o.name]
+        assert len(hidden) == 3 and {("ELi%dE" % rows) in o.name[-60:] for o in hidden} == {True}
+        assert len(parts) == 4 and all("Li0ELi128E" in o.name for o in parts)
+        assert all((o.grid >= 148) == (rows == 128) or rows == 64 for o in hidden)
+    finally:
+        c.close()
