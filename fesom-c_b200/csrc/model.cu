@@ -416,15 +416,15 @@ std::vector<FieldRef> field_table(fesomc_model *m) {
 
 // ---- state read-back ----------------------------------------------------------
 // A field whose array is page-locked is copied straight into it.  The others
-// go through page-locked staging slots of 1 MB: the calling thread enqueues
-// the device copies slot after slot, worker threads wait for a slot's copy and
-// move it to the caller's array (widening FP32), so that the caller's page
-// faults, the conversion and the transfer overlap.  Read-backs of up to 6 MB
-// fill and empty one slot in turn, without workers: starting threads costs
-// more than they save there.  Against copying each field to pageable memory
-// and waiting for it: 803 MB into fresh arrays 166 -> 35 ms (the page faults of
-// one thread were most of it), 148 MB of FP32 fields 37 -> 8.7 ms, 90 MB 40 -> 8
-// ms, 1.4 MB in 25 fields 0.62 -> 0.33 ms.
+// go through page-locked staging slots of 1 MB (the first 1.5): the calling
+// thread enqueues the device copies slot after slot, worker threads wait for a
+// slot's copy and move it to the caller's array (widening FP32), so that the
+// caller's page faults, the conversion and the transfer overlap.  Read-backs of
+// up to 6 MB fill and empty the first slot in turn, without workers: starting
+// threads costs more than they save there.  Against copying each field to
+// pageable memory and waiting for it: 803 MB into fresh arrays 166 -> 35 ms
+// (the page faults of one thread were most of it), 148 MB of FP32 fields 37 ->
+// 8.7 ms, 90 MB 40 -> 8 ms, 1.4 MB in 25 fields 0.62 -> 0.33 ms.
 // Page-locking is slow (1 to 2.5 ms per 2 MB), so the slots are made as the
 // volume read so far justifies them: the first at once (2 us: it comes out of
 // what the runtime holds for a model's small buffers), then one for every 16
@@ -441,6 +441,7 @@ std::vector<FieldRef> field_table(fesomc_model *m) {
 // path.
 constexpr size_t kSlotBytes = 1 << 20;
 constexpr int kSlots = 16;
+constexpr size_t kFirstBytes = kSlotBytes + kSlotBytes / 2;   // of the first slot, still out of what the runtime holds
 constexpr size_t kSlotsAlone = 6 * kSlotBytes;    // device bytes that need no workers
 constexpr size_t kRoundsMost = 16 * kSlotBytes;   // FP64 bytes worth one slot in turn
 constexpr size_t kBytesPerSlot = 16 * kSlotBytes; // volume that justifies a slot more
@@ -474,7 +475,7 @@ int staging_for(fesomc_model *m, const ReadBytes &b) {
     const int want = std::max(1, (int)std::min<size_t>(most, g_staging.volume / kBytesPerSlot));
     while (g_staging.n < want) {
         void *q = nullptr;
-        if (cudaMallocHost(&q, kSlotBytes) != cudaSuccess) {
+        if (cudaMallocHost(&q, g_staging.n == 0 ? kFirstBytes : kSlotBytes) != cudaSuccess) {
             (void)cudaGetLastError();
             break;
         }
@@ -555,8 +556,8 @@ int fields_in_rounds(fesomc_model *m, const std::vector<FieldOut> &fields) {
         int rc = field_source(m, o.f, &src);
         if (rc) return rc;
         for (size_t at = 0; at < bytes;) {
-            if (off == kSlotBytes && (rc = empty())) return rc;
-            const size_t n = std::min(kSlotBytes - off, bytes - at);
+            if (off == kFirstBytes && (rc = empty())) return rc;
+            const size_t n = std::min(kFirstBytes - off, bytes - at);
             CK(cudaMemcpyAsync(buf + off, src + at, n, cudaMemcpyDeviceToHost, m->stream));
             out.push_back({buf + off, o.h + at / value, n, o.f.f32});
             at += n;
@@ -667,11 +668,15 @@ int fields_to_host_staged(fesomc_model *m, const std::vector<FieldOut> &fields) 
 
 // whether a field's array in the caller's memory is page-locked
 bool page_locked(const double *h, size_t count) {
-    cudaPointerAttributes a, b;
-    if (cudaPointerGetAttributes(&a, h) == cudaSuccess && cudaPointerGetAttributes(&b, h + count - 1) == cudaSuccess)
-        return a.type == cudaMemoryTypeHost && b.type == cudaMemoryTypeHost;
-    (void)cudaGetLastError();
-    return false;
+    for (const double *p : {h, h + count - 1}) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        if (a.type != cudaMemoryTypeHost) return false;
+    }
+    return true;
 }
 
 // host double <-> device field (converting for FP32 level fields, and

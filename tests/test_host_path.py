@@ -168,7 +168,7 @@ def test_page_locked_arrays_receive_the_copy_directly(fake, fp32):
 
 @pytest.mark.parametrize("fp32", [0, 1])
 def test_staging_memory_grows_with_use_and_is_given_back(fake, fp32):
-    """The page-locked slots are made as read-backs justify them (1 MB for
+    """The page-locked slots are made as read-backs justify them (1.5 MB for
     small ones, more with the volume of larger ones, 16 MB at most), shared by
     the process's models and freed with the last of them; the values are the
     same at every stage."""
@@ -180,10 +180,10 @@ def test_staging_memory_grows_with_use_and_is_given_back(fake, fp32):
     held = fake.lib.fake_pinned_bytes()          # a model's own small buffers
     try:
         want = a.state()
-        assert fake.lib.fake_pinned_bytes() - held == MB
+        assert fake.lib.fake_pinned_bytes() - held == 3 * MB // 2
         case = cases.estuary_case("e", 200, 100, 300.0, 21, 2.0, 25.0, fp32_form=fp32)
         b = model.GpuModel(case)
-        held = fake.lib.fake_pinned_bytes() - MB
+        held = fake.lib.fake_pinned_bytes() - 3 * MB // 2
         sizes = []
         first = b.state()
         assert 64 * MB < sum(v.nbytes for k, v in first.items() if k != "_time_jd") < 128 * MB
