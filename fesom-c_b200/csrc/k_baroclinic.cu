@@ -1330,8 +1330,13 @@ static int col_b(const Dev &d) {
 // pressure_col's level sums take one lane per column, and its blocks do little
 // else: four columns where the others take one or two.  100 k nodes, FP32: 54
 // layers 0.064 -> 0.054 ms, 100 layers 0.144 -> 0.103, 126 layers 0.161 -> 0.126,
-// FP64 0.100 -> 0.091, 0.222 -> 0.168, 0.251 -> 0.249.
-static int pressure_b(const Dev &d) { return d.tune[TK_COLUMNS] == 0 && d.L > 53 ? 4 : col_b(d); }
+// FP64 0.100 -> 0.091, 0.222 -> 0.168, 0.251 -> 0.249.  Fewer layers: the count
+// that fills its warps, 149 k nodes, 44 layers 0.113 -> 0.103 ms, FP32 0.073 ->
+// 0.062, 27 layers 0.069 -> 0.064 (the others' barriers want small blocks).
+static int pressure_b(const Dev &d) {
+    if (d.tune[TK_COLUMNS] > 0) return col_b(d);
+    return d.L > 53 ? 4 : filled_columns(d.L, default_columns(d.L));
+}
 static size_t pressure_smem(const Dev &d) { return (size_t)pressure_b(d) * (d.L | 1) * sizeof(real); }
 static size_t bpg_smem(const Dev &d) {
     return (size_t)col_b(d) * (kEsReals + 12 + 2 * d.L + 1) * sizeof(real);

@@ -746,10 +746,12 @@ void launch_el2nodes(const Dev &d, const real *Ue, const real *Ve, real *Un, rea
 // kernels (up to 1024 threads before: 1.05 M nodes 0.90 -> 0.70 ms, 40 k, 30
 // layers 0.082 -> 0.054, 232 k FP32 0.133 -> 0.117); per element its slot tile, 8 slot sums, 4 acc, dmean_n and 4 edge codes
 // (81 to 119 layers: two at least, FP32 96 layers 0.554 -> 0.343 ms, 110 layers
-// 0.317 -> 0.274, 100 k nodes)
+// 0.317 -> 0.274, 100 k nodes; and the count that fills its warps, 149 k nodes,
+// FP32, 44 layers 0.185 -> 0.160, 69 layers 0.274 -> 0.241, FP64 27 layers 0.153 ->
+// 0.140)
 static int p1_elems(const Dev &d) {
     const int b = default_columns(d.L);
-    return b < 2 && d.L < 120 ? 2 : b;
+    return filled_columns(d.L, b < 2 && d.L < 120 ? 2 : b);
 }
 static size_t p1_smem(const Dev &d) {
     return (size_t)p1_elems(d) * ((2 * (kP1Slots + (d.bih_3D ? 1 : 0)) * d.L + 1 + 13) * sizeof(real) +

@@ -32,7 +32,7 @@ def test_implicit_viscosity_tiles(built, nx, ny, nsigma, kw):
     _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib, **kw), 3)
 
 
-@pytest.mark.parametrize("nsigma", [54, 55, 84, 97, 101, 106, 108, 120, 121])
+@pytest.mark.parametrize("nsigma", [18, 25, 28, 45, 54, 55, 70, 84, 97, 101, 106, 108, 120, 121])
 def test_columns_per_block(built, nsigma):
     from fesomc import cases
     _compare(lambda lib: cases.estuary_case("e", 13, 11, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib), 3)

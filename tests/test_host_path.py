@@ -278,9 +278,10 @@ def test_implicit_viscosity_tile(fake, nsigma, fp32, cols):
     assert "k_implvisc_fic_tileILi%dE" % cols in _launched(fake, 20, 10, nsigma, fp32)
 
 
-@pytest.mark.parametrize("nsigma,columns,pressure,p1", [(21, 8, 8, 8), (54, 3, 3, 3), (55, 2, 4, 2), (81, 2, 4, 2), (84, 3, 4, 3),
-                                                        (97, 1, 4, 2), (106, 3, 4, 3), (108, 1, 4, 2), (120, 1, 4, 2),
-                                                        (121, 1, 4, 1), (127, 1, 4, 1)])
+@pytest.mark.parametrize("nsigma,columns,pressure,p1", [(11, 16, 16, 16), (21, 8, 8, 8), (25, 6, 8, 8), (45, 3, 5, 5),
+                                                        (54, 3, 3, 3), (55, 2, 4, 4), (81, 2, 4, 2), (84, 3, 4, 3), (97, 1, 4, 2),
+                                                        (106, 3, 4, 3), (108, 1, 4, 2), (120, 1, 4, 2), (121, 1, 4, 1),
+                                                        (127, 1, 4, 1)])
 def test_columns_per_block(fake, nsigma, columns, pressure, p1):
     """Entities per block of the column kernels, by the level count."""
     from fesomc import cases, model
