@@ -994,12 +994,14 @@ __global__ void k_wvel(Dev d) {
 // layers 0.049, 0.064 -> 0.043, 16 k, 10 layers 0.017, 0.016 -> 0.013, 4.5 k,
 // 39 layers 0.032, 0.025 -> 0.019.
 // A column takes 32 B of shared memory per layer (FP64): where 32 of them
-// would leave an SM fewer than three blocks (73 layers on), a block takes 16,
-// and 256 threads, four times as many as its recurrences need, for the staging
-// and its divisions.  16 k nodes, 80 layers 0.091 -> 0.051 ms, 126 layers 0.222 ->
-// 0.097, 100 k nodes 0.429 -> 0.260 and 1.235 -> 0.562 (one thread per column:
-// 0.103, 0.142, 0.416, 0.710; 16 columns with 64 threads 0.354 and 0.849, with 128
-// 0.288 and 0.660).
+// leave an SM fewer than four blocks (55 layers on) a block takes 16, and 256
+// threads, four times as many as its recurrences need, for the staging and its
+// divisions; where 16 leave fewer than four (106 layers on) 8, and 128.  16 k
+// nodes, 80 layers 0.091 -> 0.051 ms, 149 k nodes, 55 layers 0.328 -> 0.278, 69
+// layers 0.404 -> 0.338, 100 k nodes, 80 layers 0.429 -> 0.260, 126 layers 1.235 ->
+// 0.55 (one thread per column 0.416, 0.710; 16 columns with 64 threads 0.849, with
+// 128 0.660, with 256 0.562); 8 columns with 128 threads at 74 layers 0.362 against
+// 0.355.
 #if !FESOMC_FP32
 constexpr int kIvBatch = 3;
 #endif
@@ -1307,16 +1309,25 @@ static void (*implvisc_reg_kernel(const Dev &d))(Dev) {
 }
 static size_t implvisc_reg_smem(const Dev &d) { return (size_t)kIrCols * (3 * (d.L | 1) + (d.NS | 1)) * sizeof(real); }
 // Few layers leave the level-parallel tiles little to share between their
-// barriers: the register tiles from five of them per SM on (elements; ms at
-// nodes, register / level-parallel tiles): 10 layers 40 k nodes 0.0183 /
+// barriers: the register tiles from five of them per SM on, three in FP32
+// (elements; ms at nodes, register / level-parallel tiles): 10 layers 40 k nodes 0.0183 /
 // 0.0198, 1.0 M 0.229 / 0.251, FP32 40 k 0.0126 / 0.0138, 100 k 0.0164 / 0.0228,
 // 1.0 M 0.095 / 0.127; 5 layers 1.0 M 0.101 / 0.176, FP32 0.054 / 0.088; 24 k
-// nodes 0.0166 / 0.0149.
-static bool implvisc_reg(const Dev &d) { return d.L >= 4 && d.L <= 10 && d.E >= 5 * 148 * kIrCols; }
+// nodes 0.0166 / 0.0149, FP32 6 layers 0.0085 / 0.0103.
+static bool implvisc_reg(const Dev &d) { return d.L >= 4 && d.L <= 10 && d.E >= (FESOMC_FP32 ? 3 : 5) * 148 * kIrCols; }
 static size_t implvisc_tile_smem(const Dev &d, int cols) { return (size_t)4 * d.L * (cols + 1) * sizeof(real); }
+// columns of a tile
+static int implvisc_cols(const Dev &d) {
+    if (FESOMC_FP32 || implvisc_tile_smem(d, 32) <= 56 * 1024) return 32;
+    return implvisc_tile_smem(d, 16) <= 56 * 1024 ? 16 : 8;
+}
+static void (*implvisc_tile_kernel(const Dev &d))(Dev) {
 #if !FESOMC_FP32
-static bool implvisc_narrow(const Dev &d) { return implvisc_tile_smem(d, 32) > 75 * 1024; }
+    if (implvisc_cols(d) == 16) return k_implvisc_fic_tile<16, 256>;
+    if (implvisc_cols(d) == 8) return k_implvisc_fic_tile<8, 128>;
 #endif
+    return k_implvisc_fic_tile<32, 128>;
+}
 
 // ---- launch wrappers --------------------------------------------------------
 // Column blocks: B entities, B * L threads, about 160 of them (at most 16
@@ -1346,12 +1357,7 @@ static size_t wvel_smem(const Dev &d) {
     return (size_t)col_b(d) * (kWvEdges * sizeof(WvEdge) + ((d.L | 1) + 2) * sizeof(real));
 }
 int config_columns(const Dev &d) {
-    cudaError_t e = cudaSuccess;
-#if !FESOMC_FP32
-    if (implvisc_narrow(d)) e = raise_smem_limit(k_implvisc_fic_tile<16, 256>, implvisc_tile_smem(d, 16));
-    else
-#endif
-        e = raise_smem_limit(k_implvisc_fic_tile<32, 128>, implvisc_tile_smem(d, 32));
+    cudaError_t e = raise_smem_limit(implvisc_tile_kernel(d), implvisc_tile_smem(d, implvisc_cols(d)));
     if (e == cudaSuccess) e = raise_smem_limit(k_bpg_elem, bpg_smem(d));
     if (e == cudaSuccess) e = raise_smem_limit(k_update3d, update3d_smem(d));
     if (e == cudaSuccess) e = raise_smem_limit(k_pressure_col, pressure_smem(d));
@@ -1406,10 +1412,10 @@ void launch_implvisc(const Dev &d, cudaStream_t s) {
     if (d.im_vert_visc) MAXL_DISPATCH(k_implvisc, grid_for(d.E, 128), 128, s, d);
     if (!d.im_vert_visc_fic) return;
     if (implvisc_reg(d)) launch_k(implvisc_reg_kernel(d), (d.E + kIrCols - 1) / kIrCols, kIrCols, implvisc_reg_smem(d), s, d);
-#if !FESOMC_FP32
-    else if (implvisc_narrow(d)) launch_k(k_implvisc_fic_tile<16, 256>, (d.E + 15) / 16, 256, implvisc_tile_smem(d, 16), s, d);
-#endif
-    else launch_k(k_implvisc_fic_tile<32, 128>, (d.E + 31) / 32, 128, implvisc_tile_smem(d, 32), s, d);
+    else {
+        const int C = implvisc_cols(d);
+        launch_k(implvisc_tile_kernel(d), (d.E + C - 1) / C, C == 16 ? 256 : 128, implvisc_tile_smem(d, C), s, d);
+    }
 }
 void launch_jac_swap(const Dev &d, cudaStream_t s) {
     const int b = tuned(d, TK_ROT, 256);

@@ -1,6 +1,6 @@
 """Kernel forms of meshes with many layers against the oracle, bit for bit:
-the implicit viscosity's tiles of 32 and 16 columns on both sides of their
-choice (72 and 73 layers) with whole and ragged last tiles, and the column
+the implicit viscosity's tiles of 32, 16 and 8 columns on both sides of their
+choices (54 and 55, 105 and 106 layers) with whole and ragged last tiles, and the column
 kernels' entities per block, which change with the level count."""
 import numpy as np
 import pytest
@@ -25,8 +25,8 @@ def _compare(case_of, steps):
         o.close()
 
 
-@pytest.mark.parametrize("nx,ny,nsigma,kw", [(12, 11, 73, {}), (12, 11, 74, {}), (19, 13, 91, {"fic_point": 0}),
-                                             (21, 12, 102, {"fic_point": 2}), (33, 17, 127, {})])
+@pytest.mark.parametrize("nx,ny,nsigma,kw", [(12, 11, 55, {}), (12, 11, 56, {}), (19, 13, 91, {"fic_point": 0}),
+                                             (21, 12, 106, {}), (21, 12, 107, {"fic_point": 2}), (33, 17, 127, {})])
 def test_implicit_viscosity_tiles(built, nx, ny, nsigma, kw):
     from fesomc import cases
     _compare(lambda lib: cases.estuary_case("e", nx, ny, 300.0, nsigma, 2.0, 25.0, stress=(0.0, 0.05), lib=lib, **kw), 3)

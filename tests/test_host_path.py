@@ -240,8 +240,9 @@ def test_vertical_diffusion_form(fake, nx, ny, nsigma, fp32, reg):
     assert ("k_vdiff_regILi%dE" % (nsigma - 1) in names) == reg and ("k_vdiff_tile" in names) != reg
 
 
-# 160x100: about 21 k elements; 280x150: 55 k
-@pytest.mark.parametrize("nx,ny,nsigma,fp32,reg", [(160, 100, 11, 0, False), (280, 150, 11, 0, True), (280, 150, 11, 1, True),
+# 160x100: about 21 k elements; 200x120: 31 k; 280x150: 55 k
+@pytest.mark.parametrize("nx,ny,nsigma,fp32,reg", [(160, 100, 11, 0, False), (160, 100, 7, 1, False), (200, 120, 7, 1, True),
+                                                   (200, 120, 7, 0, False), (280, 150, 11, 0, True), (280, 150, 11, 1, True),
                                                    (280, 150, 5, 1, True), (280, 150, 12, 0, False), (280, 150, 21, 1, False)])
 def test_implicit_viscosity_form(fake, nx, ny, nsigma, fp32, reg):
     """Register tiles for few layers on grids that fill the device."""
@@ -272,9 +273,10 @@ def test_d3end_form(fake, nx, ny, nsigma, fp32, tiles):
         g.close()
 
 
-@pytest.mark.parametrize("nsigma,fp32,cols", [(73, 0, 32), (74, 0, 16), (127, 0, 16), (127, 1, 32)])
+@pytest.mark.parametrize("nsigma,fp32,cols", [(55, 0, 32), (56, 0, 16), (106, 0, 16), (107, 0, 8), (127, 0, 8), (127, 1, 32)])
 def test_implicit_viscosity_tile(fake, nsigma, fp32, cols):
-    """FP64 tiles of 16 columns where 32 would leave an SM fewer than three."""
+    """FP64 tiles of 16 and 8 columns where 32 and 16 leave an SM fewer than
+    four."""
     assert "k_implvisc_fic_tileILi%dE" % cols in _launched(fake, 20, 10, nsigma, fp32)
 
 
