@@ -425,34 +425,37 @@ std::vector<FieldRef> field_table(fesomc_model *m) {
 // pageable memory and waiting for it: 803 MB into fresh arrays 166 -> 35 ms
 // (the page faults of one thread were most of it), 148 MB of FP32 fields 37 ->
 // 8.7 ms, 90 MB 40 -> 8 ms, 1.4 MB in 25 fields 0.62 -> 0.33 ms.
-// Page-locking is slow (1 to 2.5 ms per 2 MB), so the slots are made as the
-// volume read so far justifies them: the first at once (2 us: it comes out of
-// what the runtime holds for a model's small buffers), then one for every 16
-// MB (8 MB of FP32 fields, whose widening gains more), and no more than one for
-// every 2 MB of a read-back.  A slot saves its cost on 8 MB where the caller's
-// pages are fresh (a page fault is the dearest part) and on 35 MB where they
-// are warm.  Until there are two, FP64 fields of more than 16 MB are copied one
-// by one.  First read-back of a process's only model with all 16 made at once,
-// so, and field by field: 1.4 MB 14, 0.4, 0.6 ms; 8.5 MB 18, 1.4, 1.1; 34 MB 22,
-// 5, 2.8 (fresh pages 13, 8, 10); 88 MB 22, 10, 5.5; FP32 24, 11, 13.5; 166 MB,
-// fresh pages 27, 19, 33.
+// Page-locking is slow (1 to 2.5 ms per 2 MB, on a busy host tens of ms a
+// call), so the slots are made in three steps as the volume read so far
+// justifies them: the first at once (2 us: it comes out of what the runtime
+// holds for a model's small buffers), four from 32 MB on, all 16 from 96 MB on
+// (FP32 fields, whose widening gains more, count twice).  A MB saves its cost on
+// 8 MB where the caller's pages are fresh (a page fault is the dearest part)
+// and on 35 MB where they are warm.  With one slot, FP64 fields of more than 16
+// MB are copied one by one.  First read-back of a process's only model with all
+// 16 made at once, so, and field by field: 1.4 MB 14, 0.4, 0.6 ms; 8.5 MB 18, 1.4,
+// 1.1 (fresh pages 17, 2.4, 2.5); 34 MB 22, 8, 2.8 (fresh pages 13, 10, 10); 88 MB
+// 22, 10, 5.5; FP32 24, 11, 13.5; 166 MB, fresh pages 27, 20, 33.
 // The slots are shared by the process's models and freed with the last of
 // them.  A read-back that finds them in use by another thread takes the plain
 // path.
 constexpr size_t kSlotBytes = 1 << 20;
-constexpr int kSlots = 16;
 constexpr size_t kFirstBytes = kSlotBytes + kSlotBytes / 2;   // of the first slot, still out of what the runtime holds
 constexpr size_t kSlotsAlone = 6 * kSlotBytes;    // device bytes that need no workers
 constexpr size_t kRoundsMost = 16 * kSlotBytes;   // FP64 bytes worth one slot in turn
-constexpr size_t kBytesPerSlot = 16 * kSlotBytes; // volume that justifies a slot more
-constexpr size_t kSlotShare = 2 * kSlotBytes;     // of a read-back, for each slot it takes
+// the steps: slots, the volume that justifies them, the least read-back for them
+constexpr int kSlots = 16, kSteps = 3;
+constexpr struct {
+    int slots;
+    size_t volume, out;
+} kStagingStep[kSteps] = {{1, 0, 0}, {4, 32 * kSlotBytes, 8 * kSlotBytes}, {kSlots, 96 * kSlotBytes, 16 * kSlotBytes}};
 struct StagingPool {
     std::mutex in_use;                // held for the length of a read-back
     std::mutex mu;                    // guards the rest
     int users = 0;
-    int n = 0;                        // slots made
+    int steps = 0, n = 0;             // steps taken, slots they made
     size_t volume = 0;                // of the larger read-backs, FP32 fields counted twice
-    unsigned char *slot[kSlots] = {};
+    unsigned char *block[kSteps] = {}, *slot[kSlots] = {};
 };
 StagingPool g_staging;
 
@@ -470,18 +473,25 @@ int staging_for(fesomc_model *m, const ReadBytes &b) {
         m->stage_ref = true;
     }
     const bool alone = b.dev <= kSlotsAlone;
-    const int most = alone ? 1 : (int)std::min<size_t>(kSlots, std::max<size_t>(1, b.out / kSlotShare));
     if (!alone) g_staging.volume += b.weight;
-    const int want = std::max(1, (int)std::min<size_t>(most, g_staging.volume / kBytesPerSlot));
-    while (g_staging.n < want) {
+    int want = 1;   // steps
+    while (!alone && want < kSteps && g_staging.volume >= kStagingStep[want].volume && b.out >= kStagingStep[want].out) ++want;
+    if (g_staging.steps < want) {   // all that is missing in one allocation
+        const int n0 = g_staging.n, n1 = kStagingStep[want - 1].slots;
+        const size_t first = n0 == 0 ? kFirstBytes : kSlotBytes;
         void *q = nullptr;
-        if (cudaMallocHost(&q, g_staging.n == 0 ? kFirstBytes : kSlotBytes) != cudaSuccess) {
+        if (cudaMallocHost(&q, first + (n1 - n0 - 1) * kSlotBytes) == cudaSuccess) {
+            unsigned char *p = static_cast<unsigned char *>(q);
+            g_staging.block[g_staging.steps] = p;
+            for (int i = n0; i < n1; ++i, p += i == n0 + 1 ? first : kSlotBytes) g_staging.slot[i] = p;
+            g_staging.steps = want;
+            g_staging.n = n1;
+        } else {
             (void)cudaGetLastError();
-            break;
         }
-        g_staging.slot[g_staging.n++] = static_cast<unsigned char *>(q);
     }
-    const int ns = std::min(g_staging.n, most);
+    int ns = std::min(g_staging.n, alone ? 1 : kSlots);
+    if (b.out < kStagingStep[kSteps - 1].out) ns = std::min(ns, kStagingStep[1].slots);
     while (ns > 1 && (int)m->stage_done.size() < ns) {
         cudaEvent_t e;
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
@@ -499,8 +509,11 @@ void staging_release(fesomc_model *m) {
     std::lock_guard<std::mutex> lk(g_staging.mu);
     m->stage_ref = false;
     if (--g_staging.users > 0) return;
-    for (int i = 0; i < g_staging.n; ++i) cudaFreeHost(g_staging.slot[i]);
-    g_staging.n = 0;
+    for (unsigned char *&p : g_staging.block) {
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+    }
+    g_staging.steps = g_staging.n = 0;
     g_staging.volume = 0;
 }
 

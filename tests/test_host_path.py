@@ -187,12 +187,12 @@ def test_staging_memory_grows_with_use_and_is_given_back(fake, fp32):
         sizes = []
         first = b.state()
         assert 64 * MB < sum(v.nbytes for k, v in first.items() if k != "_time_jd") < 128 * MB
-        for _ in range(10):
-            sizes.append((fake.lib.fake_pinned_bytes() - held) // MB)
+        for _ in range(4):
+            sizes.append((fake.lib.fake_pinned_bytes() - held) / MB)
             got = b.state()
             for k, v in got.items():
                 assert np.array_equal(v, first[k]), k
-        assert sizes[0] == 4 and sizes == sorted(sizes) and sizes[-1] == 16
+        assert sizes == [4.5, 16.5, 16.5, 16.5]
         got = a.state()
         assert all(np.array_equal(got[k], v) for k, v in want.items())
         b.close()
